@@ -554,7 +554,7 @@ def paged_attention_simt(q, q_stride, k_cache, v_cache, block_table, cu_q, q_sta
     mode = _attention_mode(sink, sigmoid, mapped)
     _run(_core(), "fe_paged_attention_simt", _ptr(q), _c_ll(q_stride), _ptr(out), _c_ll(nq * d), _ptr(k_cache),
          _ptr(v_cache), _ptr(block_table), _c_int(block_table.shape[1]), _ptr(cu_q), _ptr(q_start),
-         _ptr(token_request), _c_int(T), _c_int(nq), _c_int(nkv), _c_int(d), _c_int(page_size),
+         _ptr(token_request), _c_int(cu_q.numel() - 1), _c_int(T), _c_int(nq), _c_int(nkv), _c_int(d), _c_int(page_size),
          _c_int(k_cache.shape[0]), _c_float(scale), _c_int(window), _c_int(keep), _c_int(mode), _c_int(_code(k_cache.dtype)),
          _ptr(status_word(k_cache.device)), _ptr(per_head), _c_float(softcap), _stream())
     return out
