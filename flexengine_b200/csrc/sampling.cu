@@ -14,6 +14,13 @@
 // then a running sum), the segments' masses are added up by one thread in index order, and the pass that looks for
 // the token repeats the same arithmetic, so the intervals of the tokens tile [0, total) and the result is the same
 // on every run, in every batch and with every cluster size.
+//
+// What bounds a row is how often its logits are walked (from L2 after the first time) and how many steps wait for one another.
+// A top-k row used to walk them seven times, four of them with an atomic a logit in a few bins of a histogram.  Now the pass
+// that finds the maximum also leaves every thread's own maximum; the k-th largest of a block's 1,024 is a lower bound of the
+// row's k-th largest logit (each is a logit of its own), so one more walk collects the few logits that reach the bound, and
+// threshold, ties and the groups of 256 that hold any mass come from that short list.  A list that does not fit (many
+// equal logits, or large ones all in one thread's share) and k beyond the threads' number take the radix select over the row.
 #include <math_constants.h>
 
 #define FE_PDL_CLASS 8      // FE_PDL_SAMPLING
@@ -28,6 +35,7 @@ constexpr int WARPS = THREADS / 32;
 constexpr int RADIX_LOADS = 8;      // loads on their way at once in a pass of the radix select
 constexpr int SEGMENTS = 256;       // of a row; a block of a cluster of C owns SEGMENTS / C of them, a warp SEGMENTS / C / 32
 constexpr int MAX_CLUSTER = 8;
+constexpr int LIST = 2 * THREADS;      // logits of a row (all blocks together) that the short list takes: two a thread
 
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
@@ -68,12 +76,20 @@ sample_kernel(const float* __restrict__ logits, long long ld, int V, const float
               const long long* __restrict__ draw, int* __restrict__ out, const int C) {
     griddep_wait();
     griddep_launch_dependents();
-    __shared__ float s_val[THREADS];
-    __shared__ int s_idx[THREADS];
+    __shared__ float s_val[WARPS];
+    __shared__ int s_idx[WARPS];
+    __shared__ unsigned int blk_bound;                  // this block's lower bound of the row's k-th largest key
+    __shared__ int list_count;                          // this block's logits that reach the row's bound
+    __shared__ unsigned int seg_groups[SEGMENTS];       // bit g of a segment of this block: its group g (31: 31 and up) holds mass
     __shared__ float blk_val;                           // this block's maximum and its lowest index
     __shared__ int blk_idx;
     __shared__ unsigned int hist[2][256], warp_above[8];      // hist: one per parity of the pass
     __shared__ unsigned int warp_hist[WARPS][256];      // one histogram per warp: no two warps meet in a bin
+    // the short list's keys and indices lie there first: a row takes the list or the histograms (a block that goes on to its
+    // histograms may overwrite a list which a slower one still copies, and which none of them uses then)
+    static_assert(2 * LIST <= WARPS * 256, "the list fits the histograms");
+    unsigned int* list_key = &warp_hist[0][0];
+    int* list_idx = reinterpret_cast<int*>(list_key + LIST);
     __shared__ unsigned int s_prefix, s_need;
     __shared__ float seg_mass[SEGMENTS];                // of this block's segments (the first SEGMENTS / C entries)
     __shared__ int seg_ties[SEGMENTS];
@@ -121,16 +137,32 @@ sample_kernel(const float* __restrict__ logits, long long ld, int V, const float
             if (v > best || (v == best && i < best_i)) { best = v; best_i = i; }
         }
     }
-    s_val[tid] = best; s_idx[tid] = best_i;
-    __syncthreads();
-    for (int off = THREADS / 2; off > 0; off >>= 1) {
-        if (tid < off) {
-            const float v = s_val[tid + off]; const int i = s_idx[tid + off];
-            if (v > s_val[tid] || (v == s_val[tid] && i < s_idx[tid])) { s_val[tid] = v; s_idx[tid] = i; }
+    int k = temp == 0.f ? 0 : top_k[row];
+    const bool use_k = k > 0 && k < V;
+    const bool listed = use_k && k <= THREADS / 2;
+    if (listed) {
+        // the largest t (to 24 bits) that k or more of the threads' maxima reach, bit by bit
+        const unsigned int own = ordered_key(best);
+        unsigned int t = 0;
+        for (int bit = 31; bit >= 8; --bit) {
+            const unsigned int more = t | (1u << bit);
+            if (__syncthreads_count(own >= more) >= k) t = more;
         }
-        __syncthreads();
+        if (tid == 0) blk_bound = t;
     }
-    if (tid == 0) { blk_val = s_val[0]; blk_idx = s_idx[0]; }
+    auto take = [&](float v, int i) { if (v > best || (v == best && i < best_i)) { best = v; best_i = i; } };
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) take(__shfl_xor_sync(0xffffffffu, best, off), __shfl_xor_sync(0xffffffffu, best_i, off));
+    if ((tid & 31) == 0) { s_val[tid >> 5] = best; s_idx[tid >> 5] = best_i; }
+    if (tid < SEGMENTS) { seg_ties[tid] = 0; seg_groups[tid] = 0; }
+    if (tid == 0) list_count = 0;
+    __syncthreads();
+    if (tid < 32) {
+        best = s_val[tid]; best_i = s_idx[tid];
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) take(__shfl_xor_sync(0xffffffffu, best, off), __shfl_xor_sync(0xffffffffu, best_i, off));
+        if (tid == 0) { blk_val = best; blk_idx = best_i; }
+    }
     cluster_sync();
     float max_logit = -CUDART_INF_F;
     int argmax = 0x7fffffff;
@@ -146,13 +178,76 @@ sample_kernel(const float* __restrict__ logits, long long ld, int V, const float
         return;
     }
 
-    // ---- top-k threshold by radix select on the ordered keys of the logits (division by a
-    //      positive temperature keeps the order)
-    int k = top_k[row];
-    const bool use_k = k > 0 && k < V;
+    // ---- top-k threshold on the ordered keys of the logits (division by a positive temperature keeps the order)
     unsigned int thr_key = 0;      // keep keys > thr_key, and ``need`` of the keys == thr_key
     unsigned int need = 0;
-    if (use_k) {
+    bool from_list = false;
+    if (listed) {
+        unsigned int bound = 0;
+        for (int c = 0; c < C; ++c) bound = max(bound, ld_peer(&blk_bound, c));
+        auto collect = [&](float raw, int i) {
+            const unsigned int key = ordered_key(sanitize(raw));
+            if (key >= bound) {
+                const int at = atomicAdd(&list_count, 1);
+                if (at < LIST) { list_key[at] = key; list_idx[at] = i; }
+            }
+        };
+        if (vector) {
+            const float4* x4 = reinterpret_cast<const float4*>(x);
+            const int n4 = hi >> 2;
+            for (int i = (lo >> 2) + tid; i < n4; i += 4 * THREADS) {
+                float4 part[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) part[u] = i + u * THREADS < n4 ? x4[i + u * THREADS] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int at = 4 * (i + u * THREADS);
+                    if (i + u * THREADS < n4) { collect(part[u].x, at); collect(part[u].y, at + 1); collect(part[u].z, at + 2); collect(part[u].w, at + 3); }
+                }
+            }
+        } else {
+            for (int i0 = lo + tid; i0 < hi; i0 += RADIX_LOADS * THREADS) {
+                float v[RADIX_LOADS];
+#pragma unroll
+                for (int u = 0; u < RADIX_LOADS; ++u) v[u] = i0 + u * THREADS < hi ? x[i0 + u * THREADS] : 0.f;
+#pragma unroll
+                for (int u = 0; u < RADIX_LOADS; ++u)
+                    if (i0 + u * THREADS < hi) collect(v[u], i0 + u * THREADS);
+            }
+        }
+        cluster_sync();
+        // all blocks' keys, two a thread: list position p is in block c at p - (entries of the blocks before)
+        int total = 0;
+        unsigned int key0 = 0, key1 = 0;
+        for (int c = 0; c < C; ++c) {
+            const int count = (int)ld_peer(&list_count, c);
+            const int p0 = tid - total, p1 = tid + THREADS - total;
+            if (p0 >= 0 && p0 < count) key0 = ld_peer(&list_key[min(p0, LIST - 1)], c);
+            if (p1 >= 0 && p1 < count) key1 = ld_peer(&list_key[min(p1, LIST - 1)], c);
+            total = min(total + count, LIST + 1);
+        }
+        from_list = total <= LIST;                      // the same in every block
+        if (from_list) {
+            // the k-th largest key: the largest t that k or more keys reach (a thread without an entry holds 0, below every key)
+            auto reach = [&](unsigned int t) {
+                int n = __syncthreads_count(key0 >= t);
+                if (total > THREADS) n += __syncthreads_count(key1 >= t);
+                return n;
+            };
+            for (int bit = 31; bit >= 0; --bit) {
+                const unsigned int more = thr_key | (1u << bit);
+                if (reach(more) >= k) thr_key = more;
+            }
+            need = (unsigned int)(k - reach(thr_key + 1));         // keys end at that of +inf, far below the largest number
+            for (int i = tid; i < list_count; i += THREADS) {
+                if (list_key[i] < thr_key) continue;
+                const int segment = list_idx[i] / S, mine = segment - (int)rank * per_block;
+                atomicOr(&seg_groups[mine], 1u << min((list_idx[i] - segment * S) / 256, 31));
+                if (list_key[i] == thr_key) atomicAdd(&seg_ties[mine], 1);
+            }
+        }
+    }
+    if (use_k && !from_list) {
         if (tid == 0) { s_prefix = 0; s_need = (unsigned int)k; }
         __syncthreads();
         for (int pass = 0; pass < 4; ++pass) {
@@ -252,7 +347,7 @@ sample_kernel(const float* __restrict__ logits, long long ld, int V, const float
 
     // threshold ties of every segment, and from them the ties before each, in index order
     if (use_k) {
-        for (int j = 0; j < per_warp; ++j) {
+        for (int j = 0; j < per_warp && !from_list; ++j) {
             const int mine = warp * per_warp + j;
             int seg0, seg1;
             bounds((int)rank * per_block + mine, seg0, seg1);
@@ -269,9 +364,19 @@ sample_kernel(const float* __restrict__ logits, long long ld, int V, const float
         cluster_sync();
         if (tid < SEGMENTS) ties_before[tid] = (int)ld_peer(&seg_ties[tid % per_block], tid / per_block);
         __syncthreads();
-        if (tid == 0) {
+        if (tid < 32) {
             int run = 0;
-            for (int g = 0; g < SEGMENTS; ++g) { const int t = ties_before[g]; ties_before[g] = run; run += t; }
+            for (int g = 0; g < SEGMENTS; g += 32) {
+                const int t = ties_before[g + tid];
+                int upto = t;
+#pragma unroll
+                for (int off = 1; off < 32; off <<= 1) {
+                    const int up = __shfl_up_sync(0xffffffffu, upto, off);
+                    if (tid >= off) upto += up;
+                }
+                ties_before[g + tid] = run + upto - t;
+                run += __shfl_sync(0xffffffffu, upto, 31);
+            }
         }
         __syncthreads();
     }
@@ -301,7 +406,9 @@ sample_kernel(const float* __restrict__ logits, long long ld, int V, const float
         const int tie_base = use_k ? ties_before[segment] : 0;
         float cum = 0.f;
         int ties_seen = 0;
+        const unsigned int groups = from_list ? seg_groups[mine] : 0xffffffffu;       // the others hold neither mass nor ties
         for (int base = seg0; base < seg1; base += 32 * GROUP) {
+            if (!(groups >> min((base - seg0) / (32 * GROUP), 31) & 1u)) continue;
             float v[GROUP];
             load_group(base, seg1, v);
             float part = 0.f;
@@ -316,8 +423,15 @@ sample_kernel(const float* __restrict__ logits, long long ld, int V, const float
     __syncthreads();
     if (tid == 0) {
         // accumulated by one thread in index order: nondecreasing, so the segments' intervals tile [0, total)
+        // (sixteen values are fetched together: the additions, not the loads, are what waits for one another)
         float run = 0.f;
-        for (int g = 0; g < SEGMENTS; ++g) { const float m = mass_before[g]; mass_before[g] = run; run += m; }
+        for (int g = 0; g < SEGMENTS; g += 16) {
+            float m[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) m[i] = mass_before[g + i];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) { mass_before[g + i] = run; run += m[i]; }
+        }
         mass_before[SEGMENTS] = run;
     }
     cluster_sync();                                     // every block has read the others' masses (and ties): they may leave

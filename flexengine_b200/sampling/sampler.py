@@ -9,12 +9,21 @@ else is in the batch or on how the scheduler cut the work.
 """
 from __future__ import annotations
 
+import numpy as np
 import torch
 
 
 def validate_sampling(temperature: float, top_k: int) -> None:
     if temperature < 0 or top_k < 0:
         raise ValueError("temperature and top_k must be >= 0")
+
+
+def _numbers(values, dtype, one):
+    """A sequence of numbers (or of one-element tensors) as an array."""
+    try:
+        return np.asarray(values, dtype=dtype)
+    except TypeError:
+        return np.asarray([one(v) for v in values], dtype=dtype)
 
 
 class Sampler:
@@ -33,11 +42,13 @@ class Sampler:
         """As ``sample`` but the token ids stay where the logits are (int32 [R]); nothing waits for the device."""
         if logits.dim() != 2 or logits.shape[0] != len(temperatures):
             raise ValueError("Expected logits [requests, vocab]")
-        for t, k in zip(temperatures, top_ks):
-            validate_sampling(t, k)
-        dev = logits.device
         n = len(temperatures)
-        if all(t == 0.0 for t in temperatures):
+        t64, k64 = _numbers(temperatures, np.float64, float), _numbers(top_ks, np.int64, int)
+        if (t64 < 0).any() or (k64 < 0).any():
+            for t, k in zip(temperatures, top_ks):
+                validate_sampling(t, k)
+        dev = logits.device
+        if not t64.any():
             # greedy rows need no parameters: zeros kept on the device, no copy per step
             key = (str(dev), n)
             if key not in self._zeros:
@@ -46,13 +57,13 @@ class Sampler:
                                     torch.zeros(n, dtype=torch.int64, device=dev))
             temperature, top_k, zero64 = self._zeros[key]
             return self.ops.sample(logits, temperature, top_k, zero64, zero64)
-        # one host buffer, one copy: [temperature bits | top_k | seed lo, hi | draw lo, hi] as 64-bit words
-        packed = torch.empty((4, n), dtype=torch.int64, pin_memory=dev.type == "cuda")
-        packed[0] = torch.tensor(list(temperatures), dtype=torch.float32).view(torch.int32).to(torch.int64)
-        packed[1] = torch.tensor(list(top_ks), dtype=torch.int64)
-        packed[2] = torch.tensor(list(seeds), dtype=torch.int64)
-        packed[3] = torch.tensor(list(draws), dtype=torch.int64)
+        # One host buffer, one copy, no kernel to take it apart: [seeds | draws | temperatures | top_ks] as 8, 8, 4 and 4 bytes
+        # each (four conversions and two kernels before: the host took longer than the device, 106 us for 64 rows)
+        packed = torch.empty(3 * n, dtype=torch.int64, pin_memory=dev.type == "cuda")
+        host = packed.numpy()
+        host[:n], host[n:2 * n] = _numbers(seeds, np.int64, int), _numbers(draws, np.int64, int)
+        host[2 * n:].view(np.float32)[:n] = t64
+        host[2 * n:].view(np.int32)[n:] = k64
         on_dev = packed.to(dev, non_blocking=True)
-        temperature = on_dev[0].to(torch.int32).view(torch.float32)
-        top_k = on_dev[1].to(torch.int32)
-        return self.ops.sample(logits, temperature, top_k, on_dev[2].contiguous(), on_dev[3].contiguous())
+        small = on_dev[2 * n:].view(torch.int32)
+        return self.ops.sample(logits, small[:n].view(torch.float32), small[n:], on_dev[:n], on_dev[n:2 * n])
