@@ -188,16 +188,28 @@ __device__ __forceinline__ int swizzled(int r, int c, int block_bytes) {
 }
 
 // The softmax of one row over a key tile, the 64 scores in registers.  MASKED: the tile crosses
-// the causal edge or the window's edge for some row of the warp; ``hi`` and ``lo`` are then this
-// row's last and first visible key relative to the tile, and keys below ``keep`` are visible however far back they are.
-__device__ __forceinline__ bool hidden(int key, int hi, int lo, int keep) { return key > hi || (key < lo && key >= keep); }
+// the causal edge or the window's edge for some row of the warp; what this row sees of the tile is then two words of bits, made once a
+// tile (a comparison per key with its short-circuit branches took a tile that crosses an edge from 1.1 to 3.9 us).
+struct Seen { unsigned word[2]; };
+__device__ __forceinline__ unsigned low_bits(int n) { return n <= 0 ? 0u : n >= 32 ? 0xffffffffu : (1u << n) - 1u; }
+// ``hi`` and ``lo``: the row's last and first visible key relative to the tile; keys below ``keep`` are visible however far back they are.
+__device__ __forceinline__ Seen seen_keys(int hi, int lo, int keep) {
+    Seen seen;
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+        const int at = 32 * w;
+        seen.word[w] = low_bits(hi + 1 - at) & (~low_bits(lo - at) | low_bits(keep - at));
+    }
+    return seen;
+}
+__device__ __forceinline__ bool hidden(int key, const Seen& seen) { return !(seen.word[key >> 5] >> (key & 31) & 1u); }
 __device__ __forceinline__ float max3(float a, float b, float c) {
     float m;
     asm("max.f32 %0, %1, %2, %3;\n" : "=f"(m) : "f"(a), "f"(b), "f"(c));
     return m;
 }
 template <bool MASKED>
-__device__ __forceinline__ float row_max(const unsigned* r, int hi, int lo, int keep) {
+__device__ __forceinline__ float row_max(const unsigned* r, const Seen& seen) {
     float m0 = -CUDART_INF_F, m1 = -CUDART_INF_F, m2 = -CUDART_INF_F, m3 = -CUDART_INF_F;
 #pragma unroll
     for (int i = 0; i < KEYS; i += 8) {
@@ -205,7 +217,7 @@ __device__ __forceinline__ float row_max(const unsigned* r, int hi, int lo, int 
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
             v[e] = __uint_as_float(r[i + e]);
-            if (MASKED && hidden(i + e, hi, lo, keep)) v[e] = -CUDART_INF_F;
+            if (MASKED && hidden(i + e, seen)) v[e] = -CUDART_INF_F;
         }
         m0 = max3(m0, v[0], v[1]), m1 = max3(m1, v[2], v[3]), m2 = max3(m2, v[4], v[5]), m3 = max3(m3, v[6], v[7]);
     }
@@ -214,7 +226,7 @@ __device__ __forceinline__ float row_max(const unsigned* r, int hi, int lo, int 
 // P = 2^(s scale - ref) as bfloat16 pairs over the scores' own columns (32 of the 64); returns the row's sum.
 // The multiply-adds and the sums run two floats per instruction.
 template <bool MASKED>
-__device__ __forceinline__ float row_exp(const unsigned* r, unsigned p_addr, int hi, int lo, int keep, float scale_log2, float ref) {
+__device__ __forceinline__ float row_exp(const unsigned* r, unsigned p_addr, const Seen& seen, float scale_log2, float ref) {
     float2 sum = make_float2(0.f, 0.f);
     const float2 scale2 = make_float2(scale_log2, scale_log2), ref2 = make_float2(-ref, -ref);
 #pragma unroll
@@ -226,8 +238,8 @@ __device__ __forceinline__ float row_exp(const unsigned* r, unsigned p_addr, int
             const float2 t = __ffma2_rn(make_float2(__uint_as_float(r[k]), __uint_as_float(r[k + 1])), scale2, ref2);
             float2 e = make_float2(ex2(t.x), ex2(t.y));
             if (MASKED) {
-                if (hidden(k, hi, lo, keep)) e.x = 0.f;
-                if (hidden(k + 1, hi, lo, keep)) e.y = 0.f;
+                if (hidden(k, seen)) e.x = 0.f;
+                if (hidden(k + 1, seen)) e.y = 0.f;
             }
             sum = __fadd2_rn(sum, e);
             const __nv_bfloat162 pair = __floats2bfloat162_rn(e.x, e.y);
@@ -241,7 +253,7 @@ __device__ __forceinline__ float row_exp(const unsigned* r, unsigned p_addr, int
 // Sigmoid weights instead of a softmax: P = 1 / (1 + 2^-(s scale + bias)) as bfloat16 pairs over the scores' own columns;
 // nothing is summed, a masked key weighs 0.
 template <bool MASKED>
-__device__ __forceinline__ void row_sigmoid(const unsigned* r, unsigned p_addr, int hi, int lo, int keep, float scale_log2, float bias) {
+__device__ __forceinline__ void row_sigmoid(const unsigned* r, unsigned p_addr, const Seen& seen, float scale_log2, float bias) {
     const float2 scale2 = make_float2(-scale_log2, -scale_log2), bias2 = make_float2(-bias, -bias);
 #pragma unroll
     for (int c = 0; c < KEYS; c += 32) {
@@ -252,8 +264,8 @@ __device__ __forceinline__ void row_sigmoid(const unsigned* r, unsigned p_addr, 
             const float2 t = __ffma2_rn(make_float2(__uint_as_float(r[k]), __uint_as_float(r[k + 1])), scale2, bias2);
             float2 e = make_float2(rcp(1.f + ex2(t.x)), rcp(1.f + ex2(t.y)));
             if (MASKED) {
-                if (hidden(k, hi, lo, keep)) e.x = 0.f;
-                if (hidden(k + 1, hi, lo, keep)) e.y = 0.f;
+                if (hidden(k, seen)) e.x = 0.f;
+                if (hidden(k + 1, seen)) e.y = 0.f;
             }
             const __nv_bfloat162 pair = __floats2bfloat162_rn(e.x, e.y);
             packed[i] = *reinterpret_cast<const unsigned*>(&pair);
@@ -304,12 +316,85 @@ __device__ __forceinline__ void row_map(unsigned* r, float unit, float cap_log2)
     }
 }
 
+// The step's items, one per (request, pair of row tiles), in the order in which blocks take them: those whose last query sees
+// the most key tiles first, whichever request they belong to, so that no long walk starts when the others are done (one block
+// is resident on an SM); of items with the same last key tile the earlier request's first.  No list is made: an item ends in key
+// tile e or later from a certain pair of its request on, so the number of items with last tile >= e is a sum over the
+// requests, and the e of the item-th item is found by bisection.  One warp, every lane with the same result; ``who`` = -1
+// when there are fewer items.  Portions of prompts beside decoded tokens (2,048 tokens, 12 heads in 2 groups, prompts of 255 to
+// 1,021): 70 us a layer with a grid over (pairs of the longest portion, heads, requests), most of it blocks without rows and
+// long walks begun late.
+__device__ __forceinline__ int items_from(int e, int n_q, int start, int G) {
+    // pair m's last query is min(n_q - 1, (256 (m + 1) - 1) / G): the first pair that reaches query q is 256 m > q G - 256
+    const int pairs = (n_q * G + 2 * ROWS - 1) / (2 * ROWS), q = e * KEYS - start;
+    return q <= 0 ? pairs : q >= n_q ? 0 : pairs - q * G / (2 * ROWS);
+}
+__device__ __forceinline__ void pick_item(int item, const int* __restrict__ cu_q, const int* __restrict__ q_start, int requests, int G,
+                                          int& who, int& pair) {
+    constexpr unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int n0 = lane < requests ? cu_q[lane + 1] - cu_q[lane] : 0, s0 = lane < requests ? q_start[lane] : 0;
+    auto request = [&](int base, int& n, int& s) {                  // of this lane; the first 32 stay in registers
+        n = n0, s = s0;
+        if (base > 0) {
+            const int i = base + lane;
+            n = i < requests ? cu_q[i + 1] - cu_q[i] : 0;
+            s = i < requests ? q_start[i] : 0;
+        }
+    };
+    auto total_from = [&](int e) {
+        int sum = 0;
+        for (int base = 0; base < requests; base += 32) {
+            int n, s;
+            request(base, n, s);
+            sum += items_from(e, n, s, G);
+        }
+        return __reduce_add_sync(FULL, sum);
+    };
+    int last = 0;                                                   // the largest last key tile
+    for (int base = 0; base < requests; base += 32) {
+        int n, s;
+        request(base, n, s);
+        if (n > 0) last = max(last, (s + n - 1) / KEYS);
+    }
+    last = __reduce_max_sync(FULL, last);
+    who = -1, pair = 0;
+    if (total_from(0) <= item) return;
+    int low = 0, high = last + 1;                                   // items from ``low`` on: more than ``item``; from ``high`` on: not
+    while (high - low > 1) {
+        const int mid = (low + high) >> 1;
+        if (total_from(mid) > item) low = mid;
+        else high = mid;
+    }
+    int left = item - total_from(low + 1);                          // which of the items that end in tile ``low``
+    for (int base = 0; base < requests; base += 32) {
+        int n, s;
+        request(base, n, s);
+        const int later = items_from(low + 1, n, s, G), mine = items_from(low, n, s, G) - later;
+        int upto = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(FULL, upto, o);
+            if (lane >= o) upto += v;
+        }
+        const unsigned here = __ballot_sync(FULL, left >= upto - mine && left < upto);
+        if (here) {
+            const int at = __ffs(here) - 1;
+            const int pairs = (n * G + 2 * ROWS - 1) / (2 * ROWS);
+            who = base + at;
+            pair = __shfl_sync(FULL, pairs - 1 - later - (left - (upto - mine)), at);
+            return;
+        }
+        left -= __shfl_sync(FULL, upto, 31);
+    }
+}
+
 template <int D>
 __global__ void __launch_bounds__(THREADS, 1)
 paged_prefill_tcgen05_kernel(const bf16* __restrict__ q, long long q_stride, bf16* __restrict__ out, long long out_stride,
                              const bf16* __restrict__ kc, const bf16* __restrict__ vc,
                              const int* __restrict__ block_table, int bt_stride, const int* __restrict__ cu_q,
-                             const int* __restrict__ q_start, int nq, int nkv, int ps, int num_pages, float scale_log2,
+                             const int* __restrict__ q_start, int requests, int nq, int nkv, int ps, int num_pages, float scale_log2,
                              int window, int keep, int mode, int splits, float* __restrict__ part_o, float* __restrict__ part_lse,
                              int* __restrict__ status, const float* __restrict__ per_head, float cap_log2) {
     const bool sink = mode & 1, sigmoid = mode & 2;         // bit 1: sigmoid(score + per_head[head]) instead of a softmax
@@ -319,6 +404,7 @@ paged_prefill_tcgen05_kernel(const bf16* __restrict__ q, long long q_stride, bf1
     __shared__ long long offs[2][KEYS];
     __shared__ unsigned tmem_holder;
     __shared__ volatile int give_up;
+    __shared__ int item_request, item_pair;
     constexpr int DB = D / 64;                       // 64-element blocks per row
     constexpr int Q_BYTES = DB * Q_BLOCK;            // one row tile of Q
     constexpr int KV_BYTES = DB * KV_BLOCK;          // one key tile of K or of V
@@ -330,14 +416,20 @@ paged_prefill_tcgen05_kernel(const bf16* __restrict__ q, long long q_stride, bf1
     griddep_wait();
     griddep_launch_dependents();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int kvh = blockIdx.y, r = blockIdx.z;
     const int G = nq / nkv;
+    // blockIdx.x = (item, key/value head, split of its keys); warp 0 finds the item's request and pair of row tiles
+    const int split = blockIdx.x % splits, kvh = (blockIdx.x / splits) % nkv;
+    if (warp == 0) {
+        int who, pair;
+        pick_item((int)(blockIdx.x / (splits * nkv)), cu_q, q_start, requests, G, who, pair);
+        if (lane == 0) { item_request = who; item_pair = pair; }
+    }
+    __syncthreads();
+    const int r = item_request;
+    if (r < 0) return;                                              // the grid is an upper bound of the items
     const int tok0 = cu_q[r], n_q = cu_q[r + 1] - tok0;
     const int rows = n_q * G;
-    // blockIdx.x = (pair of row tiles, split of its keys); the rows with the most keys first
-    const int split = blockIdx.x % splits;
-    const int m_pair = (gridDim.x / splits - 1 - blockIdx.x / splits) * 2 * ROWS;
-    if (m_pair >= rows) return;
+    const int m_pair = item_pair * 2 * ROWS;
     const bool two = m_pair + ROWS < rows;                          // else the second row tile is empty and left out
     const int start = q_start[r];
     // keys this block needs: from the window edge of its first query to its last query
@@ -377,8 +469,10 @@ paged_prefill_tcgen05_kernel(const bf16* __restrict__ q, long long q_stride, bf1
     const int m = m_pair + ti * ROWS + (tid & 127);
     const bool valid = softmax_thread && m < rows;
     const int qi = valid ? m / G : 0, head = kvh * G + (valid ? m % G : 0);
-    const int pos = valid ? start + qi : -1;
+    // a padding row sees what the last query sees: it is computed and never written, and must not make a tile a masked one
+    const int pos = valid ? start + qi : hi;
     const int row_lo = first_visible(pos, window);
+    const bool any_valid = __any_sync(0xffffffffu, valid);          // of the warp
     // where this thread's row starts in q and in out (in elements); other lanes fetch it by shuffle
     const long long q_off = valid ? (long long)(tok0 + qi) * q_stride + (long long)head * D : -1;
     const long long out_off = valid ? (long long)(tok0 + qi) * out_stride + (long long)head * D : -1;
@@ -517,6 +611,11 @@ paged_prefill_tcgen05_kernel(const bf16* __restrict__ q, long long q_stride, bf1
             ok = __all_sync(FULL, mbar_wait(&s_ready[ti][j & 1], (j >> 1) & 1, &give_up));
             if (!ok) break;
             tc_fence_after();
+            if (!any_valid) {                                      // padding rows only (a decoded token fills a few of 128): whatever
+                tc_fence_before();                                 // lies there is multiplied, and never written
+                mbar_arrive(&p_ready[ti][j & 1]);
+                continue;
+            }
             const unsigned s_addr = tmem_base + lane_bits + (2 * ti + (j & 1)) * 64;
             unsigned raw[KEYS];
             tmem_issue_load32(s_addr, raw);
@@ -526,17 +625,18 @@ paged_prefill_tcgen05_kernel(const bf16* __restrict__ q, long long q_stride, bf1
             tie32(raw + 32);
             const int key0 = listed_tile<KEYS>(t_begin + j, kept, lo) * KEYS;
             const bool unmasked = key0 + KEYS - 1 <= pos_min && (key0 >= lo_max || key0 + KEYS <= keep);      // for the whole warp
-            const int rel_hi = pos - key0, rel_lo = row_lo - key0, rel_keep = keep - key0;
+            Seen seen = {{0u, 0u}};
+            if (!unmasked) seen = seen_keys(pos - key0, row_lo - key0, keep - key0);
             if (sigmoid) {
-                if (unmasked) row_sigmoid<false>(raw, s_addr, rel_hi, rel_lo, rel_keep, scale_log2, bias);
-                else row_sigmoid<true>(raw, s_addr, rel_hi, rel_lo, rel_keep, scale_log2, bias);
+                if (unmasked) row_sigmoid<false>(raw, s_addr, seen, scale_log2, bias);
+                else row_sigmoid<true>(raw, s_addr, seen, scale_log2, bias);
                 tmem_store_wait();
                 tc_fence_before();
                 mbar_arrive(&p_ready[ti][j & 1]);
                 continue;
             }
             if (mapped) row_map(raw, unit, cap_log2);
-            const float mx = unmasked ? row_max<false>(raw, rel_hi, rel_lo, rel_keep) : row_max<true>(raw, rel_hi, rel_lo, rel_keep);
+            const float mx = unmasked ? row_max<false>(raw, seen) : row_max<true>(raw, seen);
             const float m_new = fmaxf(m_ref, mx * to_log2);
             if (__any_sync(FULL, m_new > m_ref + RESCALE_STEP)) {
                 // move the reference point to the new maximum: O and the sum were taken against the old one
@@ -558,8 +658,8 @@ paged_prefill_tcgen05_kernel(const bf16* __restrict__ q, long long q_stride, bf1
                 m_ref = m_new;
             }
             const float m_safe = m_ref == -CUDART_INF_F ? 0.f : m_ref;
-            row_sum += unmasked ? row_exp<false>(raw, s_addr, rel_hi, rel_lo, rel_keep, to_log2, m_safe)
-                                : row_exp<true>(raw, s_addr, rel_hi, rel_lo, rel_keep, to_log2, m_safe);
+            row_sum += unmasked ? row_exp<false>(raw, s_addr, seen, to_log2, m_safe)
+                                : row_exp<true>(raw, s_addr, seen, to_log2, m_safe);
             tmem_store_wait();
             tc_fence_before();
             mbar_arrive(&p_ready[ti][j & 1]);
@@ -671,14 +771,16 @@ int launch(const void* q, long long q_stride, void* out, long long out_stride, c
     const size_t smem = (size_t)(D / 64) * (2 * Q_BLOCK + 2 * KV_STAGES * KV_BLOCK) + 1024;
     const cudaError_t err = cudaFuncSetAttribute(paged_prefill_tcgen05_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     FE_REQUIRE(err == cudaSuccess, "paged_prefill_tcgen05: %s", cudaGetErrorString(err));
-    const long long rows = (long long)max_q_len * (nq / nkv);
-    const long long tiles = (rows + 2 * ROWS - 1) / (2 * ROWS) * splits;
-    FE_REQUIRE(tiles <= 2147483647LL && nkv <= 65535 && requests <= 65535, "paged_prefill_tcgen05: grid too large");
+    // every request's pairs of row tiles: as many as the longest one's each, and at most one more each than the rows fill
+    const long long group = nq / nkv, each = (max_q_len * group + 2 * ROWS - 1) / (2 * ROWS) * requests;
+    const long long filled = total_tokens > 0 ? total_tokens * group / (2 * ROWS) + requests : each;
+    const long long blocks = (each < filled ? each : filled) * nkv * splits;
+    FE_REQUIRE(blocks <= 2147483647LL && (long long)max_q_len * group <= 2147483647LL - 2 * ROWS, "paged_prefill_tcgen05: grid too large");
     // partial results: [token, head, split, D] float32, then [token, head, split] logarithms of the sums
     float* part_o = splits > 1 ? scratch : nullptr;
     float* part_lse = splits > 1 ? scratch + (size_t)total_tokens * nq * splits * D : nullptr;
-    fe::launch(paged_prefill_tcgen05_kernel<D>, dim3((unsigned)tiles, nkv, requests), THREADS, smem, stream, (const bf16*)q, q_stride,
-               (bf16*)out, out_stride, (const bf16*)kc, (const bf16*)vc, block_table, bt_stride, cu_q, q_start, nq, nkv, ps,
+    fe::launch(paged_prefill_tcgen05_kernel<D>, dim3((unsigned)blocks), THREADS, smem, stream, (const bf16*)q, q_stride,
+               (bf16*)out, out_stride, (const bf16*)kc, (const bf16*)vc, block_table, bt_stride, cu_q, q_start, requests, nq, nkv, ps,
                num_pages, scale * LOG2E, window, keep, sink, splits, part_o, part_lse, status, per_head, softcap * LOG2E);
     if (fe_check_launch("paged_prefill_tcgen05")) return 1;
     if (splits > 1) {
