@@ -141,11 +141,12 @@ template <int TILE> __host__ __device__ __forceinline__ int listed_tile(int i, i
 // may be touched before.  launch_dependents lets the next kernel start its own preamble; it is
 // called after the wait, so that at most one kernel is resident ahead of the one that runs
 // (called before, every later kernel of a graph piles onto the SMs and starves the running one).
-// Without the launch attribute both are no-ops, and the attribute is off unless fe_set_pdl names classes of
-// kernels: inside the CUDA graph of a decode step (28 layers, B200) a step took 3.24 ms without it; with it on the
-// weight-streaming products alone 3.36 ms when they never trigger (the dependent starts as the last block exits),
-// 4.25 ms with the trigger behind their main loop and 5.5 ms with the trigger first: the earlier the dependent's
-// blocks become resident, the slower the step.
+// Without the launch attribute both are no-ops; fe_set_pdl names the classes of kernels that get it.  What it is worth: a
+// kernel boundary costs about 2 us of idle memory, 5 of them a layer in a decode step.  Weight-streaming products and
+// elementwise kernels with it against without (B200): 32 steps of one request on the 1.5B shape 40.3 -> 34.1 ms, 16 steps of 8
+// requests on the 7B shape 26.3 -> 25.2 ms, the hybrid designs 5 to 10 %; all kernels so launched share one split of an
+// SM's memory (fe_share_carveout says why).  Decode attention, the scans and the rest gain nothing or lose (7B: 25.2 ->
+// 26.5 ms with the attention clusters, whose successor then takes the place of late clusters).
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -165,6 +166,7 @@ __device__ __forceinline__ void prefetch_l2_share(const void* base, long long by
 void fe_set_error(const char* fmt, ...);
 int fe_check_launch(const char* what);
 int fe_pdl_enabled();
+void fe_share_carveout(const void* kernel);       // the split of an SM's memory that overlapping kernels share
 int fe_sm_count();      // multiprocessors of the current device (asked once per device)
 
 // Classes of kernels for fe_set_pdl: a source file names its own before including this header.
@@ -191,6 +193,7 @@ inline void launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
     attr[0].val.programmaticStreamSerializationAllowed = (fe_pdl_enabled() & FE_PDL_CLASS) != 0;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
+    if (attr[0].val.programmaticStreamSerializationAllowed) fe_share_carveout((const void*)kernel);
     cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);       // errors surface in fe_check_launch
 }
 }  // namespace fe
