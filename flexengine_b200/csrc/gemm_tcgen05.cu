@@ -5,9 +5,10 @@
 // Blocks are persistent: one per SM, each walks over output tiles (row tiles fastest, so blocks
 // that run together share their rows of W: W is larger than L2 and then comes from HBM once).
 // Warp 0 (one lane) is the TMA producer, warp 1 (one lane) issues the MMAs and owns the TMEM
-// allocation, warps 2..5 are the epilogue: each reads its quarter of the accumulator's lanes with
+// allocation, warps 2..9 are the epilogue: each reads its quarter of the accumulator's lanes, one half of the columns, with
 // tcgen05.ld and writes the rows out.  The accumulator is double-buffered in TMEM (2 x 256
-// columns), so the epilogue of one tile runs under the MMAs of the next.  UMMA shape 128 x 256 x 16.
+// columns), so the epilogue of one tile runs under the MMAs of the next; with one warp a quarter (four in all) the gated
+// epilogue took as long as the products of a tile of K = 1,536 (24 steps of 512 clocks) and set the pace.  UMMA shape 128 x 256 x 16.
 //   plain epilogue:  a 128 x 256 output tile, bfloat16 (or float, for a product whose results are added up afterwards)
 //   SwiGLU epilogue: W is [2I, K] (gate rows, then up rows); the block loads 128 gate rows and
 //                    their 128 up rows as one 256-row B tile, so accumulator columns j and 128 + j
@@ -35,7 +36,8 @@ constexpr int BM = 128;             // rows of the output tile = UMMA M
 constexpr int BK = 64;              // k elements per stage: 128 bytes, one swizzle atom wide
 constexpr int UMMA_K = 16;
 constexpr int STAGES = 4;
-constexpr int THREADS = 192;
+constexpr int EPILOGUE_WARPS = 8;
+constexpr int THREADS = 64 + 32 * EPILOGUE_WARPS;
 constexpr long long WAIT_LIMIT = 4000000000LL;      // clock cycles
 
 enum { EPI_BF16 = 0, EPI_F32 = 1, EPI_SWIGLU = 2, EPI_GEGLU = 5, EPI_RELU2 = 6, EPI_REGLU = 7, EPI_GELU = 8 };      // 5: the gated epilogue with the tanh form of GELU
@@ -205,7 +207,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-        for (int b = 0; b < ACC_BUFFERS; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 4); }
+        for (int b = 0; b < ACC_BUFFERS; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], EPILOGUE_WARPS); }
         give_up = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
@@ -259,7 +261,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         }
     } else if (warp >= 2) {
         // ---- epilogue: warp w may read TMEM lanes 32 (w % 4) .. + 31 ----
-        const int quarter = warp & 3;
+        const int quarter = warp & 3, c_begin = ((warp - 2) >> 2) * (OUT_COLS / 2);
         int i = 0;
         for (int t = blockIdx.x; t < total_tiles && !give_up; t += gridDim.x, ++i) {
             const int buf = i & 1;
@@ -272,7 +274,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             const float rw = (row_weights && row < row_end) ? row_weights[pair_of_row[row]] : 1.f;
             const unsigned lane_addr = tmem_base + buf * BN + ((unsigned)(quarter * 32) << 16);
 #pragma unroll 1
-            for (int c = 0; c < OUT_COLS; c += 32) {
+            for (int c = c_begin; c < c_begin + OUT_COLS / 2; c += 32) {
                 float v[32];
                 tmem_load32(lane_addr + c, v);
                 if (EPI == EPI_SWIGLU) {
