@@ -182,7 +182,7 @@ int fe_sm_count();      // multiprocessors of the current device (asked once per
 namespace fe {
 // Launch with the programmatic-stream-serialization attribute (when enabled for this file's class of kernels).
 template <typename... KArgs, typename... Args>
-inline void launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+inline void launch_as(int classes, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -190,11 +190,15 @@ inline void launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = (fe_pdl_enabled() & FE_PDL_CLASS) != 0;
+    attr[0].val.programmaticStreamSerializationAllowed = (fe_pdl_enabled() & classes) != 0;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     if (attr[0].val.programmaticStreamSerializationAllowed) fe_share_carveout((const void*)kernel);
     cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);       // errors surface in fe_check_launch
+}
+template <typename... KArgs, typename... Args>
+inline void launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+    launch_as(FE_PDL_CLASS, kernel, grid, block, smem, stream, static_cast<Args&&>(args)...);
 }
 }  // namespace fe
 
