@@ -717,9 +717,7 @@ def paged_decode_balanced(q, q_stride, k_cache, v_cache, block_table, cu_q, q_st
         out = torch.empty((requests, nq * d), dtype=torch.bfloat16, device=k_cache.device)
     mapped, per_head, softcap = _score_map(sigmoid, head_bias, softcap, head_scales)
     lib = _bf16()
-    # of the call's own: steps on different streams do not share it
-    work = torch.empty(lib.fe_paged_decode_balanced_scratch_bytes(_c_int(requests), _c_int(nq), _c_int(d), _c_int(items)), dtype=torch.uint8,
-                       device=k_cache.device)
+    work = scratch(k_cache.device, lib.fe_paged_decode_balanced_scratch_bytes(_c_int(requests), _c_int(nq), _c_int(d), _c_int(items)))
     _run(lib, "fe_paged_decode_balanced", _ptr(q), _c_ll(q_stride), _ptr(out), _c_ll(out.stride(0)), _ptr(work), _ptr(k_cache),
          _ptr(v_cache), _ptr(block_table), _c_int(block_table.shape[1]), _ptr(cu_q), _ptr(q_start), _c_int(requests),
          _c_int(nq), _c_int(nkv), _c_int(d), _c_int(page_size), _c_int(k_cache.shape[0]), _c_float(scale), _c_int(window), _c_int(keep),
