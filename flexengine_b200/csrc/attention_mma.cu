@@ -300,75 +300,14 @@ constexpr int CLUSTER_MAX_SPLITS = 16;
 // STAGES: the ring of 32-key stages; STAGES - 1 tiles are on their way while one is multiplied.  A block that walks
 // only a few tiles (short contexts split many ways) spends its life waiting for memory: a deeper ring asks for its
 // tiles earlier.
-// BALANCED: the requests of a large batch differ in length, and with as many splits for each the longest one's splits are what
-// the step waits for.  So the splits are dealt out by length: the step's items are shares of at most U tiles of a request,
-// U the smallest that lets all of them (times the key/value heads) be resident at once.  The grid is that bound; a block finds
-// U by bisection over the sum of the requests' shares, and from it its request and share (a warp adds 32 requests up at a
-// time: a few hundred instructions against walks of a dozen tiles).  Partial results lie by item, and the first block of a request
-// leaves where its items begin and how many there are, for the merge.
-constexpr int BALANCED_MIN_TILES = 4;            // shorter shares cost more to begin and merge than they save
-// A step may have fewer shares than the bound: the blocks that have one are spread evenly over the grid (all of them among its first
-// blocks left some SMs with twice the others' share).
-__device__ __forceinline__ bool pick_share(int nkv, const int* __restrict__ q_start, int requests, int window, int keep,
-                                           int& first_item, int& kvh, int& b, int& split, int& splits) {
-    const int items = gridDim.x / nkv;
-    constexpr unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    auto tiles_of = [&](int i) {                 // of the list that request i walks
-        if (i >= requests) return 0;
-        const int pos = q_start[i], lo = first_visible(pos, window);
-        return kept_tiles<TK>(lo, keep) + pos / TK - lo / TK + 1;
-    };
-    const int first = tiles_of(lane);            // the first 32 requests' stay in registers
-    auto shares = [&](int base, int u) { return ((base == 0 ? first : tiles_of(base + lane)) + u - 1) / u; };
-    int longest = 0;
-    for (int base = 0; base < requests; base += 32) longest = max(longest, base == 0 ? first : tiles_of(base + lane));
-    longest = __reduce_max_sync(FULL, longest);
-    int low = BALANCED_MIN_TILES - 1, high = max(longest, BALANCED_MIN_TILES);      // ``high`` tiles a share: one item a request
-    while (high - low > 1) {
-        const int mid = (low + high) >> 1;
-        int sum = 0;
-        for (int base = 0; base < requests; base += 32) sum += shares(base, mid);
-        if (__reduce_add_sync(FULL, sum) <= items) high = mid;
-        else low = mid;
-    }
-    int total = 0;
-    for (int base = 0; base < requests; base += 32) total += shares(base, high);
-    total = __reduce_add_sync(FULL, total) * nkv;                   // blocks with a share
-    const int mine_at = (int)((long long)blockIdx.x * total / gridDim.x), next_at = (int)((long long)(blockIdx.x + 1) * total / gridDim.x);
-    if (mine_at == next_at) return false;
-    kvh = mine_at % nkv;
-    int item = mine_at / nkv;
-    first_item = item;
-    for (int base = 0; base < requests; base += 32) {
-        const int mine = shares(base, high);
-        int upto = mine;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(FULL, upto, o);
-            if (lane >= o) upto += v;
-        }
-        const unsigned here = __ballot_sync(FULL, item >= upto - mine && item < upto);
-        if (here) {
-            const int who = __ffs(here) - 1;
-            b = base + who;
-            split = item - __shfl_sync(FULL, upto - mine, who);
-            splits = __shfl_sync(FULL, mine, who);
-            return true;
-        }
-        item -= __shfl_sync(FULL, upto, 31);
-    }
-    return false;
-}
-
-template <int DMAX, bool UPPER, bool CLUSTER = false, int STAGES = 2, bool BALANCED = false>
+template <int DMAX, bool UPPER, bool CLUSTER = false, int STAGES = 2>
 __global__ void __launch_bounds__(DECODE_WARPS * 32)
 paged_decode_kernel(const bf16* __restrict__ q, long long q_stride, bf16* __restrict__ out, long long out_stride,
                     float* __restrict__ part_o, float* __restrict__ part_lse, const bf16* __restrict__ kc,
                     const bf16* __restrict__ vc, const int* __restrict__ block_table, int bt_stride,
                     const int* __restrict__ cu_q, const int* __restrict__ q_start, int nq, int nkv, int d, int ps,
                     int num_pages, float scale_log2, int window, int keep, int mode, int* __restrict__ status,
-                    const float* __restrict__ per_head, float cap_log2, int requests, int2* __restrict__ directory) {
+                    const float* __restrict__ per_head, float cap_log2) {
     griddep_wait();
     griddep_launch_dependents();
     const bool sink = mode & 1, sigmoid = mode & 2;
@@ -378,12 +317,7 @@ paged_decode_kernel(const bf16* __restrict__ q, long long q_stride, bf16* __rest
     bf16* smem = reinterpret_cast<bf16*>(smem_raw);
     constexpr int TILE = TK * pitch<DMAX>();         // elements per K (or V) stage
     constexpr int THREADS = DECODE_WARPS * 32;
-    int split = blockIdx.x, splits = gridDim.x, kvh = blockIdx.y, b = blockIdx.z;
-    int item = 0;
-    if (BALANCED) {
-        if (!pick_share(nkv, q_start, requests, window, keep, item, kvh, b, split, splits)) return;
-        if (split == 0 && kvh == 0 && threadIdx.x == 0) directory[b] = make_int2(item, splits);
-    }
+    const int split = blockIdx.x, splits = gridDim.x, kvh = blockIdx.y, b = blockIdx.z;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int G = nq / nkv;
     const int tok = cu_q[b];
@@ -523,7 +457,7 @@ paged_decode_kernel(const bf16* __restrict__ q, long long q_stride, bf16* __rest
                     *reinterpret_cast<__nv_bfloat162*>(op + col) = __floats2bfloat162_rn(o[n][2 * i] * inv, o[n][2 * i + 1] * inv);
             }
         } else {
-            const size_t slot = BALANCED ? (size_t)item * nq + head : ((size_t)b * nq + head) * splits + split;
+            const size_t slot = ((size_t)b * nq + head) * splits + split;
             float* po = part_o + slot * d;
 #pragma unroll
             for (int n = 0; n < DMAX / 8; ++n) {
@@ -642,56 +576,6 @@ __global__ void decode_combine_kernel(const float* __restrict__ part_o, const fl
             __syncthreads();                         // before the next round of columns overwrites the sums
         }
         if (grp == 0 && j < d) op[j] = __float2bfloat16_rn(acc * inv_total);
-    }
-}
-
-// The merge of the balanced form: a warp per (request, head) adds its items up in their order, weighted by what each saw of the
-// softmax sum; a request of one item has its output already.
-constexpr int GATHER_WARPS = 4;
-__global__ void __launch_bounds__(GATHER_WARPS * 32)
-decode_gather_kernel(const float* __restrict__ part_o, const float* __restrict__ part_lse, const int2* __restrict__ directory,
-                     bf16* __restrict__ out, long long out_stride, const int* __restrict__ cu_q, int nq, int d, int requests, int added) {
-    griddep_wait();
-    griddep_launch_dependents();
-    const int at = blockIdx.x * GATHER_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (at >= requests * nq) return;
-    const int b = at / nq, head = at - b * nq;
-    const int2 mine = directory[b];
-    const int first = mine.x, count = mine.y;
-    if (count == 1) return;
-    float mx = -CUDART_INF_F;
-    for (int s = lane; s < count; s += 32) mx = fmaxf(mx, part_lse[(size_t)(first + s) * nq + head]);
-    mx = warp_max(mx);
-    float4 acc[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
-    float total = 0.f;
-    for (int base = 0; base < count; base += 32) {
-        const int s = base + lane;
-        const float w = s < count && mx != -CUDART_INF_F ? ex2(part_lse[(size_t)(first + s) * nq + head] - mx) : 0.f;
-        total += w;
-        const int here = min(32, count - base);
-#pragma unroll 4
-        for (int i = 0; i < here; ++i) {
-            const float ws = __shfl_sync(0xffffffffu, w, i);
-            const float* v = part_o + ((size_t)(first + base + i) * nq + head) * d;
-#pragma unroll
-            for (int c = 0; c < 2; ++c) {
-                if (lane * 4 + 128 * c < d) {
-                    const float4 f = *reinterpret_cast<const float4*>(v + lane * 4 + 128 * c);
-                    acc[c].x += ws * f.x; acc[c].y += ws * f.y; acc[c].z += ws * f.z; acc[c].w += ws * f.w;
-                }
-            }
-        }
-    }
-    total = warp_sum(total);
-    const float inv = added ? 1.f : (total > 0.f ? 1.f / total : 0.f);      // added (sigmoid weights): parts of weight 1, summed
-    bf16* op = out + (size_t)cu_q[b] * out_stride + (size_t)head * d;
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-        const int j = lane * 4 + 128 * c;
-        if (j < d) {
-            *reinterpret_cast<__nv_bfloat162*>(op + j) = __floats2bfloat162_rn(acc[c].x * inv, acc[c].y * inv);
-            *reinterpret_cast<__nv_bfloat162*>(op + j + 2) = __floats2bfloat162_rn(acc[c].z * inv, acc[c].w * inv);
-        }
     }
 }
 
@@ -881,8 +765,7 @@ extern "C" int fe_paged_decode_mma_upcoming(const void* q, long long q_stride, v
         if (allow_smem(paged_decode_kernel<DMAX, UPPER>, decode_smem<DMAX>(), "paged_decode")) return 1;          \
         fe::launch(paged_decode_kernel<DMAX, UPPER>, grid, DECODE_WARPS * 32, decode_smem<DMAX>(), stream,                               \
             (const bf16*)q, q_stride, (bf16*)out, out_stride, part_o, part_lse, (const bf16*)kc, (const bf16*)vc, \
-            block_table, bt_stride, cu_q, q_start, nq, nkv, d, ps, num_pages, scale_log2, window, keep, sink, status, per_head, softcap * LOG2E,  \
-            requests, (int2*)nullptr);                                                                            \
+            block_table, bt_stride, cu_q, q_start, nq, nkv, d, ps, num_pages, scale_log2, window, keep, sink, status, per_head, softcap * LOG2E);  \
     } while (0)
     const bool upper = nq / nkv > 8;
     if (d <= 64) { if (upper) FE_DECODE(64, true); else FE_DECODE(64, false); }
@@ -900,57 +783,6 @@ extern "C" int fe_paged_decode_mma_upcoming(const void* q, long long q_stride, v
         return fe_check_launch("paged_decode combine");
     }
     return 0;
-}
-
-// The same attention with the splits dealt out by the requests' lengths (see BALANCED above).  ``items``: the shares that the step's
-// requests are cut into at most, ``requests`` at least; items * nkv blocks should be resident at once.  ``scratch``:
-// fe_paged_decode_balanced_scratch_bytes bytes on a 16-byte boundary.
-extern "C" long long fe_paged_decode_balanced_scratch_bytes(int requests, int nq, int d, int items) {
-    return (long long)items * nq * (d + 1) * (long long)sizeof(float) + (long long)(requests + 1) * (long long)sizeof(int2);
-}
-
-extern "C" int fe_paged_decode_balanced(const void* q, long long q_stride, void* out, long long out_stride, void* scratch, const void* kc,
-                                        const void* vc, const int* block_table, int bt_stride, const int* cu_q, const int* q_start,
-                                        int requests, int nq, int nkv, int d, int ps, int num_pages, float scale, int window, int keep,
-                                        int sink, int items, int* status, const float* per_head, float softcap, cudaStream_t stream) {
-    if (check_common("paged_decode", nq, nkv, d, ps, num_pages, window, keep, q_stride, out_stride)) return 1;
-    FE_REQUIRE(nq / nkv <= 16, "paged_decode: %d query heads per key/value head; this kernel takes up to 16", nq / nkv);
-    FE_REQUIRE(requests >= 0 && items >= requests && items >= 1 && (long long)items * nkv <= 2147483647LL && (long long)requests * nq <= 2147483647LL,
-               "paged_decode (balanced): %d items for %d requests", items, requests);
-    FE_REQUIRE(scratch != nullptr && ((size_t)scratch & 15) == 0, "paged_decode (balanced): scratch memory on a 16-byte boundary");
-    if (requests == 0) return 0;
-    float* part_o = (float*)scratch;
-    float* part_lse = part_o + (size_t)items * nq * d;
-    int2* directory = (int2*)(((size_t)(part_lse + (size_t)items * nq) + 7) & ~(size_t)7);
-    const float scale_log2 = scale * LOG2E;
-#define FE_DECODE_BALANCED(DMAX, UPPER)                                                                            \
-    do {                                                                                                          \
-        auto kernel = paged_decode_kernel<DMAX, UPPER, false, 2, true>;                                            \
-        if (allow_smem(kernel, decode_smem<DMAX>(), "paged_decode (balanced)")) return 1;                          \
-        fe::launch(kernel, items * nkv, DECODE_WARPS * 32, decode_smem<DMAX>(), stream, (const bf16*)q, q_stride, (bf16*)out, out_stride, \
-                   part_o, part_lse, (const bf16*)kc, (const bf16*)vc, block_table, bt_stride, cu_q, q_start, nq, nkv, d, ps, num_pages, \
-                   scale_log2, window, keep, sink, status, per_head, softcap * LOG2E, requests, directory);        \
-    } while (0)
-    const bool upper = nq / nkv > 8;
-    if (d <= 64) { if (upper) FE_DECODE_BALANCED(64, true); else FE_DECODE_BALANCED(64, false); }
-    else if (d <= 128) { if (upper) FE_DECODE_BALANCED(128, true); else FE_DECODE_BALANCED(128, false); }
-    else { if (upper) FE_DECODE_BALANCED(256, true); else FE_DECODE_BALANCED(256, false); }
-#undef FE_DECODE_BALANCED
-    if (fe_check_launch("paged_decode (balanced)")) return 2;
-    // the merge's blocks take their places while the shares are still walked (they are small, and all shares are resident): a
-    // boundary between the two would cost as much as the merge itself
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((requests * nq + GATHER_WARPS - 1) / GATHER_WARPS));
-    cfg.blockDim = dim3(GATHER_WARPS * 32);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = (fe_pdl_enabled() & FE_PDL_ELEMENTWISE) != 0;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, decode_gather_kernel, (const float*)part_o, (const float*)part_lse, (const int2*)directory, (bf16*)out, out_stride,
-                       cu_q, nq, d, requests, sink & 2);
-    return fe_check_launch("paged_decode gather");
 }
 
 // The same attention with the splits of a (request, key/value head) as one thread-block cluster that merges its
@@ -1050,7 +882,7 @@ extern "C" int fe_paged_decode_cluster(const void* q, long long q_stride, void* 
         cfg.dynamicSmemBytes = decode_smem<DMAX>(STAGES);                                                              \
         const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, (const bf16*)q, q_stride, (bf16*)out, out_stride,     \
             (float*)nullptr, (float*)nullptr, (const bf16*)kc, (const bf16*)vc, block_table, bt_stride, cu_q, q_start, \
-            nq, nkv, d, ps, num_pages, scale_log2, window, keep, sink, status, per_head, softcap * LOG2E, requests, (int2*)nullptr);   \
+            nq, nkv, d, ps, num_pages, scale_log2, window, keep, sink, status, per_head, softcap * LOG2E);                             \
         FE_REQUIRE(err == cudaSuccess, "paged_decode (cluster of %d): %s", splits, cudaGetErrorString(err));           \
     } while (0)
     const bool upper = nq / nkv > 8;

@@ -691,40 +691,6 @@ def paged_decode_cluster(q, q_stride, k_cache, v_cache, block_table, cu_q, q_sta
     return out
 
 
-def decode_items(requests: int, nkv: int, sms: int | None = None) -> int:
-    """Into how many shares of keys the balanced form cuts a step's requests at most: what one round of resident blocks (six an
-    SM) holds, one share a request at least."""
-    return max(requests, 6 * (sms or sm_count()) // nkv)
-
-
-BALANCED_MIN_PAIRS, BALANCED_MIN_KEYS = 128, 4096
-
-
-def decode_balanced(requests: int, nkv: int, max_ctx_len: int) -> bool:
-    """Whether decode attention deals its splits out by the requests' lengths: many (request, key/value head) pairs, so that each
-    has few splits and the longest request's are what the step waits for, and contexts so long that finding and merging the
-    shares is small against the walk.  16 requests of 2,048 to 8,192 tokens, eight heads: 76 -> 66 us, all of 8,192: 91 -> 93; below
-    the line a batch of equal lengths loses more than 5 % (64 of 2,048, four heads: 52 -> 56, of 512 to 2,048: 45 -> 41; 16 of
-    512, eight heads: 11 -> 16)."""
-    return requests * nkv >= BALANCED_MIN_PAIRS and max_ctx_len >= BALANCED_MIN_KEYS
-
-
-def paged_decode_balanced(q, q_stride, k_cache, v_cache, block_table, cu_q, q_start, requests, nq, nkv, d, page_size,
-                          scale, window, items, out=None, sink=False, sigmoid=False, head_bias=None, softcap=0.0,
-                          head_scales=None, keep=0):
-    """Tensor-core decode attention with the splits dealt out by the requests' lengths, ``items`` of them at most."""
-    if out is None:
-        out = torch.empty((requests, nq * d), dtype=torch.bfloat16, device=k_cache.device)
-    mapped, per_head, softcap = _score_map(sigmoid, head_bias, softcap, head_scales)
-    lib = _bf16()
-    work = scratch(k_cache.device, lib.fe_paged_decode_balanced_scratch_bytes(_c_int(requests), _c_int(nq), _c_int(d), _c_int(items)))
-    _run(lib, "fe_paged_decode_balanced", _ptr(q), _c_ll(q_stride), _ptr(out), _c_ll(out.stride(0)), _ptr(work), _ptr(k_cache),
-         _ptr(v_cache), _ptr(block_table), _c_int(block_table.shape[1]), _ptr(cu_q), _ptr(q_start), _c_int(requests),
-         _c_int(nq), _c_int(nkv), _c_int(d), _c_int(page_size), _c_int(k_cache.shape[0]), _c_float(scale), _c_int(window), _c_int(keep),
-         _c_int(_attention_mode(sink, sigmoid, mapped)), _c_int(items), _ptr(status_word(k_cache.device)), _ptr(per_head), _c_float(softcap), _stream())
-    return out
-
-
 def paged_prefill_mma(q, q_stride, k_cache, v_cache, block_table, cu_q, q_start, T, requests, max_q_len, nq, nkv, d,
                       page_size, scale, window, sink=False, sigmoid=False, head_bias=None, softcap=0.0,
                       head_scales=None, keep=0):
@@ -831,10 +797,6 @@ def paged_attention(qkv, k_cache, v_cache, block_table, ctx, nq, nkv, d, page_si
     if ctx.max_q_len == 1 and nq // nkv <= 16:
         # a window or a chunk bounds the keys a token walks (plus the tile of 32 that its first key lies in)
         span = ctx.max_ctx_len if window == 0 else min(ctx.max_ctx_len, abs(window) + 31 + -(-keep_first // 32) * 32)
-        if decode_balanced(requests, nkv, span):
-            return paged_decode_balanced(qkv, qkv.stride(0), k_cache, v_cache, block_table, ctx.cu_q, ctx.q_start, requests, nq, nkv, d,
-                                         page_size, scale, window, decode_items(requests, nkv), sink=sink, sigmoid=sigmoid,
-                                         head_bias=head_bias, **score)
         splits = decode_splits(requests, nkv, span)
         clustered = decode_cluster_splits(splits, span, requests * nkv,
                                           lambda s: clusters_resident(requests, nq, nkv, d, s))

@@ -102,17 +102,3 @@ def test_sample_short_list_and_its_limits(V):
             target = kernel_refs.uniform_from(int(seed[r]), 5) * float(cum[-1])
             slack = 1e-5 * float(cum[-1])          # float32 sums of up to 1,025 masses: well below 1,025 * 2^-24
             assert (float(cum[token - 1]) if token else 0.0) - slack <= target <= float(cum[token]) + slack, (k, r)
-
-
-@pytest.mark.parametrize("nq,nkv,d", [(4, 2, 64), (28, 4, 128), (5, 1, 80), (12, 1, 48), (4, 1, 256)])
-@pytest.mark.parametrize("window,sink", [(0, False), (70, True), (-100, False)])
-def test_decode_attention_balanced(nq, nkv, d, window, sink, gen, monkeypatch):
-    """Decode attention whose splits are dealt out by length: requests of one tile beside long ones, more of them than a warp has
-    lanes, as many items as requests and many more."""
-    monkeypatch.setattr(ops(), "decode_balanced", lambda *sizes: True)
-    for items in (1, 60, 400):
-        monkeypatch.setattr(ops(), "decode_items", lambda requests, heads: max(requests, items))
-        for starts in ([700], [0, 1, 31, 32, 33, 1023], [0, 5, 64, 200, 900] * 9):
-            got, want, _ = _attention_case(torch.bfloat16, nq, nkv, d, 16, [(s, 1) for s in starts], window, gen, sink=sink)
-            torch.testing.assert_close(got.float(), want.float(), **bar(torch.bfloat16))
-    ops().check_status(DEV)
