@@ -18,12 +18,17 @@ def validate_sampling(temperature: float, top_k: int) -> None:
         raise ValueError("temperature and top_k must be >= 0")
 
 
-def _numbers(values, dtype, one):
-    """A sequence of numbers (or of one-element tensors) as an array."""
+def _fill(words, values, dtype) -> None:
+    """``values`` into the numpy array ``words``: a list or tuple that numpy takes for numbers of the kind in one conversion;
+    anything else as a tensor of ``dtype``, which takes, broadcasts and refuses what a tensor does."""
     try:
-        return np.asarray(values, dtype=dtype)
-    except TypeError:
-        return np.asarray([one(v) for v in values], dtype=dtype)
+        given = np.array(values) if type(values) in (list, tuple) else None
+    except (TypeError, ValueError):
+        given = None
+    if given is not None and given.shape == words.shape and given.dtype.kind in ("fi" if dtype is torch.float32 else "i"):
+        words[:] = given
+    else:
+        torch.from_numpy(words)[:] = torch.tensor(list(values), dtype=dtype)
 
 
 class Sampler:
@@ -43,12 +48,11 @@ class Sampler:
         if logits.dim() != 2 or logits.shape[0] != len(temperatures):
             raise ValueError("Expected logits [requests, vocab]")
         n = len(temperatures)
-        t64, k64 = _numbers(temperatures, np.float64, float), _numbers(top_ks, np.int64, int)
-        if (t64 < 0).any() or (k64 < 0).any():
-            for t, k in zip(temperatures, top_ks):
+        for t, k in zip(temperatures, top_ks):
+            if t < 0 or k < 0:                           # a call a row would cost more than the comparisons
                 validate_sampling(t, k)
         dev = logits.device
-        if not t64.any():
+        if all(t == 0.0 for t in temperatures):
             # greedy rows need no parameters: zeros kept on the device, no copy per step
             key = (str(dev), n)
             if key not in self._zeros:
@@ -61,9 +65,11 @@ class Sampler:
         # each (four conversions and two kernels before: the host took longer than the device, 106 us for 64 rows)
         packed = torch.empty(3 * n, dtype=torch.int64, pin_memory=dev.type == "cuda")
         host = packed.numpy()
-        host[:n], host[n:2 * n] = _numbers(seeds, np.int64, int), _numbers(draws, np.int64, int)
-        host[2 * n:].view(np.float32)[:n] = t64
-        host[2 * n:].view(np.int32)[n:] = k64
+        with np.errstate(over="ignore"):                 # a temperature beyond float32 is an infinite one
+            _fill(host[:n], seeds, torch.int64)
+            _fill(host[n:2 * n], draws, torch.int64)
+            _fill(host[2 * n:].view(np.float32)[:n], temperatures, torch.float32)
+            _fill(host[2 * n:].view(np.int32)[n:], top_ks, torch.int64)
         on_dev = packed.to(dev, non_blocking=True)
         small = on_dev[2 * n:].view(torch.int32)
         return self.ops.sample(logits, small[:n].view(torch.float32), small[n:], on_dev[:n], on_dev[n:2 * n])

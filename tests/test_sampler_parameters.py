@@ -1,0 +1,64 @@
+"""What the sampler takes as a step's parameters: lists of numbers in one conversion, any other sequence as a tensor would take
+it; what is no number, is negative or does not fit is refused."""
+import math
+
+import numpy as np
+import pytest
+import torch
+
+from flexengine_b200.sampling import Sampler
+
+LOGITS = torch.zeros(2, 8)
+GOOD = ([0.5, 1.0], [0, 3], [1, 2], [3, 4])
+
+
+class Seen:
+    def sample(self, logits, temperature, top_k, seed, draw):
+        assert (temperature.dtype, top_k.dtype, seed.dtype, draw.dtype) == (torch.float32, torch.int32, torch.int64, torch.int64)
+        return [temperature.tolist(), top_k.tolist(), seed.tolist(), draw.tolist()]
+
+
+def taken(*parameters):
+    return Sampler(Seen()).sample_on_device(LOGITS, *parameters)
+
+
+def changed(at, values):
+    return GOOD[:at] + (values,) + GOOD[at + 1:]
+
+
+@pytest.mark.parametrize("at,values", [(0, [None, 1.0]), (0, ["0.5", 1.0]), (0, [[0.5], [1.0]]), (1, [None, 3]), (1, ["1", 3]),
+                                       (1, [[0], [1]]), (2, [None, 2]), (2, ["7", 2])])
+def test_what_is_no_number_is_refused(at, values):
+    with pytest.raises((TypeError, ValueError)):
+        taken(*changed(at, values))
+
+
+@pytest.mark.parametrize("at,values", [(0, [0.5, -1.0]), (0, [math.nan, -1.0]), (0, np.array([0.5, -1.0])), (0, torch.tensor([0.5, -1.0])),
+                                       (1, [0, -1]), (1, [-0.5, 3]), (1, np.array([0, -1])), (1, (3, -2))])
+def test_negative_parameters_are_refused(at, values):
+    with pytest.raises(ValueError, match="must be >= 0"):
+        taken(*changed(at, values))
+
+
+@pytest.mark.parametrize("at,values,error", [(1, [2 ** 70, 1], ValueError), (2, [2 ** 63, 2], ValueError), (1, [math.nan, 1], RuntimeError),
+                                             (1, [0, 1, 2], RuntimeError), (2, [1, 2, 3], RuntimeError)])
+def test_what_does_not_fit_is_refused_as_a_tensor_refuses_it(at, values, error):
+    with pytest.raises(error):
+        taken(*changed(at, values))
+
+
+@pytest.mark.parametrize("at,values,want", [
+    (0, (0.25, 2), [0.25, 2.0]), (0, np.array([0.5, 1.0], dtype=np.float32), [0.5, 1.0]), (0, torch.tensor([0.5, 1.0], dtype=torch.bfloat16), [0.5, 1.0]),
+    (0, [torch.tensor(0.5), 1.0], [0.5, 1.0]), (0, [1e39, 1.0], [math.inf, 1.0]), (0, [1e-60, 1.0], [0.0, 1.0]), (0, [True, 0.5], [1.0, 0.5]),
+    (1, (2, 5), [2, 5]), (1, [1.7, 3], [1, 3]), (1, torch.tensor([4, 5]), [4, 5]), (1, [7], [7, 7]), (1, [2 ** 32 + 3, 1], [3, 1]),
+    (2, range(5, 7), [5, 6]), (2, [-1, 2 ** 63 - 1], [-1, 2 ** 63 - 1]), (3, np.array([8, 9]), [8, 9]), (3, [6], [6, 6])])
+def test_numbers_of_any_kind_arrive(at, values, want):
+    got = taken(*changed(at, values))
+    assert got[at] == want
+    assert all(got[i] == GOOD[i] for i in range(4) if i != at)
+
+
+def test_greedy_rows_take_whatever_stands_beside_them():
+    for top_ks in ([2 ** 70, 1], [0], [1, 2, 3], (5, 5)):
+        assert taken([0.0, 0], top_ks, [1], [3]) == [[0.0, 0.0], [0, 0], [0, 0], [0, 0]]
+    assert Sampler(Seen()).sample_on_device(torch.zeros(0, 8), [], [], [], []) == [[], [], [], []]
