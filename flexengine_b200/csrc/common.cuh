@@ -137,8 +137,8 @@ template <int TILE> __host__ __device__ __forceinline__ int listed_tile(int i, i
 
 // Programmatic dependent launch: a kernel launched through fe::launch may begin while the kernel
 // before it in the stream is still running.  Everything it reads that an earlier kernel wrote,
-// and every write, must come after griddep_wait(); only data that no kernel writes (weights)
-// may be touched before.  launch_dependents lets the next kernel start its own preamble; it is
+// and every write, must come after griddep_wait(); only what stood in memory before that kernel
+// began (the weights of a model, whose steps start with other kernels) may be read before.  launch_dependents lets the next kernel start its own preamble; it is
 // called after the wait, so that at most one kernel is resident ahead of the one that runs
 // (called before, every later kernel of a graph piles onto the SMs and starves the running one).
 // Without the launch attribute both are no-ops; fe_set_pdl names the classes of kernels that get it.  What it is worth: a

@@ -56,6 +56,8 @@ struct ResidEpilogue {
 // ``next``: memory that the kernel after this one streams first (may be null): as a block leaves its loop it asks for its
 // share of the first ``next_bytes`` to be brought into L2, so that the next kernel's first loads, which would
 // otherwise go out to an idle memory system after the launch gap, are met there.
+// ``held``: W belongs to a model, whose steps begin with other kernels: it stands in memory before the kernel ahead of this one
+// began.  Any other W may be that very kernel's output, and is read when that has ended, like x.
 struct RowScale {
     const float* sumsq;         // [tiles][8] or nullptr: the input is normalised already
     int tiles;
@@ -63,6 +65,7 @@ struct RowScale {
     int width;                  // elements of a row (the mean is over them)
     const void* next;
     long long next_bytes;
+    int held;
 };
 
 // What the fused query/key/value epilogue needs beside the product: bias, rotary table, where the
@@ -196,10 +199,11 @@ skinny_gemm_kernel(const bf16* __restrict__ x, const bf16* __restrict__ W, void*
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) acc[r][nt][0] = acc[r][nt][1] = acc[r][nt][2] = acc[r][nt][3] = 0.f;
 
+    if (!scale.held && first_unit) griddep_wait();
     for (int s = s_begin; s < s_end; s += PF) {
         uint4 b[PF][NT][2];
         if (!(STAYS && ahead && s == s_begin)) load_weights(w0, w1, s);
-        // the weights above depend on no kernel; the activations below are the previous kernel's
+        // held weights depend on no kernel that may still run; the activations below are the previous kernel's
         // output, so the first batch of weight loads is already in flight while that kernel ends
         if (s == s_begin && first_unit) {
             griddep_wait();
@@ -437,16 +441,16 @@ static int check_scale(const char* what, const float* sumsq, int sumsq_tiles, in
 
 // epilogue: 0 bfloat16 [M, N]; 1 float [M, N]; 2 SwiGLU: W is [2 I, K] (gate rows, then up rows), out bfloat16 [M, I]; 5 the
 // same with the tanh form of GELU as the gate's function, 7 with relu; 6 out = relu(x W^T)^2 as bfloat16 [M, N], 8 the exact GELU.
-// ``sumsq`` (may be null): see check_scale.
+// ``sumsq`` (may be null): see check_scale.  ``held``: see RowScale (the same for the entry points below).
 extern "C" int fe_skinny_gemm_scaled(const void* x, const void* W, void* out, int M, int N, int K, int epilogue,
                                      const float* sumsq, int sumsq_tiles, float eps, const void* next, long long next_bytes,
-                                     cudaStream_t stream) {
+                                     int held, cudaStream_t stream) {
     FE_REQUIRE(M >= 1 && M <= 16, "skinny_gemm: %d rows; this kernel takes 1 to 16", M);
     FE_REQUIRE(N > 0 && K > 0 && K % KSTEP == 0, "skinny_gemm: K = %d must be a positive multiple of %d", K, KSTEP);
     FE_REQUIRE((((size_t)x | (size_t)W) & 15) == 0, "skinny_gemm: operands must be 16-byte aligned");
     if (check_scale("skinny_gemm", sumsq, sumsq_tiles, M, K)) return 1;
     FE_REQUIRE(next_bytes >= 0, "skinny_gemm: negative byte count");
-    const RowScale scale{sumsq, sumsq_tiles, eps, K, next, next_bytes};
+    const RowScale scale{sumsq, sumsq_tiles, eps, K, next, next_bytes, held};
     if (epilogue == EPI_BF16) return launch<EPI_BF16>(x, W, out, M, N, K, 0, stream, QkvEpilogue{}, ResidEpilogue{}, scale);
     if (epilogue == EPI_F32) return launch<EPI_F32>(x, W, out, M, N, K, 0, stream, QkvEpilogue{}, ResidEpilogue{}, scale);
     if (epilogue == EPI_RELU2 || epilogue == EPI_GELU)
@@ -461,7 +465,7 @@ extern "C" int fe_skinny_gemm_scaled(const void* x, const void* W, void* out, in
 
 extern "C" int fe_skinny_gemm(const void* x, const void* W, void* out, int M, int N, int K, int epilogue,
                               cudaStream_t stream) {
-    return fe_skinny_gemm_scaled(x, W, out, M, N, K, epilogue, nullptr, 0, 0.f, nullptr, 0, stream);
+    return fe_skinny_gemm_scaled(x, W, out, M, N, K, epilogue, nullptr, 0, 0.f, nullptr, 0, 0, stream);
 }
 
 // The product that ends a branch of a layer: residual[M, N] += x W^T (float, in place); scaled[M, N] = bfloat16(new
@@ -469,7 +473,7 @@ extern "C" int fe_skinny_gemm(const void* x, const void* W, void* out, int M, in
 // ``sumsq_in`` (may be null): the scales of the input rows, as for fe_skinny_gemm_scaled.  M <= 8.
 extern "C" int fe_skinny_gemm_residual(const void* x, const void* W, float* residual, const float* norm_weight, void* scaled,
                                        float* sumsq_out, int M, int N, int K, const float* sumsq_in, int sumsq_tiles,
-                                       float eps, const void* next, long long next_bytes, cudaStream_t stream) {
+                                       float eps, const void* next, long long next_bytes, int held, cudaStream_t stream) {
     FE_REQUIRE(M >= 1 && M <= 8, "skinny_gemm_residual: %d rows; this kernel takes 1 to 8", M);
     FE_REQUIRE(N > 0 && K > 0 && K % KSTEP == 0, "skinny_gemm_residual: K = %d must be a positive multiple of %d", K, KSTEP);
     FE_REQUIRE((((size_t)x | (size_t)W) & 15) == 0, "skinny_gemm_residual: operands must be 16-byte aligned");
@@ -478,7 +482,7 @@ extern "C" int fe_skinny_gemm_residual(const void* x, const void* W, float* resi
     const ResidEpilogue resid{residual, norm_weight, (bf16*)scaled, sumsq_out};
     FE_REQUIRE(next_bytes >= 0, "skinny_gemm_residual: negative byte count");
     return launch<EPI_RESID>(x, W, nullptr, M, N, K, 0, stream, QkvEpilogue{}, resid,
-                             RowScale{sumsq_in, sumsq_tiles, eps, K, next, next_bytes});
+                             RowScale{sumsq_in, sumsq_tiles, eps, K, next, next_bytes, held});
 }
 
 // The query/key/value projection of an attention layer with its epilogue fused: y = x W^T + bias,
@@ -489,7 +493,7 @@ extern "C" int fe_skinny_gemm_residual(const void* x, const void* W, float* resi
 extern "C" int fe_skinny_qkv(const void* x, const void* W, void* out, const float* bias, const int* positions,
                              const float* inv_freq, const int* slot_mapping, void* kc, void* vc, int M, int K, int nq,
                              int nkv, int d, int ps, long long num_slots, const float* sumsq, int sumsq_tiles, float eps,
-                             int* status, cudaStream_t stream) {
+                             int* status, int held, cudaStream_t stream) {
     FE_REQUIRE(M >= 1 && M <= 8, "skinny_qkv: %d rows; this kernel takes 1 to 8", M);
     FE_REQUIRE(K > 0 && K % KSTEP == 0, "skinny_qkv: K = %d must be a positive multiple of %d", K, KSTEP);
     FE_REQUIRE(d >= 16 && d % 16 == 0 && nq > 0 && nkv > 0 && ps > 0, "skinny_qkv: bad head size or counts");
@@ -498,5 +502,5 @@ extern "C" int fe_skinny_qkv(const void* x, const void* W, void* out, const floa
     if (check_scale("skinny_qkv", sumsq, sumsq_tiles, M, K)) return 1;
     QkvEpilogue e{bias, positions, inv_freq, slot_mapping, (bf16*)kc, (bf16*)vc, nq, nkv, d, ps, num_slots, status};
     return launch<EPI_QKV>(x, W, out, M, (nq + 2 * nkv) * d, K, 0, stream, e, ResidEpilogue{},
-                           RowScale{sumsq, sumsq_tiles, eps, K, nullptr, 0});
+                           RowScale{sumsq, sumsq_tiles, eps, K, nullptr, 0, held});
 }

@@ -313,7 +313,7 @@ def linear(x, w, bias=None, out_float32=False, follow=None, upcoming=None):
             table = torch.empty((-(-N // 16), 8), dtype=torch.float32, device=rows.device)
             _run(_bf16(), "fe_skinny_gemm_residual", _ptr(rows), _ptr(w), _ptr(residual), _ptr(norm_weight), _ptr(scaled),
                  _ptr(table), _c_int(M), _c_int(N), _c_int(rows.shape[1]), sumsq, tiles, eps,
-                 *_upcoming(upcoming, M, UPCOMING_TAIL_BYTES), _stream())
+                 *_upcoming(upcoming, M, UPCOMING_TAIL_BYTES), _held(w), _stream())
             return Prenormed(scaled, table, norm_eps, residual, norm_weight)
     if kernel and w.dtype == torch.bfloat16:
         wide = out_float32 or bias is not None           # a bias is added in float32, before the one rounding
@@ -353,6 +353,13 @@ def skinny_ok(x, w) -> bool:
             and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
+def _held(w):
+    """Whether the weight-streaming kernel may begin to read ``w`` while the kernel before it ends: only what a model holds
+    (``DecoderModel.bind`` marks it), for its steps begin with kernels that wait for whatever wrote it.  Any other matrix may be the
+    output of that very kernel."""
+    return _c_int(1 if getattr(w, "held", False) else 0)
+
+
 def skinny_gemm(x, w, epilogue: int = EPI_BF16, upcoming=None):
     """x [M <= 16, K] (a tensor or a Prenormed) times w [N, K]^T by streaming w once; see csrc/gemm_skinny.cu."""
     x, sumsq, tiles, eps = _rows_and_scale(x)
@@ -363,7 +370,7 @@ def skinny_gemm(x, w, epilogue: int = EPI_BF16, upcoming=None):
     else:
         out = torch.empty((M, N), dtype=torch.float32 if epilogue == EPI_F32 else torch.bfloat16, device=x.device)
     _run(_bf16(), "fe_skinny_gemm_scaled", _ptr(x), _ptr(w), _ptr(out), _c_int(M), _c_int(N), _c_int(K), _c_int(epilogue),
-         sumsq, tiles, eps, *_upcoming(upcoming, M, UPCOMING_TAIL_BYTES), _stream())
+         sumsq, tiles, eps, *_upcoming(upcoming, M, UPCOMING_TAIL_BYTES), _held(w), _stream())
     return out
 
 
@@ -514,7 +521,7 @@ def qkv_projection(h, w, bias, positions, inv_freq, rot, slot_mapping, k_cache, 
         _run(_bf16(), "fe_skinny_qkv", _ptr(rows), _ptr(w), _ptr(out), _ptr(bias), _ptr(positions), _ptr(inv_freq),
              _ptr(slot_mapping), _ptr(k_cache), _ptr(v_cache), _c_int(T), _c_int(rows.shape[1]), _c_int(nq), _c_int(nkv),
              _c_int(d), _c_int(page_size), _c_ll(k_cache.shape[0] * page_size), sumsq, tiles, eps,
-             _ptr(status_word(rows.device)), _stream())
+             _ptr(status_word(rows.device)), _held(w), _stream())
         return out
     if isinstance(h, Prenormed):
         h = h.materialize()

@@ -7,8 +7,21 @@ does arithmetic of its own: sizes and parts come from the plan.
 """
 from __future__ import annotations
 
+import torch
+
 from .base import block_factory, build_part
 from .spec import ModelPlan, PartSpec
+
+
+def _tensors_of(held):
+    """Every tensor that parts hold, those they made of their parameters and those of parts within parts among them."""
+    for value in held:
+        if isinstance(value, torch.Tensor):
+            yield value
+        elif hasattr(value, "parameter_shapes"):
+            yield from _tensors_of(vars(value).values())
+        elif isinstance(value, (list, tuple)):
+            yield from _tensors_of(value)
 
 
 class DecoderModel:
@@ -51,6 +64,8 @@ class DecoderModel:
                            if k[0] == "layer" and k[1] == i and k[2] == part_name})
         for j, part in enumerate(self.junctions):
             part.bind({k[2]: t for k, t in tensors.items() if k[0] == "junction" and k[1] == j})
+        for t in _tensors_of([p for _, p in self._outer_parts()] + [p for b in self.blocks for p in b.parts().values()] + self.junctions):
+            t.held = True       # stands while the model does: a product may begin to read it before the kernel ahead has ended
 
     def _outer_parts(self):
         """The parts outside the layers, under the names their bindings use."""
