@@ -398,8 +398,9 @@ extern "C" int fe_paged_attention_simt(const void* q, long long q_stride, void* 
     FE_REQUIRE(ps > 0 && num_pages > 0, "paged_attention: bad page size or page count");
     FE_REQUIRE(q_stride % 8 == 0, "paged_attention: query row stride %lld must be a multiple of 8 elements", q_stride);
     if (T_tokens == 0) return 0;
-    FE_REQUIRE((((size_t)kc | (size_t)vc) & 15) == 0, "paged_attention: the cache must be 16-byte aligned");
-    if (dtype == FE_F32 && d <= TILE_MAX_D)
+    FE_REQUIRE(((size_t)kc & 15) == 0, "paged_attention: the cache's keys must be 16-byte aligned");
+    // the tiled kernel copies values 16 bytes at a time; the other one reads them one by one
+    if (dtype == FE_F32 && d <= TILE_MAX_D && ((size_t)vc & 15) == 0)
         return launch_tiled((const float*)q, q_stride, (float*)out, out_stride, (const float*)kc, (const float*)vc, block_table,
                             bt_stride, cu_q, q_start, requests, T_tokens, nq, nkv, d, ps, num_pages, scale, window, keep, sink,
                             per_head, softcap, status, stream);
