@@ -1,6 +1,6 @@
 // Paged causal grouped-query attention on CUDA cores, float arithmetic throughout.
 //
-// Keys are taken in blocks of 32 that are aligned to absolute position 0; scores, running maximum, running
+// Keys are taken in blocks of 32 or 64 that are aligned to absolute position 0; scores, running maximum, running
 // sum and the value accumulator are float (online softmax, as the reference's block-wise path:
 // inference/attention/paged.py:50-70).  Key t is visible to the query at position p iff t <= p
 // (and t > p - window, or t < keep, when window > 0; t in the chunk of -window positions that holds p when window < 0)
@@ -12,15 +12,27 @@
 // order, the result for a query does not depend on how its request was cut into steps.
 //
 // Two kernels.  The tiled one serves the true 32-bit path for head sizes up to 128: a block of 32 rows shares every key it
-// loads (below).  The other, one warp per (token, query head) with one key per lane, serves larger heads in 32 bits, and
-// bfloat16 for shapes the tensor core kernels do not take (head sizes beyond 256: the rows of a wide cached latent).
+// loads (below).  The other, one warp per (token, query head), serves calls of the same heads that have little to share
+// (rows_pay), larger heads in 32 bits, and bfloat16 for shapes the tensor core kernels do not take (head sizes beyond 256: the
+// rows of a wide cached latent).
 #include <math_constants.h>
 
 #include "common.cuh"
 
 using namespace fe;
 
-template <typename T, int DPL>
+// A score from the dot product: times the scale, squashed where there is a cap.  Rounded after each step, so that no compiler
+// folds the product into what follows in one kernel and not in another.
+__device__ __forceinline__ float score_of(float dot, float scale, float cap) {
+    const float s = __fmul_rn(dot, scale);
+    return cap > 0.f ? __fmul_rn(cap, tanhf(s / cap)) : s;
+}
+
+// One warp per (token, query head), PER keys a lane at a time: lane l takes keys l, l + 32, ... of a block of 32 PER.  With
+// PER = 2 it does the arithmetic of the tiled kernel below for one row, operation by operation (blocks of 64 keys; the sum of
+// a block's weights first over keys 16 apart, then 32, then within 16), so that a row's result is the same bit for bit
+// whichever of the two takes it.
+template <typename T, int DPL, int PER>
 __global__ void paged_attention_simt_kernel(const T* __restrict__ q, long long q_stride, T* __restrict__ out,
                                             long long out_stride, const T* __restrict__ kc,
                                             const T* __restrict__ vc, const int* __restrict__ block_table,
@@ -31,6 +43,7 @@ __global__ void paged_attention_simt_kernel(const T* __restrict__ q, long long q
     griddep_wait();
     griddep_launch_dependents();
     extern __shared__ float q_smem[];
+    constexpr int KEYS = 32 * PER;
     const int lane = threadIdx.x & 31;
     const int warp_in_block = threadIdx.x >> 5;
     const long long warp = (long long)blockIdx.x * (blockDim.x >> 5) + warp_in_block;
@@ -55,57 +68,78 @@ __global__ void paged_attention_simt_kernel(const T* __restrict__ q, long long q
 
     const int lo = first_visible(pos, window);
     const int* table = block_table + (size_t)r * bt_stride;
-    const int kept = kept_tiles<32>(lo, keep), blocks = kept + pos / 32 - lo / 32 + 1;
+    const int kept = kept_tiles<KEYS>(lo, keep), blocks = kept + pos / KEYS - lo / KEYS + 1;
     for (int at = 0; at < blocks; ++at) {
-        const int kb = listed_tile<32>(at, kept, lo) * 32;
-        const int t = kb + lane;
-        bool valid = (t >= lo || t < keep) && t <= pos;
-        float s = -CUDART_INF_F;
-        long long base = 0;
-        if (valid) {
-            const int page = table[t / ps];
-            if (page < 0 || page >= num_pages) {
-                if (status) atomicOr(status, FE_STATUS_BAD_PAGE);
-                valid = false;
-            } else {
-                base = (((long long)page * nkv + kvh) * ps + (t % ps)) * d;
-                const T* kp = kc + base;
-                float dot = 0.f;
-                for (int j = 0; j < d; j += 8) {
-                    float kv[8];
-                    load8<T>(kp + j, kv);
+        const int kb = listed_tile<KEYS>(at, kept, lo) * KEYS;
+        bool valid[PER];
+        float s[PER], p[PER];
+        long long base[PER];
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) dot = fmaf(qs[j + e], kv[e], dot);
+        for (int u = 0; u < PER; ++u) {
+            const int t = kb + 32 * u + lane;
+            valid[u] = (t >= lo || t < keep) && t <= pos;
+            s[u] = -CUDART_INF_F;
+            base[u] = 0;
+            if (valid[u]) {
+                const int page = table[t / ps];
+                if (page < 0 || page >= num_pages) {
+                    if (status) atomicOr(status, FE_STATUS_BAD_PAGE);
+                    valid[u] = false;
+                } else {
+                    base[u] = (((long long)page * nkv + kvh) * ps + (t % ps)) * d;
+                    const T* kp = kc + base[u];
+                    float dot = 0.f;
+                    for (int j = 0; j < d; j += 8) {
+                        float kv[8];
+                        load8<T>(kp + j, kv);
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) dot = fmaf(qs[j + e], kv[e], dot);
+                    }
+                    s[u] = score_of(dot, scale, cap);
                 }
-                s = dot * scale;
-                if (cap > 0.f) s = cap * tanhf(s / cap);
             }
         }
-        float p;
         if (sigmoid) {
-            p = valid ? 1.f / (1.f + expf(-(s + bias))) : 0.f;
+#pragma unroll
+            for (int u = 0; u < PER; ++u) p[u] = valid[u] ? 1.f / (1.f + expf(-(s[u] + bias))) : 0.f;
             l = 1.f;                                   // the sum is not divided by anything
         } else {
-            const float bm = warp_max(s);
+            float bm = s[0];
+#pragma unroll
+            for (int u = 1; u < PER; ++u) bm = fmaxf(bm, s[u]);
+            bm = warp_max(bm);
             if (bm == -CUDART_INF_F) continue;         // nothing visible in this block (bad pages only)
             const float m_new = fmaxf(m, bm);
             const float alpha = expf(m - m_new);       // exp(-inf) = 0 on the first block
-            p = valid ? expf(s - m_new) : 0.f;
-            l = l * alpha + warp_sum(p);
+            float sum = 0.f;
+#pragma unroll
+            for (int u = 0; u < PER; ++u) {
+                p[u] = valid[u] ? expf(s[u] - m_new) : 0.f;
+                const float pair = p[u] + __shfl_xor_sync(0xffffffffu, p[u], 16);
+                sum = u == 0 ? pair : sum + pair;
+            }
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            l = fmaf(l, alpha, sum);
 #pragma unroll
             for (int i = 0; i < DPL; ++i) acc[i] *= alpha;
             m = m_new;
         }
-        const int count = min(32, pos - kb + 1);
-        for (int tt = 0; tt < count; ++tt) {
-            const float pt = __shfl_sync(0xffffffffu, p, tt);
-            const long long vb = __shfl_sync(0xffffffffu, base, tt);
-            if (pt != 0.f) {
-                const T* vp = vc + vb;
 #pragma unroll
-                for (int i = 0; i < DPL; ++i) {
-                    const int j = lane + 32 * i;
-                    if (j < d) acc[i] = fmaf(pt, to_float(vp[j]), acc[i]);
+        for (int u = 0; u < PER; ++u) {
+            const unsigned weighs = __ballot_sync(0xffffffffu, p[u] != 0.f);      // all from the window's edge to the diagonal, as a rule
+            if (weighs == 0u) continue;
+            const int count = 32 - __clz(weighs);
+            for (int tt = __ffs(weighs) - 1; tt < count; ++tt) {
+                const float pt = __shfl_sync(0xffffffffu, p[u], tt);
+                const long long vb = __shfl_sync(0xffffffffu, base[u], tt);
+                if (pt != 0.f) {
+                    const T* vp = vc + vb;
+#pragma unroll
+                    for (int i = 0; i < DPL; ++i) {
+                        const int j = lane + 32 * i;
+                        if (j < d) acc[i] = fmaf(pt, to_float(vp[j]), acc[i]);
+                    }
                 }
             }
         }
@@ -281,8 +315,7 @@ paged_attention_tiled_kernel(const float* __restrict__ q, long long q_stride, fl
             float top = -CUDART_INF_F;
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                s[i][u] *= factor[i];
-                if (cap > 0.f) s[i][u] = cap * tanhf(s[i][u] / cap);
+                s[i][u] = score_of(s[i][u], factor[i], cap);
                 if (see[i][u]) top = fmaxf(top, s[i][u]);
             }
             if (sigmoid) {
@@ -301,7 +334,7 @@ paged_attention_tiled_kernel(const float* __restrict__ q, long long q_stride, fl
             float sum = (p[i][0] + p[i][1]) + (p[i][2] + p[i][3]);
 #pragma unroll
             for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-            l[i] = l[i] * alpha + sum;
+            l[i] = fmaf(l[i], alpha, sum);
 #pragma unroll
             for (int c = 0; c < 4; ++c) { acc[i][c].x *= alpha; acc[i][c].y *= alpha; }
             m[i] = m_new;
@@ -360,6 +393,24 @@ int launch_tiled(const float* q, long long q_stride, float* out, long long out_s
     return fe_check_launch("paged_attention_tiled");
 }
 
+// Whether a call's rows are taken one warp each and not 32 a block (the same bits either way).  A block of the tiled kernel costs its
+// 8 us however few of its rows and keys are real, and one or two are resident on an SM; a warp a row costs by the key.  So: where no
+// row sees more than a few keys (40 prompts of 9, 12 heads of 128 in two groups: 12.7 us, tiled 26.9; one prompt of 9: 9.0, 15.2; a
+// window of 5 over 1,024 tokens: 36, 50); and where the blocks make several rounds with little in each (``seen`` keys times a block's
+// rows below what a block costs: 128 requests of 64 keys, 32 heads of 128: 76 us, tiled 237; 48 of 130: 110, 195; 128 of 256 with 8
+// heads of 96 over two: 201 against 159 is beyond it), if there are rows enough to hide a warp's walk (16 requests of 256 keys, 32
+// heads: 189 us, tiled 96).
+bool rows_pay(int T_tokens, int requests, int nq, int nkv, int d, long long context, int window, int keep) {
+    const long long G = nq / nkv, portion = (T_tokens + requests - 1) / requests;
+    const long long rows = portion * G, tiles = (rows + TILE_ROWS - 1) / TILE_ROWS, blocks = tiles * nkv * requests;
+    long long seen = context - (portion - 1) / 2;                     // by a row, on average of a portion
+    if (window > 0) seen = min(seen, (long long)window + keep);
+    if (window < 0) seen = min(seen, (1LL - window) / 2);
+    if (seen <= (d <= 32 ? 24 : 16)) return true;
+    const long long resident = (long long)fe_sm_count() * (d <= 80 ? 2 : 1);
+    return blocks > resident && seen * rows <= tiles * (280 + seen / 2) && seen * resident <= 50 * blocks;
+}
+
 }  // namespace
 
 template <typename T>
@@ -371,26 +422,26 @@ static int launch_simt(const void* q, long long q_stride, void* out, long long o
     const long long total = (long long)T_tokens * nq;
     const int blocks = (int)((total + warps - 1) / warps);
     const size_t smem = (size_t)warps * d * sizeof(float);
-#define FE_LAUNCH_SIMT(DPL)                                                                                      \
-    fe::launch(paged_attention_simt_kernel<T, DPL>, blocks, warps * 32, smem, stream,                                    \
+    constexpr int PER = sizeof(T) == 4 ? 2 : 1;               // in 32 bits the blocks of the tiled kernel, for the heads that it takes
+#define FE_LAUNCH_SIMT(DPL, PER)                                                                                 \
+    fe::launch(paged_attention_simt_kernel<T, DPL, PER>, blocks, warps * 32, smem, stream,                               \
         (const T*)q, q_stride, (T*)out, out_stride, (const T*)kc, (const T*)vc, block_table, bt_stride, cu_q,   \
         q_start, token_req, T_tokens, nq, nkv, d, ps, num_pages, scale, window, keep, sink, per_head, softcap, status)
-    if constexpr (sizeof(T) == 2) {                           // in 32 bits the tiled kernel takes these
-        if (d <= 32) FE_LAUNCH_SIMT(1);
-        else if (d <= 64) FE_LAUNCH_SIMT(2);
-        else if (d <= 128) FE_LAUNCH_SIMT(4);
-        if (d <= TILE_MAX_D) return fe_check_launch("paged_attention_simt");
-    }
-    if (d <= 256) FE_LAUNCH_SIMT(8);
-    else if (d <= 512) FE_LAUNCH_SIMT(16);
-    else FE_LAUNCH_SIMT(32);
+    static_assert(TILE_MAX_D == 128, "heads up to this size walk blocks of PER * 32 keys");
+    if (d <= 32) FE_LAUNCH_SIMT(1, PER);
+    else if (d <= 64) FE_LAUNCH_SIMT(2, PER);
+    else if (d <= 128) FE_LAUNCH_SIMT(4, PER);
+    else if (d <= 256) FE_LAUNCH_SIMT(8, 1);
+    else if (d <= 512) FE_LAUNCH_SIMT(16, 1);
+    else FE_LAUNCH_SIMT(32, 1);
 #undef FE_LAUNCH_SIMT
     return fe_check_launch("paged_attention_simt");
 }
 
+// ``context``: the longest context among the requests, 0 if it is not known (the block table's width then stands for it).
 extern "C" int fe_paged_attention_simt(const void* q, long long q_stride, void* out, long long out_stride,
                                        const void* kc, const void* vc, const int* block_table, int bt_stride,
-                                       const int* cu_q, const int* q_start, const int* token_req, int requests, int T_tokens,
+                                       const int* cu_q, const int* q_start, const int* token_req, int requests, int T_tokens, int context,
                                        int nq, int nkv, int d, int ps, int num_pages, float scale, int window, int keep,
                                        int sink, int dtype, int* status, const float* per_head, float softcap, cudaStream_t stream) {
     FE_REQUIRE(T_tokens >= 0 && nq > 0 && nkv > 0 && nq % nkv == 0, "paged_attention: bad head counts %d/%d", nq, nkv);
@@ -399,8 +450,10 @@ extern "C" int fe_paged_attention_simt(const void* q, long long q_stride, void* 
     FE_REQUIRE(q_stride % 8 == 0, "paged_attention: query row stride %lld must be a multiple of 8 elements", q_stride);
     if (T_tokens == 0) return 0;
     FE_REQUIRE(((size_t)kc & 15) == 0, "paged_attention: the cache's keys must be 16-byte aligned");
-    // the tiled kernel copies values 16 bytes at a time; the other one reads them one by one
-    if (dtype == FE_F32 && d <= TILE_MAX_D && ((size_t)vc & 15) == 0)
+    FE_REQUIRE(requests > 0 && context >= 0, "paged_attention: %d requests, longest context %d", requests, context);
+    // the tiled kernel copies values 16 bytes at a time as well
+    if (dtype == FE_F32 && d <= TILE_MAX_D && ((size_t)vc & 15) == 0 && nkv <= 65535 &&
+        !rows_pay(T_tokens, requests, nq, nkv, d, context > 0 ? context : (long long)bt_stride * ps, window, keep))
         return launch_tiled((const float*)q, q_stride, (float*)out, out_stride, (const float*)kc, (const float*)vc, block_table,
                             bt_stride, cu_q, q_start, requests, T_tokens, nq, nkv, d, ps, num_pages, scale, window, keep, sink,
                             per_head, softcap, status, stream);

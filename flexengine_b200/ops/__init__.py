@@ -555,13 +555,14 @@ def _score_map(sigmoid, head_bias, softcap, head_scales):
 
 def paged_attention_simt(q, q_stride, k_cache, v_cache, block_table, cu_q, q_start, token_request, T, nq, nkv, d,
                          page_size, scale, window, sink=False, sigmoid=False, head_bias=None, softcap=0.0,
-                         head_scales=None, keep=0):
+                         head_scales=None, keep=0, max_ctx_len=0):
+    """Attention on CUDA cores; ``max_ctx_len`` (0: not known) helps to choose between its kernels, whose results are the same."""
     out = torch.empty((T, nq * d), dtype=k_cache.dtype, device=k_cache.device)
     mapped, per_head, softcap = _score_map(sigmoid, head_bias, softcap, head_scales)
     mode = _attention_mode(sink, sigmoid, mapped)
     _run(_core(), "fe_paged_attention_simt", _ptr(q), _c_ll(q_stride), _ptr(out), _c_ll(nq * d), _ptr(k_cache),
          _ptr(v_cache), _ptr(block_table), _c_int(block_table.shape[1]), _ptr(cu_q), _ptr(q_start),
-         _ptr(token_request), _c_int(cu_q.numel() - 1), _c_int(T), _c_int(nq), _c_int(nkv), _c_int(d), _c_int(page_size),
+         _ptr(token_request), _c_int(cu_q.numel() - 1), _c_int(T), _c_int(max_ctx_len), _c_int(nq), _c_int(nkv), _c_int(d), _c_int(page_size),
          _c_int(k_cache.shape[0]), _c_float(scale), _c_int(window), _c_int(keep), _c_int(mode), _c_int(_code(k_cache.dtype)),
          _ptr(status_word(k_cache.device)), _ptr(per_head), _c_float(softcap), _stream())
     return out
@@ -799,7 +800,8 @@ def paged_attention(qkv, k_cache, v_cache, block_table, ctx, nq, nkv, d, page_si
     score = {"softcap": softcap, "head_scales": head_scales, "keep": keep_first}
     if qkv.dtype == torch.float32 or d > 256:          # the tensor-core kernels take head sizes up to 256
         return paged_attention_simt(qkv, qkv.stride(0), k_cache, v_cache, block_table, ctx.cu_q, ctx.q_start,
-                                    ctx.token_request, T, nq, nkv, d, page_size, scale, window, sink, sigmoid, head_bias, **score)
+                                    ctx.token_request, T, nq, nkv, d, page_size, scale, window, sink, sigmoid, head_bias,
+                                    max_ctx_len=ctx.max_ctx_len, **score)
     requests = ctx.cu_q.numel() - 1
     if ctx.max_q_len == 1 and nq // nkv <= 16:
         # a window or a chunk bounds the keys a token walks (plus the tile of 32 that its first key lies in)

@@ -1,15 +1,20 @@
-"""32-bit attention where the cache's values start on no 16-byte boundary: one by one they may be read from anywhere."""
+"""The two kernels of 32-bit attention give a row the same bits.  Values that start on no 16-byte boundary are taken by the one
+that reads them one by one, so that shifting the cache's values by one element runs a call through the other kernel."""
 import types
 
 import pytest
 import torch
 
+import kernel_refs
 from test_kernels_gpu import DEV, bar, gen, ops, rand      # noqa: F401  (gen is a fixture)
 
 pytestmark = pytest.mark.gpu
 
 PORTIONS = {"prompts": [(0, 33), (0, 200), (0, 1), (0, 64), (0, 65)], "decoded": [(s, 1) for s in (0, 15, 16, 31, 32, 63, 64, 127, 300)],
             "later portions": [(300, 40), (63, 2), (64, 129), (17, 15)]}
+SCORES = {"softmax": {}, "sink": {"sink": True}, "window": {"window": 70}, "narrow window": {"window": 5}, "window of a tile": {"window": 64},
+          "chunk": {"window": -50}, "kept": {"window": 40, "keep": 7}, "kept tile": {"window": 100, "keep": 65}, "sigmoid": {"sigmoid": True, "bias": True},
+          "squashed": {"softcap": 5.0, "scales": True}, "scaled": {"scales": True, "window": 33, "keep": 3}}
 
 
 def _case(nq, nkv, d, portions, gen, ps=16):
@@ -36,7 +41,7 @@ def _run(q, kc, vc, table, ctx, nq, nkv, d, kind, gen_state):
     return ops().paged_attention_simt(q, q.stride(0), kc, vc, table, ctx.cu_q, ctx.q_start, ctx.token_request, q.shape[0], nq, nkv, d, 16,
                                       d ** -0.5, kind.get("window", 0), sink=kind.get("sink", False), sigmoid=kind.get("sigmoid", False),
                                       head_bias=per_head if kind.get("bias") else None, softcap=kind.get("softcap", 0.0),
-                                      head_scales=per_head if kind.get("scales") else None, keep=kind.get("keep", 0))
+                                      head_scales=per_head if kind.get("scales") else None, keep=kind.get("keep", 0), max_ctx_len=ctx.max_ctx_len)
 
 
 def _shifted(values):
@@ -46,13 +51,30 @@ def _shifted(values):
     return other
 
 
-@pytest.mark.parametrize("nq,nkv,d", [(4, 4, 128), (12, 2, 128), (6, 1, 48), (4, 2, 16)])
+@pytest.mark.parametrize("nq,nkv,d", [(4, 4, 128), (12, 2, 128), (6, 1, 48), (7, 1, 80), (4, 2, 16), (2, 1, 96)])
 @pytest.mark.parametrize("portions", PORTIONS)
-def test_values_need_no_boundary(nq, nkv, d, portions, gen):
+@pytest.mark.parametrize("score", SCORES)
+def test_both_kernels_give_a_row_the_same_bits(nq, nkv, d, portions, score, gen):
     q, kc, vc, table, ctx = _case(nq, nkv, d, PORTIONS[portions], gen)
-    got = _run(q, kc, _shifted(vc), table, ctx, nq, nkv, d, {}, 3)
-    torch.testing.assert_close(got, _run(q, kc, vc, table, ctx, nq, nkv, d, {}, 3), **bar(torch.float32))
+    got = _run(q, kc, vc, table, ctx, nq, nkv, d, SCORES[score], 3)
+    assert torch.equal(_run(q, kc, _shifted(vc), table, ctx, nq, nkv, d, SCORES[score], 3), got)
     ops().check_status(DEV)
+
+
+@pytest.mark.parametrize("requests,keys", [(48, 64), (128, 17), (128, 130), (3, 16)])
+def test_many_short_requests(requests, keys, gen):
+    """Batches that the kernel of one warp a row takes, against the plain reference and a request by itself (which shares its keys'
+    tiles where it sees more than a few)."""
+    nq = nkv = 16
+    q, kc, vc, table, ctx = _case(nq, nkv, 128, [(keys - 1, 1)] * requests, gen)
+    got = _run(q, kc, vc, table, ctx, nq, nkv, 128, {}, 3)
+    want = kernel_refs.paged_attention(q, kc, vc, table, ctx, nq, nkv, 128, 16, 128 ** -0.5, 0)
+    torch.testing.assert_close(got, want, **bar(torch.float32))
+    for r in (0, requests - 1):
+        one = types.SimpleNamespace(cu_q=torch.tensor([0, 1], dtype=torch.int32, device=DEV), q_start=ctx.q_start[r:r + 1].contiguous(),
+                                    token_request=torch.zeros(1, dtype=torch.int32, device=DEV), max_ctx_len=2000)
+        alone = _run(q[r:r + 1].contiguous(), kc, vc, table[r:r + 1].contiguous(), one, nq, nkv, 128, {}, 3)
+        assert torch.equal(alone[0], got[r]), r
 
 
 def test_values_of_larger_heads_need_no_boundary_either(gen):
