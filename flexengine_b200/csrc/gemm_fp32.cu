@@ -237,7 +237,7 @@ gemm_fp32_ring_kernel(const float* __restrict__ A, const float* __restrict__ W, 
     }
 }
 
-// ---- few columns (a router, a low-rank projection) for any number of rows --------------------------------------------------
+// ---- few columns (a router, a low-rank projection) for any number of rows, and few rows where the rings do not pay -------------
 // A block of 128 threads owns 8 rows x 16 columns, one output a thread, and walks K in chunks of 64 that it stages in
 // shared memory: the tiles above would be few blocks with long loops.
 constexpr int SR = 8, SC = 16, SK = 64;
@@ -299,6 +299,60 @@ gemm_fp32_narrow_kernel(const float* __restrict__ A, const float* __restrict__ W
     if (m0 + m < M && n0 + n < N) C[(size_t)(m0 + m) * N + n0 + n] = acc + (bias ? bias[n0 + n] : 0.f);
 }
 
+// ---- rows that start on no 16-byte boundary ------------------------------------------------------------------------------
+// A block of 256 threads owns 64 x 64 of C, a thread 4 x 4 of it; every value of a step of 16 is a load of its own, which is all
+// that such rows allow, and the many blocks an SM hide them better than the larger tiles' few or a ring of 4-byte copies.
+constexpr int UM = 64, UN = 64, UK = 16, UT = 4;
+
+__global__ void __launch_bounds__(256)
+gemm_fp32_unaligned_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
+                           float* __restrict__ C, int M, int N, int K) {
+    fe::griddep_wait();
+    fe::griddep_launch_dependents();
+    __shared__ float As[UK][UM + 4];
+    __shared__ float Ws[UK][UN + 4];
+    const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
+    const int m0 = blockIdx.y * UM, n0 = blockIdx.x * UN;
+    float acc[UT][UT];
+#pragma unroll
+    for (int i = 0; i < UT; ++i)
+#pragma unroll
+        for (int j = 0; j < UT; ++j) acc[i][j] = 0.f;
+    for (int k0 = 0; k0 < K; k0 += UK) {
+#pragma unroll
+        for (int i = 0; i < UM * UK / 256; ++i) {
+            const int idx = tid + i * 256, row = idx / UK, col = idx % UK;
+            const int gm = m0 + row, gn = n0 + row, gk = k0 + col;
+            As[col][row] = (gm < M && gk < K) ? A[(size_t)gm * K + gk] : 0.f;
+            Ws[col][row] = (gn < N && gk < K) ? W[(size_t)gn * K + gk] : 0.f;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < UK; ++k) {
+            float a[UT], w[UT];
+#pragma unroll
+            for (int i = 0; i < UT; ++i) a[i] = As[k][ty * UT + i];
+#pragma unroll
+            for (int j = 0; j < UT; ++j) w[j] = Ws[k][tx * UT + j];
+#pragma unroll
+            for (int i = 0; i < UT; ++i)
+#pragma unroll
+                for (int j = 0; j < UT; ++j) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < UT; ++i) {
+        const int gm = m0 + ty * UT + i;
+        if (gm >= M) continue;
+#pragma unroll
+        for (int j = 0; j < UT; ++j) {
+            const int gn = n0 + tx * UT + j;
+            if (gn < N) C[(size_t)gm * N + gn] = acc[i][j] + (bias ? bias[gn] : 0.f);
+        }
+    }
+}
+
 template <int BM, int BN, int TM, int TN, int STAGES, int CHUNK, bool VEC>
 int launch_ring(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, cudaStream_t stream) {
     constexpr size_t smem = (size_t)STAGES * (BM + BN) * (CHUNK + 4) * sizeof(float);
@@ -310,24 +364,54 @@ int launch_ring(const float* A, const float* W, const float* bias, float* C, int
     return fe_check_launch("gemm_fp32 (ring)");
 }
 
+int launch_narrow(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, cudaStream_t stream) {
+    const dim3 grid((N + SC - 1) / SC, (M + SR - 1) / SR);
+    FE_REQUIRE(grid.y <= 65535, "gemm_fp32: too many rows (%d)", M);
+    fe::launch(gemm_fp32_narrow_kernel, grid, 128, 0, stream, A, W, bias, C, M, N, K);
+    return fe_check_launch("gemm_fp32 (narrow)");
+}
+
+// Up to 16 rows: whether blocks of 8 rows and 16 columns are done before the rings' (the same bits either way).  The lines lie
+// where the rings' blocks go into another round over the SMs and these do not, or where a copy takes more than it brings:
+//   rows of 16 bytes: K of one chunk from three rows on (5 rows x 4,864 x 64: 3.0 us, ring 3.7); 5 to 8 rows a little over a
+//     round of the ring's 32 columns (x 4,864 x 2,048: 28.3, ring 32.3; x 8,000: 36.3 against 32.7); 9 to 16 rows with these
+//     blocks on different SMs (x 1,152 x 2,048: 15.9 against 18.8; x 1,536: 22.9 against 18.8), or the ring's 16 columns, one
+//     block an SM, in their second round (x 3,072: 28.9 against 34.2; x 4,864: 44.8 against 33.0)
+//   other rows, whose ring takes a copy for every value: nearly always (16 rows x 515 x 515: 5.9 us, ring 13.2; 8 x 40,000 x 131:
+//     16.0 against 26.2), but for four rows in the middle (x 10,000 x 515: 14.3 against 11.1) and for 9 to 16 rows of many
+//     columns, which these blocks fetch twice (x 10,000 x 1,539: 61.8 against 43.8; from twice as many on with a short K)
+template <bool VEC>
+bool narrow_pays(int M, int N, int K) {
+    const int sms = fe_sm_count();
+    if (VEC) {
+        if (K <= SK) return M > 2 && N <= (M <= 8 ? 128 : 64) * sms;
+        if (M <= 8) return M > 4 && N > 32 * sms && N <= 44 * sms;
+        return N <= 8 * sms || (N > 16 * sms && N <= 32 * sms);
+    }
+    if (M <= 4) return N <= 44 * sms || N > 256 * sms;
+    return M <= 8 || N <= (K <= 256 ? 64 : 32) * sms;
+}
+
 template <bool VEC>
 int few_rows(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, cudaStream_t stream) {
+    if (narrow_pays<VEC>(M, N, K)) return launch_narrow(A, W, bias, C, M, N, K, stream);
     // 16 columns a block while 32 would leave SMs without one; a deeper ring there (fewer blocks an SM).  A vocabulary's worth of
     // columns fills the device with blocks of 128 columns, whose threads use each value of W for four rows or more.  As few
     // threads a block as the rows allow: what a block reads from shared memory is what its threads' outputs do not share.
     const int sms = fe_sm_count();
-    if (N <= 32 * sms) {
-        if (M <= 4) return launch_ring<4, 16, 1, 1, 8, 128, VEC>(A, W, bias, C, M, N, K, stream);
-        if (M <= 8) return launch_ring<8, 16, 2, 1, 8, 128, VEC>(A, W, bias, C, M, N, K, stream);
-        return launch_ring<16, 16, 2, 2, 8, 128, VEC>(A, W, bias, C, M, N, K, stream);
+    if constexpr (VEC) {
+        if (N <= 32 * sms) {
+            if (M <= 4) return launch_ring<4, 16, 1, 1, 8, 128, VEC>(A, W, bias, C, M, N, K, stream);
+            if (M <= 8) return launch_ring<8, 16, 2, 1, 8, 128, VEC>(A, W, bias, C, M, N, K, stream);
+            return launch_ring<16, 16, 2, 2, 8, 128, VEC>(A, W, bias, C, M, N, K, stream);
+        }
+        if (N <= 256 * sms && M > 4 && M <= 8) return launch_ring<8, 32, 2, 2, 4, 64, VEC>(A, W, bias, C, M, N, K, stream);
+        if (N > 256 * sms) {
+            if (M <= 4) return launch_ring<4, 128, 4, 1, 3, 64, VEC>(A, W, bias, C, M, N, K, stream);
+            if (M <= 8) return launch_ring<8, 128, 8, 1, 3, 64, VEC>(A, W, bias, C, M, N, K, stream);
+        }
     }
-    if (N <= 256 * sms) {
-        if (M <= 4) return launch_ring<4, 32, 2, 1, 4, 64, VEC>(A, W, bias, C, M, N, K, stream);
-        if (M <= 8) return launch_ring<8, 32, 2, 2, 4, 64, VEC>(A, W, bias, C, M, N, K, stream);
-    } else {
-        if (M <= 4) return launch_ring<4, 128, 4, 1, 3, 64, VEC>(A, W, bias, C, M, N, K, stream);
-        if (M <= 8) return launch_ring<8, 128, 8, 1, 3, 64, VEC>(A, W, bias, C, M, N, K, stream);
-    }
+    if (M <= 4) return launch_ring<4, 32, 2, 1, 4, 64, VEC>(A, W, bias, C, M, N, K, stream);
     return launch_ring<16, 32, 4, 2, 4, 64, VEC>(A, W, bias, C, M, N, K, stream);
 }
 
@@ -339,29 +423,53 @@ int launch_tiles(const float* A, const float* W, const float* bias, float* C, in
     return fe_check_launch("gemm_fp32");
 }
 
-template <bool VEC>
-int many_rows(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, cudaStream_t stream) {
-    // The tile whose blocks are done first: rounds of blocks over the SMs times what a block takes, which is its area over
-    // how close to the FMA rate it comes (per mille, measured: alone on an SM, and where the SMs hold two or more).
-    struct Shape { int bm, bn, alone, several; };
-    static constexpr Shape SHAPES[6] = {{128, 128, 690, 720}, {64, 48, 460, 530}, {64, 32, 390, 485},
-                                        {32, 64, 380, 490}, {32, 32, 300, 430}, {32, 16, 170, 290}};
+int launch_unaligned(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, cudaStream_t stream) {
+    const dim3 grid((N + UN - 1) / UN, (M + UM - 1) / UM);
+    FE_REQUIRE(grid.y <= 65535, "gemm_fp32: too many rows (%d)", M);
+    fe::launch(gemm_fp32_unaligned_kernel, grid, 256, 0, stream, A, W, bias, C, M, N, K);
+    return fe_check_launch("gemm_fp32 (unaligned rows)");
+}
+
+// The tile whose blocks are done first: rounds of blocks over the SMs times what a block takes, which is its area over
+// how close to the FMA rate it comes (measured: alone on an SM, and where the SMs hold two or more; per mille for rows of 16 bytes).
+struct Shape { int bm, bn, alone, several; };
+inline int first_done(const Shape* shapes, int count, int M, int N) {
     const int sms = fe_sm_count();
     int best = 0;
     long long least = 0;
-    for (int i = 0; i < 6; ++i) {
-        const Shape& s = SHAPES[i];
+    for (int i = 0; i < count; ++i) {
+        const Shape& s = shapes[i];
         const long long tiles = (long long)((M + s.bm - 1) / s.bm) * ((N + s.bn - 1) / s.bn), rounds = (tiles + sms - 1) / sms;
         const long long cost = rounds * 1000LL * s.bm * s.bn / (rounds > 1 ? s.several : s.alone);
         if (i == 0 || cost < least) best = i, least = cost;
     }
-    switch (best) {
-        case 0: return launch_tiles<VEC>(A, W, bias, C, M, N, K, stream);
-        case 1: return launch_ring<64, 48, 4, 6, 3, 64, VEC>(A, W, bias, C, M, N, K, stream);
-        case 2: return launch_ring<64, 32, 4, 4, 4, 64, VEC>(A, W, bias, C, M, N, K, stream);
-        case 3: return launch_ring<32, 64, 4, 4, 3, 64, VEC>(A, W, bias, C, M, N, K, stream);
-        case 4: return launch_ring<32, 32, 4, 2, 4, 64, VEC>(A, W, bias, C, M, N, K, stream);
-        default: return launch_ring<32, 16, 4, 1, 4, 64, VEC>(A, W, bias, C, M, N, K, stream);
+    return best;
+}
+
+int many_rows(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, cudaStream_t stream) {
+    static constexpr Shape SHAPES[6] = {{128, 128, 690, 720}, {64, 48, 460, 530}, {64, 32, 390, 485},
+                                        {32, 64, 380, 490}, {32, 32, 300, 430}, {32, 16, 170, 290}};
+    switch (first_done(SHAPES, 6, M, N)) {
+        case 0: return launch_tiles<true>(A, W, bias, C, M, N, K, stream);
+        case 1: return launch_ring<64, 48, 4, 6, 3, 64, true>(A, W, bias, C, M, N, K, stream);
+        case 2: return launch_ring<64, 32, 4, 4, 4, 64, true>(A, W, bias, C, M, N, K, stream);
+        case 3: return launch_ring<32, 64, 4, 4, 3, 64, true>(A, W, bias, C, M, N, K, stream);
+        case 4: return launch_ring<32, 32, 4, 2, 4, 64, true>(A, W, bias, C, M, N, K, stream);
+        default: return launch_ring<32, 16, 4, 1, 4, 64, true>(A, W, bias, C, M, N, K, stream);
+    }
+}
+
+// Rows that start on no 16-byte boundary: the tiles' order is another, since a ring's copies are of four bytes (relative rates
+// over 132 sizes with K of 131 to 1,539: within 2 % of the best of them on average, nowhere behind the 64 x 64 tiles.  33 rows x
+// 40,000 x 131: 42 us, by the rates of aligned rows 49; 129 rows: 102, 134; 300 x 3,072 x 515: 64, 69).
+int many_unaligned_rows(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, cudaStream_t stream) {
+    static constexpr Shape SHAPES[5] = {{128, 128, 130, 167}, {64, 48, 42, 66}, {32, 32, 43, 49}, {32, 16, 26, 45}, {UM, UN, 66, 82}};
+    switch (first_done(SHAPES, 5, M, N)) {
+        case 0: return launch_tiles<false>(A, W, bias, C, M, N, K, stream);
+        case 1: return launch_ring<64, 48, 4, 6, 3, 64, false>(A, W, bias, C, M, N, K, stream);
+        case 2: return launch_ring<32, 32, 4, 2, 4, 64, false>(A, W, bias, C, M, N, K, stream);
+        case 3: return launch_ring<32, 16, 4, 1, 4, 64, false>(A, W, bias, C, M, N, K, stream);
+        default: return launch_unaligned(A, W, bias, C, M, N, K, stream);
     }
 }
 
@@ -374,11 +482,6 @@ extern "C" int fe_gemm_fp32(const float* A, const float* W, const float* bias, f
     const bool vec = (K & 3) == 0 && (((size_t)A | (size_t)W | (size_t)C) & 15) == 0;
     if (M <= 16)
         return vec ? few_rows<true>(A, W, bias, C, M, N, K, stream) : few_rows<false>(A, W, bias, C, M, N, K, stream);
-    if (N <= 128) {
-        const dim3 few((N + SC - 1) / SC, (M + SR - 1) / SR);
-        FE_REQUIRE(few.y <= 65535, "gemm_fp32: too many rows (%d)", M);
-        fe::launch(gemm_fp32_narrow_kernel, few, 128, 0, stream, A, W, bias, C, M, N, K);
-        return fe_check_launch("gemm_fp32 (few columns)");
-    }
-    return vec ? many_rows<true>(A, W, bias, C, M, N, K, stream) : many_rows<false>(A, W, bias, C, M, N, K, stream);
+    if (N <= 128) return launch_narrow(A, W, bias, C, M, N, K, stream);
+    return vec ? many_rows(A, W, bias, C, M, N, K, stream) : many_unaligned_rows(A, W, bias, C, M, N, K, stream);
 }

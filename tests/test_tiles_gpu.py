@@ -102,3 +102,18 @@ def test_sample_short_list_and_its_limits(V):
             target = kernel_refs.uniform_from(int(seed[r]), 5) * float(cum[-1])
             slack = 1e-5 * float(cum[-1])          # float32 sums of up to 1,025 masses: well below 1,025 * 2^-24
             assert (float(cum[token - 1]) if token else 0.0) - slack <= target <= float(cum[token]) + slack, (k, r)
+
+
+@pytest.mark.parametrize("K", [64, 68, 67, 259])
+def test_gemm_fp32_at_the_lines_of_its_rules(K, gen):
+    """Widths on both sides of every line of the choice between the kernels for up to 16 rows: a row is the same bit for bit in every
+    batch, rows that start on no 16-byte boundary included."""
+    sms = ops().sm_count()
+    for line in (8, 16, 32, 44, 64, 128, 256):
+        w = rand((line * sms + 1, K), torch.float32, gen)
+        x = rand((17, K), torch.float32, gen)
+        for N in (line * sms, line * sms + 1):
+            full = ops().linear(x, w[:N])
+            torch.testing.assert_close(full.double(), x.double() @ w[:N].double().T, atol=2e-6 * math.sqrt(K) * 4, rtol=1e-5)
+            for M in (1, 3, 5, 9, 16):
+                assert torch.equal(ops().linear(x[:M].contiguous(), w[:N]), full[:M]), (N, M)
