@@ -20,7 +20,7 @@
 // that finds the maximum also leaves every thread's own maximum; the k-th largest of a block's 1,024 is a lower bound of the
 // row's k-th largest logit (each is a logit of its own), so one more walk collects the few logits that reach the bound, and
 // threshold, ties and the groups of 256 that hold any mass come from that short list.  A list that does not fit (many
-// equal logits, or large ones all in one thread's share) and k beyond the threads' number take the radix select over the row.
+// equal logits, or large ones all in one thread's share) and a k too large for one take the radix select over the row.
 #include <math_constants.h>
 
 #define FE_PDL_CLASS 8      // FE_PDL_SAMPLING
@@ -139,7 +139,11 @@ sample_kernel(const float* __restrict__ logits, long long ld, int V, const float
     }
     int k = temp == 0.f ? 0 : top_k[row];
     const bool use_k = k > 0 && k < V;
-    const bool listed = use_k && k <= THREADS / 2;
+    // Only where the list is expected to fit: with the logits spread over the threads about -1024 ln(1 - k / 1024) of a block reach its
+    // bound, and C blocks share LIST places (that many at 226 of eight blocks and at 403 of four); a row of no more logits than
+    // places always fits.  Beyond, the two walks are for nothing: one row of 152,064 with k = 256 takes 42.7 us by the radix select
+    // alone, 48.4 after a list that overflowed; 16 rows with k = 400 36 us from their lists, 58 by the select.
+    const bool listed = use_k && k <= (V <= LIST || C <= 2 ? THREADS / 2 : C <= 4 ? 400 : 216);
     if (listed) {
         // the largest t (to 24 bits) that k or more of the threads' maxima reach, bit by bit
         const unsigned int own = ordered_key(best);

@@ -117,3 +117,19 @@ def test_gemm_fp32_at_the_lines_of_its_rules(K, gen):
             torch.testing.assert_close(full.double(), x.double() @ w[:N].double().T, atol=2e-6 * math.sqrt(K) * 4, rtol=1e-5)
             for M in (1, 3, 5, 9, 16):
                 assert torch.equal(ops().linear(x[:M].contiguous(), w[:N]), full[:M]), (N, M)
+
+
+@pytest.mark.parametrize("V", [2047, 2048, 2049, 32000])
+@pytest.mark.parametrize("k", [216, 217, 400, 401, 512, 513])
+def test_sample_on_both_sides_of_the_lists_rule(V, k):
+    """A top-k of which the list is tried with as many blocks a row and not with more: the tokens are the same with every number of blocks,
+    and one of the k largest."""
+    gen = torch.Generator(DEV).manual_seed(k)
+    logits = torch.randn((3, V), generator=gen, device=DEV)
+    temperature, top_k = torch.full((3,), 0.9, device=DEV), torch.full((3,), k, dtype=torch.int32, device=DEV)
+    seed, draw = torch.arange(3, dtype=torch.int64, device=DEV), torch.full((3,), 7, dtype=torch.int64, device=DEV)
+    got = ops().sample(logits, temperature, top_k, seed, draw, blocks=1)
+    for blocks in (2, 4, 8):
+        assert torch.equal(ops().sample(logits, temperature, top_k, seed, draw, blocks=blocks), got), blocks
+    kth = logits.topk(k).values[:, -1]
+    assert bool((logits.gather(1, got[:, None].long())[:, 0] >= kth).all())
