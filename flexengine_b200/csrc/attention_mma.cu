@@ -177,8 +177,7 @@ __device__ __forceinline__ void compute_tile(const bf16* ks, const bf16* vs, con
 #pragma unroll
             for (int e = 0; e < (UPPER ? 4 : 2); ++e) {
                 const int key = first_key + j * 8 + 2 * t + (e & 1);
-                // no short circuit: a branch a key costs more than the comparisons
-                const bool vis = e < 2 ? ((key <= pos0) & ((key >= lo0) | (key < keep))) : ((key <= pos1) & ((key >= lo1) | (key < keep)));
+                const bool vis = e < 2 ? (key <= pos0 && (key >= lo0 || key < keep)) : (key <= pos1 && (key >= lo1 || key < keep));
                 if (!vis) s[j][e] = -CUDART_INF_F;
             }
         }
