@@ -417,19 +417,26 @@ paged_prefill_tcgen05_kernel(const bf16* __restrict__ q, long long q_stride, bf1
     griddep_launch_dependents();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int G = nq / nkv;
-    // blockIdx.x = (item, key/value head, split of its keys); warp 0 finds the item's request and pair of row tiles
-    const int split = blockIdx.x % splits, kvh = (blockIdx.x / splits) % nkv;
-    if (warp == 0) {
-        int who, pair;
-        pick_item((int)(blockIdx.x / (splits * nkv)), cu_q, q_start, requests, G, who, pair);
-        if (lane == 0) { item_request = who; item_pair = pair; }
+    // blockIdx.x = (item, key/value head, split of its keys).  With one request an item is one of its pairs, the last ones first; with
+    // more, warp 0 finds the item's request and pair of row tiles.
+    const int split = blockIdx.x % splits, kvh = (blockIdx.x / splits) % nkv, item = blockIdx.x / (splits * nkv);
+    int r = 0, pair_at;
+    if (requests == 1) {
+        pair_at = ((cu_q[1] - cu_q[0]) * G + 2 * ROWS - 1) / (2 * ROWS) - 1 - item;
+        if (pair_at < 0) return;
+    } else {
+        if (warp == 0) {
+            int who, pair;
+            pick_item(item, cu_q, q_start, requests, G, who, pair);
+            if (lane == 0) { item_request = who; item_pair = pair; }
+        }
+        __syncthreads();
+        r = item_request, pair_at = item_pair;
+        if (r < 0) return;                                          // the grid is an upper bound of the items
     }
-    __syncthreads();
-    const int r = item_request;
-    if (r < 0) return;                                              // the grid is an upper bound of the items
     const int tok0 = cu_q[r], n_q = cu_q[r + 1] - tok0;
     const int rows = n_q * G;
-    const int m_pair = item_pair * 2 * ROWS;
+    const int m_pair = pair_at * 2 * ROWS;
     const bool two = m_pair + ROWS < rows;                          // else the second row tile is empty and left out
     const int start = q_start[r];
     // keys this block needs: from the window edge of its first query to its last query

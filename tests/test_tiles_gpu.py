@@ -133,3 +133,27 @@ def test_sample_on_both_sides_of_the_lists_rule(V, k):
         assert torch.equal(ops().sample(logits, temperature, top_k, seed, draw, blocks=blocks), got), blocks
     kth = logits.topk(k).values[:, -1]
     assert bool((logits.gather(1, got[:, None].long())[:, 0] >= kth).all())
+
+
+@pytest.mark.parametrize("nq,nkv,d", [(12, 2, 128), (16, 16, 64), (5, 1, 128)])
+@pytest.mark.parametrize("start,n", [(0, 1), (0, 255), (0, 256), (0, 700), (900, 64), (63, 257)])
+def test_prefill_attention_of_one_request(nq, nkv, d, start, n, gen):
+    """A step's only request finds its row tiles without a search: against the plain reference, with split keys and without, and bit for
+    bit what it is beside a request that has no tokens in the step."""
+    import types
+    ps = 16
+    pages = -(-(start + n) // ps)
+    kc, vc = (rand((pages, nkv, ps, d), torch.bfloat16, gen) for _ in range(2))
+    qkv = rand((n, nq * d), torch.bfloat16, gen)
+    table = torch.arange(pages, dtype=torch.int32, device=DEV)[None].repeat(2, 1).contiguous()
+    cu, starts = torch.tensor([0, n, n], dtype=torch.int32, device=DEV), torch.tensor([start, 0], dtype=torch.int32, device=DEV)
+    ctx = types.SimpleNamespace(cu_q=cu[:2].contiguous(), q_start=starts[:1].contiguous(), token_request=torch.zeros(n, dtype=torch.int32, device=DEV))
+    want = kernel_refs.paged_attention(qkv, kc, vc, table[:1], ctx, nq, nkv, d, ps, d ** -0.5, 0)
+    for splits in (1, 3):
+        def run(requests):
+            return ops().paged_prefill_tcgen05(qkv, qkv.stride(0), kc, vc, table[:requests].contiguous(), cu[:requests + 1].contiguous(),
+                                               starts[:requests].contiguous(), n, requests, n, nq, nkv, d, ps, d ** -0.5, 0, splits=splits)
+        got = run(1)
+        torch.testing.assert_close(got.float(), want.float(), **bar(torch.bfloat16))
+        assert torch.equal(run(2), got)
+    ops().check_status(DEV)
