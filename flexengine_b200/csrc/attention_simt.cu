@@ -396,10 +396,10 @@ int launch_tiled(const float* q, long long q_stride, float* out, long long out_s
 // Whether a call's rows are taken one warp each and not 32 a block (the same bits either way).  A block of the tiled kernel costs its
 // 8 us however few of its rows and keys are real, and one or two are resident on an SM; a warp a row costs by the key.  So: where no
 // row sees more than a few keys (40 prompts of 9, 12 heads of 128 in two groups: 12.7 us, tiled 26.9; one prompt of 9: 9.0, 15.2; a
-// window of 5 over 1,024 tokens: 36, 50); and where the blocks make several rounds with little in each (``seen`` keys times a block's
-// rows below what a block costs: 128 requests of 64 keys, 32 heads of 128: 76 us, tiled 237; 48 of 130: 110, 195; 128 of 256 with 8
-// heads of 96 over two: 201 against 159 is beyond it), if there are rows enough to hide a warp's walk (16 requests of 256 keys, 32
-// heads: 189 us, tiled 96).
+// window of 5 over 1,024 tokens: 29, 50; small heads a few more keys); and where the blocks make several rounds with little in each
+// (``seen`` keys times a block's rows below what a block costs: 128 requests of 64 keys, 32 heads of 128: 76 us, tiled 237; 48 of 130
+// keys: 110, 195; beyond the line 128 of 256 keys, 16 heads of 96 in eight groups: 201, tiled 159), if there are rows enough to hide
+// a warp's walk (16 requests of 256 keys, 32 heads of 128: 189 us, tiled 96).
 bool rows_pay(int T_tokens, int requests, int nq, int nkv, int d, long long context, int window, int keep) {
     const long long G = nq / nkv, portion = (T_tokens + requests - 1) / requests;
     const long long rows = portion * G, tiles = (rows + TILE_ROWS - 1) / TILE_ROWS, blocks = tiles * nkv * requests;
