@@ -9,12 +9,6 @@
 
 using namespace fe;
 
-// Whether a kernel between two products of a dense layer may begin while the product before it ends: with up to 8 rows that is one of
-// this package's streaming products, with a prompt's worth a long one of the library.  Between, the library's product is a few
-// rounds of blocks long, and blocks that take their places early slow it down (decode of 40 requests on the 1.5B shape: 7.34 ->
-// 7.52 ms for four steps; 24 on the 7B shape: 7.74 -> 7.75).
-static int overlap_class(int rows) { return rows <= 8 || rows > 256 ? FE_PDL_CLASS : 0; }
-
 // ---------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void embedding_kernel(const int* __restrict__ ids, const T* __restrict__ table, float* __restrict__ out,

@@ -286,11 +286,11 @@ static int launch_stream_rmsnorm(float* x, int S, int T_tokens, int H, const flo
         if (threads < 64) threads = 64;
     }
 #define FE_LAUNCH_STREAM_NORM_PLAIN(SMAX)                                                                                 \
-    fe::launch(stream_rmsnorm_kernel<T, SMAX>, n_out, threads, smem, stream, x, S, T_tokens, H, read, weight, eps,       \
+    fe::launch_as(overlap_class(n_out), stream_rmsnorm_kernel<T, SMAX>, n_out, threads, smem, stream, x, S, T_tokens, H, read, weight, eps,       \
                (const T*)y, (const T*)gate, gate_bias, mix, write, rows, (T*)out, shift_mu, kept, kept_stride, seats, n_seats, \
                (T*)shifted)
 #define FE_LAUNCH_STREAM_NORM_VEC(SMAX, ITERS)                                                                            \
-    fe::launch(stream_rmsnorm_vec_kernel<T, SMAX, ITERS>, n_out, threads, smem, stream, x, S, T_tokens, H, read, weight, \
+    fe::launch_as(overlap_class(n_out), stream_rmsnorm_vec_kernel<T, SMAX, ITERS>, n_out, threads, smem, stream, x, S, T_tokens, H, read, weight, \
                eps, (const T*)y, (const T*)gate, gate_bias, mix, write, rows, (T*)out, shift_mu, kept, kept_stride, seats,       \
                n_seats, (T*)shifted)
     if (staged) {
@@ -408,10 +408,10 @@ extern "C" int fe_token_shift(const void* h, const float* mu, float* kept, long 
         const long long total = (long long)T * (D >> 3), want = (total + 255) / 256;
         const int blocks = (int)(want < 65535LL * 4 ? want : 65535LL * 4);
         if (dtype == FE_F32)
-            fe::launch(token_shift_vec_kernel<float>, blocks, 256, 0, stream, (const float*)h, mu, kept, kept_stride, seats, cu_q, token_req,
+            fe::launch_as(overlap_class(T), token_shift_vec_kernel<float>, blocks, 256, 0, stream, (const float*)h, mu, kept, kept_stride, seats, cu_q, token_req,
                        (float*)out, T, D, n_seats);
         else
-            fe::launch(token_shift_vec_kernel<bf16>, blocks, 256, 0, stream, (const bf16*)h, mu, kept, kept_stride, seats, cu_q, token_req,
+            fe::launch_as(overlap_class(T), token_shift_vec_kernel<bf16>, blocks, 256, 0, stream, (const bf16*)h, mu, kept, kept_stride, seats, cu_q, token_req,
                        (bf16*)out, T, D, n_seats);
         return fe_check_launch("token_shift");
     }
@@ -419,10 +419,10 @@ extern "C" int fe_token_shift(const void* h, const float* mu, float* kept, long 
     const int stretches = T >= 512 ? 1 : (D + threads - 1) / threads;
     const dim3 grid(T, stretches < 65535 ? stretches : 65535);
     if (dtype == FE_F32)
-        fe::launch(token_shift_kernel<float>, grid, threads, 0, stream, (const float*)h, mu, kept, kept_stride, seats, cu_q, token_req,
+        fe::launch_as(overlap_class(T), token_shift_kernel<float>, grid, threads, 0, stream, (const float*)h, mu, kept, kept_stride, seats, cu_q, token_req,
                    (float*)out, D, n_seats);
     else if (dtype == FE_BF16)
-        fe::launch(token_shift_kernel<bf16>, grid, threads, 0, stream, (const bf16*)h, mu, kept, kept_stride, seats, cu_q, token_req,
+        fe::launch_as(overlap_class(T), token_shift_kernel<bf16>, grid, threads, 0, stream, (const bf16*)h, mu, kept, kept_stride, seats, cu_q, token_req,
                    (bf16*)out, D, n_seats);
     else
         FE_REQUIRE(false, "token_shift: unknown dtype %d", dtype);
@@ -709,7 +709,7 @@ static int launch_qkv_prepare(const void* proj, long long ld, const float* conv,
         head <= KV_ROUNDS * 256 && (((size_t)proj | (size_t)kc | (size_t)vc) & 15) == 0) {
         if (!slot_mapping) return 0;
         const long long items = (long long)T_tokens * 2 * kv_heads;
-        fe::launch(kv_cache_kernel<T>, (unsigned)((items + 7) / 8), 256, 0, stream, (const T*)proj, ld, heads * dim, slot_mapping, (T*)kc, (T*)vc,
+        fe::launch_as(overlap_class(T_tokens), kv_cache_kernel<T>, (unsigned)((items + 7) / 8), 256, 0, stream, (const T*)proj, ld, heads * dim, slot_mapping, (T*)kc, (T*)vc,
                    T_tokens, kv_heads, dim, vdim, head, ps, num_slots, eps, v_norm, status);
         return fe_check_launch("kv_cache");
     }
@@ -727,7 +727,7 @@ static int launch_qkv_prepare(const void* proj, long long ld, const float* conv,
                          (((size_t)proj | (size_t)kc | (size_t)vc | (size_t)q_out | (size_t)history | (size_t)conv) & 15) == 0;
     const int per = aligned ? dim / 32 : 0;
 #define FE_LAUNCH_QKV_PREPARE(PER)                                                                                                   \
-    fe::launch(qkv_conv_rope_norm_cache_kernel<T, PER>, T_tokens, warps * 32, smem, stream, (const T*)proj, ld, conv, history,     \
+    fe::launch_as(overlap_class(T_tokens), qkv_conv_rope_norm_cache_kernel<T, PER>, T_tokens, warps * 32, smem, stream, (const T*)proj, ld, conv, history,     \
                history_stride, taps, seats, cu_q, token_req, positions, inv_freq, rot, qk_norm, eps, slot_mapping, (T*)kc, (T*)vc,  \
                (T*)q_out, T_tokens, heads, kv_heads, dim, vdim, head, ps, num_slots, n_seats, status, q_weight, k_weight, temp_coef,     \
                temp_every, v_norm)
@@ -1055,7 +1055,7 @@ extern "C" int fe_qkv_norm_rope_cache(const void* proj, long long ld, const floa
             cudaError_t err = cudaFuncSetAttribute(qkv_norm_rope_cache_four_kernel<TYPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)four_smem); \
             FE_REQUIRE(err == cudaSuccess, "qkv_norm_rope_cache: %s", cudaGetErrorString(err));                                          \
         }                                                                                                                               \
-        fe::launch(qkv_norm_rope_cache_four_kernel<TYPE>, T, 256, four_smem, stream, (const TYPE*)proj, ld, q_weight, k_weight, eps,      \
+        fe::launch_as(overlap_class(T), qkv_norm_rope_cache_four_kernel<TYPE>, T, 256, four_smem, stream, (const TYPE*)proj, ld, q_weight, k_weight, eps,      \
                    positions, inv_freq, rot, bias, gain, slot_mapping, (TYPE*)kc, (TYPE*)vc, (TYPE*)q_out, heads, kv_heads, dim, vdim,    \
                    head, ps, num_slots, status);                                                                                        \
     } while (0)
@@ -1071,7 +1071,7 @@ extern "C" int fe_qkv_norm_rope_cache(const void* proj, long long ld, const floa
             cudaError_t err = cudaFuncSetAttribute(qkv_norm_rope_cache_kernel<TYPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
             FE_REQUIRE(err == cudaSuccess, "qkv_norm_rope_cache: %s", cudaGetErrorString(err));                                          \
         }                                                                                                                               \
-        fe::launch(qkv_norm_rope_cache_kernel<TYPE>, T, threads, smem, stream, (const TYPE*)proj, ld, q_weight, k_weight, eps, positions, \
+        fe::launch_as(overlap_class(T), qkv_norm_rope_cache_kernel<TYPE>, T, threads, smem, stream, (const TYPE*)proj, ld, q_weight, k_weight, eps, positions, \
                    inv_freq, rot, interleaved, v_inv_freq, bias, gain, slot_mapping, (TYPE*)kc, (TYPE*)vc, (TYPE*)q_out, heads, kv_heads, dim, vdim,    \
                    head, ps, num_slots, status);                                                                                        \
     } while (0)
@@ -1155,20 +1155,20 @@ extern "C" int fe_head_gate(const void* mixed, const void* gates, long long ld, 
         const long long groups = total / 8, want = (groups + 255) / 256;
         const int blocks = (int)(want < 65535LL * 4 ? want : 65535LL * 4);
         if (dtype == FE_F32)
-            fe::launch(head_gate_vec_kernel<float>, blocks, 256, 0, stream, (const float*)mixed, (const float*)gates, ld, (float*)out, ldo,
+            fe::launch_as(overlap_class(T), head_gate_vec_kernel<float>, blocks, 256, 0, stream, (const float*)mixed, (const float*)gates, ld, (float*)out, ldo,
                        groups, heads, head, vdim, per_element, scale);
         else
-            fe::launch(head_gate_vec_kernel<bf16>, blocks, 256, 0, stream, (const bf16*)mixed, (const bf16*)gates, ld, (bf16*)out, ldo,
+            fe::launch_as(overlap_class(T), head_gate_vec_kernel<bf16>, blocks, 256, 0, stream, (const bf16*)mixed, (const bf16*)gates, ld, (bf16*)out, ldo,
                        groups, heads, head, vdim, per_element, scale);
         return fe_check_launch("head_gate");
     }
     const long long want = (total + 255) / 256;
     const int blocks = (int)(want < 65535LL * 4 ? want : 65535LL * 4);
     if (dtype == FE_F32)
-        fe::launch(head_gate_kernel<float>, blocks, 256, 0, stream, (const float*)mixed, (const float*)gates, ld, (float*)out, ldo, total,
+        fe::launch_as(overlap_class(T), head_gate_kernel<float>, blocks, 256, 0, stream, (const float*)mixed, (const float*)gates, ld, (float*)out, ldo, total,
                    heads, head, vdim, per_element, scale);
     else
-        fe::launch(head_gate_kernel<bf16>, blocks, 256, 0, stream, (const bf16*)mixed, (const bf16*)gates, ld, (bf16*)out, ldo, total,
+        fe::launch_as(overlap_class(T), head_gate_kernel<bf16>, blocks, 256, 0, stream, (const bf16*)mixed, (const bf16*)gates, ld, (bf16*)out, ldo, total,
                    heads, head, vdim, per_element, scale);
     return fe_check_launch("head_gate");
 }
@@ -1374,9 +1374,9 @@ extern "C" int fe_gated_activation(const void* gate_up, void* out, int T, int I,
     const long long want = (total + 255) / 256;
     const int blocks = (int)(want < 65535LL * 8 ? want : 65535LL * 8);
     if (dtype == FE_F32)
-        fe::launch(gated_activation_kernel<float>, blocks, 256, 0, stream, (const float*)gate_up, (float*)out, total, I, act);
+        fe::launch_as(overlap_class(T), gated_activation_kernel<float>, blocks, 256, 0, stream, (const float*)gate_up, (float*)out, total, I, act);
     else if (dtype == FE_BF16)
-        fe::launch(gated_activation_kernel<bf16>, blocks, 256, 0, stream, (const bf16*)gate_up, (bf16*)out, total, I, act);
+        fe::launch_as(overlap_class(T), gated_activation_kernel<bf16>, blocks, 256, 0, stream, (const bf16*)gate_up, (bf16*)out, total, I, act);
     else
         FE_REQUIRE(false, "gated_activation: unknown dtype %d", dtype);
     return fe_check_launch("gated_activation");

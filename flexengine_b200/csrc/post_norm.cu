@@ -130,10 +130,10 @@ static int launch_post_norm(float* residual, const void* delta, const float* bia
         cudaFuncSetAttribute(post_norm_kernel<T, TD, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     }
     if (vec)
-        fe::launch(post_norm_kernel<T, TD, 4>, n_out, threads, smem, stream, residual, (const TD*)delta, bias, post_w, post_eps, w, eps,
+        fe::launch_as(overlap_class(n_out), post_norm_kernel<T, TD, 4>, n_out, threads, smem, stream, residual, (const TD*)delta, bias, post_w, post_eps, w, eps,
                    (T*)out, ldo, rows, H, extra, extra_cols, T_tokens);
     else
-        fe::launch(post_norm_kernel<T, TD, 1>, n_out, threads, smem, stream, residual, (const TD*)delta, bias, post_w, post_eps, w, eps,
+        fe::launch_as(overlap_class(n_out), post_norm_kernel<T, TD, 1>, n_out, threads, smem, stream, residual, (const TD*)delta, bias, post_w, post_eps, w, eps,
                    (T*)out, ldo, rows, H, extra, extra_cols, T_tokens);
     return fe_check_launch("post_norm");
 }
@@ -203,11 +203,11 @@ extern "C" int fe_gated_activation_bias(const void* gu, int in_dtype, const floa
     const long long want = (total + 255) / 256;
     const unsigned blocks = (unsigned)(want < 65535LL * 8 ? want : 65535LL * 8);
     if (in_dtype == FE_F32 && dtype == FE_F32)
-        fe::launch(gated_activation_bias_kernel<float, float>, blocks, 256, 0, stream, (const float*)gu, bias, (float*)out, total, I, act);
+        fe::launch_as(overlap_class(T), gated_activation_bias_kernel<float, float>, blocks, 256, 0, stream, (const float*)gu, bias, (float*)out, total, I, act);
     else if (in_dtype == FE_F32 && dtype == FE_BF16)
-        fe::launch(gated_activation_bias_kernel<float, bf16>, blocks, 256, 0, stream, (const float*)gu, bias, (bf16*)out, total, I, act);
+        fe::launch_as(overlap_class(T), gated_activation_bias_kernel<float, bf16>, blocks, 256, 0, stream, (const float*)gu, bias, (bf16*)out, total, I, act);
     else if (in_dtype == FE_BF16 && dtype == FE_BF16)
-        fe::launch(gated_activation_bias_kernel<bf16, bf16>, blocks, 256, 0, stream, (const bf16*)gu, bias, (bf16*)out, total, I, act);
+        fe::launch_as(overlap_class(T), gated_activation_bias_kernel<bf16, bf16>, blocks, 256, 0, stream, (const bf16*)gu, bias, (bf16*)out, total, I, act);
     else
         FE_REQUIRE(false, "gated_activation_bias: unknown dtypes %d -> %d", in_dtype, dtype);
     return fe_check_launch("gated_activation_bias");
