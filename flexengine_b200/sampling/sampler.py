@@ -18,6 +18,12 @@ def validate_sampling(temperature: float, top_k: int) -> None:
         raise ValueError("temperature and top_k must be >= 0")
 
 
+def _none_negative(values, n: int) -> bool:
+    """Whether a list or tuple of ``n`` certainly holds nothing below zero, in one pass (a first NaN is not certain: it hides what
+    follows)."""
+    return type(values) in (list, tuple) and len(values) == n and (n == 0 or bool(min(values) >= 0))
+
+
 def _fill(words, values, dtype) -> None:
     """``values`` into the numpy array ``words``: a list or tuple that numpy takes for numbers of the kind in one conversion;
     anything else as a tensor of ``dtype``, which takes, broadcasts and refuses what a tensor does."""
@@ -48,8 +54,8 @@ class Sampler:
         if logits.dim() != 2 or logits.shape[0] != len(temperatures):
             raise ValueError("Expected logits [requests, vocab]")
         n = len(temperatures)
-        for t, k in zip(temperatures, top_ks):
-            if t < 0 or k < 0:                           # a call a row would cost more than the comparisons
+        if not (_none_negative(temperatures, n) and _none_negative(top_ks, n)):
+            for t, k in zip(temperatures, top_ks):
                 validate_sampling(t, k)
         dev = logits.device
         if all(t == 0.0 for t in temperatures):

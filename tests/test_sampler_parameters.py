@@ -59,6 +59,6 @@ def test_numbers_of_any_kind_arrive(at, values, want):
 
 
 def test_greedy_rows_take_whatever_stands_beside_them():
-    for top_ks in ([2 ** 70, 1], [0], [1, 2, 3], (5, 5)):
+    for top_ks in ([2 ** 70, 1], [0], [1, 2, 3], (5, 5), [1, 2, None], iter([1, 2])):
         assert taken([0.0, 0], top_ks, [1], [3]) == [[0.0, 0.0], [0, 0], [0, 0], [0, 0]]
     assert Sampler(Seen()).sample_on_device(torch.zeros(0, 8), [], [], [], []) == [[], [], [], []]
