@@ -858,7 +858,9 @@ extern "C" int fe_paged_decode_cluster(const void* q, long long q_stride, void* 
     attr[0].val.clusterDim.z = 1;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     // A class of its own: with blocks on every SM the successor of a step that may begin early takes the place of late clusters (7B
-    // shape, 8 requests: 25.2 -> 26.5 ms for 16 steps).  A step of fewer blocks than SMs leaves room for both.
+    // shape, 8 requests: 25.2 -> 26.5 ms for 16 steps).  A step of fewer blocks than SMs leaves room for both.  It does not ask for the
+    // split of an SM's memory that fe::launch asks for: the kernel is the one of large steps too, whose blocks then lack the shared
+    // memory to be resident at once (26.4 -> 33.5 ms), and one request gains nothing by it (36.9, 36.8 ms for 32 steps of the 1.5B shape).
     const bool small = (long long)splits * nkv * requests <= fe_sm_count();
     attr[1].val.programmaticStreamSerializationAllowed = (fe_pdl_enabled() & 16) != 0 || (small && (fe_pdl_enabled() & FE_PDL_STREAMING_GEMM) != 0);
     cfg.attrs = attr;

@@ -143,10 +143,11 @@ template <int TILE> __host__ __device__ __forceinline__ int listed_tile(int i, i
 // (called before, every later kernel of a graph piles onto the SMs and starves the running one).
 // Without the launch attribute both are no-ops; fe_set_pdl names the classes of kernels that get it.  What it is worth: a
 // kernel boundary costs about 2 us of idle memory, 5 of them a layer in a decode step.  Weight-streaming products and
-// elementwise kernels with it against without (B200): 32 steps of one request on the 1.5B shape 40.3 -> 34.1 ms, 16 steps of 8
-// requests on the 7B shape 26.3 -> 25.2 ms, the hybrid designs 5 to 10 %; all kernels so launched share one split of an
-// SM's memory (fe_share_carveout says why).  Decode attention, the scans and the rest gain nothing or lose (7B: 25.2 ->
-// 26.5 ms with the attention clusters, whose successor then takes the place of late clusters).
+// elementwise kernels with it against without (B200): 32 steps of one request on the 1.5B shape 40.4 -> 34.1 ms, 16 steps of 8
+// requests on the 7B shape 26.8 -> 25.9 ms, the hybrid designs 7 to 14 %; all kernels launched through fe::launch share one split of
+// an SM's memory (fe_share_carveout says why; the cluster form of decode attention, which begins early in small steps, keeps
+// its own).  Decode attention, the scans and the rest gain nothing or lose (7B: 25.2 -> 26.5 ms on one box with the attention
+// clusters, whose successor then takes the place of late clusters).
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
