@@ -801,7 +801,7 @@ def paged_attention(qkv, k_cache, v_cache, block_table, ctx, nq, nkv, d, page_si
     if qkv.dtype == torch.float32 or d > 256:          # the tensor-core kernels take head sizes up to 256
         return paged_attention_simt(qkv, qkv.stride(0), k_cache, v_cache, block_table, ctx.cu_q, ctx.q_start,
                                     ctx.token_request, T, nq, nkv, d, page_size, scale, window, sink, sigmoid, head_bias,
-                                    max_ctx_len=ctx.max_ctx_len, **score)
+                                    max_ctx_len=getattr(ctx, "max_ctx_len", 0), **score)
     requests = ctx.cu_q.numel() - 1
     if ctx.max_q_len == 1 and nq // nkv <= 16:
         # a window or a chunk bounds the keys a token walks (plus the tile of 32 that its first key lies in)
