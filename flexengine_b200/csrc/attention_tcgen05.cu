@@ -208,8 +208,10 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
     asm("max.f32 %0, %1, %2, %3;\n" : "=f"(m) : "f"(a), "f"(b), "f"(c));
     return m;
 }
+struct Edges { int hi, lo, keep; };           // of a row, relative to the tile
 template <bool MASKED>
-__device__ __forceinline__ float row_max(const unsigned* r, const Seen& seen) {
+__device__ __forceinline__ float row_max(const unsigned* r, const Edges& edges) {
+    const Seen seen = MASKED ? seen_keys(edges.hi, edges.lo, edges.keep) : Seen{};
     float m0 = -CUDART_INF_F, m1 = -CUDART_INF_F, m2 = -CUDART_INF_F, m3 = -CUDART_INF_F;
 #pragma unroll
     for (int i = 0; i < KEYS; i += 8) {
@@ -226,7 +228,8 @@ __device__ __forceinline__ float row_max(const unsigned* r, const Seen& seen) {
 // P = 2^(s scale - ref) as bfloat16 pairs over the scores' own columns (32 of the 64); returns the row's sum.
 // The multiply-adds and the sums run two floats per instruction.
 template <bool MASKED>
-__device__ __forceinline__ float row_exp(const unsigned* r, unsigned p_addr, const Seen& seen, float scale_log2, float ref) {
+__device__ __forceinline__ float row_exp(const unsigned* r, unsigned p_addr, const Edges& edges, float scale_log2, float ref) {
+    const Seen seen = MASKED ? seen_keys(edges.hi, edges.lo, edges.keep) : Seen{};
     float2 sum = make_float2(0.f, 0.f);
     const float2 scale2 = make_float2(scale_log2, scale_log2), ref2 = make_float2(-ref, -ref);
 #pragma unroll
@@ -253,7 +256,8 @@ __device__ __forceinline__ float row_exp(const unsigned* r, unsigned p_addr, con
 // Sigmoid weights instead of a softmax: P = 1 / (1 + 2^-(s scale + bias)) as bfloat16 pairs over the scores' own columns;
 // nothing is summed, a masked key weighs 0.
 template <bool MASKED>
-__device__ __forceinline__ void row_sigmoid(const unsigned* r, unsigned p_addr, const Seen& seen, float scale_log2, float bias) {
+__device__ __forceinline__ void row_sigmoid(const unsigned* r, unsigned p_addr, const Edges& edges, float scale_log2, float bias) {
+    const Seen seen = MASKED ? seen_keys(edges.hi, edges.lo, edges.keep) : Seen{};
     const float2 scale2 = make_float2(-scale_log2, -scale_log2), bias2 = make_float2(-bias, -bias);
 #pragma unroll
     for (int c = 0; c < KEYS; c += 32) {
@@ -405,6 +409,7 @@ paged_prefill_tcgen05_kernel(const bf16* __restrict__ q, long long q_stride, bf1
     __shared__ unsigned tmem_holder;
     __shared__ volatile int give_up;
     __shared__ int item_request, item_pair;
+    __shared__ long long row_place[2 * ROWS];        // where each row's result goes, -1 for padding rows
     constexpr int DB = D / 64;                       // 64-element blocks per row
     constexpr int Q_BYTES = DB * Q_BLOCK;            // one row tile of Q
     constexpr int KV_BYTES = DB * KV_BLOCK;          // one key tile of K or of V
@@ -480,9 +485,12 @@ paged_prefill_tcgen05_kernel(const bf16* __restrict__ q, long long q_stride, bf1
     const int pos = valid ? start + qi : hi;
     const int row_lo = first_visible(pos, window);
     const bool any_valid = __any_sync(0xffffffffu, valid);          // of the warp
-    // where this thread's row starts in q and in out (in elements); other lanes fetch it by shuffle
+    // where this thread's row starts in q (in elements; other lanes fetch it by shuffle)
     const long long q_off = valid ? (long long)(tok0 + qi) * q_stride + (long long)head * D : -1;
-    const long long out_off = valid ? (long long)(tok0 + qi) * out_stride + (long long)head * D : -1;
+    // and in out, or in the splits' partial results: kept in shared memory, so that no register holds it through the walk
+    if (tid < 2 * ROWS)
+        row_place[tid] = !valid ? -1 : splits == 1 ? (long long)(tok0 + qi) * out_stride + (long long)head * D
+                                                   : ((long long)(tok0 + qi) * nq + head) * splits + split;
     constexpr int CPR = D / 8;                       // 16-byte chunks per row
     constexpr int RPI = 32 / CPR;                    // rows a warp moves per instruction: a row's chunks side by side
     if (softmax_thread) {
@@ -632,18 +640,17 @@ paged_prefill_tcgen05_kernel(const bf16* __restrict__ q, long long q_stride, bf1
             tie32(raw + 32);
             const int key0 = listed_tile<KEYS>(t_begin + j, kept, lo) * KEYS;
             const bool unmasked = key0 + KEYS - 1 <= pos_min && (key0 >= lo_max || key0 + KEYS <= keep);      // for the whole warp
-            Seen seen = {{0u, 0u}};
-            if (!unmasked) seen = seen_keys(pos - key0, row_lo - key0, keep - key0);
+            const Edges edges = {pos - key0, row_lo - key0, keep - key0};
             if (sigmoid) {
-                if (unmasked) row_sigmoid<false>(raw, s_addr, seen, scale_log2, bias);
-                else row_sigmoid<true>(raw, s_addr, seen, scale_log2, bias);
+                if (unmasked) row_sigmoid<false>(raw, s_addr, edges, scale_log2, bias);
+                else row_sigmoid<true>(raw, s_addr, edges, scale_log2, bias);
                 tmem_store_wait();
                 tc_fence_before();
                 mbar_arrive(&p_ready[ti][j & 1]);
                 continue;
             }
             if (mapped) row_map(raw, unit, cap_log2);
-            const float mx = unmasked ? row_max<false>(raw, seen) : row_max<true>(raw, seen);
+            const float mx = unmasked ? row_max<false>(raw, edges) : row_max<true>(raw, edges);
             const float m_new = fmaxf(m_ref, mx * to_log2);
             if (__any_sync(FULL, m_new > m_ref + RESCALE_STEP)) {
                 // move the reference point to the new maximum: O and the sum were taken against the old one
@@ -665,8 +672,8 @@ paged_prefill_tcgen05_kernel(const bf16* __restrict__ q, long long q_stride, bf1
                 m_ref = m_new;
             }
             const float m_safe = m_ref == -CUDART_INF_F ? 0.f : m_ref;
-            row_sum += unmasked ? row_exp<false>(raw, s_addr, seen, to_log2, m_safe)
-                                : row_exp<true>(raw, s_addr, seen, to_log2, m_safe);
+            row_sum += unmasked ? row_exp<false>(raw, s_addr, edges, to_log2, m_safe)
+                                : row_exp<true>(raw, s_addr, edges, to_log2, m_safe);
             tmem_store_wait();
             tc_fence_before();
             mbar_arrive(&p_ready[ti][j & 1]);
@@ -695,7 +702,7 @@ paged_prefill_tcgen05_kernel(const bf16* __restrict__ q, long long q_stride, bf1
 #pragma unroll
             for (int k = 0; k < CPR; ++k) {
                 const int row_in_warp = k * RPI + lane / CPR;
-                const long long to = __shfl_sync(FULL, out_off, row_in_warp);
+                const long long to = row_place[warp * 32 + row_in_warp];
                 const uint4 v = *reinterpret_cast<const uint4*>(stage + row_in_warp * (2 * D) + ((c ^ (row_in_warp & 7)) << 4));
                 if (to >= 0) *reinterpret_cast<uint4*>(out + to + c * 8) = v;
             }
@@ -703,8 +710,7 @@ paged_prefill_tcgen05_kernel(const bf16* __restrict__ q, long long q_stride, bf1
             // this split's share of the row: O / sum in float32 and the logarithm of the sum, for the merge
             tc_fence_after();
             const float inv = row_sum > 0.f ? 1.f / row_sum : 0.f;
-            const long long slot = valid ? ((long long)(tok0 + qi) * nq + head) * splits + split : -1;
-            if (valid) part_lse[slot] = row_sum > 0.f ? m_ref + log2f(row_sum) : -CUDART_INF_F;
+            if (row_place[tid] >= 0) part_lse[row_place[tid]] = row_sum > 0.f ? m_ref + log2f(row_sum) : -CUDART_INF_F;
             float* stage = reinterpret_cast<float*>(kv_s + (size_t)ti * (ROWS * 4 * D) + (warp & 3) * (32 * 4 * D));
 #pragma unroll 1
             for (int c = 0; c < D; c += 32) {
@@ -721,7 +727,7 @@ paged_prefill_tcgen05_kernel(const bf16* __restrict__ q, long long q_stride, bf1
 #pragma unroll 4
             for (int k = 0; k < CPR4; ++k) {
                 const int row_in_warp = k * RPI4 + lane / CPR4;
-                const long long to = __shfl_sync(FULL, slot, row_in_warp);
+                const long long to = row_place[warp * 32 + row_in_warp];
                 const float4 v = *reinterpret_cast<const float4*>(stage + row_in_warp * D + ((c ^ (row_in_warp & 7)) << 2));
                 if (to >= 0) *reinterpret_cast<float4*>(part_o + to * D + c * 4) = v;
             }
