@@ -279,10 +279,21 @@ def _fits(x, w) -> str:
     return "skinny" if skinny_ok(x.scaled if isinstance(x, Prenormed) else x, w) else ""
 
 
+SPLIT_MIN_K, SPLIT_MIN_N = 1024, 512
+
+
 def gemm_fp32(x, w, bias=None):
+    """The float32 product.  Matrices of SPLIT_MIN_N rows and SPLIT_MIN_K columns or more go through the tensor cores in three bfloat16
+    parts a number (csrc/gemm_split.cu), whatever the rows of x: a row's result does not depend on the batch."""
     M, K = x.shape
     N = w.shape[0]
     out = torch.empty((M, N), dtype=torch.float32, device=x.device)
+    if K >= SPLIT_MIN_K and N >= SPLIT_MIN_N:
+        segments = int(_core().fe_gemm_split_segments(_c_int(N), _c_int(K)))
+        part = torch.empty((segments, M, N), dtype=torch.float32, device=x.device) if segments > 1 else None
+        _run(_core(), "fe_gemm_split", _ptr(x), _ptr(w), _ptr(bias), _ptr(out), _ptr(part), _c_int(M), _c_int(N), _c_int(K),
+             _ptr(status_word(x.device)), _stream())
+        return out
     _run(_core(), "fe_gemm_fp32", _ptr(x), _ptr(w), _ptr(bias), _ptr(out), _c_int(M), _c_int(N), _c_int(K), _stream())
     return out
 

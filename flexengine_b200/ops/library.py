@@ -29,7 +29,7 @@ NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17",
 # library -> its sources; each library is what one kind of work needs, so that a first call
 # compiles only that
 GROUPS = {
-    "core": ["errors.cu", "elementwise.cu", "attention_simt.cu", "gemm_fp32.cu", "sampling.cu", "stream_ops.cu", "wkv.cu",
+    "core": ["errors.cu", "elementwise.cu", "attention_simt.cu", "gemm_fp32.cu", "gemm_split.cu", "sampling.cu", "stream_ops.cu", "wkv.cu",
              "latent.cu", "routed.cu", "hyper_ops.cu", "post_norm.cu", "layer_norm.cu", "retention.cu", "delta.cu",
              "head_scan.cu", "state_space.cu"],
     # elementwise.cu once more: the layer executor launches its kernels from inside this library
