@@ -51,7 +51,8 @@ extern "C" void fe_set_pdl(int classes) { g_pdl = classes; }
 // block of the next kernel fitted where two should have (gate/up of the 7B shape: 128 us instead of 44, the reason why such
 // launches were off).  30 % is enough for two of the largest of them and leaves L1 the rows that a weight-streaming kernel reads
 // again and again: 16 decode steps of 8 requests on the 7B shape take 25.2 ms with 20 or 30 %, 26.3 with 50 %, 57 with 100 %.
-constexpr int SHARED_CARVEOUT_PERCENT = 30;
+#include <cstdlib>
+static const int SHARED_CARVEOUT_PERCENT = getenv("FE_CARVE") ? atoi(getenv("FE_CARVE")) : 100;
 
 void fe_share_carveout(const void* kernel) {
     constexpr int SLOTS = 512;

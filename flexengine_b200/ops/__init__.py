@@ -321,10 +321,11 @@ def linear(x, w, bias=None, out_float32=False, follow=None, upcoming=None):
                 and norm_weight.dtype == torch.float32 and norm_weight.numel() == N):
             scaled = torch.empty((M, N), dtype=torch.bfloat16, device=rows.device)
             _rows, sumsq, tiles, eps = _rows_and_scale(x)
-            table = torch.empty((-(-N // 16), 8), dtype=torch.float32, device=rows.device)
+            parts = min(N, sm_count(rows.device)) if rows.is_cuda else 1       # blocks of the kernel, each of which leaves its sums
+            table = torch.empty((parts, 8), dtype=torch.float32, device=rows.device)
             _run(_bf16(), "fe_skinny_gemm_residual", _ptr(rows), _ptr(w), _ptr(residual), _ptr(norm_weight), _ptr(scaled),
                  _ptr(table), _c_int(M), _c_int(N), _c_int(rows.shape[1]), sumsq, tiles, eps,
-                 *_upcoming(upcoming, M, UPCOMING_TAIL_BYTES), _held(w), _stream())
+                 *_upcoming(upcoming, M, UPCOMING_TAIL_BYTES), _ptr(status_word(rows.device)), _held(w), _stream())
             return Prenormed(scaled, table, norm_eps, residual, norm_weight)
     if kernel and w.dtype == torch.bfloat16:
         wide = out_float32 or bias is not None           # a bias is added in float32, before the one rounding
@@ -381,7 +382,7 @@ def skinny_gemm(x, w, epilogue: int = EPI_BF16, upcoming=None):
     else:
         out = torch.empty((M, N), dtype=torch.float32 if epilogue == EPI_F32 else torch.bfloat16, device=x.device)
     _run(_bf16(), "fe_skinny_gemm_scaled", _ptr(x), _ptr(w), _ptr(out), _c_int(M), _c_int(N), _c_int(K), _c_int(epilogue),
-         sumsq, tiles, eps, *_upcoming(upcoming, M, UPCOMING_TAIL_BYTES), _held(w), _stream())
+         sumsq, tiles, eps, *_upcoming(upcoming, M, UPCOMING_TAIL_BYTES), _ptr(status_word(x.device)), _held(w), _stream())
     return out
 
 
