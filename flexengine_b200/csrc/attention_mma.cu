@@ -818,7 +818,7 @@ extern "C" int fe_paged_decode_cluster_resident(int requests, int nq, int nkv, i
             return 0;                                                                                                  \
         }                                                                                                              \
         cfg.dynamicSmemBytes = decode_smem<DMAX>(STAGES);                                                              \
-        if (getenv("FE_ATT")) fe_share_carveout((const void*)kernel);                                                  \
+        if (getenv("FE_ATT")) cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100);                                                  \
         if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess) {                                  \
             cudaGetLastError();                                                                                        \
             return 0;                                                                                                  \

@@ -35,8 +35,7 @@ namespace {
 
 constexpr int WARPS = 8;
 constexpr int KSTEP = 32;       // k elements of a step (2 MMAs)
-constexpr int WARP_RING = 12288, MAX_DEPTH = 8;        // bytes and units of a warp's ring
-constexpr int RING_BYTES = WARPS * WARP_RING;
+constexpr int LARGE_RING = 13824, SMALL_RING = 10240, MAX_DEPTH = 8;        // bytes (and units) of a warp's ring
 
 enum { EPI_BF16 = 0, EPI_F32 = 1, EPI_SWIGLU = 2, EPI_QKV = 3, EPI_RESID = 4, EPI_GEGLU = 5, EPI_RELU2 = 6, EPI_REGLU = 7, EPI_GELU = 8 };   // 5: gated, the tanh form of GELU
 constexpr int ACT_RELU2 = 3;            // ``gate_act`` of the bfloat16 epilogue: the square of relu(product), no gate (entry code 6)
@@ -70,7 +69,7 @@ struct RowScale {
     int width;                  // elements of a row (the mean is over them)
     const void* next;
     long long next_bytes;
-    int held;
+    int held, beside;
 };
 
 // What the fused query/key/value epilogue needs beside the product: bias, rotary table, where the
@@ -118,7 +117,7 @@ constexpr int RED_FLOATS = 4 * 128;      // accumulator tiles a warp leaves at a
 // How a launch cuts the matrix: ``items`` (rows, or pairs of rows) over the blocks, a block's in groups of at most ``rows`` of them; a
 // unit of the stream is ``rows`` items x KB steps of k, ``plane`` bytes a step, ``slot`` bytes in all, ``depth`` units a warp's ring.
 struct Cut {
-    int items, rows, plane, slot, depth;
+    int items, rows, plane, slot, depth, ring;
 };
 
 // TILES: the 16-row tiles a group has at most (1, 2 or 4); KB = 4 / TILES steps of k are one unit, so that a unit is always four
@@ -135,7 +134,7 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap map, const bf16* __restri
     __shared__ __align__(8) unsigned long long bars[WARPS][MAX_DEPTH];
     __shared__ float scale_part[WARPS][8];
     __shared__ float square_part[TILES][8];
-    float* const red = reinterpret_cast<float*>(shared + RING_BYTES);       // [WARPS][RED_FLOATS]
+    float* const red = reinterpret_cast<float*>(shared + WARPS * cut.ring);       // [WARPS][RED_FLOATS]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     // the block's groups of items; for queries, keys and values a group lies within a head
     const int item0 = EPI == EPI_QKV ? 0 : (int)((long long)cut.items * blockIdx.x / gridDim.x);
@@ -146,7 +145,7 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap map, const bf16* __restri
     const int u_begin = warp * units / WARPS, u_end = (warp + 1) * units / WARPS;
 
     // ---- the stream of weights: one lane a warp asks for units, into the warp's own ring ------------------------------
-    const unsigned ring = smem_u32(shared) + warp * WARP_RING, bar0 = smem_u32(&bars[warp][0]);
+    const unsigned ring = smem_u32(shared) + warp * cut.ring, bar0 = smem_u32(&bars[warp][0]);
     if (lane == 0) {
         for (int i = 0; i < MAX_DEPTH; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bar0 + 8 * i) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -401,7 +400,7 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap map, const bf16* __restri
     if (dead && lane == 0 && status) atomicOr(status, FE_STATUS_WAIT_EXPIRED);
 }
 
-constexpr int SHARED_BYTES = RING_BYTES + WARPS * RED_FLOATS * 4;
+constexpr int shared_bytes(int ring) { return WARPS * (ring + RED_FLOATS * 4); }
 
 int blocks_for(int items) { const int sms = fe_sm_count(); return items < sms ? items : sms; }
 
@@ -422,17 +421,17 @@ EncodeTiled encode_fn() {
 
 // Launches a kernel; gives it its shared memory first, once a device.
 template <int NT, int EPI, bool ONE, int TILES, typename... Args>
-int launch_kernel(int blocks, cudaStream_t stream, const CUtensorMap& map, Args... args) {
+int launch_kernel(int blocks, int ring, cudaStream_t stream, const CUtensorMap& map, Args... args) {
     static std::atomic<unsigned long long> allowed{0};
     const auto kernel = skinny_gemm_kernel<NT, EPI, ONE, TILES>;
     int device = 0;
     cudaGetDevice(&device);
     if (!(allowed.load() >> (device & 63) & 1)) {
-        const cudaError_t err = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SHARED_BYTES);
+        const cudaError_t err = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, shared_bytes(LARGE_RING));
         FE_REQUIRE(err == cudaSuccess, "skinny_gemm: %s", cudaGetErrorString(err));
         allowed.fetch_or(1ull << (device & 63));
     }
-    fe::launch(kernel, blocks, WARPS * 32, SHARED_BYTES, stream, map, args...);
+    fe::launch(kernel, blocks, WARPS * 32, shared_bytes(ring), stream, map, args...);
     return fe_check_launch("skinny_gemm");
 }
 
@@ -458,8 +457,8 @@ int launch(const void* x, const void* W, void* out, int M, int N, int K, int ite
     }
     const int tiles = (rows + ITEMS - 1) / ITEMS, T = tiles == 1 ? 1 : tiles == 2 ? 2 : 4, KB = 4 / T;
     const int plane = rows * (PAIRS ? 2 : 1) * KSTEP * 2, slot = (plane * KB + 127) / 128 * 128;
-    const int depth = WARP_RING / slot < MAX_DEPTH ? WARP_RING / slot : MAX_DEPTH;
-    const Cut cut{items, rows, plane, slot, depth};
+    const int ring = scale.beside ? SMALL_RING : LARGE_RING, depth = ring / slot < MAX_DEPTH ? ring / slot : MAX_DEPTH;
+    const Cut cut{items, rows, plane, slot, depth, ring};
     EncodeTiled encode = encode_fn();
     FE_REQUIRE(encode != nullptr, "skinny_gemm: cuTensorMapEncodeTiled is not available from this driver");
     CUtensorMap map;
@@ -485,7 +484,7 @@ int launch(const void* x, const void* W, void* out, int M, int N, int K, int ite
     }
     FE_REQUIRE(rc == CUDA_SUCCESS, "skinny_gemm: cuTensorMapEncodeTiled failed with code %d", (int)rc);
 #define FE_SKINNY(NT, ONE, TILES) \
-    return launch_kernel<NT, EPI, ONE, TILES>(blocks, stream, map, (const bf16*)x, out, M, N, K, cut, qkv, resid, scale, gate_act, status)
+    return launch_kernel<NT, EPI, ONE, TILES>(blocks, ring, stream, map, (const bf16*)x, out, M, N, K, cut, qkv, resid, scale, gate_act, status)
     if (M == 1) {
         if (T == 1) FE_SKINNY(1, true, 1);
         if (T == 2) FE_SKINNY(1, true, 2);
@@ -523,13 +522,13 @@ static int check_scale(const char* what, const float* sumsq, int sumsq_tiles, in
 // ``sumsq`` (may be null): see check_scale.  ``held``: see RowScale (the same for the entry points below).
 extern "C" int fe_skinny_gemm_scaled(const void* x, const void* W, void* out, int M, int N, int K, int epilogue,
                                      const float* sumsq, int sumsq_tiles, float eps, const void* next, long long next_bytes,
-                                     int* status, int held, cudaStream_t stream) {
+                                     int* status, int beside, int held, cudaStream_t stream) {
     FE_REQUIRE(M >= 1 && M <= 16, "skinny_gemm: %d rows; this kernel takes 1 to 16", M);
     FE_REQUIRE(N > 0 && K > 0 && K % 64 == 0, "skinny_gemm: K = %d must be a positive multiple of 64", K);
     FE_REQUIRE((((size_t)x | (size_t)W) & 15) == 0, "skinny_gemm: operands must be 16-byte aligned");
     if (check_scale("skinny_gemm", sumsq, sumsq_tiles, M, K)) return 1;
     FE_REQUIRE(next_bytes >= 0, "skinny_gemm: negative byte count");
-    const RowScale scale{sumsq, sumsq_tiles, eps, K, next, next_bytes, held};
+    const RowScale scale{sumsq, sumsq_tiles, eps, K, next, next_bytes, held, beside};
     if (epilogue == EPI_BF16) return launch<EPI_BF16>(x, W, out, M, N, K, N, stream, status, QkvEpilogue{}, ResidEpilogue{}, scale);
     if (epilogue == EPI_F32) return launch<EPI_F32>(x, W, out, M, N, K, N, stream, status, QkvEpilogue{}, ResidEpilogue{}, scale);
     if (epilogue == EPI_RELU2 || epilogue == EPI_GELU)
@@ -544,7 +543,7 @@ extern "C" int fe_skinny_gemm_scaled(const void* x, const void* W, void* out, in
 
 extern "C" int fe_skinny_gemm(const void* x, const void* W, void* out, int M, int N, int K, int epilogue,
                               cudaStream_t stream) {
-    return fe_skinny_gemm_scaled(x, W, out, M, N, K, epilogue, nullptr, 0, 0.f, nullptr, 0, nullptr, 0, stream);
+    return fe_skinny_gemm_scaled(x, W, out, M, N, K, epilogue, nullptr, 0, 0.f, nullptr, 0, nullptr, 0, 0, stream);
 }
 
 // The product that ends a branch of a layer: residual[M, N] += x W^T (float, in place); scaled[M, N] = bfloat16(new
@@ -552,7 +551,7 @@ extern "C" int fe_skinny_gemm(const void* x, const void* W, void* out, int M, in
 // ``sumsq_in`` (may be null): the scales of the input rows, as for fe_skinny_gemm_scaled.  M <= 8.
 extern "C" int fe_skinny_gemm_residual(const void* x, const void* W, float* residual, const float* norm_weight, void* scaled,
                                        float* sumsq_out, int M, int N, int K, const float* sumsq_in, int sumsq_tiles,
-                                       float eps, const void* next, long long next_bytes, int* status, int held, cudaStream_t stream) {
+                                       float eps, const void* next, long long next_bytes, int* status, int beside, int held, cudaStream_t stream) {
     FE_REQUIRE(M >= 1 && M <= 8, "skinny_gemm_residual: %d rows; this kernel takes 1 to 8", M);
     FE_REQUIRE(N > 0 && K > 0 && K % 64 == 0, "skinny_gemm_residual: K = %d must be a positive multiple of 64", K);
     FE_REQUIRE((((size_t)x | (size_t)W) & 15) == 0, "skinny_gemm_residual: operands must be 16-byte aligned");
@@ -561,7 +560,7 @@ extern "C" int fe_skinny_gemm_residual(const void* x, const void* W, float* resi
     const ResidEpilogue resid{residual, norm_weight, (bf16*)scaled, sumsq_out};
     FE_REQUIRE(next_bytes >= 0, "skinny_gemm_residual: negative byte count");
     return launch<EPI_RESID>(x, W, nullptr, M, N, K, N, stream, status, QkvEpilogue{}, resid,
-                             RowScale{sumsq_in, sumsq_tiles, eps, K, next, next_bytes, held});
+                             RowScale{sumsq_in, sumsq_tiles, eps, K, next, next_bytes, held, beside});
 }
 
 // The query/key/value projection of an attention layer with its epilogue fused: y = x W^T + bias,
@@ -572,7 +571,7 @@ extern "C" int fe_skinny_gemm_residual(const void* x, const void* W, float* resi
 extern "C" int fe_skinny_qkv(const void* x, const void* W, void* out, const float* bias, const int* positions,
                              const float* inv_freq, const int* slot_mapping, void* kc, void* vc, int M, int K, int nq,
                              int nkv, int d, int ps, long long num_slots, const float* sumsq, int sumsq_tiles, float eps,
-                             int* status, int held, cudaStream_t stream) {
+                             int* status, int beside, int held, cudaStream_t stream) {
     FE_REQUIRE(M >= 1 && M <= 8, "skinny_qkv: %d rows; this kernel takes 1 to 8", M);
     FE_REQUIRE(K > 0 && K % 64 == 0, "skinny_qkv: K = %d must be a positive multiple of 64", K);
     FE_REQUIRE(d >= 16 && d % 16 == 0 && nq > 0 && nkv > 0 && ps > 0, "skinny_qkv: bad head size or counts");
@@ -581,7 +580,7 @@ extern "C" int fe_skinny_qkv(const void* x, const void* W, void* out, const floa
     if (check_scale("skinny_qkv", sumsq, sumsq_tiles, M, K)) return 1;
     QkvEpilogue e{bias, positions, inv_freq, slot_mapping, (bf16*)kc, (bf16*)vc, nq, nkv, d, ps, num_slots, status};
     return launch<EPI_QKV>(x, W, out, M, (nq + 2 * nkv) * d, K, (nq + 2 * nkv) * (d / 2), stream, status, e, ResidEpilogue{},
-                           RowScale{sumsq, sumsq_tiles, eps, K, nullptr, 0, held});
+                           RowScale{sumsq, sumsq_tiles, eps, K, nullptr, 0, held, beside});
 }
 
 // How many entries of 8 floats the residual epilogue of a product with N columns leaves in ``sumsq_out``.

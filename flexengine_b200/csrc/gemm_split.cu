@@ -90,7 +90,7 @@ __device__ __forceinline__ void split8(const float4& p, const float4& q, uint4& 
 }
 
 template <int BN> struct Sizes {
-    static constexpr int STAGES = BN == 128 ? 2 : BN == 64 ? 3 : 4;
+    static constexpr int STAGES = 2;
     static constexpr int W_PART = TILE_W * CHUNK * 2, X_PART = BN * CHUNK * 2;
     static constexpr int STAGE = 3 * (W_PART + X_PART);
     static constexpr int BYTES = STAGES * STAGE + 1024;
@@ -358,7 +358,8 @@ __global__ void __launch_bounds__(256) add_segments_kernel(const float* __restri
 template <int BN, bool VEC>
 int launch_split(const float* A, const float* W, const float* bias, float* C, float* part, int M, int N, int K, int segments, int* status, cudaStream_t stream) {
     const auto kernel = gemm_split_kernel<BN, VEC>;
-    const cudaError_t err = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Sizes<BN>::BYTES);
+    cudaError_t err = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Sizes<BN>::BYTES);
+    if (err == cudaSuccess) err = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributePreferredSharedMemoryCarveout, (Sizes<BN>::BYTES + 2048) * 100 / (228 * 1024) + 1);
     FE_REQUIRE(err == cudaSuccess, "gemm_split: %s", cudaGetErrorString(err));
     const long long m_tiles = (M + BN - 1) / BN, tiles = m_tiles * ((N + TILE_W - 1) / TILE_W) * segments;
     FE_REQUIRE(tiles < (1LL << 30), "gemm_split: too many tiles");
