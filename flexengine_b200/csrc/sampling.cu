@@ -22,6 +22,7 @@
 // threshold, ties and the groups of 256 that hold any mass come from that short list.  A list that does not fit (many
 // equal logits, or large ones all in one thread's share) and a k too large for one take the radix select over the row.
 #include <math_constants.h>
+#include <string.h>
 
 #define FE_PDL_CLASS 8      // FE_PDL_SAMPLING
 #include "common.cuh"
@@ -32,6 +33,7 @@ namespace {
 
 constexpr int THREADS = 1024;
 constexpr int WARPS = THREADS / 32;
+constexpr int WIDE = 8;             // 16-byte loads on their way at once in the passes for the maximum and for the short list
 constexpr int RADIX_LOADS = 8;      // loads on their way at once in a pass of the radix select
 constexpr int SEGMENTS = 256;       // of a row; a block of a cluster of C owns SEGMENTS / C of them, a warp SEGMENTS / C / 32
 constexpr int MAX_CLUSTER = 8;
@@ -70,10 +72,24 @@ __device__ __forceinline__ float warp_total(float v) {       // the same value i
     return v;
 }
 
+// The parameters of a step's rows: on the device, or (up to LISTED_ROWS rows) with the launch, so that lists of numbers on the host
+// need no buffer and no copy of their own.
+constexpr int LISTED_ROWS = 64;
+struct OnDevice {
+    const float* temperature;
+    const int* top_k;
+    const long long* seed;
+    const long long* draw;
+};
+struct Listed {
+    float temperature[LISTED_ROWS];
+    int top_k[LISTED_ROWS];
+    long long seed[LISTED_ROWS], draw[LISTED_ROWS];
+};
+
+template <typename Parameters>
 __global__ void __launch_bounds__(THREADS)
-sample_kernel(const float* __restrict__ logits, long long ld, int V, const float* __restrict__ temperature,
-              const int* __restrict__ top_k, const long long* __restrict__ seed,
-              const long long* __restrict__ draw, int* __restrict__ out, const int C) {
+sample_kernel(const float* __restrict__ logits, long long ld, int V, const __grid_constant__ Parameters of, int* __restrict__ out, const int C) {
     griddep_wait();
     griddep_launch_dependents();
     __shared__ float s_val[WARPS];
@@ -99,7 +115,7 @@ sample_kernel(const float* __restrict__ logits, long long ld, int V, const float
     const int row = blockIdx.x / C, tid = threadIdx.x;
     const unsigned rank = blockIdx.x % C;               // of this block in its cluster
     const float* x = logits + (size_t)row * ld;
-    const float temp = temperature[row];
+    const float temp = of.temperature[row];
     // segments of S indices (a multiple of 32); this block's slice of the row is its segments side by side
     const int S = ((V + SEGMENTS - 1) / SEGMENTS + 31) / 32 * 32;
     const int per_block = SEGMENTS / C, per_warp = per_block / WARPS;
@@ -110,17 +126,17 @@ sample_kernel(const float* __restrict__ logits, long long ld, int V, const float
     int best_i = 0x7fffffff;
     const bool vector = (V & 3) == 0 && (reinterpret_cast<size_t>(x) & 15) == 0;      // lo is a multiple of 32
     if (vector) {
-        // four logits per load, four loads in flight per thread: what bounds this pass is how many loads are on
+        // four logits per load, eight loads in flight per thread: what bounds this pass is how many loads are on
         // their way at once
         const float4* x4 = reinterpret_cast<const float4*>(x);
         const int n4 = hi >> 2;                          // hi is V or a multiple of 32
         const float4 none = make_float4(-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F);
-        for (int i = (lo >> 2) + tid; i < n4; i += 4 * THREADS) {
-            float4 part[4];
+        for (int i = (lo >> 2) + tid; i < n4; i += WIDE * THREADS) {
+            float4 part[WIDE];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) part[u] = i + u * THREADS < n4 ? x4[i + u * THREADS] : none;
+            for (int u = 0; u < WIDE; ++u) part[u] = i + u * THREADS < n4 ? x4[i + u * THREADS] : none;
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
+            for (int u = 0; u < WIDE; ++u) {
                 const int at = 4 * (i + u * THREADS);
                 const float v4[4] = {part[u].x, part[u].y, part[u].z, part[u].w};
 #pragma unroll
@@ -137,7 +153,7 @@ sample_kernel(const float* __restrict__ logits, long long ld, int V, const float
             if (v > best || (v == best && i < best_i)) { best = v; best_i = i; }
         }
     }
-    int k = temp == 0.f ? 0 : top_k[row];
+    int k = temp == 0.f ? 0 : of.top_k[row];
     const bool use_k = k > 0 && k < V;
     // Only where the list is expected to fit: with the logits spread over the threads about -1024 ln(1 - k / 1024) of a block reach its
     // bound, and C blocks share LIST places (that many at 226 of eight blocks and at 403 of four); a row of no more logits than
@@ -199,12 +215,12 @@ sample_kernel(const float* __restrict__ logits, long long ld, int V, const float
         if (vector) {
             const float4* x4 = reinterpret_cast<const float4*>(x);
             const int n4 = hi >> 2;
-            for (int i = (lo >> 2) + tid; i < n4; i += 4 * THREADS) {
-                float4 part[4];
+            for (int i = (lo >> 2) + tid; i < n4; i += WIDE * THREADS) {
+                float4 part[WIDE];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) part[u] = i + u * THREADS < n4 ? x4[i + u * THREADS] : make_float4(0.f, 0.f, 0.f, 0.f);
+                for (int u = 0; u < WIDE; ++u) part[u] = i + u * THREADS < n4 ? x4[i + u * THREADS] : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
+                for (int u = 0; u < WIDE; ++u) {
                     const int at = 4 * (i + u * THREADS);
                     if (i + u * THREADS < n4) { collect(part[u].x, at); collect(part[u].y, at + 1); collect(part[u].z, at + 2); collect(part[u].w, at + 3); }
                 }
@@ -402,25 +418,50 @@ sample_kernel(const float* __restrict__ logits, long long ld, int V, const float
     };
 
     // mass of a segment: per group, each lane adds its eight values in order, the lanes' sums are added by a fixed
-    // butterfly, and the groups' sums are added up as the walk goes
-    for (int j = 0; j < per_warp; ++j) {
-        const int mine = warp * per_warp + j, segment = (int)rank * per_block + mine;
-        int seg0, seg1;
-        bounds(segment, seg0, seg1);
-        const int tie_base = use_k ? ties_before[segment] : 0;
+    // butterfly, and the groups' sums are added up as the walk goes; the next group's values are on their way meanwhile
+    {
+        int ahead_j = 0, ahead_base = 0, ahead0 = 0, ahead1 = 0;
+        unsigned int ahead_groups = 0;
+        auto open = [&](int at) {
+            ahead_j = at;
+            if (at < per_warp) {
+                bounds((int)rank * per_block + warp * per_warp + at, ahead0, ahead1);
+                ahead_base = ahead0;
+                ahead_groups = from_list ? seg_groups[warp * per_warp + at] : 0xffffffffu;      // the others hold neither mass nor ties
+            }
+        };
+        auto settle = [&]() {                            // on to a group that holds any
+            while (ahead_j < per_warp) {
+                while (ahead_base < ahead1 && !(ahead_groups >> min((ahead_base - ahead0) / (32 * GROUP), 31) & 1u)) ahead_base += 32 * GROUP;
+                if (ahead_base < ahead1) return;
+                open(ahead_j + 1);
+            }
+        };
+        if (lane == 0)
+            for (int q = 0; q < per_warp; ++q) seg_mass[warp * per_warp + q] = 0.f;
+        open(0);
+        settle();
+        float next[GROUP];
+        if (ahead_j < per_warp) load_group(ahead_base, ahead1, next);
         float cum = 0.f;
-        int ties_seen = 0;
-        const unsigned int groups = from_list ? seg_groups[mine] : 0xffffffffu;       // the others hold neither mass nor ties
-        for (int base = seg0; base < seg1; base += 32 * GROUP) {
-            if (!(groups >> min((base - seg0) / (32 * GROUP), 31) & 1u)) continue;
+        int j = -1, ties_seen = 0;
+        while (ahead_j < per_warp) {
+            if (ahead_j != j) { cum = 0.f; ties_seen = 0; }
+            j = ahead_j;
+            const int base = ahead_base, seg1 = ahead1;
             float v[GROUP];
-            load_group(base, seg1, v);
+#pragma unroll
+            for (int c = 0; c < GROUP; ++c) v[c] = next[c];
+            ahead_base += 32 * GROUP;
+            settle();
+            if (ahead_j < per_warp) load_group(ahead_base, ahead1, next);
+            const int mine = warp * per_warp + j, tie_base = use_k ? ties_before[(int)rank * per_block + mine] : 0;
             float part = 0.f;
 #pragma unroll
             for (int c = 0; c < GROUP; ++c) part += mass_of(base + 32 * c + lane, seg1, tie_base, v[c], ties_seen);
             cum += warp_total(part);
+            if (lane == 0) seg_mass[mine] = cum;
         }
-        if (lane == 0) seg_mass[mine] = cum;
     }
     cluster_sync();
     if (tid < SEGMENTS) mass_before[tid] = __uint_as_float(ld_peer(&seg_mass[tid % per_block], tid / per_block));
@@ -440,7 +481,7 @@ sample_kernel(const float* __restrict__ logits, long long ld, int V, const float
     }
     cluster_sync();                                     // every block has read the others' masses (and ties): they may leave
     const float total = mass_before[SEGMENTS];
-    const unsigned long long bits = splitmix64(splitmix64((unsigned long long)seed[row]) + (unsigned long long)draw[row]);
+    const unsigned long long bits = splitmix64(splitmix64((unsigned long long)of.seed[row]) + (unsigned long long)of.draw[row]);
     const float u = (float)(bits >> 40) * (1.0f / 16777216.0f);
     float target = u * total;
     if (target >= total) target = nextafterf(total, 0.f);
@@ -515,7 +556,7 @@ static int clusters_resident(int blocks) {
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         int clusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&clusters, sample_kernel, &cfg) != cudaSuccess) {
+        if (cudaOccupancyMaxActiveClusters(&clusters, sample_kernel<OnDevice>, &cfg) != cudaSuccess) {
             cudaGetLastError();
             clusters = 0;
         }
@@ -532,36 +573,8 @@ static int blocks_per_row(int R) {
     return 1;
 }
 
-extern "C" int fe_sample(const float* logits, long long ld, int R, int V, const float* temperature,
-                         const int* top_k, const long long* seed, const long long* draw, int* out,
-                         cudaStream_t stream) {
-    FE_REQUIRE(R >= 0 && V > 0 && ld >= V, "sample: bad sizes R=%d V=%d ld=%lld", R, V, ld);
-    FE_REQUIRE((long long)R * MAX_CLUSTER < (1LL << 31), "sample: too many rows");
-    if (R == 0) return 0;
-    const int C = blocks_per_row(R);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(R * C));
-    cfg.blockDim = dim3(THREADS);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = C;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    const cudaError_t err = cudaLaunchKernelEx(&cfg, sample_kernel, logits, ld, V, temperature, top_k, seed, draw, out, C);
-    FE_REQUIRE(err == cudaSuccess, "sample (clusters of %d): %s", C, cudaGetErrorString(err));
-    return fe_check_launch("sample");
-}
-
-// The same with a given number of blocks a row (1, 2, 4 or 8): the tokens are the same for every number.
-extern "C" int fe_sample_blocks(const float* logits, long long ld, int R, int V, const float* temperature,
-                                const int* top_k, const long long* seed, const long long* draw, int* out,
-                                int blocks, cudaStream_t stream) {
-    FE_REQUIRE(R >= 0 && V > 0 && ld >= V, "sample: bad sizes R=%d V=%d ld=%lld", R, V, ld);
-    FE_REQUIRE(blocks == 1 || blocks == 2 || blocks == 4 || blocks == 8, "sample: %d blocks a row; 1, 2, 4 or 8", blocks);
-    if (R == 0) return 0;
+template <typename Parameters>
+static int sample_rows(const float* logits, long long ld, int R, int V, const Parameters& of, int* out, int blocks, cudaStream_t stream) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(R * blocks));
     cfg.blockDim = dim3(THREADS);
@@ -573,7 +586,41 @@ extern "C" int fe_sample_blocks(const float* logits, long long ld, int R, int V,
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const cudaError_t err = cudaLaunchKernelEx(&cfg, sample_kernel, logits, ld, V, temperature, top_k, seed, draw, out, blocks);
+    const cudaError_t err = cudaLaunchKernelEx(&cfg, sample_kernel<Parameters>, logits, ld, V, of, out, blocks);
     FE_REQUIRE(err == cudaSuccess, "sample (clusters of %d): %s", blocks, cudaGetErrorString(err));
     return fe_check_launch("sample");
+}
+
+extern "C" int fe_sample(const float* logits, long long ld, int R, int V, const float* temperature,
+                         const int* top_k, const long long* seed, const long long* draw, int* out,
+                         cudaStream_t stream) {
+    FE_REQUIRE(R >= 0 && V > 0 && ld >= V, "sample: bad sizes R=%d V=%d ld=%lld", R, V, ld);
+    FE_REQUIRE((long long)R * MAX_CLUSTER < (1LL << 31), "sample: too many rows");
+    if (R == 0) return 0;
+    return sample_rows(logits, ld, R, V, OnDevice{temperature, top_k, seed, draw}, out, blocks_per_row(R), stream);
+}
+
+// The same with the parameters of up to 64 rows in the host's memory: they travel with the launch.
+extern "C" int fe_sample_listed(const float* logits, long long ld, int R, int V, const float* temperature,
+                                const int* top_k, const long long* seed, const long long* draw, int* out,
+                                cudaStream_t stream) {
+    FE_REQUIRE(R >= 0 && V > 0 && ld >= V, "sample: bad sizes R=%d V=%d ld=%lld", R, V, ld);
+    FE_REQUIRE(R <= LISTED_ROWS, "sample: %d rows with their parameters on the host; %d at most", R, LISTED_ROWS);
+    if (R == 0) return 0;
+    Listed of;
+    memcpy(of.temperature, temperature, R * sizeof(float));
+    memcpy(of.top_k, top_k, R * sizeof(int));
+    memcpy(of.seed, seed, R * sizeof(long long));
+    memcpy(of.draw, draw, R * sizeof(long long));
+    return sample_rows(logits, ld, R, V, of, out, blocks_per_row(R), stream);
+}
+
+// The same with a given number of blocks a row (1, 2, 4 or 8): the tokens are the same for every number.
+extern "C" int fe_sample_blocks(const float* logits, long long ld, int R, int V, const float* temperature,
+                                const int* top_k, const long long* seed, const long long* draw, int* out,
+                                int blocks, cudaStream_t stream) {
+    FE_REQUIRE(R >= 0 && V > 0 && ld >= V, "sample: bad sizes R=%d V=%d ld=%lld", R, V, ld);
+    FE_REQUIRE(blocks == 1 || blocks == 2 || blocks == 4 || blocks == 8, "sample: %d blocks a row; 1, 2, 4 or 8", blocks);
+    if (R == 0) return 0;
+    return sample_rows(logits, ld, R, V, OnDevice{temperature, top_k, seed, draw}, out, blocks, stream);
 }

@@ -1735,6 +1735,22 @@ def sample(logits, temperature, top_k, seed, draw, blocks: int = 0):
     return out
 
 
+SAMPLE_LISTED_ROWS = 64         # rows whose parameters travel with the launch
+
+
+def sample_listed(logits, temperature, top_k, seed, draw):
+    """``sample`` for up to SAMPLE_LISTED_ROWS rows with the parameters in the host's memory: arrays (``array.array``) of 32-bit floats,
+    32-bit whole numbers and two of 64-bit whole numbers, one number a row."""
+    _need_cuda(logits)
+    R, V = logits.shape
+    if logits.dtype != torch.float32 or logits.stride(1) != 1:
+        raise TypeError("sample: logits must be float32 with unit column stride")
+    out = torch.empty(R, dtype=torch.int32, device=logits.device)
+    _run(_core(), "fe_sample_listed", _ptr(logits), _c_ll(logits.stride(0)), _c_int(R), _c_int(V),
+         *(a.buffer_info()[0] for a in (temperature, top_k, seed, draw)), _ptr(out), _stream())
+    return out
+
+
 # ---- a whole decoder layer as one call --------------------------------------------------------------------------
 import ctypes as _ct
 

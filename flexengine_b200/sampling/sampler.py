@@ -9,6 +9,8 @@ else is in the batch or on how the scheduler cut the work.
 """
 from __future__ import annotations
 
+from array import array
+
 import numpy as np
 import torch
 
@@ -35,6 +37,19 @@ def _fill(words, values, dtype) -> None:
         words[:] = given
     else:
         torch.from_numpy(words)[:] = torch.tensor(list(values), dtype=dtype)
+
+
+def _arrays(n, temperatures, top_ks, seeds, draws):
+    """The four as arrays of the kernel's types, where they are lists or tuples of ``n`` plain numbers that fit; None otherwise."""
+    for values in (top_ks, seeds, draws):
+        if type(values) not in (list, tuple) or len(values) != n or set(map(type, values)) != {int}:
+            return None
+    if type(temperatures) not in (list, tuple) or not set(map(type, temperatures)) <= {int, float}:
+        return None
+    try:
+        return array("f", temperatures), array("i", top_ks), array("q", seeds), array("q", draws)
+    except OverflowError:
+        return None
 
 
 class Sampler:
@@ -67,6 +82,12 @@ class Sampler:
                                     torch.zeros(n, dtype=torch.int64, device=dev))
             temperature, top_k, zero64 = self._zeros[key]
             return self.ops.sample(logits, temperature, top_k, zero64, zero64)
+        # Plain lists for a batch of ordinary size go with the launch: no buffer, no copy, no views
+        listed = getattr(self.ops, "sample_listed", None)
+        if listed is not None and 0 < n <= self.ops.SAMPLE_LISTED_ROWS and dev.type == "cuda":
+            arrays = _arrays(n, temperatures, top_ks, seeds, draws)
+            if arrays is not None:
+                return listed(logits, *arrays)
         # One host buffer, one copy, no kernel to take it apart: [seeds | draws | temperatures | top_ks] as 8, 8, 4 and 4 bytes
         # each (four conversions and two kernels before: the host took longer than the device, 106 us for 64 rows)
         packed = torch.empty(3 * n, dtype=torch.int64, pin_memory=dev.type == "cuda")
