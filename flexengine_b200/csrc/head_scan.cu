@@ -147,6 +147,35 @@ __device__ __forceinline__ void cumulate(const float* __restrict__ gates, int be
     __syncthreads();
 }
 
+// 64 rows of 64 floats into shared memory, ``pitch`` floats apart: rows from ``rows`` and columns from ``cols`` on are zeros.  Asynchronous
+// copies of 16 bytes where the rows start on 16-byte boundaries (the caller waits for them); 256 threads.
+__device__ __forceinline__ void load_tile(float* to, int pitch, const float* __restrict__ from, long long ld, int rows, int cols) {
+    const bool wide = ((reinterpret_cast<size_t>(from) | (size_t)(ld * 4)) & 15) == 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int e = threadIdx.x + 256 * j, n = e >> 4, i = (e & 15) * 4;
+        const int have = n < rows ? min(max(cols - i, 0), 4) : 0;
+        float* dst = to + n * pitch + i;
+        const float* src = from + (have > 0 ? (size_t)n * ld + i : 0);
+        if (wide) {
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(have * 4) : "memory");
+        } else {
+            *reinterpret_cast<float4*>(dst) = make_float4(have > 0 ? src[0] : 0.f, have > 1 ? src[1] : 0.f, have > 2 ? src[2] : 0.f, have > 3 ? src[3] : 0.f);
+        }
+    }
+}
+__device__ __forceinline__ void tiles_here() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+
+// acc[0..3] += a * v, two multiply-adds an instruction
+__device__ __forceinline__ void add_scaled(float (&acc)[4], float a, const float4& v) {
+    float2 lo = make_float2(acc[0], acc[1]), hi = make_float2(acc[2], acc[3]);
+    const float2 twice = make_float2(a, a);
+    lo = __ffma2_rn(twice, make_float2(v.x, v.y), lo);
+    hi = __ffma2_rn(twice, make_float2(v.z, v.w), hi);
+    acc[0] = lo.x, acc[1] = lo.y, acc[2] = hi.x, acc[3] = hi.y;
+}
+__device__ __forceinline__ float at4(const float4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
+
 // sums[row][head] <- sum_b exp(L_last - L_b) w_b k_b v_b^T over the block's tokens (and the same of the keys alone).  Grid (block of
 // tokens, request, head x tile of key channels x tile of value channels), 256 threads as 16 x 16, a thread 4 key x 4 value channels.
 __global__ void __launch_bounds__(256)
@@ -169,17 +198,21 @@ head_scan_sums_kernel(const float* __restrict__ k, long long ldk, const float* _
     const int len = min(CHUNK, end - begin);
     const int tid = threadIdx.x;
     const size_t row = chunk_row(cu_q, r) + c;
+    const int group = head / (heads / groups);
+    load_tile(ks, TILE, k + (size_t)begin * ldk + (size_t)group * d + dt * TILE, ldk, len, d - dt * TILE);
+    load_tile(vs, TILE, v + (size_t)begin * ldv + (size_t)head * dv + vt * TILE, ldv, len, dv - vt * TILE);
     cumulate(gates, begin, len, heads, head, cum, &half);
     if (tid < CHUNK) pw[tid] = tid < len ? expf((float)(cum[len - 1] - cum[tid])) * gates[plane + (size_t)(begin + tid) * heads + head] : 0.f;
     if (tid == 0 && dt == 0 && vt == 0) totals[row * heads + head] = exp_decay((float)cum[len - 1]);
+    tiles_here();
     __syncthreads();
-    const int group = head / (heads / groups);
-    for (int e = tid; e < CHUNK * TILE; e += 256) {
-        const int b = e / TILE, i = e - b * TILE;
-        const int gi = dt * TILE + i, gj = vt * TILE + i;
-        const bool in = b < len;
-        ks[e] = (in && gi < d) ? pw[b] * k[(size_t)(begin + b) * ldk + (size_t)group * d + gi] : 0.f;
-        vs[e] = (in && gj < dv) ? v[(size_t)(begin + b) * ldv + (size_t)head * dv + gj] : 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {                          // what this thread copied, times the tokens' weights
+        const int e = tid + 256 * j;
+        const float w = pw[e >> 4];
+        float4 t = *reinterpret_cast<const float4*>(ks + e * 4);
+        t.x *= w, t.y *= w, t.z *= w, t.w *= w;
+        *reinterpret_cast<float4*>(ks + e * 4) = t;
     }
     __syncthreads();
     const int ty = tid >> 4, tx = tid & 15;
@@ -188,11 +221,8 @@ head_scan_sums_kernel(const float* __restrict__ k, long long ldk, const float* _
     for (int b = 0; b < len; ++b) {
         const float4 k4 = *reinterpret_cast<const float4*>(ks + b * TILE + ty * 4);
         const float4 v4 = *reinterpret_cast<const float4*>(vs + b * TILE + tx * 4);
-        const float kk[4] = {k4.x, k4.y, k4.z, k4.w}, vv[4] = {v4.x, v4.y, v4.z, v4.w};
 #pragma unroll
-        for (int x = 0; x < 4; ++x)
-#pragma unroll
-            for (int y = 0; y < 4; ++y) acc[x][y] = fmaf(kk[x], vv[y], acc[x][y]);
+        for (int x = 0; x < 4; ++x) add_scaled(acc[x], at4(k4, x), v4);
     }
     float* to = sums + row * per + (size_t)head * d * dv;
 #pragma unroll
@@ -258,37 +288,41 @@ head_scan_products_kernel(const float* __restrict__ q, long long ldq, float quer
                           const int* __restrict__ cu_q, float* __restrict__ qk, int groups, int d, int nd) {
     griddep_wait();
     griddep_launch_dependents();
-    __shared__ __align__(16) float qT[TILE * PITCH];
-    __shared__ __align__(16) float kT[TILE * PITCH];
+    __shared__ __align__(16) float qS[CHUNK * PITCH];
+    __shared__ __align__(16) float kS[CHUNK * PITCH];
     const int c = blockIdx.x, r = blockIdx.y, group = blockIdx.z;
     const int begin = cu_q[r] + c * CHUNK, end = cu_q[r + 1];
     if (begin >= end) return;
     const int len = min(CHUNK, end - begin);
     const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-    float W[4][4] = {};
+    float W[4][4] = {};                          // query ty * 4 + x, key tx + 16 y
     for (int dt = 0; dt < nd; ++dt) {
         __syncthreads();
-        for (int e = tid; e < CHUNK * TILE; e += 256) {
-            const int n = e / TILE, i = e - n * TILE, gi = dt * TILE + i;
-            const bool in = n < len && gi < d;
-            qT[i * PITCH + n] = in ? query_scale * q[(size_t)(begin + n) * ldq + (size_t)group * d + gi] : 0.f;
-            kT[i * PITCH + n] = in ? k[(size_t)(begin + n) * ldk + (size_t)group * d + gi] : 0.f;
-        }
+        load_tile(qS, PITCH, q + (size_t)begin * ldq + (size_t)group * d + dt * TILE, ldq, len, d - dt * TILE);
+        load_tile(kS, PITCH, k + (size_t)begin * ldk + (size_t)group * d + dt * TILE, ldk, len, d - dt * TILE);
+        tiles_here();
         __syncthreads();
 #pragma unroll 4
-        for (int i = 0; i < TILE; ++i) {
-            const float4 q4 = *reinterpret_cast<const float4*>(qT + i * PITCH + ty * 4);
-            const float4 k4 = *reinterpret_cast<const float4*>(kT + i * PITCH + tx * 4);
-            const float qq[4] = {q4.x, q4.y, q4.z, q4.w}, kk[4] = {k4.x, k4.y, k4.z, k4.w};
+        for (int i = 0; i < TILE; i += 4) {
+            float4 q4[4], k4[4];
 #pragma unroll
-            for (int x = 0; x < 4; ++x)
+            for (int x = 0; x < 4; ++x) {
+                q4[x] = *reinterpret_cast<const float4*>(qS + (ty * 4 + x) * PITCH + i);
+                k4[x] = *reinterpret_cast<const float4*>(kS + (tx + 16 * x) * PITCH + i);
+            }
 #pragma unroll
-                for (int y = 0; y < 4; ++y) W[x][y] = fmaf(qq[x], kk[y], W[x][y]);
+            for (int e = 0; e < 4; ++e)
+#pragma unroll
+                for (int x = 0; x < 4; ++x)
+#pragma unroll
+                    for (int y = 0; y < 4; ++y) W[x][y] = fmaf(at4(q4[x], e), at4(k4[y], e), W[x][y]);
         }
     }
     float* to = qk + ((chunk_row(cu_q, r) + c) * groups + group) * (size_t)(CHUNK * CHUNK);
 #pragma unroll
-    for (int y = 0; y < 4; ++y) *reinterpret_cast<float4*>(to + (tx * 4 + y) * CHUNK + ty * 4) = make_float4(W[0][y], W[1][y], W[2][y], W[3][y]);
+    for (int y = 0; y < 4; ++y)
+        *reinterpret_cast<float4*>(to + (tx + 16 * y) * CHUNK + ty * 4) =
+            make_float4(query_scale * W[0][y], query_scale * W[1][y], query_scale * W[2][y], query_scale * W[3][y]);
 }
 
 // A block's outputs for a tile of value channels: W = (Q K^T) with entry (n, b) times exp(L_n - L_b) w_b where b <= n, else 0, and
@@ -309,9 +343,10 @@ head_scan_out_kernel(const float* __restrict__ q, long long ldq, float query_sca
     griddep_launch_dependents();
     extern __shared__ __align__(16) float smem[];
     double* cum = reinterpret_cast<double*>(smem);              // [CHUNK]
-    float* qT = smem + 2 * CHUNK;                // [TILE][PITCH]: key channel i of token n at i * PITCH + n
-    float* kT = qT + TILE * PITCH;               // the same of the keys; later W as [b][n]
-    float* sS = kT + TILE * PITCH;               // [TILE][TILE] the state before the block, key channel x value channel
+    float* qS = smem + 2 * CHUNK;                // [CHUNK][PITCH]: key channel i of token n at n * PITCH + i
+    float* kS = qS + CHUNK * PITCH;              // the same of the keys
+    float* kT = kS;                              // later W as [b][n]
+    float* sS = kS + CHUNK * PITCH;              // [TILE][TILE] the state before the block, key channel x value channel
     float* vS = sS + TILE * TILE;                // [CHUNK][TILE]
     float* wb = vS + CHUNK * TILE;               // [CHUNK] the tokens' weights
     float* below = wb + CHUNK;                   // [CHUNK] n_t . q_t, then the factor of the output
@@ -323,12 +358,9 @@ head_scan_out_kernel(const float* __restrict__ q, long long ldq, float query_sca
     if (begin >= end) return;
     const int len = min(CHUNK, end - begin);
     const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+    load_tile(vS, TILE, v + (size_t)begin * ldv + (size_t)head * dv + vt * TILE, ldv, len, dv - vt * TILE);
     cumulate(gates, begin, len, heads, head, cum, &half);
     if (tid < CHUNK) wb[tid] = tid < len ? gates[plane + (size_t)(begin + tid) * heads + head] : 0.f;
-    for (int e = tid; e < CHUNK * TILE; e += 256) {
-        const int b = e / TILE, j = e - b * TILE, gj = vt * TILE + j;
-        vS[e] = (b < len && gj < dv) ? v[(size_t)(begin + b) * ldv + (size_t)head * dv + gj] : 0.f;
-    }
     const float* before = sums + (chunk_row(cu_q, r) + c) * per + (size_t)head * d * dv;
     const float* keys_before = sums + (chunk_row(cu_q, r) + c) * per + (size_t)heads * d * dv + (size_t)head * d;
     float W[4][4] = {}, O[4][4] = {};
@@ -336,46 +368,55 @@ head_scan_out_kernel(const float* __restrict__ q, long long ldq, float query_sca
     float nq = 0.f;
     for (int dt = 0; dt < nd; ++dt) {
         __syncthreads();
-        for (int e = tid; e < CHUNK * TILE; e += 256) {
-            const int n = e / TILE, i = e - n * TILE, gi = dt * TILE + i;
-            const bool in = n < len && gi < d;
-            qT[i * PITCH + n] = in ? query_scale * q[(size_t)(begin + n) * ldq + (size_t)group * d + gi] : 0.f;
-            if (!SHARED) kT[i * PITCH + n] = in ? k[(size_t)(begin + n) * ldk + (size_t)group * d + gi] : 0.f;
-            const int gj = vt * TILE + i;                                       // here n walks key channels, i value channels
-            sS[e] = (dt * TILE + n < d && gj < dv) ? before[(size_t)(dt * TILE + n) * dv + gj] : 0.f;
-        }
+        load_tile(qS, PITCH, q + (size_t)begin * ldq + (size_t)group * d + dt * TILE, ldq, len, d - dt * TILE);
+        if (!SHARED) load_tile(kS, PITCH, k + (size_t)begin * ldk + (size_t)group * d + dt * TILE, ldk, len, d - dt * TILE);
+        load_tile(sS, TILE, before + (size_t)dt * TILE * dv + vt * TILE, dv, d - dt * TILE, dv - vt * TILE);
         if (divided && tid < TILE) nS[tid] = dt * TILE + tid < d ? keys_before[dt * TILE + tid] : 0.f;
+        tiles_here();
         __syncthreads();
 #pragma unroll 4
-        for (int i = 0; i < TILE; ++i) {
-            const float4 q4 = *reinterpret_cast<const float4*>(qT + i * PITCH + ty * 4);
-            const float4 k4 = SHARED ? make_float4(0.f, 0.f, 0.f, 0.f) : *reinterpret_cast<const float4*>(kT + i * PITCH + tx * 4);
-            const float4 s4 = *reinterpret_cast<const float4*>(sS + i * TILE + tx * 4);
-            const float qq[4] = {q4.x, q4.y, q4.z, q4.w}, kk[4] = {k4.x, k4.y, k4.z, k4.w}, ss[4] = {s4.x, s4.y, s4.z, s4.w};
+        for (int i = 0; i < TILE; i += 4) {
+            float4 q4[4], k4[4];
 #pragma unroll
-            for (int x = 0; x < 4; ++x)
+            for (int x = 0; x < 4; ++x) {
+                q4[x] = *reinterpret_cast<const float4*>(qS + (ty * 4 + x) * PITCH + i);
+                if (!SHARED) k4[x] = *reinterpret_cast<const float4*>(kS + (tx + 16 * x) * PITCH + i);
+            }
 #pragma unroll
-                for (int y = 0; y < 4; ++y) {
-                    if (!SHARED) W[x][y] = fmaf(qq[x], kk[y], W[x][y]);
-                    O[x][y] = fmaf(qq[x], ss[y], O[x][y]);
+            for (int e = 0; e < 4; ++e) {
+                const float4 s4 = *reinterpret_cast<const float4*>(sS + (i + e) * TILE + tx * 4);
+#pragma unroll
+                for (int x = 0; x < 4; ++x) {
+                    add_scaled(O[x], at4(q4[x], e), s4);
+                    if (!SHARED) {
+#pragma unroll
+                        for (int y = 0; y < 4; ++y) W[x][y] = fmaf(at4(q4[x], e), at4(k4[y], e), W[x][y]);
+                    }
                 }
+            }
         }
         if (divided)
-            for (int i = part; i < TILE; i += 4) nq = fmaf(qT[i * PITCH + mine], nS[i], nq);
+            for (int i = part; i < TILE; i += 4) nq = fmaf(qS[mine * PITCH + i], nS[i], nq);
     }
     __syncthreads();
     if (SHARED) {
         const float* from = qk + ((chunk_row(cu_q, r) + c) * groups + group) * (size_t)(CHUNK * CHUNK);
 #pragma unroll
         for (int y = 0; y < 4; ++y) {
-            const float4 w4 = *reinterpret_cast<const float4*>(from + (tx * 4 + y) * CHUNK + ty * 4);
+            const float4 w4 = *reinterpret_cast<const float4*>(from + (tx + 16 * y) * CHUNK + ty * 4);
             W[0][y] = w4.x, W[1][y] = w4.y, W[2][y] = w4.z, W[3][y] = w4.w;
         }
+    } else {
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+#pragma unroll
+            for (int y = 0; y < 4; ++y) W[x][y] *= query_scale;
     }
+    nq *= query_scale;
     const float skip_of = skip ? skip[head] : 0.f;
 #pragma unroll
     for (int y = 0; y < 4; ++y) {
-        const int b = tx * 4 + y;
+        const int b = tx + 16 * y;
         float w[4];
 #pragma unroll
         for (int x = 0; x < 4; ++x) {
@@ -386,7 +427,7 @@ head_scan_out_kernel(const float* __restrict__ q, long long ldq, float query_sca
     }
 #pragma unroll
     for (int x = 0; x < 4; ++x) {
-        const float a = expf((float)cum[ty * 4 + x]);
+        const float a = query_scale * expf((float)cum[ty * 4 + x]);
 #pragma unroll
         for (int y = 0; y < 4; ++y) O[x][y] *= a;
     }
@@ -406,11 +447,8 @@ head_scan_out_kernel(const float* __restrict__ q, long long ldq, float query_sca
     for (int b = 0; b < seen; ++b) {
         const float4 w4 = *reinterpret_cast<const float4*>(kT + b * PITCH + ty * 4);
         const float4 v4 = *reinterpret_cast<const float4*>(vS + b * TILE + tx * 4);
-        const float ww[4] = {w4.x, w4.y, w4.z, w4.w}, vv[4] = {v4.x, v4.y, v4.z, v4.w};
 #pragma unroll
-        for (int x = 0; x < 4; ++x)
-#pragma unroll
-            for (int y = 0; y < 4; ++y) O[x][y] = fmaf(ww[x], vv[y], O[x][y]);
+        for (int x = 0; x < 4; ++x) add_scaled(O[x], at4(w4, x), v4);
     }
     if (divided) __syncthreads();
 #pragma unroll
