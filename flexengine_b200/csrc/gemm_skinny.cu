@@ -122,8 +122,9 @@ struct Cut {
 
 // TILES: the 16-row tiles a group has at most (1, 2 or 4); KB = 4 / TILES steps of k are one unit, so that a unit is always four
 // (tile, step) pairs: eight 16-byte reads and eight multiplications that wait for one another in pairs at most.
-// ONE: a single row of x.
-template <int NT, int EPI, bool ONE, int TILES>
+// ONE: a single row of x.  WIDE: a block has so many items that every warp takes an eighth of them over all of K, adds nothing up with
+// the others and meets them at no barrier; else the warps share K.
+template <int NT, int EPI, bool ONE, int TILES, bool WIDE>
 __global__ void __launch_bounds__(WARPS * 32, NT == 1 ? 2 : 1)
 skinny_gemm_kernel(const __grid_constant__ CUtensorMap map, const bf16* __restrict__ x, void* __restrict__ out, const int M, const int N, const int K,
                    const Cut cut, const QkvEpilogue qkv, const ResidEpilogue resid, const RowScale scale, const int gate_act, int* __restrict__ status) {
@@ -137,12 +138,13 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap map, const bf16* __restri
     float* const red = reinterpret_cast<float*>(shared + WARPS * cut.ring);       // [WARPS][RED_FLOATS]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     // the block's groups of items; for queries, keys and values a group lies within a head
-    const int item0 = EPI == EPI_QKV ? 0 : (int)((long long)cut.items * blockIdx.x / gridDim.x);
-    const int item1 = EPI == EPI_QKV ? cut.items : (int)((long long)cut.items * (blockIdx.x + 1) / gridDim.x);
+    const int block0 = (int)((long long)cut.items * blockIdx.x / gridDim.x), block1 = (int)((long long)cut.items * (blockIdx.x + 1) / gridDim.x);
+    const int item0 = EPI == EPI_QKV ? 0 : WIDE ? block0 + (block1 - block0) * warp / WARPS : block0;
+    const int item1 = EPI == EPI_QKV ? cut.items : WIDE ? block0 + (block1 - block0) * (warp + 1) / WARPS : block1;
     const int first_item = EPI == EPI_QKV ? (int)blockIdx.x * cut.rows : item0, group_step = EPI == EPI_QKV ? (int)gridDim.x * cut.rows : cut.rows;
     // a warp's share of the units along K
     const int units = (K / KSTEP + KB - 1) / KB;
-    const int u_begin = warp * units / WARPS, u_end = (warp + 1) * units / WARPS;
+    const int u_begin = WIDE ? 0 : warp * units / WARPS, u_end = WIDE ? units : (warp + 1) * units / WARPS;
 
     // ---- the stream of weights: one lane a warp asks for units, into the warp's own ring ------------------------------
     const unsigned ring = smem_u32(shared) + warp * cut.ring, bar0 = smem_u32(&bars[warp][0]);
@@ -189,23 +191,29 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap map, const bf16* __restri
     auto load_set = [&](int k) {
         return k + g < k_end ? __ldcg(reinterpret_cast<const uint4*>(x + (size_t)(k + g) * KSTEP + 8 * t)) : make_uint4(0, 0, 0, 0);
     };
+    // step ``k`` of this group into place i of eight, or, past the group's end, the step that the next group begins with there
     auto load_step = [&](int i, int k) {
+        if (k >= k_end) k = k_begin + i;
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt)
             xa[i][nt] = xr[nt] != nullptr && k < k_end ? __ldcg(reinterpret_cast<const uint4*>(xr[nt] + (size_t)k * KSTEP)) : make_uint4(0, 0, 0, 0);
     };
-    auto first_rows = [&]() {
-        if constexpr (ONE) {
-#pragma unroll
-            for (int i = 0; i < SETS; ++i) xs[i] = load_set(k_begin + 8 * i);
-        } else {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) load_step(i, k_begin + i);
-        }
+    int set_k = k_begin;                          // ONE: the first step of the set that is loaded next; the groups follow one another in a ring
+    auto next_set = [&]() {
+        const uint4 v = load_set(set_k);
+        set_k += 8;
+        if (set_k >= k_end) set_k = k_begin;
+        return v;
     };
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) xr[nt] = nt * 8 + g < M ? x + (size_t)(nt * 8 + g) * K + 8 * t : nullptr;
-    first_rows();
+    if constexpr (ONE) {
+#pragma unroll
+        for (int i = 0; i < SETS; ++i) xs[i] = next_set();
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) load_step(i, k_begin + i);
+    }
     // a thread's column of the batch in the epilogues of one column tile: the same for every group
     const int my_m = PAIRS ? (tid >> 3) & 7 : (tid >> 4) & 7;
     if (scale.sumsq != nullptr) {
@@ -216,7 +224,7 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap map, const bf16* __restri
         sum += __shfl_xor_sync(0xffffffffu, sum, 16);
         if (lane < 8) scale_part[warp][lane] = sum;
     }
-    float row_scale = 1.f, squares = 0.f;
+    float row_scale = 1.f, squares = 0.f, scales[2] = {1.f, 1.f};
     int slot = 0;
     unsigned parity = 0;
     bool dead = false;                            // a wait has run out: no more waiting, the status word says so
@@ -293,15 +301,52 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap map, const bf16* __restri
             if constexpr (ONE) {                              // the next eight steps
 #pragma unroll
                 for (int i = 0; i + 1 < SETS; ++i) xs[i] = xs[i + 1];
-                xs[SETS - 1] = load_set((u0 + AHEAD) * KB + 8 * (SETS - 1));
+                xs[SETS - 1] = next_set();
             }
         }
-        if (more) first_rows();
         if (TILES == 1) {
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) acc[0][nt][e] += acc[CHAINS - 1][nt][e];
+        }
+        if constexpr (WIDE) {
+            if (scale.sumsq != nullptr && first) {
+                __syncthreads();                  // the shares of the rows' sums are there
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    float sum = 0.f;
+#pragma unroll
+                    for (int w = 0; w < WARPS; ++w) sum += scale_part[w][2 * t + c];
+                    scales[c] = rsqrtf(sum / (float)scale.width + scale.eps);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < TILES; ++j)
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                    for (int c = 0; c < 2; ++c) {
+                        const int m = nt * 8 + 2 * t + c;
+                        const float lo = acc[j][nt][c] * scales[c], hi = acc[j][nt][2 + c] * scales[c];       // accumulator rows g and g + 8
+                        if (m >= M) continue;
+                        if (EPI == EPI_SWIGLU) {
+                            const int item = start + j * 8 + g;
+                            if (item < end) reinterpret_cast<bf16*>(out)[(size_t)m * cut.items + item] = __float2bfloat16_rn(gate_function(lo, gate_act) * hi);
+                        } else {
+#pragma unroll
+                            for (int h = 0; h < 2; ++h) {
+                                const int col = start + j * 16 + g + 8 * h;
+                                float v = h ? hi : lo;
+                                if (col >= end) continue;
+                                if (EPI == EPI_BF16 && gate_act == ACT_RELU2) v = v > 0.f ? v * v : 0.f;
+                                if (EPI == EPI_BF16 && gate_act == ACT_GELU) v = gelu_erf(v);
+                                if (EPI == EPI_F32) reinterpret_cast<float*>(out)[(size_t)m * N + col] = v;
+                                else reinterpret_cast<bf16*>(out)[(size_t)m * N + col] = __float2bfloat16_rn(v);
+                            }
+                        }
+                    }
+            continue;
         }
         float* const mine = red + warp * RED_FLOATS;
         if (!first) __syncthreads();              // the group before has been read out of ``red``
@@ -420,10 +465,10 @@ EncodeTiled encode_fn() {
 }
 
 // Launches a kernel; gives it its shared memory first, once a device.
-template <int NT, int EPI, bool ONE, int TILES, typename... Args>
+template <int NT, int EPI, bool ONE, int TILES, bool WIDE, typename... Args>
 int launch_kernel(int blocks, int ring, cudaStream_t stream, const CUtensorMap& map, Args... args) {
     static std::atomic<unsigned long long> allowed{0};
-    const auto kernel = skinny_gemm_kernel<NT, EPI, ONE, TILES>;
+    const auto kernel = skinny_gemm_kernel<NT, EPI, ONE, TILES, WIDE>;
     int device = 0;
     cudaGetDevice(&device);
     if (!(allowed.load() >> (device & 63) & 1)) {
@@ -443,6 +488,7 @@ int launch(const void* x, const void* W, void* out, int M, int N, int K, int ite
     constexpr int ITEMS = PAIRS ? 8 : 16;
     const int sms = fe_sm_count(), most = M <= 8 ? 4 : 2;          // tiles a group may have
     int blocks, rows;
+    bool wide = false;
     if (EPI == EPI_QKV) {
         // groups that lie within a head: a divisor of d / 2; as few rounds of rows over the SMs as possible
         const int half = qkv.d / 2;
@@ -452,7 +498,9 @@ int launch(const void* x, const void* W, void* out, int M, int N, int K, int ite
         blocks = items / rows < sms ? items / rows : sms;
     } else {
         blocks = blocks_for(items);
-        const int own = (items + blocks - 1) / blocks, groups = (own + ITEMS * most - 1) / (ITEMS * most);
+        const int block_own = (items + blocks - 1) / blocks;
+        wide = EPI != EPI_RESID && block_own > 4 * ITEMS;          // more than half a tile for each warp
+        const int own = wide ? (block_own + WARPS - 1) / WARPS : block_own, groups = (own + ITEMS * most - 1) / (ITEMS * most);
         rows = (own + groups - 1) / groups;
     }
     const int tiles = (rows + ITEMS - 1) / ITEMS, T = tiles == 1 ? 1 : tiles == 2 ? 2 : 4, KB = 4 / T;
@@ -483,24 +531,25 @@ int launch(const void* x, const void* W, void* out, int M, int N, int K, int ite
         rc = make(3, dims, strides, box);
     }
     FE_REQUIRE(rc == CUDA_SUCCESS, "skinny_gemm: cuTensorMapEncodeTiled failed with code %d", (int)rc);
-#define FE_SKINNY(NT, ONE, TILES) \
-    return launch_kernel<NT, EPI, ONE, TILES>(blocks, ring, stream, map, (const bf16*)x, out, M, N, K, cut, qkv, resid, scale, gate_act, status)
-    if (M == 1) {
-        if (T == 1) FE_SKINNY(1, true, 1);
-        if (T == 2) FE_SKINNY(1, true, 2);
-        FE_SKINNY(1, true, 4);
+#define FE_SKINNY(NT, ONE, TILES, WIDE) \
+    return launch_kernel<NT, EPI, ONE, TILES, WIDE>(blocks, ring, stream, map, (const bf16*)x, out, M, N, K, cut, qkv, resid, scale, gate_act, status)
+#define FE_SKINNY_TILES(NT, ONE, WIDE) \
+    do { \
+        if (T == 1) FE_SKINNY(NT, ONE, 1, WIDE); \
+        if (T == 2) FE_SKINNY(NT, ONE, 2, WIDE); \
+        if constexpr (NT == 1) FE_SKINNY(NT, ONE, 4, WIDE); \
+    } while (0)
+    if constexpr (EPI != EPI_RESID && EPI != EPI_QKV) {
+        if (wide && M == 1) FE_SKINNY_TILES(1, true, true);
+        if (wide && M <= 8) FE_SKINNY_TILES(1, false, true);
+        if (wide) FE_SKINNY_TILES(2, false, true);
+        if (M > 8) FE_SKINNY_TILES(2, false, false);
     }
-    if (M <= 8) {
-        if (T == 1) FE_SKINNY(1, false, 1);
-        if (T == 2) FE_SKINNY(1, false, 2);
-        FE_SKINNY(1, false, 4);
-    }
-    if constexpr (EPI == EPI_RESID || EPI == EPI_QKV) return 1;      // refused by the entry point already
-    else {
-        if (T == 1) FE_SKINNY(2, false, 1);
-        FE_SKINNY(2, false, 2);
-    }
+    if (M == 1) FE_SKINNY_TILES(1, true, false);
+    if (M <= 8) FE_SKINNY_TILES(1, false, false);
+    return 1;                                     // refused by the entry point already
 #undef FE_SKINNY
+#undef FE_SKINNY_TILES
 }
 
 }  // namespace

@@ -94,7 +94,10 @@ template <int BN> struct Sizes {
     static constexpr int W_PART = TILE_W * CHUNK * 2, X_PART = BN * CHUNK * 2;
     static constexpr int STAGE = 3 * (W_PART + X_PART);
     static constexpr int BYTES = STAGES * STAGE + 1024;
-    static constexpr int COLUMNS = 2 * BN;                      // of tensor memory: two accumulators
+    // An MMA that adds to the accumulator of the one before it waits for that: CHAINS accumulators take turns (every fourth or every
+    // second step of a chunk's four), and the sums are added up in registers.
+    static constexpr int CHAINS = BN == 16 ? 4 : 2;
+    static constexpr int COLUMNS = 2 * CHAINS * BN;             // of tensor memory: two chunks' accumulators
 };
 
 // ``part`` (null with one segment): the segments' sums, [segments][M][N].
@@ -260,12 +263,12 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
             tc_fence_after();
             constexpr unsigned idesc = instr_desc(BN);
             constexpr int PW[6] = {2, 1, 0, 1, 0, 0}, PX[6] = {0, 1, 2, 0, 1, 0};
-            const unsigned w = base + s * S::STAGE, x = w + 3 * S::W_PART, acc = tmem + buf * BN;
+            const unsigned w = base + s * S::STAGE, x = w + 3 * S::W_PART, acc = tmem + buf * S::CHAINS * BN;
 #pragma unroll
             for (int p = 0; p < 6; ++p) {
                 const unsigned long long wd = smem_desc(w + PW[p] * S::W_PART), xd = smem_desc(x + PX[p] * S::X_PART);
 #pragma unroll
-                for (int k = 0; k < CHUNK / 16; ++k) umma(acc, wd + 2 * k, xd + 2 * k, idesc, (p > 0 || k > 0) ? 1u : 0u);
+                for (int k = 0; k < CHUNK / 16; ++k) umma(acc + k % S::CHAINS * BN, wd + 2 * k, xd + 2 * k, idesc, (p > 0 || k >= S::CHAINS) ? 1u : 0u);
             }
             umma_commit(&empty_bar[s]);
             umma_commit(&acc_full[buf]);
@@ -288,16 +291,23 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
                 __syncwarp();
                 if (!mbar_wait(&acc_full[buf], (i >> 1) & 1)) { give_up = 1; ok = false; break; }
                 tc_fence_after();
-                const unsigned from = tmem + buf * BN + col0 + ((unsigned)(quarter * 32) << 16);
-                constexpr int AT_ONCE = COLS >= 32 ? 32 : COLS;
+                const unsigned from = tmem + buf * S::CHAINS * BN + col0 + ((unsigned)(quarter * 32) << 16);
+                constexpr int AT_ONCE = COLS >= 16 ? 16 : COLS;
 #pragma unroll
                 for (int j = 0; j < COLS; j += AT_ONCE) {
-                    unsigned r[AT_ONCE];
+                    unsigned r[S::CHAINS][AT_ONCE];
 #pragma unroll
-                    for (int e = 0; e < AT_ONCE; e += 8) tmem_load8(from + j + e, r + e);
+                    for (int h = 0; h < S::CHAINS; ++h)
+#pragma unroll
+                        for (int e = 0; e < AT_ONCE; e += 8) tmem_load8(from + h * BN + j + e, r[h] + e);
                     asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
-                    for (int e = 0; e < AT_ONCE; ++e) sum[j + e] += __uint_as_float(r[e]);
+                    for (int e = 0; e < AT_ONCE; ++e) {
+                        float v = __uint_as_float(r[0][e]);
+#pragma unroll
+                        for (int h = 1; h < S::CHAINS; ++h) v += __uint_as_float(r[h][e]);
+                        sum[j + e] += v;
+                    }
                 }
                 tc_fence_before();
                 __syncwarp();

@@ -237,7 +237,11 @@ __global__ void stream_rmsnorm_vec_kernel(float* __restrict__ x, int S, int T_to
             bb[it] = (in && y) ? Quad<float>::load(gate_bias + j) : zero;
             ww[it] = in ? Quad<float>::load(weight + j) : zero;
             mm[it] = (in && shifted) ? Quad<float>::load(shift_mu + j) : zero;
-            kk[it] = (in && mine) ? Quad<float>::load(mine + j) : zero;
+        }
+#pragma unroll
+        for (int it = 0; it < N; ++it) {             // last: where they lie is itself on its way
+            const int j = (it * blockDim.x + threadIdx.x) * 4;
+            kk[it] = (j < H && mine) ? Quad<float>::load(mine + j) : zero;
         }
         __syncthreads();                             // the mixing weights are in shared memory
 #pragma unroll
