@@ -34,8 +34,8 @@ using namespace fe;
 namespace {
 
 constexpr int WARPS = 8;
-constexpr int KSTEP = 32;       // k elements of a step (2 MMAs)
-constexpr int LARGE_RING = 13824, SMALL_RING = 10240, MAX_DEPTH = 8;        // bytes (and units) of a warp's ring
+constexpr int KSTEP = 32;       // k elements of a step (2 MMAs); the stream brings two steps at a time: 128 bytes of a row
+constexpr int LARGE_RING = 13312, SMALL_RING = 10240, MAX_DEPTH = 8;        // bytes (and units) of a warp's ring
 
 enum { EPI_BF16 = 0, EPI_F32 = 1, EPI_SWIGLU = 2, EPI_QKV = 3, EPI_RESID = 4, EPI_GEGLU = 5, EPI_RELU2 = 6, EPI_REGLU = 7, EPI_GELU = 8 };   // 5: gated, the tanh form of GELU
 constexpr int ACT_RELU2 = 3;            // ``gate_act`` of the bfloat16 epilogue: the square of relu(product), no gate (entry code 6)
@@ -114,13 +114,14 @@ __device__ __forceinline__ int red_at(int row, int col) {
 
 constexpr int RED_FLOATS = 4 * 128;      // accumulator tiles a warp leaves at a time x their floats
 
-// How a launch cuts the matrix: ``items`` (rows, or pairs of rows) over the blocks, a block's in groups of at most ``rows`` of them; a
-// unit of the stream is ``rows`` items x KB steps of k, ``plane`` bytes a step, ``slot`` bytes in all, ``depth`` units a warp's ring.
+// How a launch cuts the matrix: ``items`` (rows, or pairs of rows) over the blocks, a block's (or a warp's) in groups of at most ``rows`` of
+// them; a unit of the stream is ``rows`` items x KB steps of k, ``plane`` bytes two steps, ``slot`` bytes in all, ``depth`` units a warp's ring.
+// Rows of 128 bytes, since the copy engine takes about as long for a row of 64 (271 MB: 54 us), swizzled.
 struct Cut {
     int items, rows, plane, slot, depth, ring;
 };
 
-// TILES: the 16-row tiles a group has at most (1, 2 or 4); KB = 4 / TILES steps of k are one unit, so that a unit is always four
+// TILES: the 16-row tiles a group has at most (1 or 2); KB = 4 / TILES steps of k are one unit, so that a unit is always four
 // (tile, step) pairs: eight 16-byte reads and eight multiplications that wait for one another in pairs at most.
 // ONE: a single row of x.  WIDE: a block has so many items that every warp takes an eighth of them over all of K, adds nothing up with
 // the others and meets them at no barrier; else the warps share K.
@@ -131,7 +132,7 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap map, const bf16* __restri
     constexpr bool PAIRS = EPI == EPI_SWIGLU || EPI == EPI_QKV;
     constexpr int ITEMS = PAIRS ? 8 : 16;         // items a tile takes: pairs of rows, or rows
     constexpr int KB = 4 / TILES, AHEAD = 8 / KB;           // AHEAD: units whose rows of x are on their way
-    extern __shared__ __align__(128) unsigned char shared[];
+    extern __shared__ __align__(1024) unsigned char shared[];
     __shared__ __align__(8) unsigned long long bars[WARPS][MAX_DEPTH];
     __shared__ float scale_part[WARPS][8];
     __shared__ float square_part[TILES][8];
@@ -158,17 +159,17 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap map, const bf16* __restri
     auto issue = [&](int slot) {                  // lane 0
         if (at_item >= item1) return;
         const unsigned bar = bar0 + 8 * slot, dst = ring + slot * cut.slot;
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(cut.plane * KB) : "memory");
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(cut.plane * (KB / 2)) : "memory");
         if constexpr (EPI == EPI_SWIGLU) {
             asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];\n"
-                         ::"r"(dst), "l"(&map), "r"(bar), "r"(0), "r"(at_item), "r"(0), "r"(at_u * KB) : "memory");
+                         ::"r"(dst), "l"(&map), "r"(bar), "r"(0), "r"(at_item), "r"(0), "r"(at_u * (KB / 2)) : "memory");
         } else if constexpr (EPI == EPI_QKV) {
             const int half = qkv.d >> 1, head = at_item / half;
             asm volatile("cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];\n"
-                         ::"r"(dst), "l"(&map), "r"(bar), "r"(0), "r"(at_item - head * half), "r"(0), "r"(head), "r"(at_u * KB) : "memory");
+                         ::"r"(dst), "l"(&map), "r"(bar), "r"(0), "r"(at_item - head * half), "r"(0), "r"(head), "r"(at_u * (KB / 2)) : "memory");
         } else {
             asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n"
-                         ::"r"(dst), "l"(&map), "r"(bar), "r"(0), "r"(at_item), "r"(at_u * KB) : "memory");
+                         ::"r"(dst), "l"(&map), "r"(bar), "r"(0), "r"(at_item), "r"(at_u * (KB / 2)) : "memory");
         }
         if (++at_u == u_end) {
             at_u = u_begin;
@@ -228,7 +229,6 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap map, const bf16* __restri
     int slot = 0;
     unsigned parity = 0;
     bool dead = false;                            // a wait has run out: no more waiting, the status word says so
-    const unsigned lane_at = ring + g * 64 + t * 16;          // this lane's 16 bytes of row g of a plane
 
     for (int start = first_item; start < item1; start += group_step) {
         const int end = EPI == EPI_QKV ? start + cut.rows : min(start + cut.rows, item1), n = (end - start + ITEMS - 1) / ITEMS;
@@ -262,15 +262,23 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap map, const bf16* __restri
                     while (!bar_test(bar, parity))
                         if (clock64() - since > WAIT_LIMIT) { dead = true; break; }
                 }
-                const unsigned from = lane_at + slot * cut.slot;
+                const unsigned from = ring + slot * cut.slot;
                 uint4 a0[KB][TILES], a1[KB][TILES];
+                // row ``r`` of a unit: its 16-byte piece c lies at c ^ (r & 7).  Lanes of odd and even rows that read together take the row's two
+                // halves in opposite order, so that they meet on no bank
+                auto two_steps = [&](int r, uint4& first, uint4& second) {
+                    const unsigned at = from + r * 128, odd = r & 1;
+                    const uint4 one = ld_shared16(at + (((t + 4 * odd) ^ (r & 7)) << 4)), two = ld_shared16(at + (((t + 4 - 4 * odd) ^ (r & 7)) << 4));
+                    first = odd ? two : one;
+                    second = odd ? one : two;
+                };
 #pragma unroll
-                for (int kk = 0; kk < KB; ++kk)
+                for (int pl = 0; pl < KB / 2; ++pl)
 #pragma unroll
                     for (int j = 0; j < TILES; ++j) {
-                        const unsigned at = from + kk * cut.plane + j * ITEMS * 64;
-                        a0[kk][j] = ld_shared16(at);
-                        a1[kk][j] = ld_shared16(at + (PAIRS ? cut.plane / 2 : 8 * 64));
+                        const int r = pl * cut.rows * (PAIRS ? 2 : 1) + j * ITEMS + g;
+                        two_steps(r, a0[2 * pl][j], a0[2 * pl + 1][j]);
+                        two_steps(r + (PAIRS ? cut.rows : 8), a1[2 * pl][j], a1[2 * pl + 1][j]);
                     }
 #pragma unroll
                 for (int kk = 0; kk < KB; ++kk) {
@@ -445,7 +453,9 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap map, const bf16* __restri
     if (dead && lane == 0 && status) atomicOr(status, FE_STATUS_WAIT_EXPIRED);
 }
 
-constexpr int shared_bytes(int ring) { return WARPS * (ring + RED_FLOATS * 4); }
+// Both sizes of a launch's shared memory: one block of each fits an SM, two of the larger do not.  Warps that add nothing up with the others
+// have the room for longer rings.
+constexpr int LARGE_BYTES = WARPS * (LARGE_RING + RED_FLOATS * 4), SMALL_BYTES = WARPS * (SMALL_RING + RED_FLOATS * 4);
 
 int blocks_for(int items) { const int sms = fe_sm_count(); return items < sms ? items : sms; }
 
@@ -466,17 +476,17 @@ EncodeTiled encode_fn() {
 
 // Launches a kernel; gives it its shared memory first, once a device.
 template <int NT, int EPI, bool ONE, int TILES, bool WIDE, typename... Args>
-int launch_kernel(int blocks, int ring, cudaStream_t stream, const CUtensorMap& map, Args... args) {
+int launch_kernel(int blocks, int bytes, cudaStream_t stream, const CUtensorMap& map, Args... args) {
     static std::atomic<unsigned long long> allowed{0};
     const auto kernel = skinny_gemm_kernel<NT, EPI, ONE, TILES, WIDE>;
     int device = 0;
     cudaGetDevice(&device);
     if (!(allowed.load() >> (device & 63) & 1)) {
-        const cudaError_t err = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, shared_bytes(LARGE_RING));
+        const cudaError_t err = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LARGE_BYTES);
         FE_REQUIRE(err == cudaSuccess, "skinny_gemm: %s", cudaGetErrorString(err));
         allowed.fetch_or(1ull << (device & 63));
     }
-    fe::launch(kernel, blocks, WARPS * 32, shared_bytes(ring), stream, map, args...);
+    fe::launch(kernel, blocks, WARPS * 32, bytes, stream, map, args...);
     return fe_check_launch("skinny_gemm");
 }
 
@@ -486,7 +496,7 @@ int launch(const void* x, const void* W, void* out, int M, int N, int K, int ite
            int gate_act = 0) {
     constexpr bool PAIRS = EPI == EPI_SWIGLU || EPI == EPI_QKV;
     constexpr int ITEMS = PAIRS ? 8 : 16;
-    const int sms = fe_sm_count(), most = M <= 8 ? 4 : 2;          // tiles a group may have
+    const int sms = fe_sm_count(), most = 2;                       // tiles a group may have
     int blocks, rows;
     bool wide = false;
     if (EPI == EPI_QKV) {
@@ -503,41 +513,40 @@ int launch(const void* x, const void* W, void* out, int M, int N, int K, int ite
         const int own = wide ? (block_own + WARPS - 1) / WARPS : block_own, groups = (own + ITEMS * most - 1) / (ITEMS * most);
         rows = (own + groups - 1) / groups;
     }
-    const int tiles = (rows + ITEMS - 1) / ITEMS, T = tiles == 1 ? 1 : tiles == 2 ? 2 : 4, KB = 4 / T;
-    const int plane = rows * (PAIRS ? 2 : 1) * KSTEP * 2, slot = (plane * KB + 127) / 128 * 128;
-    const int ring = scale.beside ? SMALL_RING : LARGE_RING, depth = ring / slot < MAX_DEPTH ? ring / slot : MAX_DEPTH;
+    const int tiles = (rows + ITEMS - 1) / ITEMS, T = tiles, KB = 4 / T;
+    const int plane = rows * (PAIRS ? 2 : 1) * 128, slot = (plane * (KB / 2) + 1023) / 1024 * 1024;
+    const int ring = (scale.beside ? SMALL_RING : LARGE_RING) + (wide ? RED_FLOATS * 4 : 0), depth = ring / slot < MAX_DEPTH ? ring / slot : MAX_DEPTH;
     const Cut cut{items, rows, plane, slot, depth, ring};
     EncodeTiled encode = encode_fn();
     FE_REQUIRE(encode != nullptr, "skinny_gemm: cuTensorMapEncodeTiled is not available from this driver");
     CUtensorMap map;
-    const cuuint64_t row = (cuuint64_t)K * 2, ks = (cuuint64_t)K / KSTEP;
+    const cuuint64_t row = (cuuint64_t)K * 2, ks = (cuuint64_t)K / 64;
     const cuuint32_t ones[5] = {1, 1, 1, 1, 1};
     auto make = [&](int rank, const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box) {
         return encode(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<void*>(W), dims, strides, box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                      CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                      CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     };
     CUresult rc;
     if constexpr (EPI == EPI_SWIGLU) {
-        const cuuint64_t dims[4] = {KSTEP, (cuuint64_t)items, 2, ks}, strides[3] = {row, row * items, KSTEP * 2};
-        const cuuint32_t box[4] = {KSTEP, (cuuint32_t)rows, 2, (cuuint32_t)KB};
+        const cuuint64_t dims[4] = {64, (cuuint64_t)items, 2, ks}, strides[3] = {row, row * items, 128};
+        const cuuint32_t box[4] = {64, (cuuint32_t)rows, 2, (cuuint32_t)KB / 2};
         rc = make(4, dims, strides, box);
     } else if constexpr (EPI == EPI_QKV) {
-        const cuuint64_t half = qkv.d / 2, dims[5] = {KSTEP, half, 2, (cuuint64_t)items / half, ks}, strides[4] = {row, row * half, row * 2 * half, KSTEP * 2};
-        const cuuint32_t box[5] = {KSTEP, (cuuint32_t)rows, 2, 1, (cuuint32_t)KB};
+        const cuuint64_t half = qkv.d / 2, dims[5] = {64, half, 2, (cuuint64_t)items / half, ks}, strides[4] = {row, row * half, row * 2 * half, 128};
+        const cuuint32_t box[5] = {64, (cuuint32_t)rows, 2, 1, (cuuint32_t)KB / 2};
         rc = make(5, dims, strides, box);
     } else {
-        const cuuint64_t dims[3] = {KSTEP, (cuuint64_t)N, ks}, strides[2] = {row, KSTEP * 2};
-        const cuuint32_t box[3] = {KSTEP, (cuuint32_t)rows, (cuuint32_t)KB};
+        const cuuint64_t dims[3] = {64, (cuuint64_t)N, ks}, strides[2] = {row, 128};
+        const cuuint32_t box[3] = {64, (cuuint32_t)rows, (cuuint32_t)KB / 2};
         rc = make(3, dims, strides, box);
     }
     FE_REQUIRE(rc == CUDA_SUCCESS, "skinny_gemm: cuTensorMapEncodeTiled failed with code %d", (int)rc);
 #define FE_SKINNY(NT, ONE, TILES, WIDE) \
-    return launch_kernel<NT, EPI, ONE, TILES, WIDE>(blocks, ring, stream, map, (const bf16*)x, out, M, N, K, cut, qkv, resid, scale, gate_act, status)
+    return launch_kernel<NT, EPI, ONE, TILES, WIDE>(blocks, scale.beside ? SMALL_BYTES : LARGE_BYTES, stream, map, (const bf16*)x, out, M, N, K, cut, qkv, resid, scale, gate_act, status)
 #define FE_SKINNY_TILES(NT, ONE, WIDE) \
     do { \
         if (T == 1) FE_SKINNY(NT, ONE, 1, WIDE); \
-        if (T == 2) FE_SKINNY(NT, ONE, 2, WIDE); \
-        if constexpr (NT == 1) FE_SKINNY(NT, ONE, 4, WIDE); \
+        FE_SKINNY(NT, ONE, 2, WIDE); \
     } while (0)
     if constexpr (EPI != EPI_RESID && EPI != EPI_QKV) {
         if (wide && M == 1) FE_SKINNY_TILES(1, true, true);

@@ -5,14 +5,15 @@
 // a2; a0 the upper half of the word, a1 the upper half of what is left, a2 the rest).  Products of two such parts are exact in float32, so
 // a.w is the sum of nine products that tcgen05.mma forms exactly; the three smallest (a1 w2, a2 w1, a2 w2: below 2^-22 of a.w together) are
 // left out.  What remains is how sums are rounded.  The tensor cores round their running sum towards zero, so it is kept short: a chunk of 64
-// k's starts from zero, adds its small products first and is then added to a float32 sum in registers, rounded to nearest.
+// k's starts from zero, in one sum for the largest products and two for the smaller ones, and is then added to a float32 sum in
+// registers, rounded to nearest.
 //
 // Every output is formed in the same steps whatever the batch: the chunks of a segment of K in order, then the segments in
-// order, their number chosen by N and K alone.  Rows of W are the 128 rows of the MMA tile, rows of A its columns (16, 64 or 128 by
+// order, their number chosen by N and K alone.  Rows of W are the 128 rows of the MMA tile, rows of A its columns (16 or 64 by
 // M), so that a handful of rows streams W once.
 //
 // Blocks stay for tile after tile.  Warps 0..7 read float32 rows (two chunks of loads in flight: half of a thread's registers hold one
-// while the other is cut up), write the three parts into 128-byte-swizzled tiles; one thread of warp 8 issues 24 MMAs a chunk into one of
+// while the other is cut up), write the three parts into 128-byte-swizzled tiles; one thread of warp 8 issues 12 MMAs a chunk into one of
 // two accumulators in tensor memory; warps 8..15 add the other to their registers and write the tile out at the end.  A
 // result that is no finite number is formed again as a chain of multiply-adds (an infinity has no three parts).
 #include "common.cuh"
@@ -90,14 +91,11 @@ __device__ __forceinline__ void split8(const float4& p, const float4& q, uint4& 
 }
 
 template <int BN> struct Sizes {
-    static constexpr int STAGES = 2;
+    static constexpr int STAGES = BN == 16 ? 3 : 2;
     static constexpr int W_PART = TILE_W * CHUNK * 2, X_PART = BN * CHUNK * 2;
     static constexpr int STAGE = 3 * (W_PART + X_PART);
     static constexpr int BYTES = STAGES * STAGE + 1024;
-    // An MMA that adds to the accumulator of the one before it waits for that: CHAINS accumulators take turns (every fourth or every
-    // second step of a chunk's four), and the sums are added up in registers.
-    static constexpr int CHAINS = BN == 16 ? 4 : 2;
-    static constexpr int COLUMNS = 2 * CHAINS * BN;             // of tensor memory: two chunks' accumulators
+    static constexpr int COLUMNS = BN == 16 ? 128 : 512;        // of tensor memory: two chunks' accumulators, 3 BN columns each
 };
 
 // ``part`` (null with one segment): the segments' sums, [segments][M][N].
@@ -248,9 +246,9 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
         }
     } else {
         // ---- sums: warp w reads TMEM lanes 32 (w % 4) .. + 31 (rows of W), one half of the columns (rows of A) ----
-        constexpr int COLS = BN / 2;
+        constexpr int COLS = BN / 2;                              // 8 or 32
         const int quarter = warp & 3, col0 = ((warp - SPLIT_WARPS) >> 2) * COLS;
-        // one thread issues the MMAs, a chunk ahead of the one it adds up: the smallest products of a chunk first
+        // one thread issues the MMAs, a chunk ahead of the one it adds up
         int it = blockIdx.x, ic = 0, ic1 = 0, issued = 0;
         auto issue = [&]() {
             if (it >= tiles || give_up) return;
@@ -261,15 +259,14 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
             const int s = issued % S::STAGES, buf = issued & 1;
             if (!mbar_wait(&full_bar[s], (issued / S::STAGES) & 1) || !mbar_wait(&acc_empty[buf], ((issued >> 1) & 1) ^ 1)) { give_up = 1; return; }
             tc_fence_after();
-            constexpr unsigned idesc = instr_desc(BN);
-            constexpr int PW[6] = {2, 1, 0, 1, 0, 0}, PX[6] = {0, 1, 2, 0, 1, 0};
-            const unsigned w = base + s * S::STAGE, x = w + 3 * S::W_PART, acc = tmem + buf * S::CHAINS * BN;
+            const unsigned w = base + s * S::STAGE, x = w + 3 * S::W_PART, acc = tmem + buf * 3 * BN;
+            // The parts of A's rows lie one after the other like 3 BN rows: a part of W meets as many of them as count at once.  Column
+            // block 0 of the accumulator takes w0 a0, block 1 w0 a1 + w1 a0, block 2 w0 a2 + w1 a1 + w2 a0.
 #pragma unroll
-            for (int p = 0; p < 6; ++p) {
-                const unsigned long long wd = smem_desc(w + PW[p] * S::W_PART), xd = smem_desc(x + PX[p] * S::X_PART);
+            for (int k = 0; k < CHUNK / 16; ++k)
 #pragma unroll
-                for (int k = 0; k < CHUNK / 16; ++k) umma(acc + k % S::CHAINS * BN, wd + 2 * k, xd + 2 * k, idesc, (p > 0 || k >= S::CHAINS) ? 1u : 0u);
-            }
+                for (int p = 0; p < 3; ++p)
+                    umma(acc + p * BN, smem_desc(w + p * S::W_PART) + 2 * k, smem_desc(x) + 2 * k, instr_desc((3 - p) * BN), (p > 0 || k > 0) ? 1u : 0u);
             umma_commit(&empty_bar[s]);
             umma_commit(&acc_full[buf]);
             ++issued;
@@ -291,23 +288,15 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
                 __syncwarp();
                 if (!mbar_wait(&acc_full[buf], (i >> 1) & 1)) { give_up = 1; ok = false; break; }
                 tc_fence_after();
-                const unsigned from = tmem + buf * S::CHAINS * BN + col0 + ((unsigned)(quarter * 32) << 16);
-                constexpr int AT_ONCE = COLS >= 16 ? 16 : COLS;
+                const unsigned from = tmem + buf * 3 * BN + col0 + ((unsigned)(quarter * 32) << 16);
 #pragma unroll
-                for (int j = 0; j < COLS; j += AT_ONCE) {
-                    unsigned r[S::CHAINS][AT_ONCE];
+                for (int j = 0; j < COLS; j += 8) {
+                    unsigned r[3][8];
 #pragma unroll
-                    for (int h = 0; h < S::CHAINS; ++h)
-#pragma unroll
-                        for (int e = 0; e < AT_ONCE; e += 8) tmem_load8(from + h * BN + j + e, r[h] + e);
+                    for (int h = 0; h < 3; ++h) tmem_load8(from + h * BN + j, r[h]);
                     asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
-                    for (int e = 0; e < AT_ONCE; ++e) {
-                        float v = __uint_as_float(r[0][e]);
-#pragma unroll
-                        for (int h = 1; h < S::CHAINS; ++h) v += __uint_as_float(r[h][e]);
-                        sum[j + e] += v;
-                    }
+                    for (int e = 0; e < 8; ++e) sum[j + e] += __uint_as_float(r[0][e]) + (__uint_as_float(r[1][e]) + __uint_as_float(r[2][e]));
                 }
                 tc_fence_before();
                 __syncwarp();
@@ -401,8 +390,7 @@ extern "C" int fe_gemm_split(const float* A, const float* W, const float* bias, 
 #define FE_SPLIT(BN) rc = vec ? launch_split<BN, true>(A, W, bias, C, part, M, N, K, segments, status, stream) \
                               : launch_split<BN, false>(A, W, bias, C, part, M, N, K, segments, status, stream)
     if (M <= 16) FE_SPLIT(16);
-    else if (M <= 64) FE_SPLIT(64);
-    else FE_SPLIT(128);
+    else FE_SPLIT(64);
 #undef FE_SPLIT
     if (rc || segments == 1) return rc;
     const long long total = (long long)M * N;
