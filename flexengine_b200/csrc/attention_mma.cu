@@ -26,7 +26,6 @@
 // prefill: four warps per (tile of 64 rows, key/value head, request); the warps share the
 //          key/value stages.
 #include <math_constants.h>
-#include <cstdlib>
 
 #define FE_PDL_CLASS 2      // FE_PDL_DECODE_ATTENTION
 #include "common.cuh"
@@ -818,7 +817,6 @@ extern "C" int fe_paged_decode_cluster_resident(int requests, int nq, int nkv, i
             return 0;                                                                                                  \
         }                                                                                                              \
         cfg.dynamicSmemBytes = decode_smem<DMAX>(STAGES);                                                              \
-        if (getenv("FE_ATT")) cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100);                                                  \
         if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess) {                                  \
             cudaGetLastError();                                                                                        \
             return 0;                                                                                                  \

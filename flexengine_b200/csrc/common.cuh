@@ -145,7 +145,7 @@ template <int TILE> __host__ __device__ __forceinline__ int listed_tile(int i, i
 // kernel boundary costs about 2 us of idle memory, 5 of them a layer in a decode step.  Weight-streaming products and
 // elementwise kernels with it against without (B200): 32 steps of one request on the 1.5B shape 40.4 -> 34.1 ms, 16 steps of 8
 // requests on the 7B shape 26.8 -> 25.9 ms, the hybrid designs 7 to 14 %; all kernels launched through fe::launch share one split of
-// an SM's memory (fe_shared_split says why; the cluster form of decode attention, which begins early in small steps, keeps
+// an SM's memory (fe_share_carveout says why; the cluster form of decode attention, which begins early in small steps, keeps
 // its own).  Decode attention, the scans and the rest gain nothing or lose (7B: 25.2 -> 26.5 ms on one box with the attention
 // clusters, whose successor then takes the place of late clusters).
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -167,7 +167,7 @@ __device__ __forceinline__ void prefetch_l2_share(const void* base, long long by
 void fe_set_error(const char* fmt, ...);
 int fe_check_launch(const char* what);
 int fe_pdl_enabled();
-int fe_shared_split(long long blocks);       // the split of an SM's memory that overlapping kernels of so many blocks share, in percent
+void fe_share_carveout(const void* kernel);       // the split of an SM's memory that overlapping kernels share
 int fe_sm_count();      // multiprocessors of the current device (asked once per device)
 
 // Classes of kernels for fe_set_pdl: a source file names its own before including this header.
@@ -189,13 +189,12 @@ inline void launch_as(int classes, void (*kernel)(KArgs...), dim3 grid, dim3 blo
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
+    cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = (fe_pdl_enabled() & classes) != 0;
-    attr[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
-    attr[1].val.sharedMemCarveout = fe_shared_split((long long)grid.x * grid.y * grid.z);
     cfg.attrs = attr;
-    cfg.numAttrs = attr[0].val.programmaticStreamSerializationAllowed ? 2 : 1;
+    cfg.numAttrs = 1;
+    if (attr[0].val.programmaticStreamSerializationAllowed) fe_share_carveout((const void*)kernel);
     cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);       // errors surface in fe_check_launch
 }
 template <typename... KArgs, typename... Args>

@@ -11,8 +11,6 @@ norm weights, biases and logits are float32; index tensors are int32.
 """
 from __future__ import annotations
 
-import threading
-
 import torch
 
 from . import library
@@ -323,11 +321,10 @@ def linear(x, w, bias=None, out_float32=False, follow=None, upcoming=None):
                 and norm_weight.dtype == torch.float32 and norm_weight.numel() == N):
             scaled = torch.empty((M, N), dtype=torch.bfloat16, device=rows.device)
             _rows, sumsq, tiles, eps = _rows_and_scale(x)
-            parts = min(N, sm_count(rows.device)) if rows.is_cuda else 1       # blocks of the kernel, each of which leaves its sums
-            table = torch.empty((parts, 8), dtype=torch.float32, device=rows.device)
+            table = torch.empty((-(-N // 16), 8), dtype=torch.float32, device=rows.device)
             _run(_bf16(), "fe_skinny_gemm_residual", _ptr(rows), _ptr(w), _ptr(residual), _ptr(norm_weight), _ptr(scaled),
                  _ptr(table), _c_int(M), _c_int(N), _c_int(rows.shape[1]), sumsq, tiles, eps,
-                 *_upcoming(upcoming, M, UPCOMING_TAIL_BYTES), _ptr(status_word(rows.device)), _beside(), _held(w), _stream())
+                 *_upcoming(upcoming, M, UPCOMING_TAIL_BYTES), _held(w), _stream())
             return Prenormed(scaled, table, norm_eps, residual, norm_weight)
     if kernel and w.dtype == torch.bfloat16:
         wide = out_float32 or bias is not None           # a bias is added in float32, before the one rounding
@@ -374,19 +371,6 @@ def _held(w):
     return _c_int(1 if getattr(w, "held", False) else 0)
 
 
-_ring = threading.local()
-
-
-def _beside():
-    """Whether the weight-streaming product about to be launched may take the smaller of its two sizes of shared memory: it does when this thread's
-    last launch on the stream was one of the larger size (see csrc/gemm_skinny.cu).  A wrong answer costs time only."""
-    stream = _stream()
-    last = getattr(_ring, "last", None)
-    small = last == (stream, launches)
-    _ring.last = None if small else (stream, launches + 1)
-    return _c_int(1 if small else 0)
-
-
 def skinny_gemm(x, w, epilogue: int = EPI_BF16, upcoming=None):
     """x [M <= 16, K] (a tensor or a Prenormed) times w [N, K]^T by streaming w once; see csrc/gemm_skinny.cu."""
     x, sumsq, tiles, eps = _rows_and_scale(x)
@@ -397,7 +381,7 @@ def skinny_gemm(x, w, epilogue: int = EPI_BF16, upcoming=None):
     else:
         out = torch.empty((M, N), dtype=torch.float32 if epilogue == EPI_F32 else torch.bfloat16, device=x.device)
     _run(_bf16(), "fe_skinny_gemm_scaled", _ptr(x), _ptr(w), _ptr(out), _c_int(M), _c_int(N), _c_int(K), _c_int(epilogue),
-         sumsq, tiles, eps, *_upcoming(upcoming, M, UPCOMING_TAIL_BYTES), _ptr(status_word(x.device)), _beside(), _held(w), _stream())
+         sumsq, tiles, eps, *_upcoming(upcoming, M, UPCOMING_TAIL_BYTES), _held(w), _stream())
     return out
 
 
@@ -548,7 +532,7 @@ def qkv_projection(h, w, bias, positions, inv_freq, rot, slot_mapping, k_cache, 
         _run(_bf16(), "fe_skinny_qkv", _ptr(rows), _ptr(w), _ptr(out), _ptr(bias), _ptr(positions), _ptr(inv_freq),
              _ptr(slot_mapping), _ptr(k_cache), _ptr(v_cache), _c_int(T), _c_int(rows.shape[1]), _c_int(nq), _c_int(nkv),
              _c_int(d), _c_int(page_size), _c_ll(k_cache.shape[0] * page_size), sumsq, tiles, eps,
-             _ptr(status_word(rows.device)), _beside(), _held(w), _stream())
+             _ptr(status_word(rows.device)), _held(w), _stream())
         return out
     if isinstance(h, Prenormed):
         h = h.materialize()
