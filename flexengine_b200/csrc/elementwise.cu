@@ -172,66 +172,6 @@ __global__ void add_rmsnorm_vec_kernel(float* __restrict__ residual, const TD* _
     }
 }
 
-// The same for rows of up to 16,384 elements: a row lies in the registers of a block whose size follows from H alone (four times
-// four elements a thread), so that everything a row reads, the weight among it, is asked for at once and no pass goes through
-// shared memory.  What bounds it is a row's one trip to memory and the sum over the block.
-constexpr int ROW_PIECES = 4;
-template <typename T, typename TD>
-__global__ void __launch_bounds__(1024)
-add_rmsnorm_row_kernel(float* __restrict__ residual, const TD* __restrict__ delta, const float* __restrict__ delta_scale,
-                       const float* __restrict__ weight, float eps, T* __restrict__ out, const int* __restrict__ rows, int H,
-                       int n_rows_total, int n_out, const void* __restrict__ upcoming, long long upcoming_bytes) {
-    if ((int)blockIdx.x >= n_out) {         // blocks beyond the rows: start the next kernel's weights into L2
-        prefetch_l2_share(upcoming, upcoming_bytes, (long long)(blockIdx.x - n_out) * blockDim.x + threadIdx.x,
-                          (long long)(gridDim.x - n_out) * blockDim.x);
-        return;
-    }
-    griddep_wait();
-    griddep_launch_dependents();
-    __shared__ float scratch[33];
-    const int i = blockIdx.x;
-    int r = rows ? rows[i] : i;
-    if (r < 0 || r >= n_rows_total) r = 0;
-    float* res = residual + (size_t)r * H;
-    const TD* del = delta ? delta + (size_t)r * H : nullptr;
-    float4 v[ROW_PIECES], w[ROW_PIECES], dv[ROW_PIECES];
-#pragma unroll
-    for (int p = 0; p < ROW_PIECES; ++p) {
-        const int j = (threadIdx.x + p * blockDim.x) * 4;
-        if (j >= H) continue;
-        v[p] = *reinterpret_cast<const float4*>(res + j);
-        if (del) dv[p] = Vec4<TD>::load(del + j);
-    }
-#pragma unroll
-    for (int p = 0; p < ROW_PIECES; ++p) {
-        const int j = (threadIdx.x + p * blockDim.x) * 4;
-        if (j < H) w[p] = *reinterpret_cast<const float4*>(weight + j);
-    }
-    float ss = 0.f;
-#pragma unroll
-    for (int p = 0; p < ROW_PIECES; ++p) {
-        const int j = (threadIdx.x + p * blockDim.x) * 4;
-        if (j >= H) continue;
-        if (del) {
-            float4 d = dv[p];
-            if (delta_scale) {
-                const float4 s = *reinterpret_cast<const float4*>(delta_scale + j);
-                d.x *= s.x; d.y *= s.y; d.z *= s.z; d.w *= s.w;
-            }
-            v[p].x += d.x; v[p].y += d.y; v[p].z += d.z; v[p].w += d.w;
-            if (!rows) *reinterpret_cast<float4*>(res + j) = v[p];
-        }
-        ss += v[p].x * v[p].x + v[p].y * v[p].y + v[p].z * v[p].z + v[p].w * v[p].w;
-    }
-    const float inv = rsqrtf(block_sum(ss, scratch) / (float)H + eps);
-    T* o = out + (size_t)i * H;
-#pragma unroll
-    for (int p = 0; p < ROW_PIECES; ++p) {
-        const int j = (threadIdx.x + p * blockDim.x) * 4;
-        if (j < H) Vec4<T>::store(o + j, make_float4(v[p].x * inv * w[p].x, v[p].y * inv * w[p].y, v[p].z * inv * w[p].z, v[p].w * inv * w[p].w));
-    }
-}
-
 constexpr int PREFETCH_BLOCKS = 64;
 
 template <typename T, typename TD>
@@ -243,11 +183,7 @@ static int launch_add_rmsnorm(float* residual, const void* delta, const float* d
     const bool vec = H % 4 == 0;
     const int threads = H >= 4096 ? 512 : (H >= 1024 ? 256 : 128);
     cudaError_t err = cudaSuccess;
-    const int row_threads = (H / 4 + 32 * ROW_PIECES - 1) / (32 * ROW_PIECES) * 32;
-    if (vec && row_threads <= 1024) {
-        fe::launch_as(overlap_class(n_out), add_rmsnorm_row_kernel<T, TD>, grid, row_threads, 0, stream, residual, (const TD*)delta, delta_scale, weight, eps, (T*)out,
-                   rows, H, n_rows_total, n_out, upcoming, upcoming_bytes);
-    } else if (vec) {
+    if (vec) {
         if (smem > 48 * 1024)
             err = cudaFuncSetAttribute(add_rmsnorm_vec_kernel<T, TD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         FE_REQUIRE(err == cudaSuccess, "add_rmsnorm: %s", cudaGetErrorString(err));

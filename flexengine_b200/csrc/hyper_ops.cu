@@ -215,16 +215,8 @@ __global__ void stream_rmsnorm_vec_kernel(float* __restrict__ x, int S, int T_to
         *reinterpret_cast<float4*>(u_row + j) = u;
         ss += u.x * u.x + u.y * u.y + u.z * u.z + u.w * u.w;
     };
-    // ``shifted``: row i is request i's one token of the step; the token shift of the normed row is done here as well (on the
-    // row as it was rounded, so that the kept row is what a later step reads of it)
-    float* mine = nullptr;
-    if (shifted) {
-        const int seat = seats[i];
-        if (seat >= 0 && seat < n_seats) mine = kept + (size_t)seat * kept_stride;
-    }
-    constexpr int N = ITERS > 0 ? ITERS : 1;
-    float4 ww[N], mm[N], kk[N];                      // what the end needs, asked for with the rest where a row takes so few rounds
     if (ITERS > 0) {
+        constexpr int N = ITERS > 0 ? ITERS : 1;
         float4 v[N][SMAX], yy[N], gg[N], bb[N];
 #pragma unroll
         for (int it = 0; it < N; ++it) {
@@ -235,13 +227,6 @@ __global__ void stream_rmsnorm_vec_kernel(float* __restrict__ x, int S, int T_to
             yy[it] = (in && y) ? Quad<T>::load(y + (size_t)r * H + j) : zero;
             gg[it] = (in && y) ? Quad<T>::load(gate + (size_t)r * H + j) : zero;
             bb[it] = (in && y) ? Quad<float>::load(gate_bias + j) : zero;
-            ww[it] = in ? Quad<float>::load(weight + j) : zero;
-            mm[it] = (in && shifted) ? Quad<float>::load(shift_mu + j) : zero;
-        }
-#pragma unroll
-        for (int it = 0; it < N; ++it) {             // last: where they lie is itself on its way
-            const int j = (it * blockDim.x + threadIdx.x) * 4;
-            kk[it] = (j < H && mine) ? Quad<float>::load(mine + j) : zero;
         }
         __syncthreads();                             // the mixing weights are in shared memory
 #pragma unroll
@@ -262,26 +247,24 @@ __global__ void stream_rmsnorm_vec_kernel(float* __restrict__ x, int S, int T_to
     const float total = block_sum(ss, scratch);
     const float inv = rsqrtf(total / (float)H + eps);
     T* o = out + (size_t)i * H;
-    auto finish = [&](int j, const float4& w, const float4& m, const float4& before) {
-        const float4 u = *reinterpret_cast<const float4*>(u_row + j);
+    // ``shifted``: row i is request i's one token of the step; the token shift of the normed row is done here as well (on the
+    // row as it was rounded, so that the kept row is what a later step reads of it)
+    float* mine = nullptr;
+    if (shifted) {
+        const int seat = seats[i];
+        if (seat >= 0 && seat < n_seats) mine = kept + (size_t)seat * kept_stride;
+    }
+    for (int j = threadIdx.x * 4; j < H; j += blockDim.x * 4) {
+        const float4 u = *reinterpret_cast<const float4*>(u_row + j), w = Quad<float>::load(weight + j);
         Quad<T>::store(o + j, make_float4(u.x * inv * w.x, u.y * inv * w.y, u.z * inv * w.z, u.w * inv * w.w));
         if (shifted) {
-            const float4 x = Quad<T>::load(o + j);
+            const float4 x = Quad<T>::load(o + j), m = Quad<float>::load(shift_mu + j);
+            const float4 before = mine ? Quad<float>::load(mine + j) : make_float4(0.f, 0.f, 0.f, 0.f);
             Quad<T>::store(shifted + (size_t)i * H + j, make_float4(fmaf(before.x - x.x, m.x, x.x), fmaf(before.y - x.y, m.y, x.y),
                                                                       fmaf(before.z - x.z, m.z, x.z), fmaf(before.w - x.w, m.w, x.w)));
             if (mine) Quad<float>::store(mine + j, x);
         }
-    };
-    if (ITERS > 0) {
-#pragma unroll
-        for (int it = 0; it < N; ++it) {
-            const int j = (it * blockDim.x + threadIdx.x) * 4;
-            if (j < H) finish(j, ww[it], mm[it], kk[it]);
-        }
-        return;
     }
-    for (int j = threadIdx.x * 4; j < H; j += blockDim.x * 4)
-        finish(j, Quad<float>::load(weight + j), shifted ? Quad<float>::load(shift_mu + j) : zero, mine ? Quad<float>::load(mine + j) : zero);
 }
 
 template <typename T>

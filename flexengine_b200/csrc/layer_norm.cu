@@ -103,22 +103,6 @@ __global__ void layer_norm_kernel(float* __restrict__ residual, const TD* __rest
             for (int e = 0; e < V; ++e) ys[n][e] += y_bias[j + e];
         }
     }
-    // the weights too, in rows of up to two pieces a thread: behind the sums over the block each would be a trip of its own
-    constexpr bool EARLY = N <= 2;
-    float pw[EARLY ? N : 1][V], pb[EARLY ? N : 1][V], wv[EARLY ? N : 1][V], bv[EARLY ? N : 1][V];
-    if (EARLY) {
-#pragma unroll
-        for (int n = 0; n < N; ++n) {
-            const int j = (n * blockDim.x + threadIdx.x) * V;
-            if (j >= H) continue;
-            if (delta && post_w) {
-                Piece<float, V>::load(post_w + j, pw[EARLY ? n : 0]);
-                Piece<float, V>::load(post_b + j, pb[EARLY ? n : 0]);
-            }
-            Piece<float, V>::load(w + j, wv[EARLY ? n : 0]);
-            Piece<float, V>::load(b + j, bv[EARLY ? n : 0]);
-        }
-    }
     float mean, inv;
     if (delta && post_w) {
         statistics<V, N>(ys, H, post_eps, part, mean, inv);
@@ -126,13 +110,11 @@ __global__ void layer_norm_kernel(float* __restrict__ residual, const TD* __rest
         for (int n = 0; n < N; ++n) {
             const int j = (n * blockDim.x + threadIdx.x) * V;
             if (j >= H) continue;
-            const int at = EARLY ? n : 0;
-            if (!EARLY) {
-                Piece<float, V>::load(post_w + j, pw[0]);
-                Piece<float, V>::load(post_b + j, pb[0]);
-            }
+            float pw[V], pb[V];
+            Piece<float, V>::load(post_w + j, pw);
+            Piece<float, V>::load(post_b + j, pb);
 #pragma unroll
-            for (int e = 0; e < V; ++e) ys[n][e] = fmaf((ys[n][e] - mean) * inv, pw[at][e], pb[at][e]);
+            for (int e = 0; e < V; ++e) ys[n][e] = fmaf((ys[n][e] - mean) * inv, pw[e], pb[e]);
         }
     }
     if (delta || plus) {
@@ -157,14 +139,11 @@ __global__ void layer_norm_kernel(float* __restrict__ residual, const TD* __rest
     for (int n = 0; n < N; ++n) {
         const int j = (n * blockDim.x + threadIdx.x) * V;
         if (j >= H) continue;
-        const int at = EARLY ? n : 0;
-        float v[V];
-        if (!EARLY) {
-            Piece<float, V>::load(w + j, wv[0]);
-            Piece<float, V>::load(b + j, bv[0]);
-        }
+        float wv[V], bv[V], v[V];
+        Piece<float, V>::load(w + j, wv);
+        Piece<float, V>::load(b + j, bv);
 #pragma unroll
-        for (int e = 0; e < V; ++e) v[e] = fmaf((xs[n][e] - mean) * inv, wv[at][e], bv[at][e]);
+        for (int e = 0; e < V; ++e) v[e] = fmaf((xs[n][e] - mean) * inv, wv[e], bv[e]);
         Piece<T, V>::store(o + j, v);
     }
 }
