@@ -5,16 +5,16 @@
 // a2; a0 the upper half of the word, a1 the upper half of what is left, a2 the rest).  Products of two such parts are exact in float32, so
 // a.w is the sum of nine products that tcgen05.mma forms exactly; the three smallest (a1 w2, a2 w1, a2 w2: below 2^-22 of a.w together) are
 // left out.  What remains is how sums are rounded.  The tensor cores round their running sum towards zero, so it is kept short: a chunk of 64
-// k's starts from zero, in one sum for the largest products and two for the smaller ones, and is then added to a float32 sum in
+// k's starts from zero, in one sum for the largest products and one for the others, and is then added to a float32 sum in
 // registers, rounded to nearest.
 //
 // Every output is formed in the same steps whatever the batch: the chunks of a segment of K in order, then the segments in
-// order, their number chosen by N and K alone.  Rows of W are the 128 rows of the MMA tile, rows of A its columns (16 or 64 by
+// order, their number chosen by N and K alone.  Rows of W are the 128 rows of the MMA tile, rows of A its columns (16, 64 or 128 by
 // M), so that a handful of rows streams W once.
 //
 // Blocks stay for tile after tile.  Warps 0..7 read float32 rows (two chunks of loads in flight: half of a thread's registers hold one
-// while the other is cut up), write the three parts into 128-byte-swizzled tiles; one thread of warp 8 issues 12 MMAs a chunk into one of
-// two accumulators in tensor memory; warps 8..15 add the other to their registers and write the tile out at the end.  A
+// while the other is cut up), write the three parts into 128-byte-swizzled tiles; one thread of warp 8 issues 20 MMAs a chunk into one of
+// several accumulators in tensor memory; warps 8..15 add the others to their registers and write the tile out at the end.  A
 // result that is no finite number is formed again as a chain of multiply-adds (an infinity has no three parts).
 #include "common.cuh"
 
@@ -91,11 +91,12 @@ __device__ __forceinline__ void split8(const float4& p, const float4& q, uint4& 
 }
 
 template <int BN> struct Sizes {
-    static constexpr int STAGES = BN == 16 ? 3 : 2;
+    static constexpr int STAGES = BN == 16 ? 3 : 2;             // no more: loads on their way need the rest of the SM's memory
     static constexpr int W_PART = TILE_W * CHUNK * 2, X_PART = BN * CHUNK * 2;
     static constexpr int STAGE = 3 * (W_PART + X_PART);
     static constexpr int BYTES = STAGES * STAGE + 1024;
-    static constexpr int COLUMNS = BN == 16 ? 128 : 512;        // of tensor memory: two chunks' accumulators, 3 BN columns each
+    static constexpr int BUFFERS = BN == 128 ? 2 : 4;           // chunks' accumulators, of 2 BN columns of tensor memory each
+    static constexpr int COLUMNS = BUFFERS * 2 * BN;
 };
 
 // ``part`` (null with one segment): the segments' sums, [segments][M][N].
@@ -106,7 +107,7 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
                   int* __restrict__ status) {
     using S = Sizes<BN>;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    __shared__ __align__(8) unsigned long long full_bar[S::STAGES], empty_bar[S::STAGES], acc_full[2], acc_empty[2];
+    __shared__ __align__(8) unsigned long long full_bar[S::STAGES], empty_bar[S::STAGES], acc_full[S::BUFFERS], acc_empty[S::BUFFERS];
     __shared__ unsigned tmem_holder;
     __shared__ volatile int give_up;
     const unsigned base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -123,7 +124,7 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
     };
     if (tid == 0) {
         for (int s = 0; s < S::STAGES; ++s) { mbar_init(&full_bar[s], SPLIT_WARPS); mbar_init(&empty_bar[s], 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], SUM_WARPS); }
+        for (int b = 0; b < S::BUFFERS; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], SUM_WARPS); }
         give_up = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
@@ -143,17 +144,17 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
         constexpr int ITEMS_W = TILE_W * 8 / (32 * SPLIT_WARPS), ITEMS_X = BN >= 32 ? BN * 8 / (32 * SPLIT_WARPS) : 1;
         const int row = tid >> 3, at = tid & 7;                   // item i: row + 32 i, eight k's ``at``
         const bool has_x = BN >= 32 || row < BN;
-        auto eight = [&](const float* __restrict__ src, int r, int rows, int k, float4& p, float4& q) {
+        const size_t apart = (size_t)32 * K;
+        auto eight = [&](const float* __restrict__ s, bool in, int k, float4& p, float4& q) {
             p = q = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (r >= rows || k >= K) return;
-            const float* s = src + (size_t)r * K + k;
+            if (!in || k >= K) return;
             if (VEC) {                                            // K a multiple of 4, 16-byte addresses
-                p = __ldg(reinterpret_cast<const float4*>(s));
-                if (k + 4 < K) q = __ldg(reinterpret_cast<const float4*>(s + 4));
+                p = __ldg(reinterpret_cast<const float4*>(s + k));
+                if (k + 4 < K) q = __ldg(reinterpret_cast<const float4*>(s + k + 4));
             } else {
                 float v[8];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) v[i] = k + i < K ? __ldg(s + i) : 0.f;
+                for (int i = 0; i < 8; ++i) v[i] = k + i < K ? __ldg(s + k + i) : 0.f;
                 p = make_float4(v[0], v[1], v[2], v[3]);
                 q = make_float4(v[4], v[5], v[6], v[7]);
             }
@@ -168,17 +169,23 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
         };
         // what is loaded next: chunk ``nc`` of tile ``nt``
         int nt = blockIdx.x, w0 = 0, m0 = 0, nc = 0, nc1 = 0, ns = 0;
-        auto settle = [&]() { while (nt < tiles) { place(nt, w0, m0, nc, nc1, ns); if (nc < nc1) return; nt += gridDim.x; } };
+        const float *wr = W, *xr = A;                             // this thread's first rows of the tile
+        auto settle = [&]() {
+            if (nt >= tiles) return;
+            place(nt, w0, m0, nc, nc1, ns);
+            wr = W + (size_t)(w0 + row) * K;
+            xr = A + (size_t)(m0 + row) * K;
+        };
         settle();
         auto step = [&]() { if (++nc >= nc1) { nt += gridDim.x; settle(); } };
         auto load_w = [&](float4 (&v)[2 * ITEMS_W]) {
 #pragma unroll
-            for (int i = 0; i < ITEMS_W; ++i) eight(W, w0 + row + 32 * i, N, nc * CHUNK + 8 * at, v[2 * i], v[2 * i + 1]);
+            for (int i = 0; i < ITEMS_W; ++i) eight(wr + i * apart, w0 + row + 32 * i < N, nc * CHUNK + 8 * at, v[2 * i], v[2 * i + 1]);
         };
         auto load_x = [&](float4 (&v)[2 * ITEMS_X]) {
             if (has_x) {
 #pragma unroll
-                for (int i = 0; i < ITEMS_X; ++i) eight(A, m0 + row + 32 * i, M, nc * CHUNK + 8 * at, v[2 * i], v[2 * i + 1]);
+                for (int i = 0; i < ITEMS_X; ++i) eight(xr + i * apart, m0 + row + 32 * i < M, nc * CHUNK + 8 * at, v[2 * i], v[2 * i + 1]);
             }
         };
         auto put_w = [&](unsigned to, const float4 (&v)[2 * ITEMS_W]) {
@@ -246,9 +253,9 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
         }
     } else {
         // ---- sums: warp w reads TMEM lanes 32 (w % 4) .. + 31 (rows of W), one half of the columns (rows of A) ----
-        constexpr int COLS = BN / 2;                              // 8 or 32
+        constexpr int COLS = BN / 2;
         const int quarter = warp & 3, col0 = ((warp - SPLIT_WARPS) >> 2) * COLS;
-        // one thread issues the MMAs, a chunk ahead of the one it adds up
+        // one thread issues the MMAs, a chunk or two ahead of the one it adds up
         int it = blockIdx.x, ic = 0, ic1 = 0, issued = 0;
         auto issue = [&]() {
             if (it >= tiles || give_up) return;
@@ -256,24 +263,32 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
                 int w0, m0, seg;
                 place(it, w0, m0, ic, ic1, seg);
             }
-            const int s = issued % S::STAGES, buf = issued & 1;
-            if (!mbar_wait(&full_bar[s], (issued / S::STAGES) & 1) || !mbar_wait(&acc_empty[buf], ((issued >> 1) & 1) ^ 1)) { give_up = 1; return; }
+            const int s = issued % S::STAGES, buf = issued % S::BUFFERS;
+            if (!mbar_wait(&full_bar[s], (issued / S::STAGES) & 1) || !mbar_wait(&acc_empty[buf], ((issued / S::BUFFERS) & 1) ^ 1)) { give_up = 1; return; }
             tc_fence_after();
-            const unsigned w = base + s * S::STAGE, x = w + 3 * S::W_PART, acc = tmem + buf * 3 * BN;
-            // The parts of A's rows lie one after the other like 3 BN rows: a part of W meets as many of them as count at once.  Column
-            // block 0 of the accumulator takes w0 a0, block 1 w0 a1 + w1 a0, block 2 w0 a2 + w1 a1 + w2 a0.
+            const unsigned w = base + s * S::STAGE, x = w + 3 * S::W_PART, acc = tmem + buf * 2 * BN;
+            // Column block 0 of the accumulator takes the largest products, w0 a0, block 1 the others.  The parts of A's rows lie one
+            // after the other like rows, so that w0 meets a0 and a1 at once.
+            const unsigned long long x0 = smem_desc(x), x1 = smem_desc(x + S::X_PART), x2 = smem_desc(x + 2 * S::X_PART);
+            const unsigned long long w0 = smem_desc(w), w1 = smem_desc(w + S::W_PART), w2 = smem_desc(w + 2 * S::W_PART);
 #pragma unroll
-            for (int k = 0; k < CHUNK / 16; ++k)
-#pragma unroll
-                for (int p = 0; p < 3; ++p)
-                    umma(acc + p * BN, smem_desc(w + p * S::W_PART) + 2 * k, smem_desc(x) + 2 * k, instr_desc((3 - p) * BN), (p > 0 || k > 0) ? 1u : 0u);
+            for (int k = 0; k < CHUNK / 16; ++k) {
+                umma(acc, w0 + 2 * k, x0 + 2 * k, instr_desc(2 * BN), k > 0 ? 1u : 0u);
+                umma(acc + BN, w0 + 2 * k, x2 + 2 * k, instr_desc(BN), 1u);
+                umma(acc + BN, w1 + 2 * k, x0 + 2 * k, instr_desc(BN), 1u);
+                umma(acc + BN, w1 + 2 * k, x1 + 2 * k, instr_desc(BN), 1u);
+                umma(acc + BN, w2 + 2 * k, x0 + 2 * k, instr_desc(BN), 1u);
+            }
             umma_commit(&empty_bar[s]);
             umma_commit(&acc_full[buf]);
             ++issued;
             if (++ic >= ic1) it += gridDim.x;
         };
         const bool issuer = tid == SPLIT_WARPS * 32;
-        if (issuer) issue();
+        if (issuer) {
+            issue();
+            if (S::BUFFERS > 2) issue();
+        }
         int i = 0;
         for (int t = blockIdx.x; t < tiles && !give_up; t += gridDim.x) {
             int w0, m0, c0, c1, seg;
@@ -283,20 +298,23 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
             for (int j = 0; j < COLS; ++j) sum[j] = 0.f;
             bool ok = true;
             for (int c = c0; c < c1; ++c, ++i) {
-                const int buf = i & 1;
+                const int buf = i % S::BUFFERS;
                 if (issuer) issue();
                 __syncwarp();
-                if (!mbar_wait(&acc_full[buf], (i >> 1) & 1)) { give_up = 1; ok = false; break; }
+                if (!mbar_wait(&acc_full[buf], (i / S::BUFFERS) & 1)) { give_up = 1; ok = false; break; }
                 tc_fence_after();
-                const unsigned from = tmem + buf * 3 * BN + col0 + ((unsigned)(quarter * 32) << 16);
+                const unsigned from = tmem + buf * 2 * BN + col0 + ((unsigned)(quarter * 32) << 16);
+                constexpr int AT_ONCE = COLS >= 16 ? 16 : COLS;
 #pragma unroll
-                for (int j = 0; j < COLS; j += 8) {
-                    unsigned r[3][8];
+                for (int j = 0; j < COLS; j += AT_ONCE) {
+                    unsigned r[2][AT_ONCE];
 #pragma unroll
-                    for (int h = 0; h < 3; ++h) tmem_load8(from + h * BN + j, r[h]);
+                    for (int h = 0; h < 2; ++h)
+#pragma unroll
+                        for (int e = 0; e < AT_ONCE; e += 8) tmem_load8(from + h * BN + j + e, r[h] + e);
                     asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) sum[j + e] += __uint_as_float(r[0][e]) + (__uint_as_float(r[1][e]) + __uint_as_float(r[2][e]));
+                    for (int e = 0; e < AT_ONCE; ++e) sum[j + e] += __uint_as_float(r[0][e]) + __uint_as_float(r[1][e]);
                 }
                 tc_fence_before();
                 __syncwarp();
@@ -390,7 +408,8 @@ extern "C" int fe_gemm_split(const float* A, const float* W, const float* bias, 
 #define FE_SPLIT(BN) rc = vec ? launch_split<BN, true>(A, W, bias, C, part, M, N, K, segments, status, stream) \
                               : launch_split<BN, false>(A, W, bias, C, part, M, N, K, segments, status, stream)
     if (M <= 16) FE_SPLIT(16);
-    else FE_SPLIT(64);
+    else if (M <= 64) FE_SPLIT(64);
+    else FE_SPLIT(128);
 #undef FE_SPLIT
     if (rc || segments == 1) return rc;
     const long long total = (long long)M * N;
