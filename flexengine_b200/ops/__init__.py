@@ -279,16 +279,21 @@ def _fits(x, w) -> str:
     return "skinny" if skinny_ok(x.scaled if isinstance(x, Prenormed) else x, w) else ""
 
 
-SPLIT_MIN_K, SPLIT_MIN_N = 1024, 512
+SPLIT_MIN_K, SPLIT_MIN_ELEMENTS, SPLIT_MAX_N = 1024, 1 << 23, 1 << 15
+
+
+def split_ok(N: int, K: int) -> bool:
+    """Whether the 32-bit product with a matrix [N, K] goes through the tensor cores in three bfloat16 parts a number (csrc/gemm_split.cu)
+    instead of a chain of multiply-adds on CUDA cores: by the matrix alone and never by the rows of x, so that a row's result does
+    not depend on the batch.  The lines lie where prompts gain more than steps of a few rows lose: SPLIT_FIGURES"""
+    return K >= SPLIT_MIN_K and N <= SPLIT_MAX_N and N * K >= SPLIT_MIN_ELEMENTS
 
 
 def gemm_fp32(x, w, bias=None):
-    """The float32 product.  Matrices of SPLIT_MIN_N rows and SPLIT_MIN_K columns or more go through the tensor cores in three bfloat16
-    parts a number (csrc/gemm_split.cu), whatever the rows of x: a row's result does not depend on the batch."""
     M, K = x.shape
     N = w.shape[0]
     out = torch.empty((M, N), dtype=torch.float32, device=x.device)
-    if K >= SPLIT_MIN_K and N >= SPLIT_MIN_N:
+    if split_ok(N, K):
         segments = int(_core().fe_gemm_split_segments(_c_int(N), _c_int(K)))
         part = torch.empty((segments, M, N), dtype=torch.float32, device=x.device) if segments > 1 else None
         _run(_core(), "fe_gemm_split", _ptr(x), _ptr(w), _ptr(bias), _ptr(out), _ptr(part), _c_int(M), _c_int(N), _c_int(K),
