@@ -5,15 +5,15 @@
 // a2; a0 the upper half of the word, a1 the upper half of what is left, a2 the rest).  Products of two such parts are exact in float32, so
 // a.w is the sum of nine products that tcgen05.mma forms exactly; the three smallest (a1 w2, a2 w1, a2 w2: below 2^-22 of a.w together) are
 // left out.  What remains is how sums are rounded.  The tensor cores round their running sum towards zero, so it is kept short: a chunk of 64
-// k's starts from zero, in one sum for the largest products and one for the others, and is then added to a float32 sum in
+// k's starts from zero, in one sum for the largest products and two for the others, and is then added to a float32 sum in
 // registers, rounded to nearest.
 //
 // Every output is formed in the same steps whatever the batch: the chunks of a segment of K in order, then the segments in
-// order, their number chosen by N and K alone.  Rows of W are the 128 rows of the MMA tile, rows of A its columns (16, 64 or 128 by
+// order, their number chosen by N and K alone.  Rows of W are the 128 rows of the MMA tile, rows of A its columns (16 or 64 by
 // M), so that a handful of rows streams W once.
 //
 // Blocks stay for tile after tile.  Two groups of eight warps read float32 rows, chunk about, and write the three parts into
-// 128-byte-swizzled tiles; one thread issues 20 MMAs a chunk into one of several accumulators in tensor memory; eight more warps add the
+// 128-byte-swizzled tiles; one thread issues 12 MMAs a chunk into one of several accumulators in tensor memory; eight more warps add the
 // others to their registers and write the tile out at the end.  A result that is no finite number is formed again as a chain of
 // multiply-adds (an infinity has no three parts).
 #include "common.cuh"
@@ -24,7 +24,7 @@ namespace {
 
 constexpr int TILE_W = 128;             // rows of W in a tile = UMMA M
 constexpr int CHUNK = 64;               // k's of a chunk: 128 bytes of bfloat16, one swizzle atom wide
-constexpr int GROUP_WARPS = 8, SUM_WARPS = 8;
+constexpr int GROUP_WARPS = 8, SPLIT_WARPS = 2 * GROUP_WARPS, SUM_WARPS = 8, THREADS = 32 * (SPLIT_WARPS + SUM_WARPS);
 constexpr long long WAIT_LIMIT = 4000000000LL;      // clock cycles
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -91,24 +91,21 @@ __device__ __forceinline__ void split8(const float4& p, const float4& q, uint4& 
 }
 
 template <int BN> struct Sizes {
-    static constexpr int STAGES = 2;                            // no more: loads on their way need the rest of the SM's memory
+    static constexpr int STAGES = BN == 16 ? 3 : 2;             // no more: loads on their way need the rest of the SM's memory
     static constexpr int W_PART = TILE_W * CHUNK * 2, X_PART = BN * CHUNK * 2;
     static constexpr int STAGE = 3 * (W_PART + X_PART);
     static constexpr int BYTES = STAGES * STAGE + 1024;
-    // Groups of warps that cut rows up: two take turns, but for the widest tile, whose sums need the registers.
-    static constexpr int GROUPS = BN == 128 ? 1 : 2, SPLIT_WARPS = GROUPS * GROUP_WARPS, THREADS = 32 * (SPLIT_WARPS + SUM_WARPS);
-    static constexpr int BUFFERS = BN == 128 ? 2 : 4;           // chunks' accumulators, of 2 BN columns of tensor memory each
-    static constexpr int COLUMNS = BUFFERS * 2 * BN;
+    static constexpr int BUFFERS = BN == 16 ? 4 : 2;            // chunks' accumulators, of 3 BN columns of tensor memory each
+    static constexpr int COLUMNS = BN == 16 ? 256 : 512;
 };
 
 // ``part`` (null with one segment): the segments' sums, [segments][M][N].
 template <int BN, bool VEC>
-__global__ void __launch_bounds__(Sizes<BN>::THREADS, 1)
+__global__ void __launch_bounds__(THREADS, 1)
 gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C,
                   float* __restrict__ part, const int M, const int N, const int K, const int m_tiles, const int tiles, const int segments,
                   int* __restrict__ status) {
     using S = Sizes<BN>;
-    constexpr int SPLIT_WARPS = S::SPLIT_WARPS;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ __align__(8) unsigned long long full_bar[S::STAGES], empty_bar[S::STAGES], acc_full[S::BUFFERS], acc_empty[S::BUFFERS];
     __shared__ unsigned tmem_holder;
@@ -212,7 +209,7 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
         auto stage_free = [&](int& s) {
             s = at_chunk % S::STAGES;
             if (!mbar_wait(&empty_bar[s], ((at_chunk / S::STAGES) & 1) ^ 1)) { give_up = 1; return false; }
-            at_chunk += S::GROUPS;
+            at_chunk += 2;
             return true;
         };
         // the rows of W of the next chunk are asked for before the rows of A of this one are cut up, and the other way round
@@ -223,7 +220,7 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
             if (!stage_free(s)) break;
             const unsigned to = base + s * S::STAGE;
             step();
-            if (S::GROUPS == 2 && nt < tiles) step();
+            if (nt < tiles) step();
             put_w(to, vw);
             if (nt < tiles) load_w(vw);
             put_x(to, vx);
@@ -245,19 +242,14 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
             const int s = issued % S::STAGES, buf = issued % S::BUFFERS;
             if (!mbar_wait(&full_bar[s], (issued / S::STAGES) & 1) || !mbar_wait(&acc_empty[buf], ((issued / S::BUFFERS) & 1) ^ 1)) { give_up = 1; return; }
             tc_fence_after();
-            const unsigned w = base + s * S::STAGE, x = w + 3 * S::W_PART, acc = tmem + buf * 2 * BN;
-            // Column block 0 of the accumulator takes the largest products, w0 a0, block 1 the others.  The parts of A's rows lie one
-            // after the other like rows, so that w0 meets a0 and a1 at once.
-            const unsigned long long x0 = smem_desc(x), x1 = smem_desc(x + S::X_PART), x2 = smem_desc(x + 2 * S::X_PART);
-            const unsigned long long w0 = smem_desc(w), w1 = smem_desc(w + S::W_PART), w2 = smem_desc(w + 2 * S::W_PART);
+            const unsigned w = base + s * S::STAGE, x = w + 3 * S::W_PART, acc = tmem + buf * 3 * BN;
+            // The parts of A's rows lie one after the other like 3 BN rows: a part of W meets as many of them as count at once.  Column
+            // block 0 of the accumulator takes w0 a0, block 1 w0 a1 + w1 a0, block 2 w0 a2 + w1 a1 + w2 a0.
 #pragma unroll
-            for (int k = 0; k < CHUNK / 16; ++k) {
-                umma(acc, w0 + 2 * k, x0 + 2 * k, instr_desc(2 * BN), k > 0 ? 1u : 0u);
-                umma(acc + BN, w0 + 2 * k, x2 + 2 * k, instr_desc(BN), 1u);
-                umma(acc + BN, w1 + 2 * k, x0 + 2 * k, instr_desc(BN), 1u);
-                umma(acc + BN, w1 + 2 * k, x1 + 2 * k, instr_desc(BN), 1u);
-                umma(acc + BN, w2 + 2 * k, x0 + 2 * k, instr_desc(BN), 1u);
-            }
+            for (int k = 0; k < CHUNK / 16; ++k)
+#pragma unroll
+                for (int p = 0; p < 3; ++p)
+                    umma(acc + p * BN, smem_desc(w + p * S::W_PART) + 2 * k, smem_desc(x) + 2 * k, instr_desc((3 - p) * BN), (p > 0 || k > 0) ? 1u : 0u);
             umma_commit(&empty_bar[s]);
             umma_commit(&acc_full[buf]);
             ++issued;
@@ -282,15 +274,15 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
                 __syncwarp();
                 if (!mbar_wait(&acc_full[buf], (i / S::BUFFERS) & 1)) { give_up = 1; ok = false; break; }
                 tc_fence_after();
-                const unsigned from = tmem + buf * 2 * BN + col0 + ((unsigned)(quarter * 32) << 16);
+                const unsigned from = tmem + buf * 3 * BN + col0 + ((unsigned)(quarter * 32) << 16);
 #pragma unroll
                 for (int j = 0; j < COLS; j += 8) {
-                    unsigned r[2][8];
+                    unsigned r[3][8];
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) tmem_load8(from + h * BN + j, r[h]);
+                    for (int h = 0; h < 3; ++h) tmem_load8(from + h * BN + j, r[h]);
                     asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) sum[j + e] += __uint_as_float(r[0][e]) + __uint_as_float(r[1][e]);
+                    for (int e = 0; e < 8; ++e) sum[j + e] += __uint_as_float(r[0][e]) + (__uint_as_float(r[1][e]) + __uint_as_float(r[2][e]));
                 }
                 tc_fence_before();
                 __syncwarp();
@@ -357,7 +349,7 @@ int launch_split(const float* A, const float* W, const float* bias, float* C, fl
     const long long m_tiles = (M + BN - 1) / BN, tiles = m_tiles * ((N + TILE_W - 1) / TILE_W) * segments;
     FE_REQUIRE(tiles < (1LL << 30), "gemm_split: too many tiles");
     const int sms = fe_sm_count();
-    fe::launch(kernel, (unsigned)(tiles < sms ? tiles : sms), Sizes<BN>::THREADS, Sizes<BN>::BYTES, stream, A, W, bias, C, segments > 1 ? part : (float*)nullptr, M, N, K,
+    fe::launch(kernel, (unsigned)(tiles < sms ? tiles : sms), THREADS, Sizes<BN>::BYTES, stream, A, W, bias, C, segments > 1 ? part : (float*)nullptr, M, N, K,
                (int)m_tiles, (int)tiles, segments, status);
     return fe_check_launch("gemm_split");
 }
@@ -384,8 +376,7 @@ extern "C" int fe_gemm_split(const float* A, const float* W, const float* bias, 
 #define FE_SPLIT(BN) rc = vec ? launch_split<BN, true>(A, W, bias, C, part, M, N, K, segments, status, stream) \
                               : launch_split<BN, false>(A, W, bias, C, part, M, N, K, segments, status, stream)
     if (M <= 16) FE_SPLIT(16);
-    else if (M <= 64) FE_SPLIT(64);
-    else FE_SPLIT(128);
+    else FE_SPLIT(64);
 #undef FE_SPLIT
     if (rc || segments == 1) return rc;
     const long long total = (long long)M * N;
