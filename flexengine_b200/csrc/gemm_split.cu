@@ -16,6 +16,11 @@
 // 128-byte-swizzled tiles; one thread issues 12 MMAs a chunk into one of several accumulators in tensor memory; eight more warps add the
 // others to their registers and write the tile out at the end.  A result that is no finite number is formed again as a chain of
 // multiply-adds (an infinity has no three parts).
+//
+// A chunk's way (rows from memory, cut up, through shared memory, 12 MMAs, sums) takes 1.1 to 1.5 us and is what bounds the kernel: a third of
+// the stalls are loads on their way, the tensor cores are busy 26 % and 19 % of the time (tiles of 16 and of 64 rows).  17,920 x 1,536: 33 us with
+// 1 to 16 rows (the chain of multiply-adds 24 to 41), 42 with 64 (107), 144 with 256 (278); 1,536 x 8,960: 33 (31 to 69), 40 (125), 78 (244).
+// Relative error against 64 bits, K = 1,536 / 8,960: 1.5e-7 / 1.5e-7, the chain 7.0e-7 / 1.7e-6.
 #include "common.cuh"
 
 using namespace fe;
@@ -91,7 +96,7 @@ __device__ __forceinline__ void split8(const float4& p, const float4& q, uint4& 
 }
 
 template <int BN> struct Sizes {
-    static constexpr int STAGES = BN == 16 ? 3 : 2;             // no more: loads on their way need the rest of the SM's memory
+    static constexpr int STAGES = BN == 16 ? 3 : 2;             // no more: loads on their way take lines of what is left of the SM's memory
     static constexpr int W_PART = TILE_W * CHUNK * 2, X_PART = BN * CHUNK * 2;
     static constexpr int STAGE = 3 * (W_PART + X_PART);
     static constexpr int BYTES = STAGES * STAGE + 1024;

@@ -147,6 +147,11 @@ __device__ __forceinline__ void cumulate(const float* __restrict__ gates, int be
     __syncthreads();
 }
 
+// What bounds the three kernels below was not their multiply-adds but what fed them: single floats loaded one by one, written transposed
+// (four lanes to a bank), two multiply-adds in two instructions.  Tiles now come by asynchronous copies and lie as in memory; a thread reads four
+// key channels of its rows at once, and takes keys tx, tx + 16, .. so that its reads meet on no bank.  A step's average portion of prompts
+// of up to 2,039 tokens: outputs with Q K^T from head_scan_products 154.6 -> 93.6 us (mamba2, 64 heads of 128 x 64), with their own 80.6 -> 54.3
+// (16 heads of 64 x 128), sums 61.8 -> 42.5, products 31.3 -> 17.6.
 // 64 rows of 64 floats into shared memory, ``pitch`` floats apart: rows from ``rows`` and columns from ``cols`` on are zeros.  Asynchronous
 // copies of 16 bytes where the rows start on 16-byte boundaries (the caller waits for them); 256 threads.
 __device__ __forceinline__ void load_tile(float* to, int pitch, const float* __restrict__ from, long long ld, int rows, int cols) {

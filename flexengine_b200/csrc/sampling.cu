@@ -72,8 +72,8 @@ __device__ __forceinline__ float warp_total(float v) {       // the same value i
     return v;
 }
 
-// The parameters of a step's rows: on the device, or (up to LISTED_ROWS rows) with the launch, so that lists of numbers on the host
-// need no buffer and no copy of their own.
+// The parameters of a step's rows: on the device, or (up to LISTED_ROWS rows: 1.5 KB of the launch's parameters) with the launch, so that
+// lists of numbers on the host need no buffer and no copy of their own.
 constexpr int LISTED_ROWS = 64;
 struct OnDevice {
     const float* temperature;
