@@ -1,26 +1,35 @@
-// C[M,N] = A[M,K] . W[N,K]^T (+ bias[N]) for float32 operands on the fifth-generation tensor cores, as exact as the chain of
-// float32 multiply-adds of gemm_fp32.cu or more so.
+// C[M,N] = A[M,K] . W[N,K]^T (+ bias[N]) for float32 operands on the fifth-generation tensor cores, with the error of float32
+// multiply-adds (gemm_fp32.cu) or less.
 //
-// A float32 has 24 bits of mantissa: cut off after 8 and after 16 of them it is the sum of three bfloat16 numbers, exactly (a = a0 + a1 +
-// a2; a0 the upper half of the word, a1 the upper half of what is left, a2 the rest).  Products of two such parts are exact in float32, so
-// a.w is the sum of nine products that tcgen05.mma forms exactly; the three smallest (a1 w2, a2 w1, a2 w2: below 2^-22 of a.w together) are
-// left out.  What remains is how sums are rounded.  The tensor cores round their running sum towards zero, so it is kept short: a chunk of 64
-// k's starts from zero, in one sum for the largest products and two for the others, and is then added to a float32 sum in
-// registers, rounded to nearest.
+// A float32 has 24 bits of mantissa: cut off after 8 and after 16 of them it is the sum of three bfloat16 numbers (a = a0 + a1 + a2; a0 the
+// upper half of the word, a1 the upper half of what is left, a2 the rest), exactly from 2^-110 on; of a smaller number less than 2^-133 is
+// lost, bfloat16's last place.  a1 is below 2^-7 of a's power of two and a2 below 2^-15.  Products of two parts are exact in float32, so a.w is
+// the sum of nine products that tcgen05.mma forms exactly; a2 w2, below 2^-30 of a.w, is left out.  (Without a1 w2 and a2 w1 too, up to
+// 2^-21 of a product was missing, always to the same side: rows with few numbers other than 0 were further from 64 bits than the multiply-adds.)
+// What remains is how sums are rounded.  The tensor cores round their running sum towards zero.  Of the largest products, w0 a0, it is
+// kept short: a chunk of 64 k's starts from zero and is then added to a float32 sum in registers, rounded to nearest.  The others, from
+// 2^-7 of a product down, have three sums in tensor memory, by their sizes, over all chunks of a tile, and meet the first one at its end: what they lose
+// by then is below what the first loses, and a result of few products is rounded about once.  Segments of K hand on their sums with what their rounding
+// lost, and are added up in 64 bits.
+//
+// Results that this does not serve are formed again from the rows themselves, in 64 bits: what is no finite number (an infinity has no three
+// parts), and what is below LEAST, where the lost places of small numbers could count.  They cannot for any other result: a number of LARGE
+// or more is made a NaN in shared memory, so that its results are formed again, and with all others below it a sum of K products has
+// lost less than 2 K 2^-133 LARGE, below 2^-24 of LEAST up to K = 2^16.
 //
 // Every output is formed in the same steps whatever the batch: the chunks of a segment of K in order, then the segments in
 // order, their number chosen by N and K alone.  Rows of W are the 128 rows of the MMA tile, rows of A its columns (16 or 64 by
 // M), so that a handful of rows streams W once.
 //
 // Blocks stay for tile after tile.  Two groups of eight warps read float32 rows, chunk about, and write the three parts into
-// 128-byte-swizzled tiles; one thread issues 12 MMAs a chunk into one of several accumulators in tensor memory; eight more warps add the
-// others to their registers and write the tile out at the end.  A result that is no finite number is formed again as a chain of
-// multiply-adds (an infinity has no three parts).
+// 128-byte-swizzled tiles; one thread issues 16 MMAs a chunk; eight more warps add the chunks' sums to their registers and write the
+// tile out at the end.
 //
-// A chunk's way (rows from memory, cut up, through shared memory, 12 MMAs, sums) takes 1.1 to 1.5 us and is what bounds the kernel: a third of
-// the stalls are loads on their way, the tensor cores are busy 26 % and 19 % of the time (tiles of 16 and of 64 rows).  17,920 x 1,536: 33 us with
-// 1 to 16 rows (the chain of multiply-adds 24 to 41), 42 with 64 (107), 144 with 256 (278); 1,536 x 8,960: 33 (31 to 69), 40 (125), 78 (244).
-// Relative error against 64 bits, K = 1,536 / 8,960: 1.5e-7 / 1.5e-7, the chain 7.0e-7 / 1.7e-6.
+// A chunk's way (rows from memory, cut up, through shared memory, 16 MMAs, sums) takes 1.2 to 1.5 us and is what bounds the kernel: loads
+// on their way, and shared memory, through which a number goes as four bytes, then as six, then to the tensor cores once an MMA.  17,920 x 1,536:
+// 39 us with 1 to 16 rows (the chain of multiply-adds 26 to 42), 45 with 64 (108), 151 with 256 (279); 1,536 x 8,960: 42 (33 to 70), 49 (127), 87 (246).
+// Relative error against 64 bits, K = 1,536 / 8,960: 1.2e-7 / 1.2e-7, the chain 7.0e-7 / 1.7e-6; rows of 1, 2, 8 and 32 numbers other than 0:
+// 2.5e-8, 2.6e-8, 2.8e-8, 4.2e-8, the chain 2.5e-8, 3.1e-8, 5.2e-8, 1.0e-7.
 #include "common.cuh"
 
 using namespace fe;
@@ -31,6 +40,8 @@ constexpr int TILE_W = 128;             // rows of W in a tile = UMMA M
 constexpr int CHUNK = 64;               // k's of a chunk: 128 bytes of bfloat16, one swizzle atom wide
 constexpr int GROUP_WARPS = 8, SPLIT_WARPS = 2 * GROUP_WARPS, SUM_WARPS = 8, THREADS = 32 * (SPLIT_WARPS + SUM_WARPS);
 constexpr long long WAIT_LIMIT = 4000000000LL;      // clock cycles
+constexpr float LEAST = 8.673617380e-19f, MOST = 3.402823466e38f;      // 2^-60; results outside of these bounds are formed again
+constexpr unsigned LARGE = 0x4f80;                  // 2^32, the upper half of the word
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(unsigned long long* bar, int count) {
@@ -90,6 +101,10 @@ __device__ __forceinline__ void split8(const float4& p, const float4& q, uint4& 
         m[i] = __byte_perm(ua, ub, 0x7632);
         l[i] = __byte_perm(__float_as_uint(a2), __float_as_uint(b2), 0x7632);
     }
+    unsigned most = 0;                                // of the eight, two by two: the upper halves without their signs
+#pragma unroll
+    for (int i = 0; i < 4; ++i) most = __vmaxu2(most, h[i] & 0x7fff7fffu);
+    if ((most >> 16) >= LARGE || (most & 0xffffu) >= LARGE) h[0] = 0x7fc07fc0u;
     hi = make_uint4(h[0], h[1], h[2], h[3]);
     mid = make_uint4(m[0], m[1], m[2], m[3]);
     lo = make_uint4(l[0], l[1], l[2], l[3]);
@@ -100,19 +115,66 @@ template <int BN> struct Sizes {
     static constexpr int W_PART = TILE_W * CHUNK * 2, X_PART = BN * CHUNK * 2;
     static constexpr int STAGE = 3 * (W_PART + X_PART);
     static constexpr int BYTES = STAGES * STAGE + 1024;
-    static constexpr int BUFFERS = BN == 16 ? 4 : 2;            // chunks' accumulators, of 3 BN columns of tensor memory each
+    // Columns of tensor memory: the sums of the smaller products (3 BN) of two tiles, then chunks' sums of the largest (BN each)
+    static constexpr int BUFFERS = BN == 16 ? 4 : 2;
     static constexpr int COLUMNS = BN == 16 ? 256 : 512;
+    static_assert(6 * BN + BUFFERS * BN <= COLUMNS, "tensor memory");
 };
 
-// ``part`` (null with one segment): the segments' sums, [segments][M][N].
+// ---- results formed again; every lane of a warp takes part ----
+__device__ bool all_zero(const float* __restrict__ row, int K) {
+    const int lane = threadIdx.x & 31;
+    for (int k0 = 0; k0 < K; k0 += 32)
+        if (__any_sync(0xffffffffu, k0 + lane < K && row[k0 + lane] != 0.f)) return false;
+    return true;
+}
+__device__ float product64(const float* __restrict__ a, const float* __restrict__ w, int K) {
+    double v = 0.;
+#pragma unroll 4
+    for (int k = threadIdx.x & 31; k < K; k += 32) v = fma((double)a[k], (double)w[k], v);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return (float)v;
+}
+// Whether a sum of products has to be formed again.  A sum of 0 may be one that lost all its places; where a whole row is 0 it is not.
+__device__ __forceinline__ bool outside(float v) { return !(fabsf(v) >= LEAST && fabsf(v) <= MOST); }
+
+// Rows m0 .. (32 at most) of A with each lane's row n of W: bit j of ``which`` for row m0 + j, of ``zero`` where the sum came to 0.
+__device__ __noinline__ void form_again(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C,
+                                        int m0, int n, int N, int K, unsigned which, unsigned zero) {
+    unsigned w_known = 0, w_zero = 0;                  // lanes whose row of W was looked through, and is 0
+    for (unsigned columns = __reduce_or_sync(0xffffffffu, which); columns; columns &= columns - 1) {
+        const int j = __ffs(columns) - 1;
+        const float* a = A + (size_t)(m0 + j) * K;
+        const unsigned zeros = __ballot_sync(0xffffffffu, zero >> j & 1u);
+        unsigned lanes = __ballot_sync(0xffffffffu, which >> j & 1u);
+        if (zeros && all_zero(a, K)) lanes &= ~zeros;
+        for (; lanes; lanes &= lanes - 1) {
+            const int l = __ffs(lanes) - 1, nl = __shfl_sync(0xffffffffu, n, l);
+            const unsigned bit = 1u << l;
+            const float* w = W + (size_t)nl * K;
+            if (zeros & bit) {
+                if (!(w_known & bit)) {
+                    w_known |= bit;
+                    if (all_zero(w, K)) w_zero |= bit;
+                }
+                if (w_zero & bit) continue;
+            }
+            const float v = product64(a, w, K);
+            if ((threadIdx.x & 31) == l) C[(size_t)(m0 + j) * N + nl] = v + (bias ? bias[nl] : 0.f);
+        }
+    }
+}
+
+// ``part`` (null with one segment): the segments' sums, [segments][M][N], and ``rest`` what their rounding lost.
 template <int BN, bool VEC>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C,
-                  float* __restrict__ part, const int M, const int N, const int K, const int m_tiles, const int tiles, const int segments,
-                  int* __restrict__ status) {
+                  float* __restrict__ part, bf16* __restrict__ rest, const int M, const int N, const int K, const int m_tiles, const int tiles,
+                  const int segments, int* __restrict__ status) {
     using S = Sizes<BN>;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    __shared__ __align__(8) unsigned long long full_bar[S::STAGES], empty_bar[S::STAGES], acc_full[S::BUFFERS], acc_empty[S::BUFFERS];
+    __shared__ __align__(8) unsigned long long full_bar[S::STAGES], empty_bar[S::STAGES], acc_full[S::BUFFERS], acc_empty[S::BUFFERS], small_empty[2];
     __shared__ unsigned tmem_holder;
     __shared__ volatile int give_up;
     const unsigned base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -130,6 +192,7 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
     if (tid == 0) {
         for (int s = 0; s < S::STAGES; ++s) { mbar_init(&full_bar[s], GROUP_WARPS); mbar_init(&empty_bar[s], 1); }
         for (int b = 0; b < S::BUFFERS; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], SUM_WARPS); }
+        for (int b = 0; b < 2; ++b) mbar_init(&small_empty[b], SUM_WARPS);
         give_up = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
@@ -236,25 +299,33 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
         // ---- sums: warp w reads TMEM lanes 32 (w % 4) .. + 31 (rows of W), one half of the columns (rows of A) ----
         constexpr int COLS = BN / 2;
         const int quarter = warp & 3, col0 = ((warp - SPLIT_WARPS) >> 2) * COLS;
-        // one thread issues the MMAs, a chunk or two ahead of the one it adds up
-        int it = blockIdx.x, ic = 0, ic1 = 0, issued = 0;
+        // one thread issues the MMAs, a chunk or two ahead of the one it adds up (a tile has four chunks or more)
+        int it = blockIdx.x, ic = 0, ic1 = 0, issued = 0, tile = -1;
         auto issue = [&]() {
             if (it >= tiles || give_up) return;
-            if (ic >= ic1) {
+            const bool begins = ic >= ic1;                    // a tile
+            if (begins) {
                 int w0, m0, seg;
                 place(it, w0, m0, ic, ic1, seg);
+                ++tile;
             }
             const int s = issued % S::STAGES, buf = issued % S::BUFFERS;
-            if (!mbar_wait(&full_bar[s], (issued / S::STAGES) & 1) || !mbar_wait(&acc_empty[buf], ((issued / S::BUFFERS) & 1) ^ 1)) { give_up = 1; return; }
+            if (!mbar_wait(&full_bar[s], (issued / S::STAGES) & 1) || !mbar_wait(&acc_empty[buf], ((issued / S::BUFFERS) & 1) ^ 1) ||
+                (begins && !mbar_wait(&small_empty[tile & 1], ((tile >> 1) & 1) ^ 1))) { give_up = 1; return; }
             tc_fence_after();
-            const unsigned w = base + s * S::STAGE, x = w + 3 * S::W_PART, acc = tmem + buf * 3 * BN;
-            // The parts of A's rows lie one after the other like 3 BN rows: a part of W meets as many of them as count at once.  Column
-            // block 0 of the accumulator takes w0 a0, block 1 w0 a1 + w1 a0, block 2 w0 a2 + w1 a1 + w2 a0.
+            const unsigned w = base + s * S::STAGE, x = w + 3 * S::W_PART;
+            const unsigned small = tmem + (tile & 1) * 3 * BN, large = tmem + (6 + buf) * BN;
+            // The parts of A's rows lie one after the other like 3 BN rows: a part of W meets as many of them as count at once.
+            // Block 0 of the small sums takes w0 a1 + w1 a0, block 1 w0 a2 + w1 a1 + w2 a0, block 2 w1 a2 + w2 a1.
+            const unsigned long long w0 = smem_desc(w), w1 = smem_desc(w + S::W_PART), w2 = smem_desc(w + 2 * S::W_PART);
+            const unsigned long long x0 = smem_desc(x), x1 = smem_desc(x + S::X_PART);
 #pragma unroll
-            for (int k = 0; k < CHUNK / 16; ++k)
-#pragma unroll
-                for (int p = 0; p < 3; ++p)
-                    umma(acc + p * BN, smem_desc(w + p * S::W_PART) + 2 * k, smem_desc(x) + 2 * k, instr_desc((3 - p) * BN), (p > 0 || k > 0) ? 1u : 0u);
+            for (int k = 0; k < CHUNK / 16; ++k) {
+                umma(small, w1 + 2 * k, x0 + 2 * k, instr_desc(3 * BN), (k > 0 || !begins) ? 1u : 0u);
+                umma(small, w0 + 2 * k, x1 + 2 * k, instr_desc(2 * BN), 1u);
+                umma(small + BN, w2 + 2 * k, x0 + 2 * k, instr_desc(2 * BN), 1u);
+                umma(large, w0 + 2 * k, x0 + 2 * k, instr_desc(BN), k > 0 ? 1u : 0u);
+            }
             umma_commit(&empty_bar[s]);
             umma_commit(&acc_full[buf]);
             ++issued;
@@ -265,13 +336,14 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
             issue();
             if (S::BUFFERS > 2) issue();
         }
-        int i = 0;
-        for (int t = blockIdx.x; t < tiles && !give_up; t += gridDim.x) {
+        int i = 0, turn = 0;
+        for (int t = blockIdx.x; t < tiles && !give_up; t += gridDim.x, ++turn) {
             int w0, m0, c0, c1, seg;
             place(t, w0, m0, c0, c1, seg);
             float sum[COLS];
 #pragma unroll
             for (int j = 0; j < COLS; ++j) sum[j] = 0.f;
+            const unsigned lanes = (unsigned)(quarter * 32) << 16;
             bool ok = true;
             for (int c = c0; c < c1; ++c, ++i) {
                 const int buf = i % S::BUFFERS;
@@ -279,36 +351,54 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
                 __syncwarp();
                 if (!mbar_wait(&acc_full[buf], (i / S::BUFFERS) & 1)) { give_up = 1; ok = false; break; }
                 tc_fence_after();
-                const unsigned from = tmem + buf * 3 * BN + col0 + ((unsigned)(quarter * 32) << 16);
+                const unsigned from = tmem + (6 + buf) * BN + col0 + lanes;
+                constexpr int PART = COLS < 16 ? COLS : 16;
 #pragma unroll
-                for (int j = 0; j < COLS; j += 8) {
-                    unsigned r[3][8];
+                for (int j0 = 0; j0 < COLS; j0 += PART) {
+                    unsigned r[PART];
 #pragma unroll
-                    for (int h = 0; h < 3; ++h) tmem_load8(from + h * BN + j, r[h]);
+                    for (int j = 0; j < PART; j += 8) tmem_load8(from + j0 + j, r + j);
                     asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) sum[j + e] += __uint_as_float(r[0][e]) + (__uint_as_float(r[1][e]) + __uint_as_float(r[2][e]));
+                    for (int j = 0; j < PART; ++j) sum[j0 + j] += __uint_as_float(r[j]);
                 }
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&acc_empty[buf]);
             }
             if (!ok) break;
+            // the last chunk's MMAs are done, and so are those of the small sums
             const int n = w0 + quarter * 32 + lane;
-            if (n >= N) continue;
-            const float add = part == nullptr && bias != nullptr ? bias[n] : 0.f;
-            float* const out = part == nullptr ? C : part + (size_t)seg * M * N;
+            const bool whole = part == nullptr;              // else the segments' sums are looked at when they are added up
+            const float add = whole && bias != nullptr && n < N ? bias[n] : 0.f;
+            float* const out = whole ? C : part + (size_t)seg * M * N;
+            unsigned which = 0, zero = 0;
+            const unsigned from = tmem + (turn & 1) * 3 * BN + col0 + lanes;
 #pragma unroll
-            for (int j = 0; j < COLS; ++j) {
-                const int m = m0 + col0 + j;
-                if (m >= M) continue;
-                float v = sum[j];
-                if (!(fabsf(v) <= 3.402823466e38f)) {
-                    v = 0.f;
-                    for (int k = c0 * CHUNK; k < min(K, c1 * CHUNK); ++k) v = fmaf(A[(size_t)m * K + k], W[(size_t)n * K + k], v);
+            for (int j0 = 0; j0 < COLS; j0 += 8) {
+                unsigned r[3][8];
+#pragma unroll
+                for (int h = 0; h < 3; ++h) tmem_load8(from + h * BN + j0, r[h]);
+                asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    const int j = j0 + e, m = m0 + col0 + j;
+                    const float large = sum[j], small = __uint_as_float(r[0][e]) + (__uint_as_float(r[1][e]) + __uint_as_float(r[2][e]));
+                    const float v = large + small;
+                    if (n >= N || m >= M) continue;
+                    out[(size_t)m * N + n] = v + add;
+                    if (!whole) {                            // what large + small lost (Knuth's two-sum)
+                        const float p = v - large;
+                        rest[((size_t)seg * M + m) * N + n] = from_float<bf16>((large - (v - p)) + (small - p));
+                    }
+                    if (outside(v)) which |= 1u << j;
+                    if (v == 0.f) zero |= 1u << j;
                 }
-                out[(size_t)m * N + n] = v + add;
             }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&small_empty[turn & 1]);
+            if (whole && __any_sync(0xffffffffu, which != 0)) form_again(A, W, bias, C, m0 + col0, n, N, K, which, zero);
         }
     }
     __syncthreads();
@@ -318,35 +408,66 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
     if (warp == SPLIT_WARPS) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "n"(S::COLUMNS) : "memory");
 }
 
-// C = the segments' sums in order, + bias.
-__global__ void __launch_bounds__(256) add_segments_kernel(const float* __restrict__ part, const float* __restrict__ bias, float* __restrict__ C,
-                                                           const long long total, const int N, const int segments) {
+// C = the segments' sums in order, + bias.  A thread takes four numbers; a warp those of its lanes that are to be formed again.
+__global__ void __launch_bounds__(256) add_segments_kernel(const float* __restrict__ part, const bf16* __restrict__ rest, const float* __restrict__ A,
+                                                           const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C,
+                                                           const long long total, const int N, const int K, const int segments) {
     griddep_wait();
     griddep_launch_dependents();
     const long long i = ((long long)blockIdx.x * 256 + threadIdx.x) * 4;
-    if (i >= total) return;
-    if ((total & 3) == 0 && (N & 3) == 0) {
-        float4 v = *reinterpret_cast<const float4*>(part + i);
-        for (int s = 1; s < segments; ++s) {
+    const int count = (int)max(0LL, min(total - i, 4LL));
+    double sum[4] = {0., 0., 0., 0.};
+    if (count == 4 && (total & 3) == 0) {
+        for (int s = 0; s < segments; ++s) {
             const float4 p = *reinterpret_cast<const float4*>(part + s * total + i);
-            v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
+            const uint2 q = *reinterpret_cast<const uint2*>(rest + s * total + i);
+            sum[0] += (double)p.x + (double)__uint_as_float(q.x << 16);
+            sum[1] += (double)p.y + (double)__uint_as_float(q.x & 0xffff0000u);
+            sum[2] += (double)p.z + (double)__uint_as_float(q.y << 16);
+            sum[3] += (double)p.w + (double)__uint_as_float(q.y & 0xffff0000u);
         }
-        if (bias) {
-            const int n = (int)(i % N);
-            v.x += bias[n]; v.y += bias[n + 1]; v.z += bias[n + 2]; v.w += bias[n + 3];
+    } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            if (e >= count) continue;
+            for (int s = 0; s < segments; ++s) sum[e] += (double)part[s * total + i + e] + (double)to_float<bf16>(rest[s * total + i + e]);
         }
-        C[i] = v.x; C[i + 1] = v.y; C[i + 2] = v.z; C[i + 3] = v.w;
-        return;
     }
-    for (long long j = i; j < min(total, i + 4); ++j) {
-        float v = part[j];
-        for (int s = 1; s < segments; ++s) v += part[s * total + j];
-        C[j] = v + (bias ? bias[j % N] : 0.f);
+    float v[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[e] = (float)sum[e];
+    unsigned which = 0;
+    const int n0 = count > 0 ? (int)(i % N) : 0;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        if (e >= count) continue;
+        const int n = n0 + e < N ? n0 + e : (n0 + e) % N;
+        C[i + e] = v[e] + (bias ? bias[n] : 0.f);
+        if (outside(v[e])) which |= (v[e] == 0.f ? 17u : 1u) << e;
+    }
+    long long m_known = -1;
+    bool m_zero = false;                               // whether row m_known of A is 0
+    for (unsigned lanes = __ballot_sync(0xffffffffu, which != 0); lanes; lanes &= lanes - 1) {
+        const int l = __ffs(lanes) - 1;
+        const unsigned of = __shfl_sync(0xffffffffu, which, l);
+        const long long from = __shfl_sync(0xffffffffu, i, l);
+        for (int e = 0; e < 4; ++e) {
+            if (!(of >> e & 1u)) continue;
+            const long long m = (from + e) / N;
+            const int n = (int)((from + e) % N);
+            const float *a = A + (size_t)m * K, *w = W + (size_t)n * K;
+            if (of >> (e + 4) & 1u) {
+                if (m != m_known) m_known = m, m_zero = all_zero(a, K);
+                if (m_zero || all_zero(w, K)) continue;
+            }
+            const float again = product64(a, w, K);
+            if ((threadIdx.x & 31) == l) C[from + e] = again + (bias ? bias[n] : 0.f);
+        }
     }
 }
 
 template <int BN, bool VEC>
-int launch_split(const float* A, const float* W, const float* bias, float* C, float* part, int M, int N, int K, int segments, int* status, cudaStream_t stream) {
+int launch_split(const float* A, const float* W, const float* bias, float* C, float* part, bf16* rest, int M, int N, int K, int segments, int* status, cudaStream_t stream) {
     const auto kernel = gemm_split_kernel<BN, VEC>;
     cudaError_t err = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Sizes<BN>::BYTES);
     if (err == cudaSuccess) err = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributePreferredSharedMemoryCarveout, (Sizes<BN>::BYTES + 2048) * 100 / (228 * 1024) + 1);
@@ -354,7 +475,7 @@ int launch_split(const float* A, const float* W, const float* bias, float* C, fl
     const long long m_tiles = (M + BN - 1) / BN, tiles = m_tiles * ((N + TILE_W - 1) / TILE_W) * segments;
     FE_REQUIRE(tiles < (1LL << 30), "gemm_split: too many tiles");
     const int sms = fe_sm_count();
-    fe::launch(kernel, (unsigned)(tiles < sms ? tiles : sms), THREADS, Sizes<BN>::BYTES, stream, A, W, bias, C, segments > 1 ? part : (float*)nullptr, M, N, K,
+    fe::launch(kernel, (unsigned)(tiles < sms ? tiles : sms), THREADS, Sizes<BN>::BYTES, stream, A, W, bias, C, segments > 1 ? part : (float*)nullptr, rest, M, N, K,
                (int)m_tiles, (int)tiles, segments, status);
     return fe_check_launch("gemm_split");
 }
@@ -369,22 +490,23 @@ extern "C" int fe_gemm_split_segments(int N, int K) {
     return s < 1 ? 1 : s;
 }
 
-// ``part``: room for segments x M x N floats (16-byte aligned); not read with one segment.
+// ``part``: 16-byte aligned room for segments x M x N numbers of six bytes; not read with one segment.
 extern "C" int fe_gemm_split(const float* A, const float* W, const float* bias, float* C, float* part, int M, int N, int K, int* status,
                              cudaStream_t stream) {
-    FE_REQUIRE(M >= 0 && N > 0 && K > 0, "gemm_split: bad sizes M=%d N=%d K=%d", M, N, K);
+    FE_REQUIRE(M >= 0 && N > 0 && K > 3 * CHUNK, "gemm_split: bad sizes M=%d N=%d K=%d", M, N, K);
     if (M == 0) return 0;
     const int segments = fe_gemm_split_segments(N, K);
     FE_REQUIRE(segments == 1 || (part != nullptr && ((size_t)part & 15) == 0), "gemm_split: no room for the sums of %d segments", segments);
+    const long long total = (long long)M * N;
+    bf16* rest = reinterpret_cast<bf16*>(part + segments * total);
     const bool vec = (K & 3) == 0 && (((size_t)A | (size_t)W) & 15) == 0;
     int rc;
-#define FE_SPLIT(BN) rc = vec ? launch_split<BN, true>(A, W, bias, C, part, M, N, K, segments, status, stream) \
-                              : launch_split<BN, false>(A, W, bias, C, part, M, N, K, segments, status, stream)
+#define FE_SPLIT(BN) rc = vec ? launch_split<BN, true>(A, W, bias, C, part, rest, M, N, K, segments, status, stream) \
+                              : launch_split<BN, false>(A, W, bias, C, part, rest, M, N, K, segments, status, stream)
     if (M <= 16) FE_SPLIT(16);
     else FE_SPLIT(64);
 #undef FE_SPLIT
     if (rc || segments == 1) return rc;
-    const long long total = (long long)M * N;
-    fe::launch(add_segments_kernel, (unsigned)((total + 1023) / 1024), 256, 0, stream, (const float*)part, bias, C, total, N, segments);
+    fe::launch(add_segments_kernel, (unsigned)((total + 1023) / 1024), 256, 0, stream, (const float*)part, (const bf16*)rest, A, W, bias, C, total, N, K, segments);
     return fe_check_launch("gemm_split (segments)");
 }

@@ -47,3 +47,68 @@ def test_what_is_no_finite_number_comes_out_as_from_the_chain(gen):
     torch.testing.assert_close(got[finite], want[finite], atol=1e-3, rtol=1e-5)
     x[5], w[9] = 3e38, 2.0                        # a sum beyond the largest number
     assert float(ops().linear(x, w)[5, 9]) == float("inf")
+
+
+FEW = [(8200, 1024), (1536, 8960), (129, 65537)]              # one segment, several, rows on no 16-byte boundary
+
+
+def both(x, w):
+    """The product's result and the chain's, with what 64 bits give."""
+    return ops().linear(x, w), chain(x, w), x.double() @ w.double().T
+
+
+@pytest.mark.parametrize("N,K", FEW)
+@pytest.mark.parametrize("nonzeros", [1, 2, 8, 16])
+def test_rows_of_few_numbers_are_as_close_as_by_multiply_adds(N, K, nonzeros, gen):
+    """What a product leaves out, a sum of few products shows.  One product: the four sums of a chunk (the larger by 2^7 each) are exact
+    but for their last places, so that a result is rounded once to float32, after a sum rounded 2^-7 below it: (1 + 2^-4) 2^-24."""
+    x = torch.zeros(80, K, device=DEV)
+    for r in range(80):
+        x[r, torch.randperm(K, device=DEV, generator=gen)[:nonzeros]] = rand((nonzeros,), torch.float32, gen)
+    x[0, x[0] != 0] = 1 + 2 ** -7 - 2 ** -23                  # all places below the first eight at their largest
+    w = rand((N, K), torch.float32, gen)
+    w[:64] = 1 + 2 ** -7 - 2 ** -23
+    got, by_chain, want = both(x, w)
+    if nonzeros == 1:
+        assert bool(((got.double() - want).abs() <= (1 + 2 ** -4) * 2 ** -24 * want.abs()).all())
+    # 1 %: the second rounding, and how far norms of this many errors are from their mean
+    assert float((got.double() - want).norm()) <= 1.01 * float((by_chain.double() - want).norm())
+
+
+@pytest.mark.parametrize("N,K", FEW)
+@pytest.mark.parametrize("scales", [(-30, 0), (-34, 0), (-36, 0), (-38, 0), (-41, 0), (0, -36), (-37, 37), (37, -37), (-18, -18), (-20, -20)])
+def test_small_numbers_keep_their_places(N, K, scales, gen):
+    """Rows or matrices whose third parts, or second ones, are below what bfloat16 holds (1e-40), alone or met by large numbers."""
+    def scaled(shape, e):
+        v = rand(shape, torch.float32, gen)
+        return v * 10.0 ** (e / 2) * 10.0 ** (e / 2)
+    x, w = scaled((20, K), scales[0]), scaled((N, K), scales[1])
+    x[3] = 0
+    w[5] = 0
+    got, by_chain, want = both(x, w)
+    assert float((got.double() - want).norm()) <= 1.01 * float((by_chain.double() - want).norm())
+    assert not bool(got[3].any()) and not bool(got[:, 5].any())
+    assert torch.equal(ops().linear(x[:9].contiguous(), w), got[:9])
+
+
+def test_a_small_number_beside_ordinary_ones_counts_where_the_others_meet_zeros(gen):
+    """Also where what meets it is a large number, so that the result is an ordinary one."""
+    x, w = rand((20, 8960), torch.float32, gen), rand((1536, 8960), torch.float32, gen)
+    x[4, 7], w[9], w[9, 7] = 1.2345678e-36, 0.0, 1.0
+    x[5, 8], w[10], w[10, 8] = 1.2345678e-36, 0.0, 7.6543211e36
+    got, by_chain, _ = both(x, w)
+    assert float(got[4, 9]) == float(by_chain[4, 9]) and float(got[5, 10]) == float(by_chain[5, 10])
+
+
+def test_not_finite_over_several_segments(gen):
+    x, w = rand((20, 8960), torch.float32, gen), rand((1536, 8960), torch.float32, gen)
+    x[3, 5], x[4, 6], w[7, 9], w[8, 8000] = float("inf"), float("nan"), float("-inf"), float("inf")
+    x[5, 100], x[5, 8900] = float("inf"), float("-inf")        # both signs, in segments of their own
+    x[6, 100], x[6, 8900], w[9] = 3e38, -3e38, 2.0             # beyond the largest number on the way, not at the end
+    got, want, exact = both(x, w)
+    for test in (torch.isnan, torch.isposinf, torch.isneginf):
+        keep = torch.ones_like(got, dtype=torch.bool)
+        keep[6] = False
+        assert torch.equal(test(got)[keep], test(want)[keep])
+    finite = torch.isfinite(want) & torch.isfinite(got)
+    assert float((got[finite].double() - exact[finite]).norm()) <= float((want[finite].double() - exact[finite]).norm())
