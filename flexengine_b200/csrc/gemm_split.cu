@@ -207,6 +207,13 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
     tc_fence_after();
     const unsigned tmem = tmem_holder;
 
+    // After a wait that ran out, here or in another warp, all lanes of a warp leave together: their votes and barriers are the warp's.
+    auto go_on = [&](bool arrived) {
+        if (__all_sync(0xffffffffu, arrived && !give_up)) return true;
+        give_up = 1;
+        return false;
+    };
+
     if (warp < SPLIT_WARPS) {
         // ---- float32 rows into three bfloat16 parts: an item is eight k's of a row ----
         constexpr int ITEMS_W = TILE_W * 8 / (32 * GROUP_WARPS), ITEMS_X = BN >= 32 ? BN * 8 / (32 * GROUP_WARPS) : 1;
@@ -276,14 +283,14 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
         int at_chunk = turn;
         auto stage_free = [&](int& s) {
             s = at_chunk % S::STAGES;
-            if (!mbar_wait(&empty_bar[s], ((at_chunk / S::STAGES) & 1) ^ 1)) { give_up = 1; return false; }
+            if (!go_on(mbar_wait(&empty_bar[s], ((at_chunk / S::STAGES) & 1) ^ 1))) return false;
             at_chunk += 2;
             return true;
         };
         // the rows of W of the next chunk are asked for before the rows of A of this one are cut up, and the other way round
         float4 vw[2 * ITEMS_W], vx[2 * ITEMS_X];
         if (nt < tiles) { load_w(vw); load_x(vx); }
-        while (nt < tiles && !give_up) {
+        while (nt < tiles) {
             int s;
             if (!stage_free(s)) break;
             const unsigned to = base + s * S::STAGE;
@@ -337,7 +344,7 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
             if (S::BUFFERS > 2) issue();
         }
         int i = 0, turn = 0;
-        for (int t = blockIdx.x; t < tiles && !give_up; t += gridDim.x, ++turn) {
+        for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++turn) {
             int w0, m0, c0, c1, seg;
             place(t, w0, m0, c0, c1, seg);
             float sum[COLS];
@@ -349,7 +356,7 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
                 const int buf = i % S::BUFFERS;
                 if (issuer) issue();
                 __syncwarp();
-                if (!mbar_wait(&acc_full[buf], (i / S::BUFFERS) & 1)) { give_up = 1; ok = false; break; }
+                if (!(ok = go_on(mbar_wait(&acc_full[buf], (i / S::BUFFERS) & 1)))) break;
                 tc_fence_after();
                 const unsigned from = tmem + (6 + buf) * BN + col0 + lanes;
                 constexpr int PART = COLS < 16 ? COLS : 16;
@@ -400,6 +407,8 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
             if (lane == 0) mbar_arrive(&small_empty[turn & 1]);
             if (whole && __any_sync(0xffffffffu, which != 0)) form_again(A, W, bias, C, m0 + col0, n, N, K, which, zero);
         }
+        // Only after a wait that ran out are any MMAs still at work here: they end before the tensor memory is given back
+        if (issuer && issued > 0) mbar_wait(&acc_full[(issued - 1) % S::BUFFERS], ((issued - 1) / S::BUFFERS) & 1);
     }
     __syncthreads();
     if (give_up && tid == 0 && status) atomicOr(status, FE_STATUS_WAIT_EXPIRED);
