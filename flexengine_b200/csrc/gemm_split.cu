@@ -22,12 +22,12 @@
 // M), so that a handful of rows streams W once.
 //
 // Blocks stay for tile after tile.  Two groups of eight warps read float32 rows, chunk about, and write the three parts into
-// 128-byte-swizzled tiles; one thread issues 16 MMAs a chunk; eight more warps add the chunks' sums to their registers and write the
-// tile out at the end.
+// 128-byte-swizzled tiles; a thread of its own issues 16 MMAs a chunk; eight more warps add the chunks' sums to their registers and
+// write the tile out at the end, while MMAs of the next one run.
 //
-// A chunk's way (rows from memory, cut up, through shared memory, 16 MMAs, sums) takes 1.2 to 1.5 us and is what bounds the kernel: loads
-// on their way, and shared memory, through which a number goes as four bytes, then as six, then to the tensor cores once an MMA.  17,920 x 1,536:
-// 39 us with 1 to 16 rows (the chain of multiply-adds 26 to 42), 45 with 64 (108), 151 with 256 (279); 1,536 x 8,960: 42 (33 to 70), 49 (127), 87 (246).
+// A chunk's way (rows from memory, cut up, through shared memory, 16 MMAs, sums) takes 1.0 to 1.3 us and is what bounds the kernel: with no MMA
+// but one a step 17,920 x 1,536 takes 30 and 122 us (4 and 256 rows), with no stores to shared memory 27 and 107; asking rows into L2 ahead of time
+// makes it slower (33, 138).  17,920 x 1,536: 31 us with 1 to 16 rows (the chain of multiply-adds 24 to 40), 40 with 64 (106), 135 with 256 (278).
 // Relative error against 64 bits, K = 1,536 / 8,960: 1.2e-7 / 1.2e-7, the chain 7.0e-7 / 1.7e-6; rows of 1, 2, 8 and 32 numbers other than 0:
 // 2.5e-8, 2.6e-8, 2.8e-8, 4.2e-8, the chain 2.5e-8, 3.1e-8, 5.2e-8, 1.0e-7.
 #include "common.cuh"
@@ -38,7 +38,7 @@ namespace {
 
 constexpr int TILE_W = 128;             // rows of W in a tile = UMMA M
 constexpr int CHUNK = 64;               // k's of a chunk: 128 bytes of bfloat16, one swizzle atom wide
-constexpr int GROUP_WARPS = 8, SPLIT_WARPS = 2 * GROUP_WARPS, SUM_WARPS = 8, THREADS = 32 * (SPLIT_WARPS + SUM_WARPS);
+constexpr int GROUP_WARPS = 8, SPLIT_WARPS = 2 * GROUP_WARPS, SUM_WARPS = 8, THREADS = 32 * (SPLIT_WARPS + SUM_WARPS + 4);
 constexpr long long WAIT_LIMIT = 4000000000LL;      // clock cycles
 constexpr float LEAST = 8.673617380e-19f, MOST = 3.402823466e38f;      // 2^-60; results outside of these bounds are formed again
 constexpr unsigned LARGE = 0x4f80;                  // 2^32, the upper half of the word
@@ -186,8 +186,8 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
         const int u = t / segments;
         m0 = u % m_tiles * BN;
         w0 = u / m_tiles * TILE_W;
-        c0 = (int)((long long)chunks * s / segments);
-        c1 = (int)((long long)chunks * (s + 1) / segments);
+        c0 = (int)((unsigned)chunks * s / segments);           // 2^25 chunks and 64 segments at most
+        c1 = (int)((unsigned)chunks * (s + 1) / segments);
     };
     if (tid == 0) {
         for (int s = 0; s < S::STAGES; ++s) { mbar_init(&full_bar[s], GROUP_WARPS); mbar_init(&empty_bar[s], 1); }
@@ -214,7 +214,10 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
         return false;
     };
 
+    // Registers: 28 warps of 72 at launch, 64,512 together.  The sixteen that cut up hold 48 numbers on their way and take 80 each (with 72, 256 rows x
+    // 17,920 x 1,536: 191 us instead of 143), which the issuing thread's four warps give: 16 x 80 + 8 x 72 + 4 x 40 = 28 x 72.
     if (warp < SPLIT_WARPS) {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 80;\n" ::: "memory");
         // ---- float32 rows into three bfloat16 parts: an item is eight k's of a row ----
         constexpr int ITEMS_W = TILE_W * 8 / (32 * GROUP_WARPS), ITEMS_X = BN >= 32 ? BN * 8 / (32 * GROUP_WARPS) : 1;
         // two groups of eight warps take turns: while one waits for its loads, a free stage or its stores, the other is at work
@@ -302,47 +305,10 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
             if (nt < tiles) load_x(vx);
             done(s);
         }
-    } else {
+    } else if (warp < SPLIT_WARPS + SUM_WARPS) {
         // ---- sums: warp w reads TMEM lanes 32 (w % 4) .. + 31 (rows of W), one half of the columns (rows of A) ----
         constexpr int COLS = BN / 2;
         const int quarter = warp & 3, col0 = ((warp - SPLIT_WARPS) >> 2) * COLS;
-        // one thread issues the MMAs, a chunk or two ahead of the one it adds up (a tile has four chunks or more)
-        int it = blockIdx.x, ic = 0, ic1 = 0, issued = 0, tile = -1;
-        auto issue = [&]() {
-            if (it >= tiles || give_up) return;
-            const bool begins = ic >= ic1;                    // a tile
-            if (begins) {
-                int w0, m0, seg;
-                place(it, w0, m0, ic, ic1, seg);
-                ++tile;
-            }
-            const int s = issued % S::STAGES, buf = issued % S::BUFFERS;
-            if (!mbar_wait(&full_bar[s], (issued / S::STAGES) & 1) || !mbar_wait(&acc_empty[buf], ((issued / S::BUFFERS) & 1) ^ 1) ||
-                (begins && !mbar_wait(&small_empty[tile & 1], ((tile >> 1) & 1) ^ 1))) { give_up = 1; return; }
-            tc_fence_after();
-            const unsigned w = base + s * S::STAGE, x = w + 3 * S::W_PART;
-            const unsigned small = tmem + (tile & 1) * 3 * BN, large = tmem + (6 + buf) * BN;
-            // The parts of A's rows lie one after the other like 3 BN rows: a part of W meets as many of them as count at once.
-            // Block 0 of the small sums takes w0 a1 + w1 a0, block 1 w0 a2 + w1 a1 + w2 a0, block 2 w1 a2 + w2 a1.
-            const unsigned long long w0 = smem_desc(w), w1 = smem_desc(w + S::W_PART), w2 = smem_desc(w + 2 * S::W_PART);
-            const unsigned long long x0 = smem_desc(x), x1 = smem_desc(x + S::X_PART);
-#pragma unroll
-            for (int k = 0; k < CHUNK / 16; ++k) {
-                umma(small, w1 + 2 * k, x0 + 2 * k, instr_desc(3 * BN), (k > 0 || !begins) ? 1u : 0u);
-                umma(small, w0 + 2 * k, x1 + 2 * k, instr_desc(2 * BN), 1u);
-                umma(small + BN, w2 + 2 * k, x0 + 2 * k, instr_desc(2 * BN), 1u);
-                umma(large, w0 + 2 * k, x0 + 2 * k, instr_desc(BN), k > 0 ? 1u : 0u);
-            }
-            umma_commit(&empty_bar[s]);
-            umma_commit(&acc_full[buf]);
-            ++issued;
-            if (++ic >= ic1) it += gridDim.x;
-        };
-        const bool issuer = tid == SPLIT_WARPS * 32;
-        if (issuer) {
-            issue();
-            if (S::BUFFERS > 2) issue();
-        }
         int i = 0, turn = 0;
         for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++turn) {
             int w0, m0, c0, c1, seg;
@@ -354,8 +320,6 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
             bool ok = true;
             for (int c = c0; c < c1; ++c, ++i) {
                 const int buf = i % S::BUFFERS;
-                if (issuer) issue();
-                __syncwarp();
                 if (!(ok = go_on(mbar_wait(&acc_full[buf], (i / S::BUFFERS) & 1)))) break;
                 tc_fence_after();
                 const unsigned from = tmem + (6 + buf) * BN + col0 + lanes;
@@ -378,7 +342,10 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
             const int n = w0 + quarter * 32 + lane;
             const bool whole = part == nullptr;              // else the segments' sums are looked at when they are added up
             const float add = whole && bias != nullptr && n < N ? bias[n] : 0.f;
-            float* const out = whole ? C : part + (size_t)seg * M * N;
+            const int rows = n < N ? M - m0 - col0 : 0;
+            const size_t first = (size_t)(m0 + col0) * N + n;
+            float* out = (whole ? C : part + (size_t)seg * M * N) + first;
+            bf16* left = whole ? nullptr : rest + (size_t)seg * M * N + first;
             unsigned which = 0, zero = 0;
             const unsigned from = tmem + (turn & 1) * 3 * BN + col0 + lanes;
 #pragma unroll
@@ -389,17 +356,20 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
                 asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
                 for (int e = 0; e < 8; ++e) {
-                    const int j = j0 + e, m = m0 + col0 + j;
+                    const int j = j0 + e;
                     const float large = sum[j], small = __uint_as_float(r[0][e]) + (__uint_as_float(r[1][e]) + __uint_as_float(r[2][e]));
                     const float v = large + small;
-                    if (n >= N || m >= M) continue;
-                    out[(size_t)m * N + n] = v + add;
-                    if (!whole) {                            // what large + small lost (Knuth's two-sum)
-                        const float p = v - large;
-                        rest[((size_t)seg * M + m) * N + n] = from_float<bf16>((large - (v - p)) + (small - p));
+                    if (j < rows) {
+                        *out = v + add;
+                        if (!whole) {                        // what large + small lost (Knuth's two-sum)
+                            const float p = v - large;
+                            *left = from_float<bf16>((large - (v - p)) + (small - p));
+                        }
+                        if (outside(v)) which |= 1u << j;
+                        if (v == 0.f) zero |= 1u << j;
                     }
-                    if (outside(v)) which |= 1u << j;
-                    if (v == 0.f) zero |= 1u << j;
+                    out += N;
+                    left += N;
                 }
             }
             tc_fence_before();
@@ -407,8 +377,42 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
             if (lane == 0) mbar_arrive(&small_empty[turn & 1]);
             if (whole && __any_sync(0xffffffffu, which != 0)) form_again(A, W, bias, C, m0 + col0, n, N, K, which, zero);
         }
-        // Only after a wait that ran out are any MMAs still at work here: they end before the tensor memory is given back
-        if (issuer && issued > 0) mbar_wait(&acc_full[(issued - 1) % S::BUFFERS], ((issued - 1) / S::BUFFERS) & 1);
+    } else {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 40;\n" ::: "memory");
+        if (warp == SPLIT_WARPS + SUM_WARPS && lane == 0) {
+            // ---- one thread issues the MMAs; three warps only give registers ----
+            int issued = 0, tile = 0;
+            bool ok = true;
+            for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++tile) {
+                int w0, m0, c0, c1, seg;
+                place(t, w0, m0, c0, c1, seg);
+                for (int c = c0; c < c1; ++c, ++issued) {
+                    const int s = issued % S::STAGES, buf = issued % S::BUFFERS;
+                    ok = mbar_wait(&full_bar[s], (issued / S::STAGES) & 1) && mbar_wait(&acc_empty[buf], ((issued / S::BUFFERS) & 1) ^ 1) &&
+                         (c > c0 || mbar_wait(&small_empty[tile & 1], ((tile >> 1) & 1) ^ 1)) && !give_up;
+                    if (!ok) break;
+                    tc_fence_after();
+                    const unsigned w = base + s * S::STAGE, x = w + 3 * S::W_PART;
+                    const unsigned small = tmem + (tile & 1) * 3 * BN, large = tmem + (6 + buf) * BN;
+                    // The parts of A's rows lie one after the other like 3 BN rows: a part of W meets as many of them as count at once.
+                    // Block 0 of the small sums takes w0 a1 + w1 a0, block 1 w0 a2 + w1 a1 + w2 a0, block 2 w1 a2 + w2 a1.
+                    const unsigned long long dw0 = smem_desc(w), dw1 = smem_desc(w + S::W_PART), dw2 = smem_desc(w + 2 * S::W_PART);
+                    const unsigned long long dx0 = smem_desc(x), dx1 = smem_desc(x + S::X_PART);
+#pragma unroll
+                    for (int k = 0; k < CHUNK / 16; ++k) {
+                        umma(small, dw1 + 2 * k, dx0 + 2 * k, instr_desc(3 * BN), (k > 0 || c > c0) ? 1u : 0u);
+                        umma(small, dw0 + 2 * k, dx1 + 2 * k, instr_desc(2 * BN), 1u);
+                        umma(small + BN, dw2 + 2 * k, dx0 + 2 * k, instr_desc(2 * BN), 1u);
+                        umma(large, dw0 + 2 * k, dx0 + 2 * k, instr_desc(BN), k > 0 ? 1u : 0u);
+                    }
+                    umma_commit(&empty_bar[s]);
+                    umma_commit(&acc_full[buf]);
+                }
+            }
+            if (!ok) give_up = 1;
+            // Only after a wait that ran out are any MMAs still at work when the sums are done: they end before the tensor memory is given back
+            if (issued > 0) mbar_wait(&acc_full[(issued - 1) % S::BUFFERS], ((issued - 1) / S::BUFFERS) & 1);
+        }
     }
     __syncthreads();
     if (give_up && tid == 0 && status) atomicOr(status, FE_STATUS_WAIT_EXPIRED);
@@ -427,6 +431,7 @@ __global__ void __launch_bounds__(256) add_segments_kernel(const float* __restri
     const int count = (int)max(0LL, min(total - i, 4LL));
     double sum[4] = {0., 0., 0., 0.};
     if (count == 4 && (total & 3) == 0) {
+#pragma unroll 4
         for (int s = 0; s < segments; ++s) {
             const float4 p = *reinterpret_cast<const float4*>(part + s * total + i);
             const uint2 q = *reinterpret_cast<const uint2*>(rest + s * total + i);
