@@ -166,11 +166,12 @@ __device__ __noinline__ void form_again(const float* __restrict__ A, const float
     }
 }
 
-// ``part`` (null with one segment): the segments' sums, [segments][M][N], and ``rest`` what their rounding lost.
+// ``part`` (null with one segment): the segments' sums, [segments][M / 4, rounded up][N][4], and ``rest`` what their rounding lost: a thread has
+// rows of A one after the other, and writes four at once.
 template <int BN, bool VEC>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C,
-                  float* __restrict__ part, bf16* __restrict__ rest, const int M, const int N, const int K, const int m_tiles, const int tiles,
+                  float4* __restrict__ part, uint2* __restrict__ rest, const int M, const int N, const int K, const int m_tiles, const int tiles,
                   const int segments, int* __restrict__ status) {
     using S = Sizes<BN>;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -339,13 +340,11 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
             }
             if (!ok) break;
             // the last chunk's MMAs are done, and so are those of the small sums
-            const int n = w0 + quarter * 32 + lane;
+            const int n = w0 + quarter * 32 + lane, rows = n < N ? M - m0 - col0 : 0;
             const bool whole = part == nullptr;              // else the segments' sums are looked at when they are added up
             const float add = whole && bias != nullptr && n < N ? bias[n] : 0.f;
-            const int rows = n < N ? M - m0 - col0 : 0;
-            const size_t first = (size_t)(m0 + col0) * N + n;
-            float* out = (whole ? C : part + (size_t)seg * M * N) + first;
-            bf16* left = whole ? nullptr : rest + (size_t)seg * M * N + first;
+            float* out = C + (size_t)(m0 + col0) * N + n;
+            size_t four = ((size_t)seg * ((M + 3) / 4) + (m0 + col0) / 4) * N + n;
             unsigned which = 0, zero = 0;
             const unsigned from = tmem + (turn & 1) * 3 * BN + col0 + lanes;
 #pragma unroll
@@ -355,21 +354,33 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
                 for (int h = 0; h < 3; ++h) tmem_load8(from + h * BN + j0, r[h]);
                 asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    const int j = j0 + e;
-                    const float large = sum[j], small = __uint_as_float(r[0][e]) + (__uint_as_float(r[1][e]) + __uint_as_float(r[2][e]));
-                    const float v = large + small;
-                    if (j < rows) {
+                for (int e = 0; e < 8; ++e) r[0][e] = __float_as_uint(__uint_as_float(r[0][e]) + (__uint_as_float(r[1][e]) + __uint_as_float(r[2][e])));
+                if (whole) {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e, out += N) {
+                        const int j = j0 + e;
+                        const float v = sum[j] + __uint_as_float(r[0][e]);
+                        if (j >= rows) continue;
                         *out = v + add;
-                        if (!whole) {                        // what large + small lost (Knuth's two-sum)
-                            const float p = v - large;
-                            *left = from_float<bf16>((large - (v - p)) + (small - p));
-                        }
                         if (outside(v)) which |= 1u << j;
                         if (v == 0.f) zero |= 1u << j;
                     }
-                    out += N;
-                    left += N;
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 8; e += 4, four += N) {
+                        float v[4], lost[4];
+#pragma unroll
+                        for (int i4 = 0; i4 < 4; ++i4) {     // and what large + small lose (Knuth's two-sum)
+                            const float large = sum[j0 + e + i4], small = __uint_as_float(r[0][e + i4]);
+                            v[i4] = large + small;
+                            const float p = v[i4] - large;
+                            lost[i4] = (large - (v[i4] - p)) + (small - p);
+                        }
+                        if (j0 + e >= rows) continue;
+                        part[four] = make_float4(v[0], v[1], v[2], v[3]);
+                        const __nv_bfloat162 a = __floats2bfloat162_rn(lost[0], lost[1]), b = __floats2bfloat162_rn(lost[2], lost[3]);
+                        rest[four] = make_uint2(*reinterpret_cast<const unsigned*>(&a), *reinterpret_cast<const unsigned*>(&b));
+                    }
                 }
             }
             tc_fence_before();
@@ -421,67 +432,49 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
     if (warp == SPLIT_WARPS) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "n"(S::COLUMNS) : "memory");
 }
 
-// C = the segments' sums in order, + bias.  A thread takes four numbers; a warp those of its lanes that are to be formed again.
-__global__ void __launch_bounds__(256) add_segments_kernel(const float* __restrict__ part, const bf16* __restrict__ rest, const float* __restrict__ A,
+// C = the segments' sums in order, + bias.  A thread takes four rows of A and a row of W; a warp what is to be formed again.
+__global__ void __launch_bounds__(256) add_segments_kernel(const float4* __restrict__ part, const uint2* __restrict__ rest, const float* __restrict__ A,
                                                            const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C,
-                                                           const long long total, const int N, const int K, const int segments) {
+                                                           const int M, const int N, const int K, const int segments) {
     griddep_wait();
     griddep_launch_dependents();
-    const long long i = ((long long)blockIdx.x * 256 + threadIdx.x) * 4;
-    const int count = (int)max(0LL, min(total - i, 4LL));
+    const long long i = (long long)blockIdx.x * 256 + threadIdx.x, all = (long long)((M + 3) / 4) * N;
+    const int m = i < all ? (int)(i / N) * 4 : M, n = (int)(i % N);
     double sum[4] = {0., 0., 0., 0.};
-    if (count == 4 && (total & 3) == 0) {
+    if (m < M) {
 #pragma unroll 4
         for (int s = 0; s < segments; ++s) {
-            const float4 p = *reinterpret_cast<const float4*>(part + s * total + i);
-            const uint2 q = *reinterpret_cast<const uint2*>(rest + s * total + i);
+            const float4 p = part[s * all + i];
+            const uint2 q = rest[s * all + i];
             sum[0] += (double)p.x + (double)__uint_as_float(q.x << 16);
             sum[1] += (double)p.y + (double)__uint_as_float(q.x & 0xffff0000u);
             sum[2] += (double)p.z + (double)__uint_as_float(q.y << 16);
             sum[3] += (double)p.w + (double)__uint_as_float(q.y & 0xffff0000u);
         }
-    } else {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            if (e >= count) continue;
-            for (int s = 0; s < segments; ++s) sum[e] += (double)part[s * total + i + e] + (double)to_float<bf16>(rest[s * total + i + e]);
-        }
     }
-    float v[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) v[e] = (float)sum[e];
-    unsigned which = 0;
-    const int n0 = count > 0 ? (int)(i % N) : 0;
+    unsigned which = 0, zero = 0;
+    const float add = bias ? bias[n] : 0.f;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-        if (e >= count) continue;
-        const int n = n0 + e < N ? n0 + e : (n0 + e) % N;
-        C[i + e] = v[e] + (bias ? bias[n] : 0.f);
-        if (outside(v[e])) which |= (v[e] == 0.f ? 17u : 1u) << e;
+        if (m + e >= M) continue;
+        const float v = (float)sum[e];
+        C[(size_t)(m + e) * N + n] = v + add;
+        if (outside(v)) which |= 1u << e;
+        if (v == 0.f) zero |= 1u << e;
     }
-    long long m_known = -1;
-    bool m_zero = false;                               // whether row m_known of A is 0
-    for (unsigned lanes = __ballot_sync(0xffffffffu, which != 0); lanes; lanes &= lanes - 1) {
-        const int l = __ffs(lanes) - 1;
-        const unsigned of = __shfl_sync(0xffffffffu, which, l);
-        const long long from = __shfl_sync(0xffffffffu, i, l);
-        for (int e = 0; e < 4; ++e) {
-            if (!(of >> e & 1u)) continue;
-            const long long m = (from + e) / N;
-            const int n = (int)((from + e) % N);
-            const float *a = A + (size_t)m * K, *w = W + (size_t)n * K;
-            if (of >> (e + 4) & 1u) {
-                if (m != m_known) m_known = m, m_zero = all_zero(a, K);
-                if (m_zero || all_zero(w, K)) continue;
-            }
-            const float again = product64(a, w, K);
-            if ((threadIdx.x & 31) == l) C[from + e] = again + (bias ? bias[n] : 0.f);
-        }
+    if (!__any_sync(0xffffffffu, which != 0)) return;
+    // The lanes' rows of W meet the same four rows of A, unless the warp reaches over the end of them
+    const int first = __shfl_sync(0xffffffffu, m, 0);
+    form_again(A, W, bias, C, first, n, N, K, m == first ? which : 0u, m == first ? zero : 0u);
+    for (unsigned others = __ballot_sync(0xffffffffu, m != first && which != 0); others; others &= others - 1) {
+        const int l = __ffs(others) - 1;
+        const bool mine = (threadIdx.x & 31) == l;
+        form_again(A, W, bias, C, __shfl_sync(0xffffffffu, m, l), n, N, K, mine ? which : 0u, mine ? zero : 0u);
     }
 }
 
 template <int BN, bool VEC>
-int launch_split(const float* A, const float* W, const float* bias, float* C, float* part, bf16* rest, int M, int N, int K, int segments, int* status, cudaStream_t stream) {
+int launch_split(const float* A, const float* W, const float* bias, float* C, float4* part, uint2* rest, int M, int N, int K, int segments, int* status, cudaStream_t stream) {
     const auto kernel = gemm_split_kernel<BN, VEC>;
     cudaError_t err = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Sizes<BN>::BYTES);
     if (err == cudaSuccess) err = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributePreferredSharedMemoryCarveout, (Sizes<BN>::BYTES + 2048) * 100 / (228 * 1024) + 1);
@@ -489,38 +482,57 @@ int launch_split(const float* A, const float* W, const float* bias, float* C, fl
     const long long m_tiles = (M + BN - 1) / BN, tiles = m_tiles * ((N + TILE_W - 1) / TILE_W) * segments;
     FE_REQUIRE(tiles < (1LL << 30), "gemm_split: too many tiles");
     const int sms = fe_sm_count();
-    fe::launch(kernel, (unsigned)(tiles < sms ? tiles : sms), THREADS, Sizes<BN>::BYTES, stream, A, W, bias, C, segments > 1 ? part : (float*)nullptr, rest, M, N, K,
+    fe::launch(kernel, (unsigned)(tiles < sms ? tiles : sms), THREADS, Sizes<BN>::BYTES, stream, A, W, bias, C, segments > 1 ? part : (float4*)nullptr, rest, M, N, K,
                (int)m_tiles, (int)tiles, segments, status);
     return fe_check_launch("gemm_split");
 }
 
+// Into how many segments K is cut, by N and K alone, so that a step of few rows has every SM at work: the least of rounds over the SMs x (a
+// segment's chunks and one to begin), two for adding up and one for every 16,384 numbers added, in the time of a chunk.  (As many
+// as gave every SM a tile of 128 rows with 256 of them were taken before: tiles have 64 rows, or 16, and 72 blocks stood on 148 SMs for
+// 1,536 x 8,960.)  Segments before and now, us with 4, 64 and 256 rows before and now, and the chain's with 4: 1,536 x 8,960 6, 12: 34, 43, 77 and 26, 30, 78 (31);
+// 4,608 x 3,584 2, 4: 36, 47, 88 and 25, 30, 88 (21); 3,584 x 18,944 2, 5: 154, 195, 385 and 70, 90, 315 (99); 5,120 x 13,824 1, 7: 238, 279, 564 and
+// 75, 96, 335 (116); 27,648 x 5,120 1, 2: 166, 213, 615 and 132, 181, 661 (122).
+int segments_of(int N, int K) {
+    const int sms = fe_sm_count(), tiles = (N + TILE_W - 1) / TILE_W, chunks = (K + CHUNK - 1) / CHUNK;
+    int best = 1;
+    long long least = 0;
+    for (int s = 1; s <= 64 && s <= chunks / 4; ++s) {
+        const long long rounds = ((long long)tiles * s + sms - 1) / sms;
+        const long long cost = 16384 * (rounds * ((chunks + s - 1) / s + 1) + (s > 1 ? 2 : 0)) + (s > 1 ? (long long)s * N : 0);
+        if (s == 1 || cost < least) best = s, least = cost;
+    }
+    return best;
+}
 }  // namespace
 
-// Into how many segments K is cut, by N and K alone: as many as give every SM a tile with 256 rows, of four chunks or more.
-extern "C" int fe_gemm_split_segments(int N, int K) {
-    const int sms = fe_sm_count(), tiles = 2 * ((N + TILE_W - 1) / TILE_W), chunks = (K + CHUNK - 1) / CHUNK;
-    int s = sms / tiles;
-    if (s > chunks / 4) s = chunks / 4;
-    return s < 1 ? 1 : s;
+extern "C" int fe_gemm_split_segments(int N, int K) { return segments_of(N, K); }
+
+// Bytes of room that a product needs for its segments' sums.
+extern "C" long long fe_gemm_split_room(int M, int N, int K) {
+    const int segments = segments_of(N, K);
+    if (segments == 1 || M <= 0) return 0;
+    return 24LL * segments * N * ((M + 3LL) / 4);
 }
 
-// ``part``: 16-byte aligned room for segments x M x N numbers of six bytes; not read with one segment.
+// ``part``: 16-byte aligned room of fe_gemm_split_room bytes; not read with one segment.
 extern "C" int fe_gemm_split(const float* A, const float* W, const float* bias, float* C, float* part, int M, int N, int K, int* status,
                              cudaStream_t stream) {
     FE_REQUIRE(M >= 0 && N > 0 && K > 3 * CHUNK, "gemm_split: bad sizes M=%d N=%d K=%d", M, N, K);
     if (M == 0) return 0;
-    const int segments = fe_gemm_split_segments(N, K);
+    const int segments = segments_of(N, K);
     FE_REQUIRE(segments == 1 || (part != nullptr && ((size_t)part & 15) == 0), "gemm_split: no room for the sums of %d segments", segments);
-    const long long total = (long long)M * N;
-    bf16* rest = reinterpret_cast<bf16*>(part + segments * total);
     const bool vec = (K & 3) == 0 && (((size_t)A | (size_t)W) & 15) == 0;
+    const long long fours = (long long)((M + 3) / 4) * N;
+    float4* sums = reinterpret_cast<float4*>(part);
+    uint2* rest = reinterpret_cast<uint2*>(sums + segments * fours);
     int rc;
-#define FE_SPLIT(BN) rc = vec ? launch_split<BN, true>(A, W, bias, C, part, rest, M, N, K, segments, status, stream) \
-                              : launch_split<BN, false>(A, W, bias, C, part, rest, M, N, K, segments, status, stream)
+#define FE_SPLIT(BN) rc = vec ? launch_split<BN, true>(A, W, bias, C, sums, rest, M, N, K, segments, status, stream) \
+                              : launch_split<BN, false>(A, W, bias, C, sums, rest, M, N, K, segments, status, stream)
     if (M <= 16) FE_SPLIT(16);
     else FE_SPLIT(64);
 #undef FE_SPLIT
     if (rc || segments == 1) return rc;
-    fe::launch(add_segments_kernel, (unsigned)((total + 1023) / 1024), 256, 0, stream, (const float*)part, (const bf16*)rest, A, W, bias, C, total, N, K, segments);
+    fe::launch(add_segments_kernel, (unsigned)((fours + 255) / 256), 256, 0, stream, (const float4*)sums, (const uint2*)rest, A, W, bias, C, M, N, K, segments);
     return fe_check_launch("gemm_split (segments)");
 }

@@ -296,8 +296,8 @@ def gemm_fp32(x, w, bias=None):
     N = w.shape[0]
     out = torch.empty((M, N), dtype=torch.float32, device=x.device)
     if split_ok(N, K):
-        segments = int(_core().fe_gemm_split_segments(_c_int(N), _c_int(K)))
-        part = torch.empty(segments * M * N * 6, dtype=torch.uint8, device=x.device) if segments > 1 else None
+        room = _core().fe_gemm_split_room(_c_int(M), _c_int(N), _c_int(K))
+        part = torch.empty(room, dtype=torch.uint8, device=x.device) if room else None
         _run(_core(), "fe_gemm_split", _ptr(x), _ptr(w), _ptr(bias), _ptr(out), _ptr(part), _c_int(M), _c_int(N), _c_int(K),
              _ptr(status_word(x.device)), _stream())
         return out

@@ -2,6 +2,7 @@
 import pytest
 import torch
 
+from flexengine_b200.bench.shapes import SHAPES
 from test_kernels_gpu import DEV, gen, ops, rand      # noqa: F401  (gen is a fixture)
 
 pytestmark = pytest.mark.gpu
@@ -112,3 +113,16 @@ def test_not_finite_over_several_segments(gen):
         assert torch.equal(test(got)[keep], test(want)[keep])
     finite = torch.isfinite(want) & torch.isfinite(got)
     assert float((got[finite].double() - exact[finite]).norm()) <= float((want[finite].double() - exact[finite]).norm())
+
+
+def test_every_sm_has_work_at_few_rows():
+    """The layers' matrices of the benchmark's three shapes: a step of few rows is within a quarter of its chunks dealt out evenly."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for cfg in SHAPES.values():
+        h, i = cfg["hidden_size"], cfg["intermediate_size"]
+        heads = cfg["num_attention_heads"] * cfg["head_dim"]
+        for N, K in ((heads + 2 * cfg["num_key_value_heads"] * cfg["head_dim"], h), (h, heads), (2 * i, h), (h, i)):
+            segments = int(ops()._core().fe_gemm_split_segments(N, K))
+            tiles, chunks = -(-N // 128), -(-K // 64)
+            if ops().split_ok(N, K):
+                assert -(-tiles * segments // sms) * -(-chunks // segments) <= 1.25 * tiles * chunks / sms + 1, (N, K, segments)
