@@ -504,15 +504,27 @@ int segments_of(int N, int K) {
     }
     return best;
 }
+// The segments' sums of all rows of a long prompt are a large part of the memory that is left beside the pages (302 MB for 8,192 rows x 1,536 x
+// 8,960): rows go in parts of nearly the same size, whole tiles each, which share one room.
+constexpr long long ROOM = 64LL << 20;              // bytes at most, or those of 64 rows
+int rows_at_once(int M, int N, int segments) {
+    if (segments == 1) return M;
+    long long most = ROOM / (6LL * segments * N) / 64 * 64;
+    if (most < 64) most = 64;
+    const long long parts = (M + most - 1) / most;
+    return (int)((M + parts * 64 - 1) / (parts * 64) * 64);
+}
+
 }  // namespace
 
 extern "C" int fe_gemm_split_segments(int N, int K) { return segments_of(N, K); }
 
-// Bytes of room that a product needs for its segments' sums.
+// Bytes of room that a product needs for its segments' sums: bounded, whatever the rows.
 extern "C" long long fe_gemm_split_room(int M, int N, int K) {
     const int segments = segments_of(N, K);
     if (segments == 1 || M <= 0) return 0;
-    return 24LL * segments * N * ((M + 3LL) / 4);
+    const long long rows = rows_at_once(M, N, segments);
+    return 24LL * segments * N * (((rows < M ? rows : M) + 3) / 4);
 }
 
 // ``part``: 16-byte aligned room of fe_gemm_split_room bytes; not read with one segment.
@@ -523,16 +535,25 @@ extern "C" int fe_gemm_split(const float* A, const float* W, const float* bias, 
     const int segments = segments_of(N, K);
     FE_REQUIRE(segments == 1 || (part != nullptr && ((size_t)part & 15) == 0), "gemm_split: no room for the sums of %d segments", segments);
     const bool vec = (K & 3) == 0 && (((size_t)A | (size_t)W) & 15) == 0;
-    const long long fours = (long long)((M + 3) / 4) * N;
-    float4* sums = reinterpret_cast<float4*>(part);
-    uint2* rest = reinterpret_cast<uint2*>(sums + segments * fours);
-    int rc;
-#define FE_SPLIT(BN) rc = vec ? launch_split<BN, true>(A, W, bias, C, sums, rest, M, N, K, segments, status, stream) \
-                              : launch_split<BN, false>(A, W, bias, C, sums, rest, M, N, K, segments, status, stream)
-    if (M <= 16) FE_SPLIT(16);
-    else FE_SPLIT(64);
+    const int at_once = rows_at_once(M, N, segments);
+    for (long long m0 = 0; m0 < M; m0 += at_once) {
+        const int rows = (int)(M - m0 < at_once ? M - m0 : at_once);
+        const float* a = A + m0 * K;
+        float* c = C + m0 * N;
+        const long long fours = (long long)((rows + 3) / 4) * N;
+        float4* sums = reinterpret_cast<float4*>(part);
+        uint2* rest = reinterpret_cast<uint2*>(sums + segments * fours);
+        int rc;
+#define FE_SPLIT(BN) rc = vec ? launch_split<BN, true>(a, W, bias, c, sums, rest, rows, N, K, segments, status, stream) \
+                              : launch_split<BN, false>(a, W, bias, c, sums, rest, rows, N, K, segments, status, stream)
+        if (rows <= 16) FE_SPLIT(16);
+        else FE_SPLIT(64);
 #undef FE_SPLIT
-    if (rc || segments == 1) return rc;
-    fe::launch(add_segments_kernel, (unsigned)((fours + 255) / 256), 256, 0, stream, (const float4*)sums, (const uint2*)rest, A, W, bias, C, M, N, K, segments);
-    return fe_check_launch("gemm_split (segments)");
+        if (rc) return rc;
+        if (segments == 1) continue;
+        fe::launch(add_segments_kernel, (unsigned)((fours + 255) / 256), 256, 0, stream, (const float4*)sums, (const uint2*)rest, a, W, bias, c, rows, N, K, segments);
+        rc = fe_check_launch("gemm_split (segments)");
+        if (rc) return rc;
+    }
+    return 0;
 }

@@ -126,3 +126,21 @@ def test_every_sm_has_work_at_few_rows():
             tiles, chunks = -(-N // 128), -(-K // 64)
             if ops().split_ok(N, K):
                 assert -(-tiles * segments // sms) * -(-chunks // segments) <= 1.25 * tiles * chunks / sms + 1, (N, K, segments)
+
+
+@pytest.mark.parametrize("N,K,M", [(1536, 8960, 1300), (5120, 13824, 450), (129, 65537, 20000)])
+def test_room_for_segments_is_bounded_whatever_the_rows(N, K, M, gen):
+    """The rows go in parts that share one room of 64 MiB; each row as it is by itself."""
+    x, w = rand((M, K), torch.float32, gen) if N != 129 else torch.zeros(M, K, device=DEV), rand((N, K), torch.float32, gen)
+    if N == 129:
+        x[::37] = rand((x[::37].shape[0], K), torch.float32, gen)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    full = ops().linear(x, w)
+    torch.cuda.synchronize()
+    assert torch.cuda.max_memory_allocated() - before <= 4 * M * N + (64 << 20) + (1 << 21)
+    for at in (0, 5, M // 2 - 3, M - 70, M - 9):
+        assert torch.equal(ops().linear(x[at:at + 67].contiguous(), w), full[at:at + 67]), at
+        assert torch.equal(ops().linear(x[at:at + 9].contiguous(), w), full[at:at + 9]), at
+    ops().check_status(DEV)
