@@ -283,11 +283,14 @@ SPLIT_MIN_K, SPLIT_MIN_ELEMENTS, SPLIT_MAX_N = 1024, 1 << 23, 1 << 15
 
 
 def split_ok(N: int, K: int) -> bool:
-    """Whether the 32-bit product with a matrix [N, K] goes through the tensor cores in three bfloat16 parts a number (csrc/gemm_split.cu)
-    instead of a chain of multiply-adds on CUDA cores: by the matrix alone and never by the rows of x, so that a row's result does
-    not depend on the batch.  The lines lie where prompts gain much and steps of a few rows
-    lose little: 17,920 x 1,536 with 256 rows 278 -> 144 us and with 4 rows 27 -> 33, 1,536 x 8,960 244 -> 78 and 31 -> 33; below, 2,048 x 1,536 55 -> 32
-    and 7 -> 14; a vocabulary of 151,936, of which a step wants few rows, 158 -> 246 with 4."""
+    """Whether the 32-bit product with a matrix [N, K] of a layer goes through the tensor cores in three bfloat16 parts a number
+    (csrc/gemm_split.cu) instead of a chain of multiply-adds on CUDA cores: by the matrix alone and never by the rows of x, so that a
+    row's result does not depend on the batch.  The lines lie where prompts gain much and steps of a few rows little or nothing: the
+    layers' matrices of the 7B and 14B shapes inside of them, us with 4 and 256 rows by the chain and in parts: 4,608 x 3,584 21, 241 and 25, 88;
+    3,584 x 3,584 21, 253 and 23, 74; 3,584 x 18,944 99, 1,323 and 70, 315; 7,168 x 5,120 49, 495 and 45, 185; 5,120 x 5,120 45, 462 and
+    35, 140; 27,648 x 5,120 122, 1,424 and 132, 661; 5,120 x 13,824 116, 1,238 and 75, 335; of the 1.5B shape 17,920 x 1,536 26, 277 and 31, 133,
+    1,536 x 8,960 31, 244 and 26, 78: a decode step takes as long as by the chain or less.  Below the lines few rows lose more (2,048 x 1,536 7,
+    55 and 14, 30), and so they do with more rows of W (37,888 x 3,584 108, 1,349 and 127, 582)."""
     return K >= SPLIT_MIN_K and N <= SPLIT_MAX_N and N * K >= SPLIT_MIN_ELEMENTS
 
 
@@ -295,7 +298,7 @@ def gemm_fp32(x, w, bias=None):
     M, K = x.shape
     N = w.shape[0]
     out = torch.empty((M, N), dtype=torch.float32, device=x.device)
-    if split_ok(N, K):
+    if split_ok(N, K) and not getattr(w, "vocabulary", False):       # marked by DecoderModel.bind: met by few rows whatever its size
         room = _core().fe_gemm_split_room(_c_int(M), _c_int(N), _c_int(K))
         part = torch.empty(room, dtype=torch.uint8, device=x.device) if room else None
         _run(_core(), "fe_gemm_split", _ptr(x), _ptr(w), _ptr(bias), _ptr(out), _ptr(part), _c_int(M), _c_int(N), _c_int(K),

@@ -66,6 +66,8 @@ class DecoderModel:
             part.bind({k[2]: t for k, t in tensors.items() if k[0] == "junction" and k[1] == j})
         for t in _tensors_of([p for _, p in self._outer_parts()] + [p for b in self.blocks for p in b.parts().values()] + self.junctions):
             t.held = True       # stands while the model does: a product may begin to read it before the kernel ahead has ended
+        if self.lm_head is not None:
+            self.lm_head.vocabulary = True       # of a step only the rows meet it whose logits are wanted: few
 
     def _outer_parts(self):
         """The parts outside the layers, under the names their bindings use."""

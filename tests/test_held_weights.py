@@ -84,3 +84,28 @@ def test_products_of_a_matrix_the_kernel_before_made(K, rows):
         want.append(ops.linear_gated(x, w, N // 2, "silu"))
     for a, b in zip(got, want):
         assert torch.equal(a, b)
+
+
+def test_a_vocabulary_keeps_the_chain_of_multiply_adds_whatever_its_size(monkeypatch):
+    """A step wants few rows of logits, which the product in three parts would not serve faster; what a model calls its head is by
+    the model's word and not by the rows, so that a row's logits do not depend on the batch."""
+    class Core:
+        fe_gemm_split_room = staticmethod(lambda M, N, K: 0)
+    seen = []
+    for name, value in (("_need_cuda", lambda *t: None), ("_core", lambda: Core), ("_ptr", lambda t: None), ("_stream", lambda: None),
+                        ("status_word", lambda device: None), ("_run", lambda lib, name, *args: seen.append(name))):
+        monkeypatch.setattr(ops, name, value)
+    w = torch.empty(8192, 1024)
+    for rows in (1, 300):
+        ops.linear(torch.empty(rows, 1024), w)
+    w.vocabulary = True
+    for rows in (1, 300):
+        ops.linear(torch.empty(rows, 1024), w)
+    assert seen == ["fe_gemm_split"] * 2 + ["fe_gemm_fp32"] * 2
+
+
+@pytest.mark.parametrize("tied", [True, False])
+def test_a_bound_model_says_which_matrix_is_its_vocabulary(tied):
+    _typed, _plan, model = random_model(dict(QWEN, tie_word_embeddings=tied), seed=1, dtype="float32", device="cpu")
+    assert model.head.weight.vocabulary
+    assert not any(getattr(t, "vocabulary", False) for block in model.blocks for part in block.parts().values() for t in vars(part).values())
