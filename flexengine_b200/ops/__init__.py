@@ -11,6 +11,8 @@ norm weights, biases and logits are float32; index tensors are int32.
 """
 from __future__ import annotations
 
+from array import array
+
 import torch
 
 from . import library
@@ -1739,6 +1741,11 @@ def sample_listed(logits, temperature, top_k, seed, draw):
     R, V = logits.shape
     if logits.dtype != torch.float32 or logits.stride(1) != 1:
         raise TypeError("sample: logits must be float32 with unit column stride")
+    for a, typecode in zip((temperature, top_k, seed, draw), "fiqq"):      # what lies at their addresses is read as it is
+        if not isinstance(a, array) or a.typecode != typecode:
+            raise TypeError("sample_listed: arrays of typecodes f, i, q and q")
+        if len(a) != R:
+            raise ValueError(f"sample_listed: {len(a)} parameters for {R} rows")
     out = torch.empty(R, dtype=torch.int32, device=logits.device)
     _run(_core(), "fe_sample_listed", _ptr(logits), _c_ll(logits.stride(0)), _c_int(R), _c_int(V),
          *(a.buffer_info()[0] for a in (temperature, top_k, seed, draw)), _ptr(out), _stream())

@@ -1,6 +1,7 @@
 """What the sampler takes as a step's parameters: lists of numbers in one conversion, any other sequence as a tensor would take
 it; what is no number, is negative or does not fit is refused."""
 import math
+from array import array
 
 import numpy as np
 import pytest
@@ -62,3 +63,19 @@ def test_greedy_rows_take_whatever_stands_beside_them():
     for top_ks in ([2 ** 70, 1], [0], [1, 2, 3], (5, 5), [1, 2, None], iter([1, 2])):
         assert taken([0.0, 0], top_ks, [1], [3]) == [[0.0, 0.0], [0, 0], [0, 0], [0, 0]]
     assert Sampler(Seen()).sample_on_device(torch.zeros(0, 8), [], [], [], []) == [[], [], [], []]
+
+
+@pytest.mark.parametrize("at,wrong,error", [(0, array("d", [0.5, 1.0]), TypeError), (0, [0.5, 1.0], TypeError), (1, array("q", [0, 3]), TypeError),
+                                            (2, array("i", [1, 2]), TypeError), (3, array("Q", [3, 4]), TypeError), (0, array("f", [0.5]), ValueError),
+                                            (1, array("i", [0]), ValueError), (2, array("q", [1, 2, 3]), ValueError), (3, array("q"), ValueError)])
+def test_listed_parameters_of_another_length_or_type_are_refused_before_they_are_read(at, wrong, error, monkeypatch):
+    from flexengine_b200 import ops
+    taken = []
+    for name, value in (("_need_cuda", lambda *t: None), ("_core", lambda: None), ("_stream", lambda: None), ("_run", lambda *args: taken.append(args))):
+        monkeypatch.setattr(ops, name, value)
+    good = (array("f", [0.5, 1.0]), array("i", [0, 3]), array("q", [1, 2]), array("q", [3, 4]))
+    ops.sample_listed(LOGITS, *good)
+    assert len(taken) == 1
+    with pytest.raises(error):
+        ops.sample_listed(LOGITS, *good[:at], wrong, *good[at + 1:])
+    assert len(taken) == 1
