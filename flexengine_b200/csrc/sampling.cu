@@ -72,9 +72,10 @@ __device__ __forceinline__ float warp_total(float v) {       // the same value i
     return v;
 }
 
-// The parameters of a step's rows: on the device, or (up to LISTED_ROWS rows: 1.5 KB of the launch's parameters) with the launch, so that
-// lists of numbers on the host need no buffer and no copy of their own.
-constexpr int LISTED_ROWS = 64;
+// The parameters of a step's rows: on the device, or with the launch, so that lists of numbers on the host need no buffer and no copy of
+// their own: up to LISTED_ROWS rows of 24 bytes, as many as the 4 KB of a launch's parameters hold beside the other five.
+// 128 rows of 32,000 with the launch 31 us a call, through a buffer 60; 64 rows 27 and 51 (1.5 KB of parameters or 4 KB make no difference).
+constexpr int LISTED_ROWS = 168;
 struct OnDevice {
     const float* temperature;
     const int* top_k;
@@ -86,6 +87,7 @@ struct Listed {
     int top_k[LISTED_ROWS];
     long long seed[LISTED_ROWS], draw[LISTED_ROWS];
 };
+static_assert(sizeof(Listed) + 48 <= 4096, "a launch's parameters");
 
 template <typename Parameters>
 __global__ void __launch_bounds__(THREADS)
@@ -600,7 +602,7 @@ extern "C" int fe_sample(const float* logits, long long ld, int R, int V, const 
     return sample_rows(logits, ld, R, V, OnDevice{temperature, top_k, seed, draw}, out, blocks_per_row(R), stream);
 }
 
-// The same with the parameters of up to 64 rows in the host's memory: they travel with the launch.
+// The same with the parameters of up to LISTED_ROWS rows in the host's memory: they travel with the launch.
 extern "C" int fe_sample_listed(const float* logits, long long ld, int R, int V, const float* temperature,
                                 const int* top_k, const long long* seed, const long long* draw, int* out,
                                 cudaStream_t stream) {

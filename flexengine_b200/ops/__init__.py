@@ -1731,7 +1731,7 @@ def sample(logits, temperature, top_k, seed, draw, blocks: int = 0):
     return out
 
 
-SAMPLE_LISTED_ROWS = 64         # rows whose parameters travel with the launch
+SAMPLE_LISTED_ROWS = 168        # rows whose parameters travel with the launch (csrc/sampling.cu)
 
 
 def sample_listed(logits, temperature, top_k, seed, draw):

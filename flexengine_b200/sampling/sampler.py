@@ -82,7 +82,7 @@ class Sampler:
                                     torch.zeros(n, dtype=torch.int64, device=dev))
             temperature, top_k, zero64 = self._zeros[key]
             return self.ops.sample(logits, temperature, top_k, zero64, zero64)
-        # Plain lists for a batch of ordinary size go with the launch: no buffer, no copy, no views
+        # Plain lists go with the launch as far as they fit into its parameters: no buffer, no copy, no views
         # (64 rows, with the kernel's own gain: a call among others 50 to 52 -> 40 us, alone 95 to 100 -> 65)
         listed = getattr(self.ops, "sample_listed", None)
         if listed is not None and 0 < n <= self.ops.SAMPLE_LISTED_ROWS and dev.type == "cuda":

@@ -79,3 +79,26 @@ def test_listed_parameters_of_another_length_or_type_are_refused_before_they_are
     with pytest.raises(error):
         ops.sample_listed(LOGITS, *good[:at], wrong, *good[at + 1:])
     assert len(taken) == 1
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("vocab,pitch", [(32000, 32000), (4099, 4103)])
+@pytest.mark.parametrize("rows", [1, 63, 64, 65, 167, 168, 169])
+def test_lists_give_the_tokens_of_tensors(rows, vocab, pitch):
+    """Parameters as plain lists (with the launch, as far as they fit into one) and the same numbers as tensors, row for row; rows on
+    16-byte boundaries and not."""
+    from flexengine_b200 import ops
+    dev = "cuda:0"
+    gen = torch.Generator(device=dev).manual_seed(rows)
+    logits = torch.empty(rows, pitch, device=dev)[:, :vocab].copy_(torch.randn(rows, vocab, device=dev, generator=gen) * 3)
+    temperatures = [(0.0, 0.7, 1, 1.3)[(i + 1) % 4] for i in range(rows)]
+    top_ks = [(0, 40, 1, 2000, vocab + 7)[i % 5] for i in range(rows)]
+    seeds = [(i * 0x9E3779B97F4A7C15 + 77) % 2 ** 64 - 2 ** 63 for i in range(rows)]
+    draws = [i * i if i % 3 else 2 ** 62 + i for i in range(rows)]
+    got = Sampler().sample_on_device(logits, temperatures, top_ks, seeds, draws)
+    want = ops.sample(logits, torch.tensor(temperatures, dtype=torch.float32, device=dev), torch.tensor(top_ks, dtype=torch.int32, device=dev),
+                      torch.tensor(seeds, device=dev), torch.tensor(draws, device=dev))
+    assert torch.equal(got, want)
+    if rows > 1:          # each parameter counts: with two of them exchanged the tokens are others
+        other = Sampler().sample_on_device(logits, temperatures, top_ks, draws, seeds)
+        assert not torch.equal(other, want)
