@@ -771,6 +771,49 @@ def test_head_scan_kernels_against_the_references(heads, groups, dim, vdim, divi
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("divided", [False, True])
+@pytest.mark.parametrize("heads,groups,dim,vdim", [(4, 2, 64, 128), (8, 4, 128, 64), (1, 1, 129, 69), (1, 1, 130, 70), (1, 1, 131, 71), (2, 2, 68, 132)])
+def test_head_scan_of_rows_on_16_byte_boundaries(heads, groups, dim, vdim, divided):
+    """Rows that start on 16-byte boundaries come by asynchronous copies, whole and in part (one to three numbers of the last four), with
+    zeros behind them: the same bits as the same rows one number further, which are loaded one by one, and what the reference gives."""
+    from flexengine_b200 import ops
+    dev = "cuda:0"
+    gen = torch.Generator().manual_seed(11)
+    per = heads * (dim * vdim + dim)
+    for lengths in (PORTIONS, [2] * 9):
+        cu, slots, T = one_step(lengths, SEATS)
+        q, k, v = (torch.randn(T, n, generator=gen) for n in (groups * dim, groups * dim, heads * vdim))
+        gates = torch.stack([-torch.rand(T, heads, generator=gen) ** 4 * 30.0, torch.rand(T, heads, generator=gen), torch.rand(T, heads, generator=gen)])
+        state = torch.randn(9, per + 5, generator=gen) * 0.5
+        extra = {"divided": 1e-6} if divided else {"skip": torch.randn(heads, generator=gen)}
+        want_state = state.clone()
+        want = kernel_refs.head_scan(q, k, v, gates, want_state, slots, cu, heads, groups, dim, vdim, query_scale=0.3, **extra)
+
+        def run(shift):
+            def rows(x):
+                pitch = (x.shape[1] + 7) // 4 * 4 + (shift > 0)
+                held = torch.full((T * pitch + shift,), float("nan"), device=dev)       # nothing beside the rows may count
+                out = held[shift:].view(T, pitch)[:, :x.shape[1]]
+                assert (out.data_ptr() % 16 == 0 and pitch % 4 == 0) == (shift == 0)
+                return out.copy_(x)
+            moved = state.to(dev)
+            on_device = {n: (t.to(dev) if torch.is_tensor(t) else t) for n, t in extra.items()}
+            got = ops.head_scan(rows(q), rows(k), rows(v), gates.to(dev), moved, slots.to(dev), cu.to(dev), heads, groups, dim, vdim, query_scale=0.3,
+                                max_q_len=max(lengths), **on_device)
+            return got, moved
+        got, moved = run(0)
+        apart, moved_apart = run(1)
+        held = torch.isfinite(got)
+        assert torch.equal(got[held], apart[held]) and torch.equal(held, torch.isfinite(apart)) and torch.equal(moved, moved_apart)
+        if divided:
+            assert held.all()
+            near(torch.tanh(got.cpu() / 50.0), torch.tanh(want / 50.0), 2e-3, "outputs")
+        else:
+            near(got, want, 3e-5, "outputs")
+        near(moved, want_state, 3e-5, "states")
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("heads", [1, 3, 8])
 def test_memory_gates_against_the_reference(heads):
     from flexengine_b200 import ops
