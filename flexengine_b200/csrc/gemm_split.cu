@@ -81,10 +81,17 @@ __device__ __forceinline__ void umma_commit(unsigned long long* bar) {
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
 
-// eight accumulator columns of this thread's TMEM lane (wait::ld is the caller's)
+// eight accumulator columns of this thread's TMEM lane; tmem_arrived is the caller's, before anything reads them
 __device__ __forceinline__ void tmem_load8(unsigned taddr, unsigned* r) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
+}
+
+// Waits for the loads before it.  The empty statement makes the registers its result, so that no addition moves up before the wait.
+template <int COUNT> __device__ __forceinline__ void tmem_arrived(unsigned* r) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < COUNT; ++i) asm volatile("" : "+r"(r[i]));
 }
 
 // Eight floats -> their three parts, eight bfloat16 each.
@@ -330,7 +337,7 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
                     unsigned r[PART];
 #pragma unroll
                     for (int j = 0; j < PART; j += 8) tmem_load8(from + j0 + j, r + j);
-                    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+                    tmem_arrived<PART>(r);
 #pragma unroll
                     for (int j = 0; j < PART; ++j) sum[j0 + j] += __uint_as_float(r[j]);
                 }
@@ -352,7 +359,7 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
                 unsigned r[3][8];
 #pragma unroll
                 for (int h = 0; h < 3; ++h) tmem_load8(from + h * BN + j0, r[h]);
-                asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+                tmem_arrived<24>(&r[0][0]);
 #pragma unroll
                 for (int e = 0; e < 8; ++e) r[0][e] = __float_as_uint(__uint_as_float(r[0][e]) + (__uint_as_float(r[1][e]) + __uint_as_float(r[2][e])));
                 if (whole) {
