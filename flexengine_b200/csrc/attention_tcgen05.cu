@@ -30,7 +30,7 @@
 // the block then records it in the status word, leaves its loops and frees its tensor memory.
 #include <math_constants.h>
 
-#include "common.cuh"
+#include "tcgen05.cuh"
 
 using namespace fe;
 
@@ -46,19 +46,6 @@ constexpr int TMEM_COLS = 512;   // score buffer b of row tile i at column 64 (2
 constexpr long long WAIT_LIMIT = 2000000000LL;
 constexpr float RESCALE_STEP = 8.f;      // log2 of the growth of a row's maximum that moves its reference point
 
-__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(unsigned long long* bar, int count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ bool mbar_test(unsigned long long* bar, unsigned parity) {
-    unsigned ok;
-    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-                 : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-    return ok != 0;
-}
 // false when the wait ran out or another thread of the block has given up; sets the flag itself then
 __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity, volatile int* give_up) {
     if (mbar_test(bar, parity)) return true;
@@ -77,79 +64,23 @@ __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src,
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait_but() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void loader_barrier() { asm volatile("bar.sync 1, 128;\n" ::: "memory"); }
 
-// Shared-memory descriptors, 128-byte swizzle.  K-major: rows 128 bytes apart, 8-row groups 1024
-// bytes apart.  MN-major (V as it lies in the cache: one row per key, 64 head elements = 128 bytes
-// of a row per block): 64-element blocks along the head dimension ``lbo`` bytes apart, 8-key groups
-// 1024 bytes apart.
-__device__ __forceinline__ unsigned long long desc_k_major(const void* p) {
-    const unsigned long long addr = smem_u32(p);
-    return ((addr & 0x3FFFFull) >> 4) | ((1024ull >> 4) << 32) | (1ull << 46) | (2ull << 61);
-}
+// Shared-memory descriptor of an MN-major operand, 128-byte swizzle (V as it lies in the cache: one row per key, 64 head elements = 128 bytes
+// of a row per block): 64-element blocks along the head dimension ``lbo`` bytes apart, 8-key groups 1024 bytes apart.
 __device__ __forceinline__ unsigned long long desc_mn_major(const void* p, unsigned lbo_bytes) {
     const unsigned long long addr = smem_u32(p);
     return ((addr & 0x3FFFFull) >> 4) | ((unsigned long long)(lbo_bytes >> 4) << 16) | ((1024ull >> 4) << 32) | (1ull << 46) |
            (2ull << 61);
-}
-// float accumulator, bfloat16 operands; b_mn: B is MN-major
-__host__ __device__ constexpr unsigned instr_desc(int m, int n, bool b_mn) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((b_mn ? 1u : 0u) << 16) | ((unsigned)(n >> 3) << 17) | ((unsigned)(m >> 4) << 24);
-}
-// D[tmem] (+)= A[smem] B[smem]
-__device__ __forceinline__ void umma_ss(unsigned tmem_d, unsigned long long adesc, unsigned long long bdesc, unsigned idesc,
-                                        unsigned accumulate) {
-    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-                 ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
 // D[tmem] (+)= A[tmem] B[smem]: A lies row per lane, two bfloat16 per 32-bit column
 __device__ __forceinline__ void umma_ts(unsigned tmem_d, unsigned tmem_a, unsigned long long bdesc, unsigned idesc,
                                         unsigned accumulate) {
     asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
                  ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void umma_commit(unsigned long long* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void tmem_load32(unsigned taddr, float* v) {
-    unsigned r[32];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr) : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-}
-// Four loads of 32 columns in flight at once: issue all, then one wait; the empty statements tie the
-// registers to the wait so that nothing reads them before it.
-__device__ __forceinline__ void tmem_issue_load32(unsigned taddr, unsigned* r) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr) : "memory");
-}
-__device__ __forceinline__ void tmem_load_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
-__device__ __forceinline__ void tie32(unsigned* r) {
-    asm volatile("" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]),
-                      "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]), "+r"(r[16]),
-                      "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]), "+r"(r[24]),
-                      "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31]) :: "memory");
 }
 __device__ __forceinline__ void tmem_store32(unsigned taddr, const float* v) {
     asm volatile(
@@ -576,7 +507,7 @@ paged_prefill_tcgen05_kernel(const bf16* __restrict__ q, long long q_stride, bf1
                 const unsigned dst = s_col + (j & 1) * 64;
 #pragma unroll
                 for (int ks = 0; ks < D / 16; ++ks)
-                    umma_ss(dst, q_desc + (((ks >> 2) * Q_BLOCK + (ks & 3) * 32) >> 4),
+                    umma(dst, q_desc + (((ks >> 2) * Q_BLOCK + (ks & 3) * 32) >> 4),
                             k_desc + (((ks >> 2) * KV_BLOCK + (ks & 3) * 32) >> 4), idesc_s, ks > 0 ? 1u : 0u);
                 umma_commit(&s_ready[i][j & 1]);
             };
@@ -635,9 +566,7 @@ paged_prefill_tcgen05_kernel(const bf16* __restrict__ q, long long q_stride, bf1
             unsigned raw[KEYS];
             tmem_issue_load32(s_addr, raw);
             tmem_issue_load32(s_addr + 32, raw + 32);
-            tmem_load_wait();
-            tie32(raw);
-            tie32(raw + 32);
+            tmem_arrived<KEYS>(raw);
             const int key0 = listed_tile<KEYS>(t_begin + j, kept, lo) * KEYS;
             const bool unmasked = key0 + KEYS - 1 <= pos_min && (key0 >= lo_max || key0 + KEYS <= keep);      // for the whole warp
             const Edges edges = {pos - key0, row_lo - key0, keep - key0};

@@ -28,9 +28,9 @@
 // A chunk's way (rows from memory, cut up, through shared memory, 16 MMAs, sums) takes 1.0 to 1.3 us and is what bounds the kernel: with no MMA
 // but one a step 17,920 x 1,536 takes 30 and 122 us (4 and 256 rows), with no stores to shared memory 27 and 107; asking rows into L2 ahead of time
 // makes it slower (33, 138).  17,920 x 1,536: 31 us with 1 to 16 rows (the chain of multiply-adds 24 to 40), 40 with 64 (106), 135 with 256 (278).
-// Relative error against 64 bits, K = 1,536 / 8,960: 1.2e-7 / 1.2e-7, the chain 7.0e-7 / 1.7e-6; rows of 1, 2, 8 and 32 numbers other than 0:
-// 2.5e-8, 2.6e-8, 2.8e-8, 4.2e-8, the chain 2.5e-8, 3.1e-8, 5.2e-8, 1.0e-7.
-#include "common.cuh"
+// Relative error against 64 bits, K = 1,536 / 8,960: 1.2e-7 / 1.0e-7, the chain 7.0e-7 / 1.7e-6; rows of 1, 2, 8 and 32 numbers other than 0:
+// 2.5e-8, 2.6e-8, 2.8e-8, 4.2e-8, the chain 2.5e-8, 3.1e-8, 5.2e-8, 1.0e-7.  All of 256 x 1,536 results (K = 8,960) formed again take 3.4 ms.
+#include "tcgen05.cuh"
 
 using namespace fe;
 
@@ -39,60 +39,8 @@ namespace {
 constexpr int TILE_W = 128;             // rows of W in a tile = UMMA M
 constexpr int CHUNK = 64;               // k's of a chunk: 128 bytes of bfloat16, one swizzle atom wide
 constexpr int GROUP_WARPS = 8, SPLIT_WARPS = 2 * GROUP_WARPS, SUM_WARPS = 8, THREADS = 32 * (SPLIT_WARPS + SUM_WARPS + 4);
-constexpr long long WAIT_LIMIT = 4000000000LL;      // clock cycles
 constexpr float LEAST = 8.673617380e-19f, MOST = 3.402823466e38f;      // 2^-60; results outside of these bounds are formed again
 constexpr unsigned LARGE = 0x4f80;                  // 2^32, the upper half of the word
-
-__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(unsigned long long* bar, int count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ bool mbar_test(unsigned long long* bar, unsigned parity) {
-    unsigned ok;
-    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-                 : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity) {
-    if (mbar_test(bar, parity)) return true;
-    const long long t0 = clock64();
-    while (!mbar_test(bar, parity)) {
-        if (clock64() - t0 > WAIT_LIMIT) return false;
-    }
-    return true;
-}
-
-// K-major operand, 128-byte swizzle, rows 128 bytes apart, groups of 8 rows 1024 bytes apart (as in gemm_tcgen05.cu).
-__device__ __forceinline__ unsigned long long smem_desc(unsigned addr) {
-    return (((unsigned long long)addr & 0x3FFFFull) >> 4) | ((1024ull >> 4) << 32) | (1ull << 46) | (2ull << 61);
-}
-// float accumulator, bfloat16 operands, both K-major, 128 x n tile
-__host__ __device__ constexpr unsigned instr_desc(int n) { return (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(n >> 3) << 17) | ((unsigned)(TILE_W >> 4) << 24); }
-__device__ __forceinline__ void umma(unsigned tmem_d, unsigned long long adesc, unsigned long long bdesc, unsigned idesc, unsigned accumulate) {
-    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-                 ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void umma_commit(unsigned long long* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
-
-// eight accumulator columns of this thread's TMEM lane; tmem_arrived is the caller's, before anything reads them
-__device__ __forceinline__ void tmem_load8(unsigned taddr, unsigned* r) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
-}
-
-// Waits for the loads before it.  The empty statement makes the registers its result, so that no addition moves up before the wait.
-template <int COUNT> __device__ __forceinline__ void tmem_arrived(unsigned* r) {
-    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < COUNT; ++i) asm volatile("" : "+r"(r[i]));
-}
 
 // Eight floats -> their three parts, eight bfloat16 each.
 __device__ __forceinline__ void split8(const float4& p, const float4& q, uint4& hi, uint4& mid, uint4& lo) {
@@ -204,10 +152,7 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
         give_up = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
-    if (warp == SPLIT_WARPS) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_holder)), "n"(S::COLUMNS) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
-    }
+    if (warp == SPLIT_WARPS) tmem_alloc<S::COLUMNS>(&tmem_holder);
     griddep_wait();
     griddep_launch_dependents();
     tc_fence_before();
@@ -414,14 +359,14 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
                     const unsigned small = tmem + (tile & 1) * 3 * BN, large = tmem + (6 + buf) * BN;
                     // The parts of A's rows lie one after the other like 3 BN rows: a part of W meets as many of them as count at once.
                     // Block 0 of the small sums takes w0 a1 + w1 a0, block 1 w0 a2 + w1 a1 + w2 a0, block 2 w1 a2 + w2 a1.
-                    const unsigned long long dw0 = smem_desc(w), dw1 = smem_desc(w + S::W_PART), dw2 = smem_desc(w + 2 * S::W_PART);
-                    const unsigned long long dx0 = smem_desc(x), dx1 = smem_desc(x + S::X_PART);
+                    const unsigned long long dw0 = desc_k_major(w), dw1 = desc_k_major(w + S::W_PART), dw2 = desc_k_major(w + 2 * S::W_PART);
+                    const unsigned long long dx0 = desc_k_major(x), dx1 = desc_k_major(x + S::X_PART);
 #pragma unroll
                     for (int k = 0; k < CHUNK / 16; ++k) {
-                        umma(small, dw1 + 2 * k, dx0 + 2 * k, instr_desc(3 * BN), (k > 0 || c > c0) ? 1u : 0u);
-                        umma(small, dw0 + 2 * k, dx1 + 2 * k, instr_desc(2 * BN), 1u);
-                        umma(small + BN, dw2 + 2 * k, dx0 + 2 * k, instr_desc(2 * BN), 1u);
-                        umma(large, dw0 + 2 * k, dx0 + 2 * k, instr_desc(BN), k > 0 ? 1u : 0u);
+                        umma(small, dw1 + 2 * k, dx0 + 2 * k, instr_desc(TILE_W, 3 * BN), (k > 0 || c > c0) ? 1u : 0u);
+                        umma(small, dw0 + 2 * k, dx1 + 2 * k, instr_desc(TILE_W, 2 * BN), 1u);
+                        umma(small + BN, dw2 + 2 * k, dx0 + 2 * k, instr_desc(TILE_W, 2 * BN), 1u);
+                        umma(large, dw0 + 2 * k, dx0 + 2 * k, instr_desc(TILE_W, BN), k > 0 ? 1u : 0u);
                     }
                     umma_commit(&empty_bar[s]);
                     umma_commit(&acc_full[buf]);
@@ -436,7 +381,7 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
     if (give_up && tid == 0 && status) atomicOr(status, FE_STATUS_WAIT_EXPIRED);
     tc_fence_before();
     __syncthreads();
-    if (warp == SPLIT_WARPS) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "n"(S::COLUMNS) : "memory");
+    if (warp == SPLIT_WARPS) tmem_dealloc<S::COLUMNS>(tmem);
 }
 
 // C = the segments' sums in order, + bias.  A thread takes four rows of A and a row of W; a warp what is to be formed again.

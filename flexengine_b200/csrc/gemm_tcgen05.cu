@@ -26,7 +26,7 @@
 // multicast.
 #include <cuda.h>
 
-#include "common.cuh"
+#include "tcgen05.cuh"
 
 using namespace fe;
 
@@ -38,7 +38,6 @@ constexpr int UMMA_K = 16;
 constexpr int STAGES = 4;
 constexpr int EPILOGUE_WARPS = 8;
 constexpr int THREADS = 64 + 32 * EPILOGUE_WARPS;
-constexpr long long WAIT_LIMIT = 4000000000LL;      // clock cycles
 
 enum { EPI_BF16 = 0, EPI_F32 = 1, EPI_SWIGLU = 2, EPI_GEGLU = 5, EPI_RELU2 = 6, EPI_REGLU = 7, EPI_GELU = 8 };      // 5: the gated epilogue with the tanh form of GELU
 constexpr int ACT_RELU2 = 3;            // ``gate_act`` of the bfloat16 epilogue: the square of relu(product), no gate (entry code 6)
@@ -61,91 +60,15 @@ __device__ __forceinline__ float gated_value(float g, float u, int act, float li
     return gate_function(g, act) * u;
 }
 
-__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(unsigned long long* bar, int count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(bar)) : "memory");
-}
 __device__ __forceinline__ void mbar_arrive_expect_tx(unsigned long long* bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ bool mbar_test(unsigned long long* bar, unsigned parity) {
-    unsigned ok;
-    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-                 : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity) {
-    if (mbar_test(bar, parity)) return true;
-    const long long t0 = clock64();
-    while (!mbar_test(bar, parity)) {
-        if (clock64() - t0 > WAIT_LIMIT) return false;
-    }
-    return true;
-}
-
 // 2-D tiled TMA load: coordinates (c0 = element along K, c1 = row).  c0 * 2 bytes is always a
 // multiple of 128 here, so the 16-byte rule on the innermost coordinate holds.
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, int c0, int c1,
                                             unsigned long long* bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n"
                  ::"r"(smem_u32(smem_dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1) : "memory");
-}
-
-// Shared-memory matrix descriptor: K-major operand, 128-byte swizzle, rows 128 bytes apart, groups
-// of 8 rows 1024 bytes apart.
-__device__ __forceinline__ unsigned long long smem_desc(const void* p) {
-    const unsigned long long addr = smem_u32(p);
-    return ((addr & 0x3FFFFull) >> 4)          // start address
-           | (0ull << 16)                      // leading-dimension byte offset: unused for swizzled K-major
-           | ((1024ull >> 4) << 32)            // stride-dimension byte offset between 8-row groups
-           | (1ull << 46)                      // descriptor version of this architecture
-           | (2ull << 61);                     // 128-byte swizzle
-}
-
-// Instruction descriptor: float accumulator, bfloat16 A and B, both K-major, M x N tile.
-__host__ __device__ constexpr unsigned instr_desc(int m, int n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(n >> 3) << 17) | ((unsigned)(m >> 4) << 24);
-}
-
-__device__ __forceinline__ void umma(unsigned tmem_d, unsigned long long adesc, unsigned long long bdesc, unsigned idesc,
-                                     unsigned accumulate) {
-    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-                 ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-// Arrives on ``bar`` once every MMA issued so far by this thread has finished (and read its operands).
-__device__ __forceinline__ void umma_commit(unsigned long long* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
-
-// 32 consecutive accumulator columns of this thread's TMEM lane.
-__device__ __forceinline__ void tmem_load32(unsigned taddr, float* v) {
-    unsigned r[32];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr) : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-template <int NCOLS> __device__ __forceinline__ void tmem_alloc(unsigned* holder) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(holder)), "n"(NCOLS) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
-}
-template <int NCOLS> __device__ __forceinline__ void tmem_dealloc(unsigned taddr) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(taddr), "n"(NCOLS) : "memory");
 }
 
 // The order of the tiles: row tiles fastest inside a panel of PANEL row tiles, the panels one after the other.  Blocks
@@ -249,7 +172,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 if (!mbar_wait(&full_bar[s], use & 1)) { give_up = 1; break; }
                 tc_fence_after();
                 const unsigned char* a = smem + s * STAGE_BYTES;
-                const unsigned long long adesc = smem_desc(a), bdesc = smem_desc(a + A_BYTES);
+                const unsigned long long adesc = desc_k_major(a), bdesc = desc_k_major(a + A_BYTES);
 #pragma unroll
                 for (int k = 0; k < BK / UMMA_K; ++k) {
                     // 16 elements along K = 32 bytes inside the swizzle atom: +2 in the address field
