@@ -74,7 +74,7 @@ __device__ __forceinline__ float warp_total(float v) {       // the same value i
 
 // The parameters of a step's rows: on the device, or with the launch, so that lists of numbers on the host need no buffer and no copy of
 // their own: up to LISTED_ROWS rows of 24 bytes, as many as the 4 KB of a launch's parameters hold beside the other five.
-// 128 rows of 32,000 with the launch 31 us a call, through a buffer 60; 64 rows 27 and 51 (1.5 KB of parameters or 4 KB make no difference).
+// 128 rows of 32,000 with the launch 31 us a call, through a buffer 60; 64 rows 27 and 51.
 constexpr int LISTED_ROWS = 168;
 struct OnDevice {
     const float* temperature;
@@ -82,12 +82,12 @@ struct OnDevice {
     const long long* seed;
     const long long* draw;
 };
-struct Listed {
-    float temperature[LISTED_ROWS];
-    int top_k[LISTED_ROWS];
-    long long seed[LISTED_ROWS], draw[LISTED_ROWS];
+template <int ROWS> struct Listed {
+    float temperature[ROWS];
+    int top_k[ROWS];
+    long long seed[ROWS], draw[ROWS];
 };
-static_assert(sizeof(Listed) + 48 <= 4096, "a launch's parameters");
+static_assert(sizeof(Listed<LISTED_ROWS>) + 48 <= 4096, "a launch's parameters");
 
 template <typename Parameters>
 __global__ void __launch_bounds__(THREADS)
@@ -602,19 +602,28 @@ extern "C" int fe_sample(const float* logits, long long ld, int R, int V, const 
     return sample_rows(logits, ld, R, V, OnDevice{temperature, top_k, seed, draw}, out, blocks_per_row(R), stream);
 }
 
-// The same with the parameters of up to LISTED_ROWS rows in the host's memory: they travel with the launch.
+template <int ROWS>
+static int sample_listed(const float* logits, long long ld, int R, int V, const float* temperature, const int* top_k, const long long* seed,
+                         const long long* draw, int* out, cudaStream_t stream) {
+    Listed<ROWS> of;
+    memcpy(of.temperature, temperature, R * sizeof(float));
+    memcpy(of.top_k, top_k, R * sizeof(int));
+    memcpy(of.seed, seed, R * sizeof(long long));
+    memcpy(of.draw, draw, R * sizeof(long long));
+    return sample_rows(logits, ld, R, V, of, out, blocks_per_row(R), stream);
+}
+
+// The same with the parameters of up to LISTED_ROWS rows in the host's memory: they travel with the launch, in 1, 2 or 4 KB, since a launch pays
+// for what it carries (64 rows a call: 39.4 us with 1.5 KB, 39.6 with 4).
 extern "C" int fe_sample_listed(const float* logits, long long ld, int R, int V, const float* temperature,
                                 const int* top_k, const long long* seed, const long long* draw, int* out,
                                 cudaStream_t stream) {
     FE_REQUIRE(R >= 0 && V > 0 && ld >= V, "sample: bad sizes R=%d V=%d ld=%lld", R, V, ld);
     FE_REQUIRE(R <= LISTED_ROWS, "sample: %d rows with their parameters on the host; %d at most", R, LISTED_ROWS);
     if (R == 0) return 0;
-    Listed of;
-    memcpy(of.temperature, temperature, R * sizeof(float));
-    memcpy(of.top_k, top_k, R * sizeof(int));
-    memcpy(of.seed, seed, R * sizeof(long long));
-    memcpy(of.draw, draw, R * sizeof(long long));
-    return sample_rows(logits, ld, R, V, of, out, blocks_per_row(R), stream);
+    if (R <= LISTED_ROWS / 4) return sample_listed<LISTED_ROWS / 4>(logits, ld, R, V, temperature, top_k, seed, draw, out, stream);
+    if (R <= LISTED_ROWS / 2) return sample_listed<LISTED_ROWS / 2>(logits, ld, R, V, temperature, top_k, seed, draw, out, stream);
+    return sample_listed<LISTED_ROWS>(logits, ld, R, V, temperature, top_k, seed, draw, out, stream);
 }
 
 // The same with a given number of blocks a row (1, 2, 4 or 8): the tokens are the same for every number.

@@ -83,7 +83,7 @@ def test_listed_parameters_of_another_length_or_type_are_refused_before_they_are
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("vocab,pitch", [(32000, 32000), (4099, 4103)])
-@pytest.mark.parametrize("rows", [1, 63, 64, 65, 167, 168, 169])
+@pytest.mark.parametrize("rows", [1, 42, 43, 64, 84, 85, 168, 169])
 def test_lists_give_the_tokens_of_tensors(rows, vocab, pitch):
     """Parameters as plain lists (with the launch, as far as they fit into one) and the same numbers as tensors, row for row; rows on
     16-byte boundaries and not."""
