@@ -79,14 +79,32 @@ template <int BN> struct Sizes {
 // ---- results formed again; every lane of a warp takes part ----
 __device__ bool all_zero(const float* __restrict__ row, int K) {
     const int lane = threadIdx.x & 31;
-    for (int k0 = 0; k0 < K; k0 += 32)
-        if (__any_sync(0xffffffffu, k0 + lane < K && row[k0 + lane] != 0.f)) return false;
+    for (int k0 = lane; k0 < K + lane; k0 += 512) {      // sixteen loads at once: a row of W that is 0 is looked through to its end
+        float v[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = row[min(k0 + 32 * i, K - 1)];
+        unsigned any = 0;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) any |= __float_as_uint(v[i]) << 1;
+        if (__any_sync(0xffffffffu, any != 0)) return false;
+    }
     return true;
 }
 __device__ float product64(const float* __restrict__ a, const float* __restrict__ w, int K) {
+    const int lane = threadIdx.x & 31;
     double v = 0.;
-#pragma unroll 4
-    for (int k = threadIdx.x & 31; k < K; k += 32) v = fma((double)a[k], (double)w[k], v);
+    for (int k0 = lane; k0 < K + lane; k0 += 512) {
+        float x[16], y[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const int k = k0 + 32 * i;
+            x[i] = k < K ? a[k] : 0.f;
+            y[i] = k < K ? w[k] : 0.f;
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v = fma((double)x[i], (double)y[i], v);
+        if (__any_sync(0xffffffffu, v != v)) return __uint_as_float(0x7fc00000u);      // and stays so
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return (float)v;
@@ -385,12 +403,13 @@ gemm_split_kernel(const float* __restrict__ A, const float* __restrict__ W, cons
 }
 
 // C = the segments' sums in order, + bias.  A thread takes four rows of A and a row of W; a warp what is to be formed again.
-__global__ void __launch_bounds__(256) add_segments_kernel(const float4* __restrict__ part, const uint2* __restrict__ rest, const float* __restrict__ A,
+constexpr int ADDING = 64;               // threads: blocks on many SMs at few rows, too
+__global__ void __launch_bounds__(ADDING) add_segments_kernel(const float4* __restrict__ part, const uint2* __restrict__ rest, const float* __restrict__ A,
                                                            const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ C,
                                                            const int M, const int N, const int K, const int segments) {
     griddep_wait();
     griddep_launch_dependents();
-    const long long i = (long long)blockIdx.x * 256 + threadIdx.x, all = (long long)((M + 3) / 4) * N;
+    const long long i = (long long)blockIdx.x * ADDING + threadIdx.x, all = (long long)((M + 3) / 4) * N;
     const int m = i < all ? (int)(i / N) * 4 : M, n = (int)(i % N);
     double sum[4] = {0., 0., 0., 0.};
     if (m < M) {
@@ -450,8 +469,8 @@ int segments_of(int N, int K) {
     int best = 1;
     long long least = 0;
     for (int s = 1; s <= 64 && s <= chunks / 4; ++s) {
-        const long long rounds = ((long long)tiles * s + sms - 1) / sms;
-        const long long cost = 16384 * (rounds * ((chunks + s - 1) / s + 1) + (s > 1 ? 2 : 0)) + (s > 1 ? (long long)s * N : 0);
+        const unsigned rounds = ((unsigned)tiles * s + sms - 1) / sms, each = ((unsigned)chunks + s - 1) / s + 1;
+        const long long cost = 16384LL * ((long long)rounds * each + (s > 1 ? 2 : 0)) + (s > 1 ? (long long)s * N : 0);
         if (s == 1 || cost < least) best = s, least = cost;
     }
     return best;
@@ -503,7 +522,7 @@ extern "C" int fe_gemm_split(const float* A, const float* W, const float* bias, 
 #undef FE_SPLIT
         if (rc) return rc;
         if (segments == 1) continue;
-        fe::launch(add_segments_kernel, (unsigned)((fours + 255) / 256), 256, 0, stream, (const float4*)sums, (const uint2*)rest, a, W, bias, c, rows, N, K, segments);
+        fe::launch(add_segments_kernel, (unsigned)((fours + ADDING - 1) / ADDING), ADDING, 0, stream, (const float4*)sums, (const uint2*)rest, a, W, bias, c, rows, N, K, segments);
         rc = fe_check_launch("gemm_split (segments)");
         if (rc) return rc;
     }

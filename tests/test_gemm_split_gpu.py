@@ -40,7 +40,7 @@ def test_split_product(N, K, sign, gen):
 def test_what_is_no_finite_number_comes_out_as_from_the_chain(gen):
     x, w = rand((20, 1024), torch.float32, gen), rand((8200, 1024), torch.float32, gen)
     x[3, 5], x[4, 6], w[7, 9] = float("inf"), float("nan"), float("-inf")
-    w[11, 0], x[6, 0] = 1e-30, 1e-30              # a part below the smallest normal number
+    w[11, 0], x[6, 0] = 1e-30, 1e-30              # lost beside ordinary numbers (whole rows of small ones have tests of their own)
     got, want = ops().linear(x, w), chain(x, w)
     assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isposinf(got), torch.isposinf(want))
     assert torch.equal(torch.isneginf(got), torch.isneginf(want))
@@ -144,3 +144,21 @@ def test_room_for_segments_is_bounded_whatever_the_rows(N, K, M, gen):
         assert torch.equal(ops().linear(x[at:at + 67].contiguous(), w), full[at:at + 67]), at
         assert torch.equal(ops().linear(x[at:at + 9].contiguous(), w), full[at:at + 9]), at
     ops().check_status(DEV)
+
+
+@pytest.mark.parametrize("N,K", [(8200, 1024), (1536, 8960)])
+def test_numbers_that_lose_places_are_found_in_every_tile(N, K, gen):
+    """One small number each in a few rows, far apart in rows and in K: a block's later tiles, segments and places that were used before."""
+    x, w = rand((200, K), torch.float32, gen), rand((N, K), torch.float32, gen)
+    rows, columns, ks = [0, 63, 64, 150, 199], [1, 127, 128, 700, N - 1], [3, 64, K // 2, K - 65, K - 1]
+    for m, k in zip(rows, ks):
+        x[m], x[m, k] = 0.0, 1.2345678e-37
+    for n, k in zip(columns, reversed(ks)):
+        w[n], w[n, k] = 0.0, 7.6543211e-39
+    got, by_chain, want = both(x, w)
+    for m in rows:                                # sums of one product: the same rounding, or 64 bits' own
+        assert float((got[m].double() - want[m]).norm()) <= 1.01 * float((by_chain[m].double() - want[m]).norm()), m
+    for n in columns:
+        assert float((got[:, n].double() - want[:, n]).norm()) <= 1.01 * float((by_chain[:, n].double() - want[:, n]).norm()), n
+    for M in (1, 16, 65):
+        assert torch.equal(ops().linear(x[:M].contiguous(), w), got[:M])
