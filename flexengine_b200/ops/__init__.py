@@ -311,9 +311,9 @@ def gemm_fp32(x, w, bias=None):
 
 
 def linear(x, w, bias=None, out_float32=False, follow=None, upcoming=None):
-    """y = x w^T (+ bias); x [M, K], w [N, K].  A float32 weight runs the true 32-bit product
-    (CUDA cores, no reduced-precision mode) whatever the activation dtype; a bfloat16 weight
-    runs on tensor cores with float32 accumulation.
+    """y = x w^T (+ bias); x [M, K], w [N, K].  A float32 weight runs the true 32-bit product whatever
+    the activation dtype, with the error of float32 multiply-adds or less (a chain of them on CUDA cores; matrices that ``split_ok``
+    names on tensor cores in three bfloat16 parts a number); a bfloat16 weight runs on tensor cores with float32 accumulation.
 
     ``follow`` = (residual, norm weight, eps): the product ends a branch of a layer; its result is to be added to
     the float32 residual stream [M, N] and an RMSNorm reads the sum next.  Where the weight-streaming kernel runs (a
