@@ -29,7 +29,10 @@
 // but one a step 17,920 x 1,536 takes 30 and 122 us (4 and 256 rows), with no stores to shared memory 27 and 107; asking rows into L2 ahead of time
 // makes it slower (33, 138).  17,920 x 1,536: 31 us with 1 to 16 rows (the chain of multiply-adds 24 to 40), 40 with 64 (106), 135 with 256 (278).
 // Relative error against 64 bits, K = 1,536 / 8,960: 1.2e-7 / 1.0e-7, the chain 7.0e-7 / 1.7e-6; rows of 1, 2, 8 and 32 numbers other than 0:
-// 2.5e-8, 2.6e-8, 2.8e-8, 4.2e-8, the chain 2.5e-8, 3.1e-8, 5.2e-8, 1.0e-7.  All of 256 x 1,536 results (K = 8,960) formed again take 3.4 ms.
+// 2.5e-8, 2.6e-8, 2.8e-8, 4.2e-8, the chain 2.5e-8, 3.1e-8, 5.2e-8, 1.0e-7.
+// Forming again is for what hardly ever is: all of 256 x 1,536 results (K = 8,960) take 3.4 ms; a row of NaN among 256 rows 156 us instead of 85, 128 rows
+// of W that are 0 395, looked through 16 numbers a lane at a time.  (Flags of the rows that lost places, which would tell such rows from others, cost
+// every product 5 to 9 %, by the registers of the warps that cut up.)
 #include "tcgen05.cuh"
 
 using namespace fe;
